@@ -72,6 +72,27 @@ def test_gpu_gdn_matches_oracle():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 3, 64, 32, 2), (2, 4, 128, 128, 4), (2, 2, 64, 256, 9)])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 263])
+def test_gpu_gdn_row_blocks_columns_and_taps(dims, n):
+    """Rows around the blocks of eight, column counts from two blocks a head to sixteen, few and many taps, a head count whose gate
+    rows are not 8-byte aligned; the second call continues from the stored state. fp32 state: sums of up to 128 terms."""
+    d = GDNDims(*dims)
+    g = torch.Generator().manual_seed(n)
+    P = _params(d, g)
+    Pg = {k: v.float().cuda().contiguous() for k, v in P.items()}
+    st_c, st_g = GDNState(d, 2, "cpu"), GDNState(d, 2, "cuda")
+    for start, rows in ((0, n), (n, 3)):
+        proj = torch.randn(rows, d.proj_out, generator=g).to(torch.bfloat16)
+        pos, slot = torch.arange(start, start + rows, dtype=torch.int32), torch.ones(rows, dtype=torch.int32)
+        ref = gdn_reference(proj, pos, slot, st_c, d, eps=1e-6, **P)
+        out = gdn_forward(proj.cuda(), pos.cuda(), slot.cuda(), st_g, d, eps=1e-6, **Pg).float().cpu()
+        assert float((out - ref).norm() / ref.norm()) < 4e-3              # bf16 output: 2^-9 at most per value
+        assert float((st_g.rec.cpu() - st_c.rec).norm() / st_c.rec.norm()) < 1e-5
+        assert torch.equal(st_g.conv.cpu(), st_c.conv)
+
+
+@pytest.mark.gpu
 def test_gpu_hybrid_model_generates_and_matches_whole_prefill():
     dev = torch.device("cuda:0")
     cfg = HybridConfig.tiny_hybrid()

@@ -2,9 +2,9 @@
 //   gdn_prepare    parallel over rows: causal short convolution + SiLU over the q|k|v channels (taps from earlier rows
 //                  of the same slot in the batch, else from the slot's convolution state), L2 norm of q and k per head,
 //                  q scale, decay exp(g) and beta per value head
-//   gdn_recurrent  one CTA per (value head, slot): walks the slot's rows in order with the state column of every thread
+//   gdn_recurrent  one CTA per (16 columns of a value head's state, slot): walks the slot's rows in order with the state
 //                  in registers:  S *= decay;  delta = (v - S^T k) * beta;  S += k (x) delta;  o = S^T q;
-//                  stores the state, and (head 0) rolls the slot's convolution state forward
+//                  stores the state and rolls the slot's convolution state forward
 //   gdn_gated_norm y = rmsnorm(o) * w * silu(z)
 // KDA (Kimi delta attention) is the same recurrence with one decay per key channel, S = diag(exp(g)) S, where
 //   g = -5 sigmoid(exp(A_log[h]) (f + dt_bias)) and f is a low-rank projection of the input; its output gate is sigmoid(z)
@@ -39,100 +39,295 @@ VE_DEVINL int rows_before(const int* slot, const int* pos, int i, int lim) {
   return r;
 }
 
-// grid (2*nk + nv + 1, rows), block = max(dk, dv) threads. Unit < nk: q head; < 2nk: k head; < 2nk+nv: v head; last: gates.
-__global__ void gdn_prepare_kernel(const GdnArgs a) {
-  __shared__ float red[33];
+// One warp per unit, eight warps a block; each warp walks `per` rows of its unit. Unit < nk: q head; < 2nk: k head; < 2nk+nv: v head;
+// last: gates. The filter of a lane's channels stays in registers, and so do the last KC - 1 inputs where a row continues the one in
+// front of it. Bound by the bf16 rows read and the fp32 rows written (126 MB at 2048 rows of 10240 channels, 20 us at the copy rate): a
+// block per (unit, row) with three barriers took 237 us there, a warp per row that fetched filter and taps again for each 155 us, this form 120 us.
+template <int NE, int KC>         // 32-channel pieces of the widest head; taps (0: any number)
+__global__ void __launch_bounds__(256) gdn_prepare_kernel(const GdnArgs a, int per) {
   grid_dep_launch();
   grid_dep_wait();
-  const int unit = blockIdx.x, i = blockIdx.y, tid = threadIdx.x;
-  const int s = a.slot[i];
-  if (s < 0) return;
+  const int lane = threadIdx.x & 31;
+  const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (unit > 2 * a.nk + a.nv) return;
   const int C = 2 * a.nk * a.dk + a.nv * a.dv;
+  const int i0 = blockIdx.y * per, i1 = min(a.rows, i0 + per);
   if (unit == 2 * a.nk + a.nv) {
-    if (tid < a.nv) {
+    for (int i = i0; i < i1; ++i) {
+      if (a.slot[i] < 0) continue;
       const __nv_bfloat16* row = a.proj + (long)i * a.ld + C + a.nv * a.dv;
-      const float b = bf2f(row[tid]), av = bf2f(row[a.nv + tid]);
-      const float x = av + a.dt_bias[tid];
-      const float sp = x > 20.f ? x : log1pf(__expf(x));
-      a.gb[(long)i * 2 * a.nv + tid] = __expf(-__expf(a.A_log[tid]) * sp);
-      a.gb[(long)i * 2 * a.nv + a.nv + tid] = 1.f / (1.f + __expf(-b));
+      for (int j = lane; j < a.nv; j += 32) {
+        const float b = bf2f(row[j]), av = bf2f(row[a.nv + j]);
+        const float x = av + a.dt_bias[j];
+        const float sp = x > 20.f ? x : log1pf(__expf(x));
+        a.gb[(long)i * 2 * a.nv + j] = __expf(-__expf(a.A_log[j]) * sp);
+        a.gb[(long)i * 2 * a.nv + a.nv + j] = 1.f / (1.f + __expf(-b));
+      }
     }
     return;
   }
   const bool is_v = unit >= 2 * a.nk;
   const int width = is_v ? a.dv : a.dk;
   const int c0 = is_v ? 2 * a.nk * a.dk + (unit - 2 * a.nk) * a.dv : unit * a.dk;
-  const int p = a.pos[i];
-  const int r = rows_before(a.slot, a.pos, i, a.kc - 1);
-  float val = 0.f;
-  if (tid < width) {
-    const int c = c0 + tid;
-    float acc = 0.f;
-    for (int d = 0; d < a.kc; ++d) {               // d = distance into the past of the tap
-      if (p - d < 0) break;
-      float x;
-      if (d <= r) x = bf2f(a.proj[(long)(i - d) * a.ld + c]);
-      else x = a.conv_state[((long)s * (a.kc - 1) + (a.kc - 1 - (d - r))) * C + c];
-      acc += x * a.conv_w[(long)c * a.kc + (a.kc - 1 - d)];
+  const int kc = KC ? KC : a.kc;
+  constexpr int KR = KC ? KC : 1;
+  float w[NE][KR], x[NE][KR];                          // filter, newest input last; inputs by distance into the past
+  if (KC)
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+#pragma unroll
+      for (int d = 0; d < KR; ++d) {
+        w[e][d] = e * 32 + lane < width ? a.conv_w[(long)(c0 + e * 32 + lane) * KC + (KC - 1 - d)] : 0.f;
+        x[e][d] = 0.f;
+      }
+  int s0 = -1, p0 = 0;                                 // slot and position of the row whose inputs x holds
+  for (int i = i0; i < i1; ++i) {
+    const int s = a.slot[i];
+    if (s < 0) { s0 = -1; continue; }
+    const int p = a.pos[i];
+    const bool next = KC && s == s0 && p == p0 + 1;
+    const int r = next ? 0 : rows_before(a.slot, a.pos, i, kc - 1);
+    auto tap = [&](int d, int c) -> float {            // input at distance d (zero in front of the sequence)
+      if (p - d < 0) return 0.f;
+      return d <= r ? bf2f(a.proj[(long)(i - d) * a.ld + c]) : a.conv_state[((long)s * (kc - 1) + (kc - 1 - (d - r))) * C + c];
+    };
+    float acc[NE], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      acc[e] = 0.f;
+      const int t = e * 32 + lane, c = c0 + t;
+      if (t < width) {
+        if (KC) {
+#pragma unroll
+          for (int d = KR - 1; d > 0; --d) x[e][d] = next ? x[e][d - 1] : tap(d, c);
+          x[e][0] = bf2f(a.proj[(long)i * a.ld + c]);
+#pragma unroll
+          for (int d = 0; d < KR; ++d) acc[e] += x[e][d] * w[e][d];
+        } else {
+          for (int d = 0; d < kc; ++d) acc[e] += tap(d, c) * a.conv_w[(long)c * kc + (kc - 1 - d)];
+        }
+        acc[e] = siluf(acc[e]);
+      }
+      ss = fmaf(acc[e], acc[e], ss);
     }
-    val = siluf(acc);
+    s0 = s;
+    p0 = p;
+    float inv = 1.f;
+    if (!is_v) inv = rsqrtf(warp_sum(ss) + 1e-6f) * (unit < a.nk ? rsqrtf((float)a.dk) : 1.f);
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+      if (e * 32 + lane < width) a.u[(long)i * C + c0 + e * 32 + lane] = acc[e] * inv;
   }
-  if (!is_v) {
-    const float ss = block_sum(val * val, red);
-    const float inv = rsqrtf(ss + 1e-6f) * (unit < a.nk ? rsqrtf((float)a.dk) : 1.f);
-    val *= inv;
-  }
-  if (tid < width) a.u[(long)i * C + c0 + tid] = val;
 }
 
-// grid (nv, slots), block dv threads; thread = one column of the head's state.
-template <int DK>
-__global__ void __launch_bounds__(256) gdn_recurrent_kernel(const GdnArgs a) {
-  __shared__ float ks[DK], qs[DK], ds[DK];
-  grid_dep_launch();
+// Two fp32 values in one register pair, for the packed FMA of sm_100.
+VE_DEVINL uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+VE_DEVINL float2 unpack2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+VE_DEVINL uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+VE_DEVINL uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+VE_DEVINL void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+VE_DEVINL void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// grid (dv / 16, nv, slots), 64 threads: 16 columns of one head's state; eight lanes share two columns, DK / 8 keys of each in the
+// registers of a lane.
+//
+// The recurrence is a serial chain over the rows, so what counts is the chain's length per row and how many chains run beside one another.
+// With a column per thread (DK registers, 48 blocks for 48 heads) every row waited for its own q, k and gates from L2 between two barriers:
+// 2.03 us a row, 4163 us for 2048 rows of 48 heads. Here the rows come in blocks of eight through a cp.async ring that runs two blocks
+// ahead, the chain of a row is 3 * DK / 8 packed FMAs and three shuffles (the output sums of a block are reduced together behind it, 14
+// shuffles instead of 48), and 384 blocks share the chip. Shared-memory reads of k and q (512 bytes a warp and 16-byte load, also where
+// lanes read the same) bind next: with one column a lane they took 384 cycles a row on an SM with three blocks, 0.65 us a row in all
+// against 0.31 us now (2048 rows of 48 heads: 650 us), of which a row's chain of dependent instructions is most.
+constexpr int kGdnRows = 8, kGdnStages = 3, kGdnCols = 16;
+template <int DK, bool KDA>
+struct GdnStage {
+  float k[kGdnRows][DK], q[kGdnRows][DK], d[KDA ? kGdnRows : 1][KDA ? DK : 4];
+  float v[kGdnRows][kGdnCols];
+  float gb[kGdnRows][2];
+};
+
+template <int DK, bool KDA>
+__global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
+  extern __shared__ __align__(16) uint8_t gdn_smem[];
+  GdnStage<DK, KDA>* const ring = reinterpret_cast<GdnStage<DK, KDA>*>(gdn_smem);
+  __shared__ int s_first[2], s_count[2];
+  constexpr int NP = DK / 16;                          // register pairs of a lane's part of a column
+  constexpr int NT = 64;
+  // Blocks of the kernel behind wait on the SMs once they may start, and their polling halves the pace of these few warps (2048 rows:
+  // 0.31 us a row without them, 0.55 us with them): a long walk lets them in only when it ends.
+  const bool brief = a.rows <= 32;
+  if (brief) grid_dep_launch();
   grid_dep_wait();
-  const int h = blockIdx.x, s = blockIdx.y, col = threadIdx.x;
+  const int c0 = blockIdx.x * kGdnCols, h = blockIdx.y, s = blockIdx.z;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = lane & 7;
+  const int col = warp * 8 + (lane >> 3) * 2;           // first of this lane's two columns within the block
   // rows of this slot (consecutive)
-  int first = -1, count = 0;
-  for (int i = 0; i < a.rows; ++i)
-    if (a.slot[i] == s) { if (first < 0) first = i; ++count; }
+  int first = a.rows, count = 0;
+  for (int i = tid; i < a.rows; i += NT)
+    if (a.slot[i] == s) { first = min(first, i); ++count; }
+  first = __reduce_min_sync(0xffffffffu, first);
+  count = __reduce_add_sync(0xffffffffu, count);
+  if (lane == 0) { s_first[warp] = first; s_count[warp] = count; }
+  __syncthreads();
+  first = min(s_first[0], s_first[1]);
+  count = s_count[0] + s_count[1];
   if (count == 0) return;
-  const int C = 2 * a.nk * a.dk + a.nv * a.dv;
+  const int C = 2 * a.nk * DK + a.nv * a.dv;
   const int kh = h / (a.nv / a.nk);
   const bool fresh = a.pos[first] == 0;
-  float* st = a.rec_state + (((long)s * a.nv + h) * DK) * a.dv + col;
-  float S[DK];
-#pragma unroll
-  for (int k = 0; k < DK; ++k) S[k] = fresh ? 0.f : st[(long)k * a.dv];
-  for (int r = 0; r < count; ++r) {
-    const int i = first + r;
-    const float* ui = a.u + (long)i * C;
-    const float decay = a.gb[(long)i * 2 * a.nv + h], beta = a.gb[(long)i * 2 * a.nv + a.nv + h];
-    for (int t = col; t < DK; t += blockDim.x) {
-      qs[t] = ui[kh * DK + t];
-      ks[t] = ui[a.nk * DK + kh * DK + t];
-      ds[t] = a.kdec ? a.kdec[((long)i * a.nv + h) * DK + t] : decay;
+
+  auto load = [&](int blk) {                            // one block of rows into its ring stage
+    if (blk * kGdnRows < count) {
+      GdnStage<DK, KDA>& st = ring[blk % kGdnStages];
+      const int n = min(kGdnRows, count - blk * kGdnRows);
+      const long i0 = first + blk * kGdnRows;
+      constexpr int Q = DK / 4;                          // 16-byte pieces of a key
+      for (int j = tid; j < n * Q; j += NT) {
+        const int r = j / Q, c = (j % Q) * 4;
+        const float* ui = a.u + (i0 + r) * C + kh * DK + c;
+        cp_async16(&st.q[r][c], ui);
+        cp_async16(&st.k[r][c], ui + a.nk * DK);
+        if (KDA) cp_async16(&st.d[r][c], a.kdec + ((i0 + r) * a.nv + h) * DK + c);
+      }
+      if (tid < n * 4) cp_async16(&st.v[tid >> 2][(tid & 3) * 4], a.u + (i0 + (tid >> 2)) * C + 2 * a.nk * DK + h * a.dv + c0 + (tid & 3) * 4);
+      else if (tid >= 32 && tid < 32 + n * 2) {
+        const int r = (tid - 32) >> 1, w = tid & 1;
+        cp_async4(&st.gb[r][w], a.gb + (i0 + r) * 2 * a.nv + w * a.nv + h);
+      }
     }
-    __syncthreads();
-    const float v = ui[2 * a.nk * DK + h * a.dv + col];
-    float mem = 0.f;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
 #pragma unroll
-    for (int k = 0; k < DK; ++k) { S[k] *= ds[k]; mem = fmaf(S[k], ks[k], mem); }
-    const float delta = (v - mem) * beta;
-    float o = 0.f;
+  for (int b = 0; b < kGdnStages - 1; ++b) load(b);
+
+  // pair j of this lane: keys (j / 2 * 8 + part) * 4 + (j % 2) * 2 and the next one, columns col and col + 1
+  float* const stp = a.rec_state + (((long)s * a.nv + h) * DK) * a.dv + c0 + col;
+  uint64_t S[2][NP];
 #pragma unroll
-    for (int k = 0; k < DK; ++k) { S[k] = fmaf(ks[k], delta, S[k]); o = fmaf(S[k], qs[k], o); }
-    a.o[(long)i * a.nv * a.dv + h * a.dv + col] = o;
-    __syncthreads();
+  for (int j = 0; j < NP; ++j) {
+    const long k = ((j >> 1) * 8 + part) * 4 + (j & 1) * 2;
+    float2 lo = make_float2(0.f, 0.f), hi = lo;
+    if (!fresh) { lo = *reinterpret_cast<const float2*>(stp + k * a.dv); hi = *reinterpret_cast<const float2*>(stp + (k + 1) * a.dv); }
+    S[0][j] = pack2(lo.x, hi.x);
+    S[1][j] = pack2(lo.y, hi.y);
   }
+  float o[2][kGdnRows];
+  auto row = [&](const GdnStage<DK, KDA>& st, int r) {
+    uint64_t k2[NP], m[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+    const float2 g = *reinterpret_cast<const float2*>(st.gb[r]);
+    const float2 v = *reinterpret_cast<const float2*>(&st.v[r][col]);
+    const uint64_t dec = pack2(g.x, g.x);
 #pragma unroll
-  for (int k = 0; k < DK; ++k) st[(long)k * a.dv] = S[k];
+    for (int j = 0; j < NP; j += 2) {
+      const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(&st.k[r][((j >> 1) * 8 + part) * 4]);
+      k2[j] = kv.x; k2[j + 1] = kv.y;
+      ulonglong2 d = make_ulonglong2(dec, dec);
+      if (KDA) d = *reinterpret_cast<const ulonglong2*>(&st.d[r][((j >> 1) * 8 + part) * 4]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        S[c][j] = mul2(S[c][j], d.x);
+        S[c][j + 1] = mul2(S[c][j + 1], d.y);
+        m[c][0] = fma2(S[c][j], k2[j], m[c][0]);
+        m[c][1] = fma2(S[c][j + 1], k2[j + 1], m[c][1]);
+      }
+    }
+    float mem[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float2 x = unpack2(m[c][0]), y = unpack2(m[c][1]);
+      mem[c] = (x.x + x.y) + (y.x + y.y);
+    }
+#pragma unroll
+    for (int w = 1; w < 8; w <<= 1) {
+      mem[0] += __shfl_xor_sync(0xffffffffu, mem[0], w);
+      mem[1] += __shfl_xor_sync(0xffffffffu, mem[1], w);
+    }
+    const float d0 = (v.x - mem[0]) * g.y, d1 = (v.y - mem[1]) * g.y;
+    const uint64_t dl[2] = {pack2(d0, d0), pack2(d1, d1)};
+    uint64_t q[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll
+    for (int j = 0; j < NP; j += 2) {
+      const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(&st.q[r][((j >> 1) * 8 + part) * 4]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        S[c][j] = fma2(k2[j], dl[c], S[c][j]);
+        S[c][j + 1] = fma2(k2[j + 1], dl[c], S[c][j + 1]);
+        q[c][0] = fma2(S[c][j], qv.x, q[c][0]);
+        q[c][1] = fma2(S[c][j + 1], qv.y, q[c][1]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float2 x = unpack2(q[c][0]), y = unpack2(q[c][1]);
+      o[c][r] = (x.x + x.y) + (y.x + y.y);
+    }
+  };
+  const int blocks = (count + kGdnRows - 1) / kGdnRows;
+  for (int blk = 0; blk < blocks; ++blk) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kGdnStages - 2) : "memory");
+    __syncthreads();                                     // this block's rows have landed; the stage in front of it is free
+    load(blk + kGdnStages - 1);
+    const GdnStage<DK, KDA>& st = ring[blk % kGdnStages];
+    const int n = min(kGdnRows, count - blk * kGdnRows);
+    if (n == kGdnRows) {
+#pragma unroll
+      for (int r = 0; r < kGdnRows; ++r) row(st, r);
+    } else {
+#pragma unroll
+      for (int r = 0; r < kGdnRows; ++r) {
+        o[0][r] = o[1][r] = 0.f;
+        if (r < n) row(st, r);
+      }
+    }
+    // sums over the eight lanes of a column: lane `part` ends with row `part`
+#pragma unroll
+    for (int w = 4; w >= 1; w >>= 1) {
+      const bool up = part & w;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < w; ++j) {
+          const float send = up ? o[c][j] : o[c][j + w], keep = up ? o[c][j + w] : o[c][j];
+          o[c][j] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        }
+    }
+    if (part < n)
+      *reinterpret_cast<float2*>(a.o + ((long)(first + blk * kGdnRows + part) * a.nv + h) * a.dv + c0 + col) = make_float2(o[0][0], o[1][0]);
+  }
+  if (!brief) grid_dep_launch();
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const long k = ((j >> 1) * 8 + part) * 4 + (j & 1) * 2;
+    const float2 x = unpack2(S[0][j]), y = unpack2(S[1][j]);
+    *reinterpret_cast<float2*>(stp + k * a.dv) = make_float2(x.x, y.x);
+    *reinterpret_cast<float2*>(stp + (k + 1) * a.dv) = make_float2(x.y, y.y);
+  }
   {
-    // roll the convolution state: the newest kc-1 inputs of the slot, oldest first. The channels are dealt to the head
+    // roll the convolution state: the newest kc-1 inputs of the slot, oldest first. The channels are dealt to the
     // blocks of the slot (every channel is independent), so no block walks all of them alone.
     const int n1 = a.kc - 1;
     float* cs = a.conv_state + (long)s * n1 * C;
-    for (int c = h * blockDim.x + col; c < C; c += gridDim.x * blockDim.x) {
+    for (int c = (h * gridDim.x + blockIdx.x) * NT + tid; c < C; c += gridDim.x * gridDim.y * NT) {
       float old[8], nw[8];
       for (int t = 0; t < n1; ++t) old[t] = fresh ? 0.f : cs[(long)t * C + c];
       for (int t = 0; t < n1; ++t) {
@@ -145,20 +340,39 @@ __global__ void __launch_bounds__(256) gdn_recurrent_kernel(const GdnArgs a) {
   }
 }
 
-// grid (nv, rows), block dv threads.
-template <bool SIGMOID>
-__global__ void gdn_gated_norm_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ proj, long ld,
-                                      const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int nv, int dv,
+// One warp per (row, head), eight a block: bound by 6 bytes read and 2 written per value. V: values of a lane's step (4 where the gate's
+// rows are 8-byte aligned, else 1).
+template <bool SIGMOID, int V>
+__global__ void __launch_bounds__(256) gdn_gated_norm_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ proj, long ld,
+                                      const float* __restrict__ w, __nv_bfloat16* __restrict__ out, long units, int nv, int dv,
                                       int z_off, float eps) {
-  __shared__ float red[33];
   grid_dep_launch();
   grid_dep_wait();
-  const int h = blockIdx.x, i = blockIdx.y, col = threadIdx.x;
-  const float x = o[((long)i * nv + h) * dv + col];
-  const float ss = block_sum(x * x, red);
-  const float z = bf2f(proj[(long)i * ld + z_off + h * dv + col]);
-  const float gate = SIGMOID ? 1.f / (1.f + __expf(-z)) : siluf(z);
-  out[((long)i * nv + h) * dv + col] = f2bf(x * rsqrtf(ss / dv + eps) * w[col] * gate);
+  const long unit = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (unit >= units) return;
+  const int lane = threadIdx.x & 31;
+  const long i = unit / nv;
+  const int h = (int)(unit % nv);
+  const float* ob = o + unit * dv;
+  float ss = 0.f;
+  for (int c = lane * V; c < dv; c += 32 * V)
+#pragma unroll
+    for (int e = 0; e < V; ++e) ss = fmaf(ob[c + e], ob[c + e], ss);
+  const float rs = rsqrtf(warp_sum(ss) / dv + eps);
+  const __nv_bfloat16* zb = proj + i * ld + z_off + h * dv;
+  for (int c = lane * V; c < dv; c += 32 * V) {
+    __align__(8) __nv_bfloat16 z[V], y[V];
+    if (V == 4) *reinterpret_cast<uint2*>(z) = *reinterpret_cast<const uint2*>(zb + c);
+    else z[0] = zb[c];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const float zf = bf2f(z[e]);
+      const float gate = SIGMOID ? 1.f / (1.f + __expf(-zf)) : siluf(zf);
+      y[e] = f2bf(ob[c + e] * rs * w[c + e] * gate);
+    }
+    if (V == 4) *reinterpret_cast<uint2*>(out + unit * dv + c) = *reinterpret_cast<const uint2*>(y);
+    else out[unit * dv + c] = y[0];
+  }
 }
 
 // KDA decay per key channel: kdec[row][j] = exp(-5 sigmoid(exp(A_log[j / dk]) (f[row][j] + dt_bias[j]))). grid (rows, channel chunks).
@@ -177,6 +391,34 @@ __global__ void kda_decay_kernel(const __nv_bfloat16* __restrict__ f, long ld, c
 
 using namespace ve;
 
+template <int DK, bool KDA>
+static int launch_recurrent_dk(const GdnArgs& a, cudaStream_t st) {
+  constexpr int smem = kGdnStages * (int)sizeof(GdnStage<DK, KDA>);
+  static_assert(smem <= 48 * 1024, "no opt-in to large shared memory is made");
+  launch_pdl(gdn_recurrent_kernel<DK, KDA>, dim3(a.dv / kGdnCols, a.nv, a.slots), dim3(64), smem, st, a);
+  VE_CHECK_LAUNCH();
+}
+template <bool KDA>
+static int launch_recurrent(const GdnArgs& a, cudaStream_t st) {
+  // rows of u and kdec are read in 16-byte pieces, the state and o in pairs: dk, dv and with them every offset are multiples of 32 floats
+  if (((uintptr_t)a.u & 15) || ((uintptr_t)a.kdec & 15) || ((uintptr_t)a.rec_state & 7) || ((uintptr_t)a.o & 7)) return cudaErrorMisalignedAddress;
+  if (a.dk == 128) return launch_recurrent_dk<128, KDA>(a, st);
+  if (a.dk == 64) return launch_recurrent_dk<64, KDA>(a, st);
+  return cudaErrorInvalidValue;
+}
+template <bool SIGMOID>
+static int launch_gated_norm(const void* o, const void* z, long ld, const void* w, void* out, int rows, int nv, int dv, int z_off,
+                             float eps, cudaStream_t st) {
+  const long units = (long)rows * nv;
+  const dim3 grid((unsigned)((units + 7) / 8));
+  const bool vec = !((uintptr_t)z & 7) && ld % 4 == 0 && z_off % 4 == 0 && !((uintptr_t)out & 7);
+  if (vec) launch_pdl(gdn_gated_norm_kernel<SIGMOID, 4>, grid, dim3(256), 0, st, (const float*)o, (const __nv_bfloat16*)z, ld,
+                      (const float*)w, (__nv_bfloat16*)out, units, nv, dv, z_off, eps);
+  else launch_pdl(gdn_gated_norm_kernel<SIGMOID, 1>, grid, dim3(256), 0, st, (const float*)o, (const __nv_bfloat16*)z, ld,
+                  (const float*)w, (__nv_bfloat16*)out, units, nv, dv, z_off, eps);
+  VE_CHECK_LAUNCH();
+}
+
 extern "C" {
 
 int ve_gdn_prepare(const void* proj, long ld, const void* pos, const void* slot, void* conv_state, const void* conv_w,
@@ -187,10 +429,13 @@ int ve_gdn_prepare(const void* proj, long ld, const void* pos, const void* slot,
   GdnArgs a{(const __nv_bfloat16*)proj, ld, (const int*)pos, (const int*)slot, (float*)conv_state, nullptr,
             (const float*)conv_w, (const float*)A_log, (const float*)dt_bias, (float*)u, (float*)gb, nullptr,
             rows, nk, nv, dk, dv, kc, slots, nullptr};
-  int threads = dk > dv ? dk : dv;
-  if (threads < nv) threads = nv;
-  threads = (threads + 31) / 32 * 32;
-  launch_pdl(gdn_prepare_kernel, dim3(2 * nk + nv + 1, rows), dim3(threads), 0, st, a);
+  const int units = 2 * nk + nv + 1, width = dk > dv ? dk : dv;
+  // a warp walks 16 rows as soon as that still gives every SM some blocks, else each row has its own warps
+  const int per = rows >= 256 ? 16 : 1;
+  const dim3 grid((units + 7) / 8, (rows + per - 1) / per);
+  if (width <= 128 && kc == 4) launch_pdl(gdn_prepare_kernel<4, 4>, grid, dim3(256), 0, st, a, per);
+  else if (width <= 128) launch_pdl(gdn_prepare_kernel<4, 0>, grid, dim3(256), 0, st, a, per);
+  else launch_pdl(gdn_prepare_kernel<8, 0>, grid, dim3(256), 0, st, a, per);
   VE_CHECK_LAUNCH();
 }
 
@@ -201,10 +446,7 @@ int ve_gdn_recurrent(const void* proj, long ld, const void* pos, const void* slo
   if (kc < 2 || kc > 9 || dv > 256 || dv % 32 || nv % nk) return cudaErrorInvalidValue;
   GdnArgs a{(const __nv_bfloat16*)proj, ld, (const int*)pos, (const int*)slot, (float*)conv_state, (float*)rec_state,
             nullptr, nullptr, nullptr, (float*)u, (float*)gb, (float*)o, rows, nk, nv, dk, dv, kc, slots, nullptr};
-  if (dk == 128) launch_pdl(gdn_recurrent_kernel<128>, dim3(nv, slots), dim3(dv), 0, st, a);
-  else if (dk == 64) launch_pdl(gdn_recurrent_kernel<64>, dim3(nv, slots), dim3(dv), 0, st, a);
-  else return cudaErrorInvalidValue;
-  VE_CHECK_LAUNCH();
+  return launch_recurrent<false>(a, st);
 }
 
 // The recurrence with one decay per key channel (kdec [rows][nv * dk], already exponentiated).
@@ -215,10 +457,7 @@ int ve_kda_recurrent(const void* proj, long ld, const void* pos, const void* slo
   if (kc < 2 || kc > 9 || dv > 256 || dv % 32 || nv % nk || !kdec) return cudaErrorInvalidValue;
   GdnArgs a{(const __nv_bfloat16*)proj, ld, (const int*)pos, (const int*)slot, (float*)conv_state, (float*)rec_state,
             nullptr, nullptr, nullptr, (float*)u, (float*)gb, (float*)o, rows, nk, nv, dk, dv, kc, slots, (const float*)kdec};
-  if (dk == 128) launch_pdl(gdn_recurrent_kernel<128>, dim3(nv, slots), dim3(dv), 0, st, a);
-  else if (dk == 64) launch_pdl(gdn_recurrent_kernel<64>, dim3(nv, slots), dim3(dv), 0, st, a);
-  else return cudaErrorInvalidValue;
-  VE_CHECK_LAUNCH();
+  return launch_recurrent<true>(a, st);
 }
 
 int ve_kda_decay(const void* f, long ld, const void* A_log, const void* dt_bias, void* kdec, int rows, int nv, int dk,
@@ -234,9 +473,7 @@ int ve_gdn_gated_norm(const void* o, const void* proj, long ld, const void* w, v
                       int conv_dim, int kc, float eps, cudaStream_t st) {
   if (rows <= 0) return 0;
   if (dv > 1024 || dv % 32) return cudaErrorInvalidValue;
-  launch_pdl(gdn_gated_norm_kernel<false>, dim3(nv, rows), dim3(dv), 0, st, (const float*)o, (const __nv_bfloat16*)proj, ld,
-             (const float*)w, (__nv_bfloat16*)out, nv, dv, conv_dim, eps);
-  VE_CHECK_LAUNCH();
+  return launch_gated_norm<false>(o, proj, ld, w, out, rows, nv, dv, conv_dim, eps, st);
 }
 
 // y = rmsnorm(o) * w * sigmoid(z); z [rows, nv * dv] bf16 with row stride ld.
@@ -244,9 +481,7 @@ int ve_kda_gated_norm(const void* o, const void* z, long ld, const void* w, void
                       cudaStream_t st) {
   if (rows <= 0) return 0;
   if (dv > 1024 || dv % 32) return cudaErrorInvalidValue;
-  launch_pdl(gdn_gated_norm_kernel<true>, dim3(nv, rows), dim3(dv), 0, st, (const float*)o, (const __nv_bfloat16*)z, ld,
-             (const float*)w, (__nv_bfloat16*)out, nv, dv, 0, eps);
-  VE_CHECK_LAUNCH();
+  return launch_gated_norm<true>(o, z, ld, w, out, rows, nv, dv, 0, eps, st);
 }
 
 }  // extern "C"

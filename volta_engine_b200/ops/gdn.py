@@ -149,7 +149,7 @@ def gdn_forward(proj, pos, slot, st: GDNState, d: GDNDims, conv_w, A_log, dt_bia
     n = proj.shape[0]
     dev = proj.device
     C, nv = d.conv_dim, d.n_v
-    if scratch is None or scratch[0].shape[0] < n:
+    if scratch is None or scratch[0].shape[0] < n or (scratch[0].data_ptr() | scratch[2].data_ptr()) % 16:
         scratch = (torch.empty(n, C, dtype=torch.float32, device=dev), torch.empty(n, 2 * nv, dtype=torch.float32, device=dev),
                    torch.empty(n, nv * d.dv, dtype=torch.float32, device=dev))
     u, gb, o = scratch
