@@ -3,274 +3,16 @@
 //   Q8_0, Q4_0, Q4_1, Q5_0, Q5_1, IQ4_NL (32-value blocks), Q2_K, Q3_K, Q4_K, Q5_K, Q6_K, IQ4_XS and the codebook
 //   formats IQ1_S, IQ1_M, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S (256-value super-blocks), bf16 activations, fp32
 //   accumulation.
-// One warp per output row; a lane decodes 32 consecutive weights at a time straight from the packed row and
-// multiplies them with the activations of every batch row, so the weights are read exactly once.
-// Summation order per row is fixed (lane-strided chunks, then a butterfly), independent of M.
+// Summation order of an output is fixed by K alone (chunks of 32 weights dealt to eight warps, warp sums added in order), so it does
+// not depend on M, on N or on what else is in the batch.
 // Reference counterparts: src/kernels/cuda/gguf/gguf_linear.cu:38-160 (gemv on q8_1 activations) and the
 // vendored dequantize kernels; block layouts as in quant/gguf.py.
-#include "common.cuh"
+#include "gguf_blocks.cuh"
 
 namespace ve {
 
-enum GgmlType { kQ4_0 = 2, kQ4_1 = 3, kQ5_0 = 6, kQ5_1 = 7, kQ8_0 = 8, kQ2_K = 10, kQ3_K = 11, kQ4_K = 12, kQ5_K = 13,
-                kQ6_K = 14, kIQ2_XXS = 16, kIQ2_XS = 17, kIQ3_XXS = 18, kIQ1_S = 19, kIQ4_NL = 20, kIQ3_S = 21, kIQ2_S = 22,
-                kIQ4_XS = 23, kIQ1_M = 29 };
-
-// Codebook formats (IQ1 / IQ2 / IQ3): one table of grid vectors and sign bytes in device memory, uploaded once per device
-// by the host (ve_gguf_set_iq_grids). Byte offsets of the parts, as in quant/gguf_iq.py:
-//   0 sign bytes [128] | 128 iq2xxs [256][8] | 2176 iq2xs [512][8] | 6272 iq2s [1024][8] | 14464 iq3xxs [256][4]
-//   | 15488 iq3s [512][4] | 17536 iq1s [2048][8] (int8)
-__constant__ const uint8_t* kIqGrids;
-constexpr int kOffSigns = 0, kOff2xxs = 128, kOff2xs = 2176, kOff2s = 6272, kOff3xxs = 14464, kOff3s = 15488, kOff1s = 17536;
-
-// 8 grid bytes times a scale with the signs of `sb` (bit j set = element j negative)
-VE_DEVINL void put8(const uint8_t* __restrict__ g, uint32_t sb, float db, float* w) {
-  const uint2 v = *reinterpret_cast<const uint2*>(g);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    w[j] = ((sb >> j) & 1 ? -db : db) * (float)((v.x >> (8 * j)) & 255);
-    w[j + 4] = ((sb >> (j + 4)) & 1 ? -db : db) * (float)((v.y >> (8 * j)) & 255);
-  }
-}
-VE_DEVINL void put4(const uint8_t* __restrict__ g, uint32_t sb, float db, float* w) {
-  const uint32_t v = *reinterpret_cast<const uint32_t*>(g);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) w[j] = ((sb >> j) & 1 ? -db : db) * (float)((v >> (8 * j)) & 255);
-}
-// 8 ternary grid values (int8) plus a shift, times a scale
-VE_DEVINL void put8_shift(const uint8_t* __restrict__ g, float delta, float dl, float* w) {
-  const uint2 v = *reinterpret_cast<const uint2*>(g);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    w[j] = dl * ((float)(int8_t)((v.x >> (8 * j)) & 255) + delta);
-    w[j + 4] = dl * ((float)(int8_t)((v.y >> (8 * j)) & 255) + delta);
-  }
-}
-
-// the 16 non-uniform levels of the IQ4 formats
-__constant__ int8_t kIq4Levels[16] = {-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113};
-
-VE_DEVINL void scale_min_k4(const uint8_t* s, int sb, int& sc, int& mn) {
-  if (sb < 4) { sc = s[sb] & 63; mn = s[sb + 4] & 63; }
-  else { sc = (s[sb + 4] & 15) | ((s[sb - 4] >> 6) << 4); mn = (s[sb + 4] >> 4) | ((s[sb] >> 6) << 4); }
-}
-
-VE_DEVINL float h2f(const uint8_t* p) {
-  return __half2float(__ushort_as_half((unsigned short)(p[0] | (p[1] << 8))));
-}
-
-// Decode the 32 weights of chunk `c` of a packed row into w[32].
-template <int TYPE>
-VE_DEVINL void decode32(const uint8_t* __restrict__ row, int c, float* w) {
-  if (TYPE == kQ8_0) {
-    const uint8_t* b = row + (size_t)c * 34;
-    const float d = h2f(b);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) w[j] = d * (float)(int8_t)b[2 + j];
-  } else if (TYPE == kQ4_0) {
-    const uint8_t* b = row + (size_t)c * 18;
-    const float d = h2f(b);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      w[j] = d * (float)((int)(b[2 + j] & 15) - 8);
-      w[j + 16] = d * (float)((int)(b[2 + j] >> 4) - 8);
-    }
-  } else if (TYPE == kQ4_K) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 144;
-    const int sb = c & 7;                       // sub-block 0..7
-    const float d = h2f(b), dmin = h2f(b + 2);
-    const uint8_t* s = b + 4;
-    int sc, mn;
-    scale_min_k4(s, sb, sc, mn);
-    const float d1 = d * (float)sc, m1 = dmin * (float)mn;
-    const uint8_t* q = b + 16 + (sb >> 1) * 32;
-    const int shift = (sb & 1) * 4;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) w[j] = d1 * (float)((q[j] >> shift) & 15) - m1;
-  } else if (TYPE == kQ4_1) {
-    const uint8_t* b = row + (size_t)c * 20;
-    const float d = h2f(b), m = h2f(b + 2);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      w[j] = fmaf(d, (float)(b[4 + j] & 15), m);
-      w[j + 16] = fmaf(d, (float)(b[4 + j] >> 4), m);
-    }
-  } else if (TYPE == kQ5_0 || TYPE == kQ5_1) {
-    const int hdr = TYPE == kQ5_0 ? 2 : 4;
-    const uint8_t* b = row + (size_t)c * (TYPE == kQ5_0 ? 22 : 24);
-    const float d = h2f(b), m = TYPE == kQ5_0 ? 0.f : h2f(b + 2);
-    const uint32_t qh = b[hdr] | (b[hdr + 1] << 8) | (b[hdr + 2] << 16) | ((uint32_t)b[hdr + 3] << 24);
-    const int off = TYPE == kQ5_0 ? 16 : 0;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int q0 = (b[hdr + 4 + j] & 15) | (((qh >> j) & 1) << 4);
-      const int q1 = (b[hdr + 4 + j] >> 4) | (((qh >> (j + 16)) & 1) << 4);
-      w[j] = fmaf(d, (float)(q0 - off), m);
-      w[j + 16] = fmaf(d, (float)(q1 - off), m);
-    }
-  } else if (TYPE == kIQ4_NL) {
-    const uint8_t* b = row + (size_t)c * 18;
-    const float d = h2f(b);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      w[j] = d * (float)kIq4Levels[b[2 + j] & 15];
-      w[j + 16] = d * (float)kIq4Levels[b[2 + j] >> 4];
-    }
-  } else if (TYPE == kIQ4_XS) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 136;
-    const int ib = c & 7;
-    const int sh = b[2] | (b[3] << 8);
-    const int ls = ((b[4 + (ib >> 1)] >> (4 * (ib & 1))) & 15) | (((sh >> (2 * ib)) & 3) << 4);
-    const float dl = h2f(b) * (float)(ls - 32);
-    const uint8_t* q = b + 8 + ib * 16;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      w[j] = dl * (float)kIq4Levels[q[j] & 15];
-      w[j + 16] = dl * (float)kIq4Levels[q[j] >> 4];
-    }
-  } else if (TYPE == kIQ2_XXS) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 66;
-    const uint8_t* q = b + 2 + (c & 7) * 8;
-    const uint32_t aux = q[4] | (q[5] << 8) | (q[6] << 16) | ((uint32_t)q[7] << 24);
-    const float db = h2f(b) * (0.5f + (float)(aux >> 28)) * 0.25f;
-#pragma unroll
-    for (int l = 0; l < 4; ++l)
-      put8(kIqGrids + kOff2xxs + q[l] * 8, kIqGrids[kOffSigns + ((aux >> (7 * l)) & 127)], db, w + 8 * l);
-  } else if (TYPE == kIQ2_XS) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 74;
-    const int ib = c & 7;
-    const uint8_t* q = b + 2 + ib * 8;
-    const int sc = b[66 + ib];
-    const float d = h2f(b);
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const int v = q[2 * l] | (q[2 * l + 1] << 8);
-      const float db = d * (0.5f + (float)(l < 2 ? (sc & 15) : (sc >> 4))) * 0.25f;
-      put8(kIqGrids + kOff2xs + (v & 511) * 8, kIqGrids[kOffSigns + (v >> 9)], db, w + 8 * l);
-    }
-  } else if (TYPE == kIQ2_S) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 82;
-    const int ib = c & 7;
-    const uint8_t* q = b + 2 + ib * 4;
-    const uint8_t* sg = b + 34 + ib * 4;
-    const int qh = b[66 + ib], sc = b[74 + ib];
-    const float d = h2f(b);
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const float db = d * (0.5f + (float)(l < 2 ? (sc & 15) : (sc >> 4))) * 0.25f;
-      put8(kIqGrids + kOff2s + (q[l] | ((qh << (8 - 2 * l)) & 0x300)) * 8, sg[l], db, w + 8 * l);
-    }
-  } else if (TYPE == kIQ3_XXS) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 98;
-    const int ib = c & 7;
-    const uint8_t* q = b + 2 + ib * 8;
-    const uint8_t* a = b + 66 + ib * 4;
-    const uint32_t aux = a[0] | (a[1] << 8) | (a[2] << 16) | ((uint32_t)a[3] << 24);
-    const float db = h2f(b) * (0.5f + (float)(aux >> 28)) * 0.5f;
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const uint32_t sb = kIqGrids[kOffSigns + ((aux >> (7 * l)) & 127)];
-      put4(kIqGrids + kOff3xxs + q[2 * l] * 4, sb, db, w + 8 * l);
-      put4(kIqGrids + kOff3xxs + q[2 * l + 1] * 4, sb >> 4, db, w + 8 * l + 4);
-    }
-  } else if (TYPE == kIQ3_S) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 110;
-    const int ib = c & 7;
-    const uint8_t* q = b + 2 + ib * 8;
-    const int qh = b[66 + ib];
-    const uint8_t* sg = b + 74 + ib * 4;
-    const int nib = (b[106 + (ib >> 1)] >> (4 * (ib & 1))) & 15;
-    const float db = h2f(b) * (float)(1 + 2 * nib);
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      put4(kIqGrids + kOff3s + (q[2 * l] | ((qh << (8 - 2 * l)) & 256)) * 4, sg[l], db, w + 8 * l);
-      put4(kIqGrids + kOff3s + (q[2 * l + 1] | ((qh << (7 - 2 * l)) & 256)) * 4, sg[l] >> 4, db, w + 8 * l + 4);
-    }
-  } else if (TYPE == kIQ1_S) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 50;
-    const int ib = c & 7;
-    const uint8_t* q = b + 2 + ib * 4;
-    const int qh = b[34 + 2 * ib] | (b[35 + 2 * ib] << 8);
-    const float dl = h2f(b) * (float)(2 * ((qh >> 12) & 7) + 1);
-    const float delta = (qh & 0x8000) ? -0.125f : 0.125f;
-#pragma unroll
-    for (int l = 0; l < 4; ++l)
-      put8_shift(kIqGrids + kOff1s + (q[l] | (((qh >> (3 * l)) & 7) << 8)) * 8, delta, dl, w + 8 * l);
-  } else if (TYPE == kIQ1_M) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 56;
-    const int ib = c & 7;
-    const uint8_t* q = b + ib * 4;
-    const int q0 = b[32 + 2 * ib], q1 = b[33 + 2 * ib];
-    const uint8_t* s8 = b + 48;
-    const int s0 = s8[0] | (s8[1] << 8), s1 = s8[2] | (s8[3] << 8), s2 = s8[4] | (s8[5] << 8), s3 = s8[6] | (s8[7] << 8);
-    const unsigned short bits = (unsigned short)((s0 >> 12) | ((s1 >> 8) & 0x00f0) | ((s2 >> 4) & 0x0f00) | (s3 & 0xf000));
-    const float d = __half2float(__ushort_as_half(bits));
-    const int sw = (ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3;
-    const float dl1 = d * (float)(2 * ((sw >> (6 * (ib & 1))) & 7) + 1);
-    const float dl2 = d * (float)(2 * ((sw >> (6 * (ib & 1) + 3)) & 7) + 1);
-    put8_shift(kIqGrids + kOff1s + (q[0] | ((q0 << 8) & 0x700)) * 8, (q0 & 0x08) ? -0.125f : 0.125f, dl1, w);
-    put8_shift(kIqGrids + kOff1s + (q[1] | ((q0 << 4) & 0x700)) * 8, (q0 & 0x80) ? -0.125f : 0.125f, dl1, w + 8);
-    put8_shift(kIqGrids + kOff1s + (q[2] | ((q1 << 8) & 0x700)) * 8, (q1 & 0x08) ? -0.125f : 0.125f, dl2, w + 16);
-    put8_shift(kIqGrids + kOff1s + (q[3] | ((q1 << 4) & 0x700)) * 8, (q1 & 0x80) ? -0.125f : 0.125f, dl2, w + 24);
-  } else if (TYPE == kQ2_K) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 84;
-    const int half = (c >> 2) & 1, sft = (c & 3) * 2;
-    const float d = h2f(b + 80), dmin = h2f(b + 82);
-    const uint8_t* q = b + 16 + half * 32;
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      const int s = b[half * 8 + (c & 3) * 2 + part];
-      const float dl = d * (float)(s & 15), ml = dmin * (float)(s >> 4);
-#pragma unroll
-      for (int l = 0; l < 16; ++l) w[part * 16 + l] = dl * (float)((q[part * 16 + l] >> sft) & 3) - ml;
-    }
-  } else if (TYPE == kQ3_K) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 110;
-    const int half = (c >> 2) & 1, j4 = c & 3, sft = j4 * 2, bit = half * 4 + j4;
-    const float d = h2f(b + 108);
-    const uint8_t* hm = b;
-    const uint8_t* q = b + 32 + half * 32;
-    const uint8_t* s12 = b + 96;
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      const int i = half * 8 + j4 * 2 + part;                 // scale index 0..15
-      const int lo = i < 8 ? (s12[i] & 15) : (s12[i - 8] >> 4);
-      const int hi = (s12[8 + (i & 3)] >> (2 * (i >> 2))) & 3;
-      const float dl = d * (float)((lo | (hi << 4)) - 32);
-#pragma unroll
-      for (int l = 0; l < 16; ++l) {
-        const int e = part * 16 + l;
-        w[e] = dl * (float)((int)((q[e] >> sft) & 3) - (((hm[e] >> bit) & 1) ? 0 : 4));
-      }
-    }
-  } else if (TYPE == kQ5_K) {
-    const uint8_t* b = row + (size_t)(c >> 3) * 176;
-    const int sb = c & 7;
-    const float d = h2f(b), dmin = h2f(b + 2);
-    int sc, mn;
-    scale_min_k4(b + 4, sb, sc, mn);
-    const float d1 = d * (float)sc, m1 = dmin * (float)mn;
-    const uint8_t* qh = b + 16;
-    const uint8_t* q = b + 48 + (sb >> 1) * 32;
-    const int shift = (sb & 1) * 4;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) w[j] = d1 * (float)(((q[j] >> shift) & 15) | (((qh[j] >> sb) & 1) << 4)) - m1;
-  } else {  // Q6_K
-    const uint8_t* b = row + (size_t)(c >> 3) * 210;
-    const int sub = c & 7, half = sub >> 2, qtr = sub & 3;
-    const uint8_t* ql = b + half * 64 + (qtr & 1) * 32;
-    const uint8_t* qh = b + 128 + half * 32;
-    const int8_t* sc = reinterpret_cast<const int8_t*>(b + 192) + half * 8 + qtr * 2;
-    const float d = h2f(b + 208);
-    const int lshift = (qtr >> 1) * 4, hshift = qtr * 2;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const int q = (int)(((ql[j] >> lshift) & 15) | (((qh[j] >> hshift) & 3) << 4)) - 32;
-      w[j] = d * (float)sc[j >> 4] * (float)q;
-    }
-  }
-}
-
+// Rows whose blocks lie at odd addresses (gguf_mma_kernel reads words): one warp per output row, a lane decodes 32 consecutive weights
+// at a time byte by byte.
 template <int TYPE>
 __global__ void __launch_bounds__(256) gguf_gemv_kernel(const uint8_t* __restrict__ W, long row_bytes,
                                                         const __nv_bfloat16* __restrict__ x, long x_stride,
@@ -316,7 +58,7 @@ __global__ void __launch_bounds__(256) gguf_gemv_kernel(const uint8_t* __restric
   }
 }
 
-// Routed experts stored as GGUF blocks (decode / verify rows): grid (output rows / 4 or / 8, routes), one warp per output
+// The same for routed experts: grid (output rows / 4 or / 8, routes), one warp per output
 // row (FUSE: per gate / up pair, the gated activation applied before the store). W holds the experts of this rank back to
 // back ([e_local][N][row_bytes]); route r reads activation row r / x_div and the expert ids[r] - e0; routes of experts
 // that live elsewhere store zeros. The per-row sum runs in the order of the dense mat-vec (lane-strided 32-weight
@@ -384,6 +126,239 @@ __global__ void __launch_bounds__(128) gguf_moe_gemv_kernel(const uint8_t* __res
   }
 }
 
+struct GgufGemvArgs {
+  const uint8_t* W; long row_bytes; const uint8_t* W_end;
+  const __nv_bfloat16* x; long x_stride;
+  __nv_bfloat16* out; float* out_f32; long out_stride;
+  int M, N, K, tiles;
+  // routed experts: route r reads activation row r / x_div and expert ids[r] - e0 of the bank; a route of another rank's expert gives zeros
+  const int* ids; int e0, e_local, x_div, act, tiles_per_route;
+  float limit;
+};
+
+// MODE 0: out[m, n] = sum_k W[n, k] x[m, k] for up to 8 * NT rows m. MODE 1: the same for routed experts, one activation row a route.
+// MODE 2: routed gate / up pair, gate in rows n and up in rows N / 2 + n of the expert, the gated activation applied before the store.
+//
+// A tile is 16 * RT weight rows (MODE 2: eight gate and eight up rows). The eight warps of a block deal its units of 256 weights along K
+// (128 for Q8_0) between them; each warp copies its units through a ring of its own with 16-byte cp.async and turns them into operand
+// fragments, whose products with all activation rows are one tensor-core instruction per 16 weights. Blocks are persistent over tiles and the
+// ring runs on into the next tile. What bounds it is the weights' DRAM traffic, or for the formats of four bits and less decoding, 1.5 to 3
+// instructions a weight. A lane that decoded 32 consecutive weights of its own straight from global memory (one warp a row) read
+// single bytes up to 4352 bytes apart and multiplied every row of x in fp32: 365 us for the average matrix of a 27B-class Q4_K layer at
+// four rows, 538 us for Q8_0 at eight rows of the larger latent-attention shapes.
+template <int TYPE, int MODE, int NT, int RT>
+struct GemvCfg {
+  using F = Fmt<TYPE>;
+  static constexpr int kPitch = ((F::kUnit + 14 + 15) / 16 | 1) * 16;     // 16-byte pieces of a row's unit at any 2-byte offset; odd: no bank conflicts
+  static constexpr int kStage = 16 * RT * kPitch;
+  static constexpr int kStages = RT == 2 ? 2 : 3;
+  static constexpr int kCols = MODE == 0 ? 8 * NT : 1;
+  static constexpr int kRed = 8 * 16 * RT * kCols;                          // floats, one of two buffers
+  static constexpr int kTab = (F::kTabBytes + 15) / 16 * 16;
+  static constexpr int kSmem = kTab + 2 * kRed * 4 + 8 * kStages * kStage;
+};
+
+template <int TYPE, int MODE, int NT, int RT>
+__global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) {
+  using F = Fmt<TYPE>;
+  using C = GemvCfg<TYPE, MODE, NT, RT>;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  uint8_t* const tab = smem_raw;
+  float* const red = reinterpret_cast<float*>(smem_raw + C::kTab);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  uint8_t* const ring = smem_raw + C::kTab + 2 * C::kRed * 4 + warp * C::kStages * C::kStage;
+  grid_dep_launch();
+  if (C::kTab) load_table<TYPE>(tab);
+  if (MODE != 0) grid_dep_wait();                       // the routes come from the kernel in front (weights do not: MODE 0 starts on them)
+
+  const int chunks = p.K >> 5;
+  const int units = (chunks + F::kChunks - 1) / F::kChunks;
+  const int mine = warp < units ? (units - warp + 7) / 8 : 0;            // units warp, warp + 8, ...
+  const int ntile = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int items = mine * ntile;
+  const int half_n = p.N >> 1;
+
+  // rows of this lane's quad in tile i: 2 * RT of them (fragment rows g and g + 8); false: the tile's expert is not here
+  auto rows_of = [&](int i, const uint8_t** rp) -> bool {
+    int tile = (int)blockIdx.x + i * (int)gridDim.x;
+    const uint8_t* base = p.W;
+    if (MODE != 0) {
+      const int route = tile / p.tiles_per_route;
+      tile -= route * p.tiles_per_route;
+      const int e = p.ids[route] - p.e0;
+      if (e < 0 || e >= p.e_local) return false;
+      base += (size_t)e * p.N * p.row_bytes;
+    }
+#pragma unroll
+    for (int r = 0; r < 2 * RT; ++r) {
+      int n;
+      if (MODE == 2) n = min(tile * 8 + g, half_n - 1) + r * half_n;
+      else n = min(tile * 16 * RT + r * 8 + g, p.N - 1);                  // rows behind the matrix repeat its last one
+      rp[r] = base + (size_t)n * p.row_bytes;
+    }
+    return true;
+  };
+  const uint8_t* lp[2 * RT];                            // rows of the tile being loaded
+  bool l_here = false;
+  int l_tile = -1, l_item = 0;
+  auto load = [&]() {                                   // the next unit into its ring stage
+    if (l_item < items) {
+      const int ti = l_item / mine, ui = warp + 8 * (l_item - ti * mine);
+      if (ti != l_tile) { l_here = rows_of(ti, lp); l_tile = ti; }
+      if (l_here) {
+        const int bytes = F::kBig ? F::kBytes : min(F::kChunks, chunks - ui * F::kChunks) * F::kBytes;
+        uint8_t* dst = ring + (l_item % C::kStages) * C::kStage;
+#pragma unroll
+        for (int r = 0; r < 2 * RT; ++r) {
+          const uint8_t* src = lp[r] + (size_t)ui * F::kUnit;
+          const int off = (int)((uintptr_t)src & 15);   // whole 16-byte pieces: they lie inside the allocation, but for a piece that
+          src -= off;                                     // the matrix ends in, which is cut there
+          const int n16 = (off + bytes + 15) >> 4;
+          for (int j = t; j < n16; j += 4) {
+            const long left = p.W_end - (src + j * 16);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (r * 8 + g) * C::kPitch + j * 16)),
+                         "l"(src + j * 16), "r"(left < 16 ? (int)left : 16)
+                         : "memory");
+          }
+        }
+      }
+    }
+    ++l_item;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < C::kStages - 1; ++s) load();
+  if (C::kTab) __syncthreads();
+  if (MODE == 0) grid_dep_wait();
+
+  int item = 0;
+  for (int ti = 0; ti < ntile; ++ti) {
+    const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
+    const uint8_t* rp[2 * RT];
+    const bool here = rows_of(ti, rp);
+    const __nv_bfloat16* xr = p.x + (MODE != 0 ? (long)(tile / p.tiles_per_route / p.x_div) * p.x_stride : 0) + 4 * t;
+    float acc[RT][NT][4];
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+    for (int w = 0; w < mine; ++w, ++item) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(C::kStages - 2) : "memory");
+      __syncwarp();                                       // every lane's pieces are here, and every lane is done with the stage in front
+      load();
+      if (!here) continue;
+      const uint8_t* st = ring + (item % C::kStages) * C::kStage;
+      const int ui = warp + 8 * w, c0 = ui * F::kChunks;
+      const uint8_t* up[2 * RT];
+#pragma unroll
+      for (int r = 0; r < 2 * RT; ++r)
+        up[r] = st + (r * 8 + g) * C::kPitch + (int)((uintptr_t)(rp[r] + (size_t)ui * F::kUnit) & 15);
+#pragma unroll
+      for (int h = 0; h < F::kChunks; h += 4) {
+        uint2 xv[4][NT][2];                               // this lane's activations of four chunks
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const bool live = (MODE != 0 ? g == 0 : j * 8 + g < p.M) && (F::kBig || c0 + h + c < chunks);
+            const __nv_bfloat16* q = xr + (MODE == 0 ? (long)(j * 8 + g) * p.x_stride : 0) + (long)(c0 + h + c) * 32;
+            xv[c][j][0] = live ? *reinterpret_cast<const uint2*>(q) : make_uint2(0u, 0u);
+            xv[c][j][1] = live ? *reinterpret_cast<const uint2*>(q + 16) : make_uint2(0u, 0u);
+          }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (!F::kBig && c0 + h + c >= chunks) break;
+          float sx[NT][2][2];                             // sums of x over the group (formats with minima), columns 2 t and 2 t + 1
+          if (F::kMin) {
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              constexpr uint32_t one = 0x3F803F80u;
+              float d[4] = {0.f, 0.f, 0.f, 0.f};
+              mma_bf16_16816(d, one, one, one, one, xv[c][j][0].x, xv[c][j][0].y);
+              if (F::kMin == 2) { sx[j][0][0] = d[0]; sx[j][0][1] = d[1]; d[0] = d[1] = d[2] = d[3] = 0.f; }
+              mma_bf16_16816(d, one, one, one, one, xv[c][j][1].x, xv[c][j][1].y);
+              sx[j][F::kMin - 1][0] = d[0]; sx[j][F::kMin - 1][1] = d[1];
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < RT; ++i) {
+            uint32_t fa[4], fb[4];
+            float sa[2], sb[2], ma[2], mb[2];
+            frag<TYPE>(up[2 * i], h + c, t, tab, fa, sa, ma);
+            frag<TYPE>(up[2 * i + 1], h + c, t, tab, fb, sb, mb);
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              float* ac = acc[i][j];
+              float d[4] = {0.f, 0.f, 0.f, 0.f};
+              mma_bf16_16816(d, fa[0], fb[0], fa[1], fb[1], xv[c][j][0].x, xv[c][j][0].y);
+              if (F::kScale16) {
+                ac[0] = fmaf(sa[0], d[0], ac[0]); ac[1] = fmaf(sa[0], d[1], ac[1]);
+                ac[2] = fmaf(sb[0], d[2], ac[2]); ac[3] = fmaf(sb[0], d[3], ac[3]);
+                d[0] = d[1] = d[2] = d[3] = 0.f;
+              }
+              mma_bf16_16816(d, fa[2], fb[2], fa[3], fb[3], xv[c][j][1].x, xv[c][j][1].y);
+              constexpr int q = F::kScale16 ? 1 : 0;
+              ac[0] = fmaf(sa[q], d[0], ac[0]); ac[1] = fmaf(sa[q], d[1], ac[1]);
+              ac[2] = fmaf(sb[q], d[2], ac[2]); ac[3] = fmaf(sb[q], d[3], ac[3]);
+#pragma unroll
+              for (int k = 0; k < F::kMin; ++k) {
+                ac[0] = fmaf(-ma[k], sx[j][k][0], ac[0]); ac[1] = fmaf(-ma[k], sx[j][k][1], ac[1]);
+                ac[2] = fmaf(-mb[k], sx[j][k][0], ac[2]); ac[3] = fmaf(-mb[k], sx[j][k][1], ac[3]);
+              }
+            }
+          }
+        }
+      }
+    }
+    // warp sums -> shared memory [warp][column][row], added in warp order
+    float* rb = red + (ti & 1) * C::kRed;
+    if (MODE == 0) {
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            rb[(warp * C::kCols + j * 8 + 2 * t + (e & 1)) * 16 * RT + i * 16 + (e >> 1) * 8 + g] = acc[i][j][e];
+    } else if (t == 0) {
+      rb[warp * 16 + g] = acc[0][0][0];
+      rb[warp * 16 + 8 + g] = acc[0][0][2];
+    }
+    __syncthreads();                                      // (the other buffer's sums were read in front of this barrier)
+    const int nw = min(8, units);
+    if (MODE == 0) {
+      for (int i = threadIdx.x; i < 16 * RT * C::kCols; i += 256) {
+        const int row = i % (16 * RT), m = i / (16 * RT), n = tile * 16 * RT + row;
+        if (m < p.M && n < p.N) {
+          float v = 0.f;
+          for (int w = 0; w < nw; ++w) v += rb[w * C::kRed / 8 + i];
+          if (p.out_f32) p.out_f32[(long)m * p.out_stride + n] = v;
+          else p.out[(long)m * p.out_stride + n] = f2bf(v);
+        }
+      }
+    } else if (threadIdx.x < (MODE == 2 ? 8 : 16)) {
+      const int route = tile / p.tiles_per_route, n = (tile - route * p.tiles_per_route) * (MODE == 2 ? 8 : 16) + threadIdx.x;
+      if (n < (MODE == 2 ? half_n : p.N)) {
+        float v = 0.f, u = 0.f;
+        if (here) {
+          for (int w = 0; w < nw; ++w) v += rb[w * 16 + threadIdx.x];
+          if (MODE == 2) {
+            for (int w = 0; w < nw; ++w) u += rb[w * 16 + 8 + threadIdx.x];
+            // the unfused pair rounds both projections to bf16 before the activation: the same rounding points here
+            float gate = bf2f(f2bf(v)), upv = bf2f(f2bf(u));
+            if (p.limit > 0.f) { gate = fminf(gate, p.limit); upv = fminf(fmaxf(upv, -p.limit), p.limit); }
+            v = (p.act ? 0.5f * gate * (1.f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate)))
+                       : gate / (1.f + __expf(-gate))) * upv;
+          }
+        }
+        p.out[(long)route * p.out_stride + n] = f2bf(v);
+      }
+    }
+  }
+}
+
 template <int TYPE>
 __global__ void gguf_dequant_kernel(const uint8_t* __restrict__ W, long row_bytes, __nv_bfloat16* __restrict__ out,
                                     long N, int K) {
@@ -403,6 +378,94 @@ __global__ void gguf_dequant_kernel(const uint8_t* __restrict__ W, long row_byte
 }  // namespace ve
 
 using namespace ve;
+
+template <int TYPE, int MODE, int NT, int RT>
+static int launch_gguf_mma(GgufGemvArgs a, cudaStream_t st) {
+  using C = GemvCfg<TYPE, MODE, NT, RT>;
+  static_assert(C::kSmem <= 200 * 1024, "shared memory of an SM");
+  static int per_sm = 0;                                 // resident blocks an SM, found once (the same on every B200)
+  int n = per_sm;
+  if (n == 0) {
+    cudaError_t e = cudaFuncSetAttribute(gguf_mma_kernel<TYPE, MODE, NT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gguf_mma_kernel<TYPE, MODE, NT, RT>, 256, C::kSmem);
+    if (e != cudaSuccess) return (int)e;
+    if (n < 1) n = 1;
+    per_sm = n;
+  }
+  const int grid = a.tiles < 148 * n ? a.tiles : 148 * n;
+  launch_pdl(gguf_mma_kernel<TYPE, MODE, NT, RT>, dim3(grid), dim3(256), C::kSmem, st, a);
+  VE_CHECK_LAUNCH();
+}
+
+// fields of a block are read from shared memory in words of their natural alignment, which the row addresses must keep
+template <int TYPE>
+static bool block_aligned(const void* W, long row_bytes) {
+  return (((uintptr_t)W | (uintptr_t)row_bytes) & (Fmt<TYPE>::kWords ? 3 : 1)) == 0;
+}
+
+template <int TYPE>
+static int run_gguf_gemv(GgufGemvArgs a, cudaStream_t st) {
+  if (!block_aligned<TYPE>(a.W, a.row_bytes)) {          // blocks at odd addresses: byte by byte
+    gguf_gemv_kernel<TYPE><<<(a.N + 7) / 8, 256, 0, st>>>(a.W, a.row_bytes, a.x, a.x_stride, a.out, a.out_stride, a.out_f32, a.M, a.N, a.K);
+    VE_CHECK_LAUNCH();
+  }
+  // 32 weight rows a tile where several rows of x would otherwise be read again for every 16 of a large matrix; the sums are the same
+  a.tiles = (a.N + 15) / 16;
+  if (a.M <= 4 || (a.M <= 8 && a.N < 32 * 148)) return launch_gguf_mma<TYPE, 0, 1, 1>(a, st);
+  a.tiles = (a.N + 31) / 32;
+  if (a.M <= 8) return launch_gguf_mma<TYPE, 0, 1, 2>(a, st);
+  return launch_gguf_mma<TYPE, 0, 2, 2>(a, st);
+}
+
+template <int TYPE>
+static int run_gguf_moe(GgufGemvArgs a, int routes, int fuse_act, cudaStream_t st) {
+  if (!block_aligned<TYPE>(a.W, a.row_bytes)) {
+    const dim3 grid(((fuse_act ? a.N / 2 : a.N) + 3) / 4, routes);
+    if (fuse_act)
+      gguf_moe_gemv_kernel<TYPE, 1><<<grid, 128, 0, st>>>(a.W, a.row_bytes, a.ids, a.e0, a.e_local, a.x, a.x_stride, a.x_div, a.out,
+                                                          a.out_stride, a.N, a.K, a.act, a.limit);
+    else
+      gguf_moe_gemv_kernel<TYPE, 0><<<grid, 128, 0, st>>>(a.W, a.row_bytes, a.ids, a.e0, a.e_local, a.x, a.x_stride, a.x_div, a.out,
+                                                          a.out_stride, a.N, a.K, a.act, a.limit);
+    VE_CHECK_LAUNCH();
+  }
+  a.tiles_per_route = fuse_act ? (a.N / 2 + 7) / 8 : (a.N + 15) / 16;
+  a.tiles = a.tiles_per_route * routes;
+  return fuse_act ? launch_gguf_mma<TYPE, 2, 1, 1>(a, st) : launch_gguf_mma<TYPE, 1, 1, 1>(a, st);
+}
+
+template <int TYPE>
+static int run_gguf_dequant(const uint8_t* W, long row_bytes, __nv_bfloat16* out, long N, int K, cudaStream_t st) {
+  const long total = N * (K / 32);
+  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+  gguf_dequant_kernel<TYPE><<<blocks, 256, 0, st>>>(W, row_bytes, out, N, K);
+  VE_CHECK_LAUNCH();
+}
+
+// CALL(type) for the block type of a launch
+#define VE_GGUF_TYPES(ggml_type, CALL)      \
+  switch (ggml_type) {                      \
+    case kQ8_0: return CALL(kQ8_0);         \
+    case kQ4_0: return CALL(kQ4_0);         \
+    case kQ4_K: return CALL(kQ4_K);         \
+    case kQ6_K: return CALL(kQ6_K);         \
+    case kQ4_1: return CALL(kQ4_1);         \
+    case kQ5_0: return CALL(kQ5_0);         \
+    case kQ5_1: return CALL(kQ5_1);         \
+    case kQ2_K: return CALL(kQ2_K);         \
+    case kQ3_K: return CALL(kQ3_K);         \
+    case kQ5_K: return CALL(kQ5_K);         \
+    case kIQ4_NL: return CALL(kIQ4_NL);     \
+    case kIQ4_XS: return CALL(kIQ4_XS);     \
+    case kIQ2_XXS: return CALL(kIQ2_XXS);   \
+    case kIQ2_XS: return CALL(kIQ2_XS);     \
+    case kIQ2_S: return CALL(kIQ2_S);       \
+    case kIQ3_XXS: return CALL(kIQ3_XXS);   \
+    case kIQ3_S: return CALL(kIQ3_S);       \
+    case kIQ1_S: return CALL(kIQ1_S);       \
+    case kIQ1_M: return CALL(kIQ1_M);       \
+    default: return cudaErrorInvalidValue;  \
+  }
 
 // which devices have had their grid table set (a codebook format launched without it would read through a null pointer)
 static bool g_iq_ready[64];
@@ -434,36 +497,11 @@ int ve_gguf_gemv(const void* W, int ggml_type, long row_bytes, const void* x, lo
   if (M <= 0 || M > 16 || N <= 0 || K % 32) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
   if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
-  const int blocks = (N + 7) / 8;
-  __nv_bfloat16* ob = out_is_f32 ? nullptr : (__nv_bfloat16*)out;
-  float* of = out_is_f32 ? (float*)out : nullptr;
-#define VE_GG(T)                                                                                                  \
-  gguf_gemv_kernel<T><<<blocks, 256, 0, st>>>((const uint8_t*)W, row_bytes, (const __nv_bfloat16*)x, x_stride, ob, \
-                                              out_stride, of, M, N, K)
-  switch (ggml_type) {
-    case kQ8_0: VE_GG(kQ8_0); break;
-    case kQ4_0: VE_GG(kQ4_0); break;
-    case kQ4_K: VE_GG(kQ4_K); break;
-    case kQ6_K: VE_GG(kQ6_K); break;
-    case kQ4_1: VE_GG(kQ4_1); break;
-    case kQ5_0: VE_GG(kQ5_0); break;
-    case kQ5_1: VE_GG(kQ5_1); break;
-    case kQ2_K: VE_GG(kQ2_K); break;
-    case kQ3_K: VE_GG(kQ3_K); break;
-    case kQ5_K: VE_GG(kQ5_K); break;
-    case kIQ4_NL: VE_GG(kIQ4_NL); break;
-    case kIQ4_XS: VE_GG(kIQ4_XS); break;
-    case kIQ2_XXS: VE_GG(kIQ2_XXS); break;
-    case kIQ2_XS: VE_GG(kIQ2_XS); break;
-    case kIQ2_S: VE_GG(kIQ2_S); break;
-    case kIQ3_XXS: VE_GG(kIQ3_XXS); break;
-    case kIQ3_S: VE_GG(kIQ3_S); break;
-    case kIQ1_S: VE_GG(kIQ1_S); break;
-    case kIQ1_M: VE_GG(kIQ1_M); break;
-    default: return cudaErrorInvalidValue;
-  }
-#undef VE_GG
-  VE_CHECK_LAUNCH();
+  GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)N * row_bytes, (const __nv_bfloat16*)x, x_stride,
+                 out_is_f32 ? nullptr : (__nv_bfloat16*)out, out_is_f32 ? (float*)out : nullptr, out_stride, M, N, K};
+#define VE_CALL(T) run_gguf_gemv<T>(a, st)
+  VE_GGUF_TYPES(ggml_type, VE_CALL)
+#undef VE_CALL
 }
 
 // Routed-expert mat-vec over GGUF blocks; see gguf_moe_gemv_kernel. fuse_act: W rows are [gate (N/2) | up (N/2)] and the
@@ -475,76 +513,20 @@ int ve_gguf_moe_gemv(const void* W, int ggml_type, long row_bytes, const void* i
   if (N <= 0 || K % 32 || x_div <= 0 || (fuse_act && N % 2)) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
   if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
-  const int outs = fuse_act ? N / 2 : N;
-  const dim3 grid((outs + 3) / 4, routes);
-#define VE_GM(T)                                                                                                       \
-  do {                                                                                                                 \
-    if (fuse_act)                                                                                                      \
-      gguf_moe_gemv_kernel<T, 1><<<grid, 128, 0, st>>>((const uint8_t*)W, row_bytes, (const int*)ids, e0, e_local,       \
-                                                       (const __nv_bfloat16*)x, x_stride, x_div, (__nv_bfloat16*)out,    \
-                                                       out_stride, N, K, act, limit);                                    \
-    else                                                                                                               \
-      gguf_moe_gemv_kernel<T, 0><<<grid, 128, 0, st>>>((const uint8_t*)W, row_bytes, (const int*)ids, e0, e_local,       \
-                                                       (const __nv_bfloat16*)x, x_stride, x_div, (__nv_bfloat16*)out,    \
-                                                       out_stride, N, K, act, limit);                                    \
-  } while (0)
-  switch (ggml_type) {
-    case kQ8_0: VE_GM(kQ8_0); break;
-    case kQ4_0: VE_GM(kQ4_0); break;
-    case kQ4_K: VE_GM(kQ4_K); break;
-    case kQ6_K: VE_GM(kQ6_K); break;
-    case kQ4_1: VE_GM(kQ4_1); break;
-    case kQ5_0: VE_GM(kQ5_0); break;
-    case kQ5_1: VE_GM(kQ5_1); break;
-    case kQ2_K: VE_GM(kQ2_K); break;
-    case kQ3_K: VE_GM(kQ3_K); break;
-    case kQ5_K: VE_GM(kQ5_K); break;
-    case kIQ4_NL: VE_GM(kIQ4_NL); break;
-    case kIQ4_XS: VE_GM(kIQ4_XS); break;
-    case kIQ2_XXS: VE_GM(kIQ2_XXS); break;
-    case kIQ2_XS: VE_GM(kIQ2_XS); break;
-    case kIQ2_S: VE_GM(kIQ2_S); break;
-    case kIQ3_XXS: VE_GM(kIQ3_XXS); break;
-    case kIQ3_S: VE_GM(kIQ3_S); break;
-    case kIQ1_S: VE_GM(kIQ1_S); break;
-    case kIQ1_M: VE_GM(kIQ1_M); break;
-    default: return cudaErrorInvalidValue;
-  }
-#undef VE_GM
-  VE_CHECK_LAUNCH();
+  GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)e_local * N * row_bytes, (const __nv_bfloat16*)x, x_stride,
+                 (__nv_bfloat16*)out, nullptr, out_stride, 1, N, K, 0, (const int*)ids, e0, e_local, x_div, act, 0, limit};
+#define VE_CALL(T) run_gguf_moe<T>(a, routes, fuse_act, st)
+  VE_GGUF_TYPES(ggml_type, VE_CALL)
+#undef VE_CALL
 }
 
 int ve_gguf_dequant(const void* W, int ggml_type, long row_bytes, void* out, long N, int K, cudaStream_t st) {
   if (N <= 0 || K % 32) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
   if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
-  const long total = N * (K / 32);
-  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-#define VE_GD(T) gguf_dequant_kernel<T><<<blocks, 256, 0, st>>>((const uint8_t*)W, row_bytes, (__nv_bfloat16*)out, N, K)
-  switch (ggml_type) {
-    case kQ8_0: VE_GD(kQ8_0); break;
-    case kQ4_0: VE_GD(kQ4_0); break;
-    case kQ4_K: VE_GD(kQ4_K); break;
-    case kQ6_K: VE_GD(kQ6_K); break;
-    case kQ4_1: VE_GD(kQ4_1); break;
-    case kQ5_0: VE_GD(kQ5_0); break;
-    case kQ5_1: VE_GD(kQ5_1); break;
-    case kQ2_K: VE_GD(kQ2_K); break;
-    case kQ3_K: VE_GD(kQ3_K); break;
-    case kQ5_K: VE_GD(kQ5_K); break;
-    case kIQ4_NL: VE_GD(kIQ4_NL); break;
-    case kIQ4_XS: VE_GD(kIQ4_XS); break;
-    case kIQ2_XXS: VE_GD(kIQ2_XXS); break;
-    case kIQ2_XS: VE_GD(kIQ2_XS); break;
-    case kIQ2_S: VE_GD(kIQ2_S); break;
-    case kIQ3_XXS: VE_GD(kIQ3_XXS); break;
-    case kIQ3_S: VE_GD(kIQ3_S); break;
-    case kIQ1_S: VE_GD(kIQ1_S); break;
-    case kIQ1_M: VE_GD(kIQ1_M); break;
-    default: return cudaErrorInvalidValue;
-  }
-#undef VE_GD
-  VE_CHECK_LAUNCH();
+#define VE_CALL(T) run_gguf_dequant<T>((const uint8_t*)W, row_bytes, (__nv_bfloat16*)out, N, K, st)
+  VE_GGUF_TYPES(ggml_type, VE_CALL)
+#undef VE_CALL
 }
 
 }  // extern "C"
