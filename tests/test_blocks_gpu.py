@@ -35,3 +35,50 @@ def test_gguf_matvec_edges(t, shift):
         for M in (1, 4, 5, 8, 9):
             assert torch.equal(lin.forward(x[:M].cuda(), out_f32=True), full[:M]), (t, N, K, M)
         assert _rel(lin.forward(x[:3].cuda()).cpu(), want[:3]) < 2 ** -8      # bf16 output: half a unit in the last place
+
+
+@pytest.mark.parametrize("spec", ["gguf_q8_0+q4_0", "gguf_q4_k+q5_1", "gguf_iq1_m+iq2_xs", "gguf_q6_k+q3_k", "gguf_q2_k+iq4_xs"])
+@pytest.mark.parametrize("rows", [17, 130, 700])
+def test_gguf_experts_decoded_in_tiles(spec, rows):
+    """The grouped GEMM that decodes blocks in its tile loader against decoding the bank to bf16 first: the same operands, sums of the same
+    MMA. Experts with no row, one row and several tiles; feature counts that are no multiple of 128; a share of experts elsewhere."""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank, parse_expert_quant
+    gt, dt = parse_expert_quant(spec)
+    E, I, H, k = 6, 256 + 64 * (gq.BLOCK[dt][0] == 32), 512, 3
+    bank = GGUFExpertBank.random(E, I, H, gt, dt, e0=2, seed=rows, amp=0.05, device="cuda")
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(9, generator=g)[:k] for _ in range(rows)]).to(torch.int32)
+    ids[:, 0] = 5
+    ids[ids == 4] = 8
+    ids[0, 1] = 4                                   # expert 4: one row; 0, 1 and 8: elsewhere
+    ids = ids.cuda()
+    assert bank._decodes_in_tiles(rows * k)
+    got, want = bank.routes_prefill(x, ids, 0, 0.0), bank._routes_prefill_slabs(x, ids, 0, 0.0)
+    away = ((ids < 2) | (ids >= 8)).reshape(-1)
+    assert not got[away].any()
+    assert _rel(got, want) < 1e-3
+    from volta_engine_b200.ops import kernels as K
+    assert K.check_status("cuda") == 0
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("cb", [0, 1, 2])
+def test_exl3_experts_decoded_in_tiles(bits, cb):
+    """The same for trellis codes; K of the down projection is no multiple of the 256 weights a unit holds."""
+    from volta_engine_b200.ops.moe_exl3 import EXL3ExpertBank
+    E, I, H, k, rows = 4, 128, 384, 2, 150
+    bank = EXL3ExpertBank.random(E, I, H, bits, e0=1, seed=bits, device="cuda", std=0.05)
+    bank.cb = cb
+    g = torch.Generator().manual_seed(bits)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(6, generator=g)[:k] for _ in range(rows)]).to(torch.int32).cuda()
+    got, want = bank.routes_prefill(x, ids, 0, 0.0), bank._routes_prefill_slabs(x, ids, 0)
+    away = ((ids < 1) | (ids >= 5)).reshape(-1)
+    assert not got[away].any() and not want[away].any()
+    assert _rel(got, want) < 1e-3
+    few = bank.routes_decode(x[:5], ids[:5], 0, 0.0)
+    assert not few[away[:5 * k]].any()
+    assert _rel(few, want[:5 * k]) < 2e-2           # fp16 activations against bf16 ones
+    from volta_engine_b200.ops import kernels as K
+    assert K.check_status("cuda") == 0

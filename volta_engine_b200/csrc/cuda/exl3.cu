@@ -13,67 +13,9 @@
 // value = lo half + hi half.
 // Reference counterparts: src/kernels/slang/ref_trellis.slang:1-130 (format statement),
 // src/kernels/cuda/trellis/ (decode GEMV / GEMM), src/backend/cpu/linear_trellis.cpp:129-239.
-#include "common.cuh"
-#include <cuda_fp16.h>
+#include "exl3_blocks.cuh"
 
 namespace ve {
-
-// Two windows -> packed half2 bits of the two decoded values (low half = first window).
-template <int CB>
-VE_DEVINL uint32_t exl3_decode2(uint32_t w0, uint32_t w1) {
-  if (CB == 2) {
-    const uint32_t h0 = __dp4a(w0 * 0x83DCD12Du, 0x01010101u, 0x6400u);   // fp16 bits of 1024 + s
-    const uint32_t h1 = __dp4a(w1 * 0x83DCD12Du, 0x01010101u, 0x6400u);
-    const uint32_t pk = __byte_perm(h0, h1, 0x5410);                       // low halves of h0, h1 (their high halves are 0)
-    const __half2 a = __half2half2(__ushort_as_half((unsigned short)0x1eee));
-    const __half2 b = __half2half2(__ushort_as_half((unsigned short)0xc931));
-    const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&pk), a, b);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  } else {
-    uint32_t x0, x1;
-    if (CB == 0) { x0 = w0 * 89226354u + 64248484u; x1 = w1 * 89226354u + 64248484u; }
-    else { x0 = w0 * 0xCBAC1FEDu; x1 = w1 * 0xCBAC1FEDu; }
-    x0 = (x0 & 0x8fff8fffu) ^ 0x3b603b60u;
-    x1 = (x1 & 0x8fff8fffu) ^ 0x3b603b60u;
-    const uint32_t lo = __byte_perm(x0, x1, 0x5410), hi = __byte_perm(x0, x1, 0x7632);
-    const __half2 v = __hadd2(*reinterpret_cast<const __half2*>(&lo), *reinterpret_cast<const __half2*>(&hi));
-    return *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-
-// Words a lane needs from its tile and the bit offset of its first window inside them.
-template <int BITS> struct Exl3Lane {
-  static constexpr int NW = BITS <= 4 ? 2 : 3;
-  int w0, off;
-  VE_DEVINL explicit Exl3Lane(int lane) {
-    const int total = 256 * BITS;
-    const int s0 = (8 * lane * BITS + BITS - 16 + total) % total;
-    w0 = s0 >> 5; off = s0 & 31;
-  }
-  VE_DEVINL void load(const uint32_t* __restrict__ tile, uint32_t* w) const {
-#pragma unroll
-    for (int j = 0; j < NW; ++j) { int idx = w0 + j; if (idx >= 8 * BITS) idx -= 8 * BITS; w[j] = __ldg(tile + idx); }
-  }
-  // The lane's 8 windows -> four packed half2 (B fragments b0,b1 of column block 0, then of block 1).
-  template <int CB> VE_DEVINL void decode(const uint32_t* w, uint32_t* frag) const {
-    uint32_t q[3];
-    q[0] = __funnelshift_l(w[1], w[0], off);
-    q[1] = __funnelshift_l(NW > 2 ? w[2] : 0u, w[1], off);
-    q[2] = NW > 2 ? (w[2] << off) : 0u;
-    uint32_t win[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = i * BITS, j = t >> 5, sh = t & 31;          // window i = bits [sh, sh + 16) below the top of q[j] : q[j + 1]
-      if (sh <= 16) {
-        win[i] = (q[j] >> (16 - sh)) & 0xffffu;                 // inside one word: a single bit-field extract
-      } else {
-        win[i] = __funnelshift_r(q[j + 1 > 2 ? 2 : j + 1], q[j], 48 - sh) & 0xffffu;
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p) frag[p] = exl3_decode2<CB>(win[2 * p], win[2 * p + 1]);
-  }
-};
 
 VE_DEVINL void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -247,6 +189,7 @@ struct HadArgs {
   const void* in; const void* in2; void* out;
   const __half* scale; const __half* scale2;
   const int* expert; long scale_stride;
+  const int* src;                // null: input row = row / in_div; else src[row] / in_div
   int rows, C, post, in_div, rows_per_group, act;
 };
 
@@ -268,12 +211,17 @@ __global__ void __launch_bounds__(256) had128_kernel(HadArgs a) {
     long soff = col;
     if (a.expert) {
       const int e = a.expert[row / a.rows_per_group];
-      if (e < 0) continue;
+      if (e < 0) {                                     // another rank's route: zeros
+        const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!a.src) had_store4<DO>(a.out, (size_t)row * a.C + col, zero);      // (rows behind the sorted routes stay unwritten)
+        continue;
+      }
       soff += (long)e * a.scale_stride;
     }
+    const size_t in_row = (size_t)((a.src ? a.src[row] : row) / a.in_div) * a.C;
     float s[4] = {1.f, 1.f, 1.f, 1.f}, v[4];
     if (a.scale) had_load4<2>(a.scale, soff, s);
-    had_load4<DI>(a.in, (size_t)(row / a.in_div) * a.C + col, v);
+    had_load4<DI>(a.in, in_row + col, v);
     if (!a.post) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] *= s[j];
@@ -286,7 +234,7 @@ __global__ void __launch_bounds__(256) had128_kernel(HadArgs a) {
     if (a.in2) {
       float u[4], s2[4] = {1.f, 1.f, 1.f, 1.f};
       if (a.scale2) had_load4<2>(a.scale2, soff, s2);
-      had_load4<DI>(a.in2, (size_t)(row / a.in_div) * a.C + col, u);
+      had_load4<DI>(a.in2, in_row + col, u);
       wht128(u, lane);
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = act_apply(v[j], a.act) * (u[j] * s2[j]);
@@ -410,12 +358,13 @@ static int exl3_reconstruct_n(const void* codes, void* out, int K, int N, int bi
 extern "C" {
 
 // dt codes: 0 bf16, 1 fp32, 2 fp16. Supported (in -> out): bf16->fp16, fp32->bf16, fp32->fp16, fp16->fp16, bf16->bf16.
+// expert: scale row of every output row (negative: zeros are written); src: input row times in_div of every output row.
 int ve_had128(const void* in, const void* in2, void* out, const void* scale, const void* scale2, const void* expert,
-              long scale_stride, int rows, int C, int post, int in_div, int rows_per_group, int act, int dt_in,
+              const void* src, long scale_stride, int rows, int C, int post, int in_div, int rows_per_group, int act, int dt_in,
               int dt_out, cudaStream_t st) {
   if (rows < 1 || C % 128 || in_div < 1 || rows_per_group < 1) return cudaErrorInvalidValue;
   HadArgs a{in, in2, out, (const __half*)scale, (const __half*)scale2, (const int*)expert, scale_stride,
-            rows, C, post, in_div, rows_per_group, act};
+            (const int*)src, rows, C, post, in_div, rows_per_group, act};
   const long blocks_needed = ((long)rows * (C / 128) + 7) / 8;
   const int blocks = (int)(blocks_needed < 148 * 8 ? blocks_needed : 148 * 8);
   if (dt_in == 0 && dt_out == 2) had128_kernel<0, 2><<<blocks, 256, 0, st>>>(a);

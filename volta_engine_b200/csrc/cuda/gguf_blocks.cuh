@@ -520,3 +520,34 @@ VE_DEVINL void frag(const uint8_t* u, int c, int t, const uint8_t* tab, uint32_t
 }
 
 }  // namespace ve
+
+// CALL(type) for the block type of a launch
+#define VE_GGUF_TYPES(ggml_type, CALL)      \
+  switch (ggml_type) {                      \
+    case kQ8_0: return CALL(kQ8_0);         \
+    case kQ4_0: return CALL(kQ4_0);         \
+    case kQ4_K: return CALL(kQ4_K);         \
+    case kQ6_K: return CALL(kQ6_K);         \
+    case kQ4_1: return CALL(kQ4_1);         \
+    case kQ5_0: return CALL(kQ5_0);         \
+    case kQ5_1: return CALL(kQ5_1);         \
+    case kQ2_K: return CALL(kQ2_K);         \
+    case kQ3_K: return CALL(kQ3_K);         \
+    case kQ5_K: return CALL(kQ5_K);         \
+    case kIQ4_NL: return CALL(kIQ4_NL);     \
+    case kIQ4_XS: return CALL(kIQ4_XS);     \
+    case kIQ2_XXS: return CALL(kIQ2_XXS);   \
+    case kIQ2_XS: return CALL(kIQ2_XS);     \
+    case kIQ2_S: return CALL(kIQ2_S);       \
+    case kIQ3_XXS: return CALL(kIQ3_XXS);   \
+    case kIQ3_S: return CALL(kIQ3_S);       \
+    case kIQ1_S: return CALL(kIQ1_S);       \
+    case kIQ1_M: return CALL(kIQ1_M);       \
+    default: return cudaErrorInvalidValue;  \
+  }
+
+namespace ve {
+// false: a codebook format whose grid table has not been set on the current device (gguf_gemv.cu)
+bool iq_grids_ready(int ggml_type);
+int set_iq_grids_gemm(const void* table);                   // gemm_blocks.cu
+}  // namespace ve

@@ -442,41 +442,18 @@ static int run_gguf_dequant(const uint8_t* W, long row_bytes, __nv_bfloat16* out
   VE_CHECK_LAUNCH();
 }
 
-// CALL(type) for the block type of a launch
-#define VE_GGUF_TYPES(ggml_type, CALL)      \
-  switch (ggml_type) {                      \
-    case kQ8_0: return CALL(kQ8_0);         \
-    case kQ4_0: return CALL(kQ4_0);         \
-    case kQ4_K: return CALL(kQ4_K);         \
-    case kQ6_K: return CALL(kQ6_K);         \
-    case kQ4_1: return CALL(kQ4_1);         \
-    case kQ5_0: return CALL(kQ5_0);         \
-    case kQ5_1: return CALL(kQ5_1);         \
-    case kQ2_K: return CALL(kQ2_K);         \
-    case kQ3_K: return CALL(kQ3_K);         \
-    case kQ5_K: return CALL(kQ5_K);         \
-    case kIQ4_NL: return CALL(kIQ4_NL);     \
-    case kIQ4_XS: return CALL(kIQ4_XS);     \
-    case kIQ2_XXS: return CALL(kIQ2_XXS);   \
-    case kIQ2_XS: return CALL(kIQ2_XS);     \
-    case kIQ2_S: return CALL(kIQ2_S);       \
-    case kIQ3_XXS: return CALL(kIQ3_XXS);   \
-    case kIQ3_S: return CALL(kIQ3_S);       \
-    case kIQ1_S: return CALL(kIQ1_S);       \
-    case kIQ1_M: return CALL(kIQ1_M);       \
-    default: return cudaErrorInvalidValue;  \
-  }
-
 // which devices have had their grid table set (a codebook format launched without it would read through a null pointer)
 static bool g_iq_ready[64];
 
 static bool iq_type(int t) {
   return t == kIQ2_XXS || t == kIQ2_XS || t == kIQ2_S || t == kIQ3_XXS || t == kIQ3_S || t == kIQ1_S || t == kIQ1_M;
 }
-static bool iq_ready() {
+namespace ve {
+bool iq_grids_ready(int ggml_type) {
   int dev = 0;
-  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_iq_ready[dev];
+  return !iq_type(ggml_type) || (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_iq_ready[dev]);
 }
+}  // namespace ve
 
 extern "C" {
 
@@ -488,6 +465,8 @@ int ve_gguf_set_iq_grids(const void* table) {
   if (dev < 0 || dev >= 64 || !table || ((uintptr_t)table & 15)) return cudaErrorInvalidValue;
   e = cudaMemcpyToSymbol(kIqGrids, &table, sizeof(table));
   if (e != cudaSuccess) return (int)e;
+  const int rc = set_iq_grids_gemm(table);
+  if (rc) return rc;
   g_iq_ready[dev] = true;
   return 0;
 }
@@ -496,7 +475,7 @@ int ve_gguf_gemv(const void* W, int ggml_type, long row_bytes, const void* x, lo
                  int out_is_f32, int M, int N, int K, cudaStream_t st) {
   if (M <= 0 || M > 16 || N <= 0 || K % 32) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
-  if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
+  if (!iq_grids_ready(ggml_type)) return cudaErrorNotReady;
   GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)N * row_bytes, (const __nv_bfloat16*)x, x_stride,
                  out_is_f32 ? nullptr : (__nv_bfloat16*)out, out_is_f32 ? (float*)out : nullptr, out_stride, M, N, K};
 #define VE_CALL(T) run_gguf_gemv<T>(a, st)
@@ -512,7 +491,7 @@ int ve_gguf_moe_gemv(const void* W, int ggml_type, long row_bytes, const void* i
   if (routes <= 0) return 0;
   if (N <= 0 || K % 32 || x_div <= 0 || (fuse_act && N % 2)) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
-  if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
+  if (!iq_grids_ready(ggml_type)) return cudaErrorNotReady;
   GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)e_local * N * row_bytes, (const __nv_bfloat16*)x, x_stride,
                  (__nv_bfloat16*)out, nullptr, out_stride, 1, N, K, 0, (const int*)ids, e0, e_local, x_div, act, 0, limit};
 #define VE_CALL(T) run_gguf_moe<T>(a, routes, fuse_act, st)
@@ -523,7 +502,7 @@ int ve_gguf_moe_gemv(const void* W, int ggml_type, long row_bytes, const void* i
 int ve_gguf_dequant(const void* W, int ggml_type, long row_bytes, void* out, long N, int K, cudaStream_t st) {
   if (N <= 0 || K % 32) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
-  if (iq_type(ggml_type) && !iq_ready()) return cudaErrorNotReady;
+  if (!iq_grids_ready(ggml_type)) return cudaErrorNotReady;
 #define VE_CALL(T) run_gguf_dequant<T>((const uint8_t*)W, row_bytes, (__nv_bfloat16*)out, N, K, st)
   VE_GGUF_TYPES(ggml_type, VE_CALL)
 #undef VE_CALL

@@ -17,14 +17,14 @@ _DT = {torch.bfloat16: 0, torch.float32: 1, torch.float16: 2}
 
 
 def had128(x, scale=None, *, post=False, out_dtype=None, out=None, x2=None, scale2=None, act=0, expert=None,
-           scale_stride=0, in_div=1, rows_per_group=1, rows=None):
+           scale_stride=0, in_div=1, rows_per_group=1, rows=None, src=None):
     """GPU Hadamard rotation over blocks of 128 with the EXL3 channel scales folded in (see ve_had128)."""
     C = x.shape[-1]
     rows = rows if rows is not None else x.numel() // C
     out_dtype = out_dtype or x.dtype
     if out is None:
         out = torch.empty(rows, C, dtype=out_dtype, device=x.device)
-    call("had128", "pppppp" + "liiiiiiii", ptr(x), ptr(x2), ptr(out), ptr(scale), ptr(scale2), ptr(expert),
+    call("had128", "ppppppp" + "liiiiiiii", ptr(x), ptr(x2), ptr(out), ptr(scale), ptr(scale2), ptr(expert), ptr(src),
          int(scale_stride), rows, C, 1 if post else 0, in_div, rows_per_group, act, _DT[x.dtype], _DT[out.dtype])
     return out
 

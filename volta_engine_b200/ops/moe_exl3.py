@@ -10,9 +10,9 @@ expert costs rotations around each of its three matrices:
     launch that rotates both projections back, applies their output scales and the gated activation
     (``had128(x2=, act=)``); the same again around the down projection. Routes of experts owned by other ranks come out
     as zeros;
-  * prefill chunks: routes sorted by expert, then per slab of experts: codes -> bf16 cores (``exl3_reconstruct_batch``)
-    into a bounded scratch, rows rotated with their expert's scales, grouped tcgen05 GEMMs over the slab's tiles, rotated
-    back; the slab's rows are scattered back into route order (no host synchronisation);
+  * prefill chunks: routes sorted by expert, rows rotated with their expert's scales, grouped tcgen05 GEMMs that decode the
+    tiles in their tile loader (``gemm_grouped_exl3``), rotated back and put into route order (no host synchronisation). Many rows an
+    expert: per slab of experts codes -> bf16 cores (``exl3_reconstruct_batch``) into a bounded scratch and the bf16 grouped GEMM;
   * CPU: the fp32 statement (``quant.exl3.linear_reference`` per route).
 Reference: src/kernels/cuda/trellis/exl3_moe_coop.cu:1034-1205 (rotation kernel, gate / up mat-vec per expert run, down
 mat-vec), exl3_moe_kernel.cuh (prefill work items), inc/engine/modules/moe.h:79-195.
@@ -26,6 +26,7 @@ from ..quant import exl3 as ex
 from . import kernels as K
 from .linear_exl3 import exl3_gemv, had128
 
+FUSED_ROWS = 512              # rows an expert up to which the grouped GEMM decodes the codes itself
 SLAB_BYTES = 2 << 30
 
 
@@ -79,26 +80,22 @@ class EXL3ExpertBank:
         rows, H = x.shape
         k = ids.shape[1]
         R, I, dev = rows * k, self.inter, x.device
-        e = ids.reshape(-1) - self.e0
-        e = torch.where((e >= 0) & (e < self.e_local), e, torch.full_like(e, -1)).to(torch.int32).contiguous()
+        e = torch.empty(R, dtype=torch.int32, device=dev)
+        call("moe_row_experts", "pppiipi", ptr(ids), None, None, self.e0, self.e_local, ptr(e), R)
         per_gu, per_dn = self.gate[0].numel(), self.down[0].numel()
         s = self.s
         f16 = torch.float16
-        xg = had128(x, s["g_suh"], out_dtype=f16, expert=e, scale_stride=H, in_div=k, rows=R, out=torch.zeros(R, H, dtype=f16, device=dev))
-        xu = had128(x, s["u_suh"], out_dtype=f16, expert=e, scale_stride=H, in_div=k, rows=R, out=torch.zeros(R, H, dtype=f16, device=dev))
-        ga = exl3_gemv(self.gate, xg, 1, H, I, self.bits, self.cb, out=torch.zeros(R, I, dtype=torch.float32, device=dev),
-                       expert=e, expert_stride=per_gu, groups=R)
-        ua = exl3_gemv(self.up, xu, 1, H, I, self.bits, self.cb, out=torch.zeros(R, I, dtype=torch.float32, device=dev),
-                       expert=e, expert_stride=per_gu, groups=R)
-        a = had128(ga, s["g_svh"], post=True, out_dtype=f16, x2=ua, scale2=s["u_svh"], act=act, expert=e, scale_stride=I,
-                   rows=R, out=torch.zeros(R, I, dtype=f16, device=dev))
+        # (rotations write zeros for routes of other ranks' experts, mat-vecs leave theirs unwritten)
+        xg = had128(x, s["g_suh"], out_dtype=f16, expert=e, scale_stride=H, in_div=k, rows=R)
+        xu = had128(x, s["u_suh"], out_dtype=f16, expert=e, scale_stride=H, in_div=k, rows=R)
+        ga = exl3_gemv(self.gate, xg, 1, H, I, self.bits, self.cb, expert=e, expert_stride=per_gu, groups=R)
+        ua = exl3_gemv(self.up, xu, 1, H, I, self.bits, self.cb, expert=e, expert_stride=per_gu, groups=R)
+        a = had128(ga, s["g_svh"], post=True, out_dtype=f16, x2=ua, scale2=s["u_svh"], act=act, expert=e, scale_stride=I, rows=R)
         if limit > 0:
             raise NotImplementedError("clamped gated activation on the EXL3 expert path")
-        xd = had128(a, s["d_suh"], out_dtype=f16, expert=e, scale_stride=I, rows=R, out=torch.zeros(R, I, dtype=f16, device=dev))
-        da = exl3_gemv(self.down, xd, 1, I, H, self.bits, self.cb, out=torch.zeros(R, H, dtype=torch.float32, device=dev),
-                       expert=e, expert_stride=per_dn, groups=R)
-        return had128(da, s["d_svh"], post=True, out_dtype=x.dtype, expert=e, scale_stride=H, rows=R,
-                      out=torch.zeros(R, H, dtype=x.dtype, device=dev))
+        xd = had128(a, s["d_suh"], out_dtype=f16, expert=e, scale_stride=I, rows=R)
+        da = exl3_gemv(self.down, xd, 1, I, H, self.bits, self.cb, expert=e, expert_stride=per_dn, groups=R)
+        return had128(da, s["d_svh"], post=True, out_dtype=x.dtype, expert=e, scale_stride=H, rows=R)
 
     # ------------------------------------------------------------------------------------------ prefill chunks
     def slab_experts(self) -> int:
@@ -108,6 +105,44 @@ class EXL3ExpertBank:
     def routes_prefill(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
         if limit > 0:
             raise NotImplementedError("clamped gated activation on the EXL3 expert path")
+        rows, H = x.shape
+        k = ids.shape[1]
+        R, I, dev, E = rows * k, self.inter, x.device, self.e_local
+        if R > FUSED_ROWS * E or (self.gate.data_ptr() | self.up.data_ptr() | self.down.data_ptr()) % 16:
+            return self._routes_prefill_slabs(x, ids, act)
+        bf = torch.bfloat16
+        st = K.status_word(dev)
+        s = self.s
+        max_tiles = R // 128 + E + 1
+        inv = torch.empty(R, dtype=torch.int32, device=dev)
+        srt = torch.empty(R, dtype=torch.int32, device=dev)
+        e_rows = torch.empty(R, dtype=torch.int32, device=dev)
+        tab = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
+        totals = torch.empty(2, dtype=torch.int32, device=dev)
+        call("moe_sort", "piiiipppip", ptr(ids), R, self.e0, E, 128, ptr(inv), ptr(srt), ptr(tab), max_tiles, ptr(totals))
+        # expert of every sorted row; rows behind the local routes carry -1: no kernel writes them and no tile in use reads them
+        call("moe_row_experts", "pppiipi", ptr(ids), ptr(srt), ptr(totals), self.e0, E, ptr(e_rows), R)
+
+        def grouped(codes, rot, K_, N):
+            out = torch.empty(R, N, dtype=bf, device=dev)
+            call("gemm_grouped_exl3", "piiplpliiiipip", ptr(codes), self.bits, self.cb, ptr(rot), rot.stride(0), ptr(out), out.stride(0), R,
+                 E, N, K_, ptr(tab), max_tiles, ptr(st))
+            return out
+        x = x.contiguous()
+        xr = had128(x, s["g_suh"], out_dtype=bf, expert=e_rows, scale_stride=H, rows=R, src=srt, in_div=k)
+        ga = grouped(self.gate, xr, H, I)
+        had128(x, s["u_suh"], out_dtype=bf, expert=e_rows, scale_stride=H, rows=R, src=srt, in_div=k, out=xr)
+        ua = grouped(self.up, xr, H, I)
+        a = had128(ga, s["g_svh"], post=True, out_dtype=bf, x2=ua, scale2=s["u_svh"], act=act, expert=e_rows, scale_stride=I, rows=R)
+        xd = had128(a, s["d_suh"], out_dtype=bf, expert=e_rows, scale_stride=I, rows=R)
+        da = grouped(self.down, xd, I, H)
+        ds = had128(da, s["d_svh"], post=True, out_dtype=x.dtype, expert=e_rows, scale_stride=H, rows=R)
+        d = torch.empty(R, H, dtype=x.dtype, device=dev)
+        call("moe_unsort", "plppii", ptr(ds), ds.stride(0), ptr(inv), ptr(d), R, H)
+        return d
+
+    def _routes_prefill_slabs(self, x: torch.Tensor, ids: torch.Tensor, act: int) -> torch.Tensor:
+        """The same per slab of experts: codes -> bf16 scratch, then the bf16 grouped GEMM."""
         rows, H = x.shape
         k = ids.shape[1]
         R, I, dev = rows * k, self.inter, x.device

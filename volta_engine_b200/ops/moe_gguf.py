@@ -6,9 +6,10 @@ for gate / up with a wider one for down). Three ways through it:
 
   * decode / verify rows (<= 16): the fused dequant mat-vec per route (csrc/cuda/gguf_gemv.cu ``gguf_moe_gemv``), gated
     activation inside the gate|up launch, rows of experts owned by other ranks come out as zeros;
-  * prefill chunks: routes sorted by expert, then per slab of experts: blocks -> bf16 (``gguf_dequant``) into a bounded
-    scratch, grouped tcgen05 GEMMs over the slab's tiles, activation, down projection; the slab's rows are scattered back
-    into route order. No host synchronisation: the tile table of every slab is built on the device;
+  * prefill chunks: routes sorted by expert, then grouped tcgen05 GEMMs that decode the blocks in their tile loader
+    (``gemm_grouped_gguf``), with the activation between them; the rows are put back into route order. Many rows an expert: per slab of
+    experts the blocks -> bf16 (``gguf_dequant``) into a bounded scratch and the bf16 grouped GEMM. No host synchronisation: the tile
+    table is built on the device;
   * CPU: the fp32 statement (dequantise, matmul, bf16 rounding between the stages).
 Reference: src/kernels/cuda/gguf/gguf_moe.cu:38-1042 (MoEGguf: per-route mat-vec and grouped tiles),
 inc/engine/modules/moe_gguf.h.
@@ -22,6 +23,7 @@ from ..quant import gguf as gq
 from . import kernels as K
 from .linear_gguf import FUSED_TYPES, ensure_iq_grids
 
+FUSED_ROWS = 512              # rows an expert up to which the grouped GEMM decodes the blocks itself
 SLAB_BYTES = 2 << 30          # bf16 scratch for the dequantised experts of one slab (gate|up and down share it)
 
 
@@ -102,8 +104,42 @@ class GGUFExpertBank:
         per = 2 * self.inter * self.hidden * 2 + self.hidden * self.inter * 2
         return max(1, min(self.e_local, SLAB_BYTES // per))
 
+    def _decodes_in_tiles(self, routes: int) -> bool:
+        """Whether the grouped GEMM decodes the blocks in its tile loader, once per 128 rows of an expert. FUSED_ROWS says up to how
+        many rows an expert this is the faster way; blocks at odd addresses and rows that are no multiple of 16 bytes stay with the other."""
+        words = 4 if gq.row_bytes(self.gu_type, self.hidden) % 4 == 0 and gq.row_bytes(self.dn_type, self.inter) % 4 == 0 else 2
+        return (routes <= FUSED_ROWS * self.e_local and self.hidden % 8 == 0 and self.inter % 8 == 0
+                and self.gu_raw.data_ptr() % words == 0 and self.dn_raw.data_ptr() % words == 0)
+
     def routes_prefill(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
         """Same result layout as :meth:`routes_decode` for a chunk of rows, through the grouped tensor-core GEMM."""
+        rows, H = x.shape
+        k = ids.shape[1]
+        routes, I, dev, E = rows * k, self.inter, x.device, self.e_local
+        if not self._decodes_in_tiles(routes):
+            return self._routes_prefill_slabs(x, ids, act, limit)
+        st = K.status_word(dev)
+        max_tiles = routes // 128 + E + 1
+        inv = torch.empty(routes, dtype=torch.int32, device=dev)
+        srt = torch.empty(routes, dtype=torch.int32, device=dev)
+        tab = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
+        totals = torch.empty(2, dtype=torch.int32, device=dev)
+        call("moe_sort", "piiiipppip", ptr(ids), routes, self.e0, E, 128, ptr(inv), ptr(srt), ptr(tab), max_tiles, ptr(totals))
+        # rows behind the local routes are neither written nor read by the tiles in use
+        xs = torch.empty(routes, H, dtype=x.dtype, device=dev)
+        call("moe_gather", "plppiplii", ptr(x), x.stride(0), ptr(srt), ptr(totals), k, ptr(xs), xs.stride(0), H, routes)
+        gu = torch.empty(routes, 2 * I, dtype=x.dtype, device=dev)
+        call("gemm_grouped_gguf", "pilplpliiiipip", ptr(self.gu_raw), self.gu_type, self.gu_raw.shape[2], ptr(xs), xs.stride(0), ptr(gu),
+             gu.stride(0), routes, E, 2 * I, H, ptr(tab), max_tiles, ptr(st))
+        a = K.gated_act(gu, I, act, limit)
+        call("gemm_grouped_gguf", "pilplpliiiipip", ptr(self.dn_raw), self.dn_type, self.dn_raw.shape[2], ptr(a), a.stride(0), ptr(xs),
+             xs.stride(0), routes, E, H, I, ptr(tab), max_tiles, ptr(st))
+        d = torch.empty(routes, H, dtype=x.dtype, device=dev)
+        call("moe_unsort", "plppii", ptr(xs), xs.stride(0), ptr(inv), ptr(d), routes, H)
+        return d
+
+    def _routes_prefill_slabs(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
+        """The same per slab of experts: blocks -> bf16 scratch, then the bf16 grouped GEMM."""
         rows, H = x.shape
         k = ids.shape[1]
         routes, I, dev = rows * k, self.inter, x.device

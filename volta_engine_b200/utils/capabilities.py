@@ -24,7 +24,8 @@ TABLE = {
     "nvfp4_dequant": ("NVFP4 quantise", P), "bf16_gemv_f32": ("LinearPlainGEMV", P),
     "exl3_gemv": ("LinearTrellis", P), "exl3_reconstruct": ("LinearTrellis", P), "exl3_reconstruct_batch": ("MoE (EXL3 experts)", P), "exl3_viterbi": ("EXL3 quantiser", P), "exl3_viterbi_scratch": ("EXL3 quantiser", P), "had128": ("LinearTrellis", P),
     "gguf_gemv": ("LinearGguf", P), "gguf_dequant": ("LinearGguf", P), "gguf_set_iq_grids": ("LinearGguf", P),
-    "gguf_moe_gemv": ("MoEGguf", P),
+    "gguf_moe_gemv": ("MoEGguf", P), "gemm_grouped_gguf": ("MoEGguf", P), "gemm_grouped_exl3": ("MoE (EXL3 experts)", P),
+    "moe_unsort": ("MoE", P), "moe_row_experts": ("MoE (EXL3 experts)", P),
     "mla_rope_store": ("MLALatent", P), "mla_absorb_q": ("MLALatent", P), "mla_decode": ("MLALatent", P),
     "mla_expand_out": ("MLALatent", P),
     "latent_rope_store": ("LatentAttention", P), "latent_absorb": ("LatentAttention", P), "latent_attn": ("LatentAttention", P),
