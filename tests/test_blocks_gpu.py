@@ -82,3 +82,16 @@ def test_exl3_experts_decoded_in_tiles(bits, cb):
     assert _rel(few, want[:5 * k]) < 2e-2           # fp16 activations against bf16 ones
     from volta_engine_b200.ops import kernels as K
     assert K.check_status("cuda") == 0
+
+
+@pytest.mark.parametrize("N,K", [(1, 8), (17, 40), (512, 7168), (2368, 264), (2369, 1032), (5000, 2048)])
+def test_bf16_matvec_edges(N, K):
+    """Row counts on both sides of the warp-count rule, K that ends inside a 32-wide step, every count of activation rows up to more than
+    one pass; fp32 sums of exact products (1e-5), a row's result independent of the rows beside it."""
+    from volta_engine_b200.ops import kernels as K_
+    g = torch.Generator().manual_seed(N)
+    W, x = torch.randn(N, K, generator=g).to(torch.bfloat16), torch.randn(21, K, generator=g).to(torch.bfloat16)
+    full = K_.bf16_gemv_f32(W.cuda(), x.cuda())
+    assert _rel(full.cpu(), x.double() @ W.double().t()) < 1e-5
+    for M in (1, 2, 3, 7, 8, 9, 16):
+        assert torch.equal(K_.bf16_gemv_f32(W.cuda(), x[:M].cuda()), full[:M]), M

@@ -132,65 +132,77 @@ nvfp4_gemv_kernel(const uint8_t* __restrict__ Wp, const uint8_t* __restrict__ Ws
   }
 }
 
-// fp32-output variant for the LM head (logits stay fp32 for argmax / top-k / LSE).
-template <int MR>
-__global__ void __launch_bounds__(kGemvWarps * 32)
+// bf16 weights, fp32 output (LM head, routers: logits stay fp32 for argmax / top-k / LSE), up to 8 * NT activation rows in one pass.
+//
+// Bound by the weights' DRAM traffic (1.55 GB and 235 us for a 151936 x 5120 head), so they are read once whatever M is: a block takes 16 * NT
+// weight rows, its warps deal 32-wide steps of K, and each product with all activation rows is two tensor-core instructions per 16 rows
+// and step. (In passes of four activation rows with fp32 FMAs 16 rows took four reads: 1072 us for the head and four routers of the
+// 512-expert model, against 94 us for one row of the head.) Lane (g, t) holds k = 8 t .. 8 t + 7 of a step for weight rows g and g + 8 and
+// activation row g, whole 16-byte loads; both operands use the same order of k. The sum of a step leaves the tensor core and is added in
+// fp32. Steps, warps and their order follow from N and K alone: a row's result does not depend on the rows beside it.
+template <int NT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
 bf16_gemv_f32_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ x, long x_stride,
-                     float* __restrict__ out, long out_stride, int M, int N, int K, int m0) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n0 = blockIdx.x * kGemvRows;
-  __shared__ float part[kGemvWarps][kGemvRows][MR];
+                     float* __restrict__ out, long out_stride, int M, int N, int K) {
+  constexpr int ROWS = 16 * NT, COLS = 8 * NT, U = 4 / NT;      // U: steps in flight a warp (eight 16-byte weight loads a lane)
+  __shared__ float part[WARPS][COLS][ROWS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * ROWS;
   grid_dep_launch();
-  grid_dep_wait();                   // x is the output of the kernel in front (this launch is a programmatic dependent)
-  float acc[kGemvRows][MR];
+  grid_dep_wait();                   // x and, where they were just decoded, the weights come from kernels in front
+  const __nv_bfloat16 *wr[2 * NT], *xr[NT];
 #pragma unroll
-  for (int r = 0; r < kGemvRows; ++r)
+  for (int r = 0; r < 2 * NT; ++r) wr[r] = W + (long)min(n0 + r * 8 + g, N - 1) * K + 8 * t;
 #pragma unroll
-    for (int m = 0; m < MR; ++m) acc[r][m] = 0.f;
-  const int kchunks = K >> 3;
-  for (int c = threadIdx.x; c < kchunks; c += kGemvWarps * 32) {
-    float2 xv[MR][4];
+  for (int j = 0; j < NT; ++j) xr[j] = x + (long)min(j * 8 + g, M - 1) * x_stride + 8 * t;
+  float acc[NT][NT][4];
 #pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4*>(x + (long)min(m0 + m, M - 1) * x_stride + (long)c * 8);
-      const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+  for (int i = 0; i < NT; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        xv[m][j] = make_float2(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xffff0000u));
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+  const int steps = (K + 31) / 32;
+  for (int c0 = warp; c0 < steps; c0 += WARPS * U) {
+    uint4 w[U][2 * NT], v[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c0 + u * WARPS) * 32;
+      const bool live = k + 8 * t < K;
+#pragma unroll
+      for (int r = 0; r < 2 * NT; ++r) w[u][r] = live ? __ldcs(reinterpret_cast<const uint4*>(wr[r] + k)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        v[u][j] = live && j * 8 + g < M ? *reinterpret_cast<const uint4*>(xr[j] + k) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) {
-      const int n = min(n0 + r, N - 1);
-      const uint4 t = __ldcs(reinterpret_cast<const uint4*>(W + (long)n * K) + c);
-      const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 wf = make_float2(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xffff0000u));
+      for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int m = 0; m < MR; ++m) {
-          acc[r][m] = fmaf(wf.x, xv[m][j].x, acc[r][m]);
-          acc[r][m] = fmaf(wf.y, xv[m][j].y, acc[r][m]);
+        for (int j = 0; j < NT; ++j) {
+          const uint4 a = w[u][2 * i], b = w[u][2 * i + 1], y = v[u][j];
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16_16816(d, a.x, b.x, a.y, b.y, y.x, y.y);
+          mma_bf16_16816(d, a.z, b.z, a.w, b.w, y.z, y.w);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][j][e] += d[e];
         }
-      }
-    }
   }
 #pragma unroll
-  for (int r = 0; r < kGemvRows; ++r)
+  for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      float v = acc[r][m];
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) part[warp][r][m] = v;
-    }
+      for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t + (e & 1)][i * 16 + (e >> 1) * 8 + g] = acc[i][j][e];
   __syncthreads();
-  if (threadIdx.x < kGemvRows * MR) {
-    const int r = threadIdx.x / MR, m = threadIdx.x % MR;
-    if (n0 + r < N && m0 + m < M) {
-      float v = 0.f;
+  for (int i = threadIdx.x; i < COLS * ROWS; i += 32 * WARPS) {
+    const int m = i / ROWS, n = n0 + i % ROWS;
+    if (m < M && n < N) {
+      float sum = 0.f;
 #pragma unroll
-      for (int w = 0; w < kGemvWarps; ++w) v += part[w][r][m];
-      out[(long)(m0 + m) * out_stride + n0 + r] = v;
+      for (int q = 0; q < WARPS; ++q) sum += part[q][m][i % ROWS];
+      out[(long)m * out_stride + n] = sum;
     }
   }
 }
@@ -231,22 +243,18 @@ int ve_nvfp4_gemv(const void* Wp, const void* Ws, float gscale, const void* x, l
 int ve_bf16_gemv_f32(const void* W, const void* x, long x_stride, void* out, long out_stride, int M, int N, int K,
                      cudaStream_t st) {
   if (K % 8 || M <= 0 || N <= 0) return cudaErrorInvalidValue;
-  const int blocks = (N + kGemvRows - 1) / kGemvRows;
-  int m0 = 0;
-  while (m0 < M) {
-    const int left = M - m0;
-#define VE_LAUNCH(MR)                                                                                        \
-  launch_pdl(bf16_gemv_f32_kernel<MR>, dim3(blocks), dim3(kGemvWarps * 32), 0, st, (const __nv_bfloat16*)W, \
-             (const __nv_bfloat16*)x, x_stride, (float*)out, out_stride, M, N, K, m0)
-    if (left >= 4) {
-      VE_LAUNCH(4);
-      m0 += 4;
-    } else if (left >= 2) {
-      VE_LAUNCH(2);
-      m0 += 2;
+  for (int m0 = 0; m0 < M; m0 += 16) {
+    const int m = M - m0 < 16 ? M - m0 : 16, nt = m > 8 ? 2 : 1;
+    const __nv_bfloat16* xm = (const __nv_bfloat16*)x + (long)m0 * x_stride;
+    float* om = (float*)out + (long)m0 * out_stride;
+    const dim3 grid((N + 16 * nt - 1) / (16 * nt));
+    // few weight rows (a router: 256 to 512): 16 warps share a block's K, so that its chain of loads stays short
+#define VE_LAUNCH(NT, WARPS)                                                                                               \
+  launch_pdl(bf16_gemv_f32_kernel<NT, WARPS>, grid, dim3(32 * WARPS), 0, st, (const __nv_bfloat16*)W, xm, x_stride, om, out_stride, m, N, K)
+    if (N <= 16 * 148) {
+      if (nt == 1) VE_LAUNCH(1, 16); else VE_LAUNCH(2, 16);
     } else {
-      VE_LAUNCH(1);
-      m0 += 1;
+      if (nt == 1) VE_LAUNCH(1, 4); else VE_LAUNCH(2, 4);
     }
 #undef VE_LAUNCH
   }
