@@ -18,9 +18,9 @@ struct TileOut {
 };
 
 // Called by four warps (etid 0..127, `quarter` = the TMEM lane quarter of the calling warp) once the accumulator is complete and the
-// staging memory (COLS * 528 bytes) is free. n0: feature of lane 0; t0: token of column 0. Ends with a barrier of the 128 threads.
+// staging memory (COLS * 528 bytes) is free; `bar`: the named barrier on which they meet. n0: feature of lane 0; t0: token of column 0. Ends with a barrier of the 128 threads.
 template <int COLS>
-VE_DEVINL void store_tile(uint8_t* stage, uint32_t tmem, int quarter, int etid, int n0, int t0, const TileOut& o) {
+VE_DEVINL void store_tile(uint8_t* stage, uint32_t tmem, int quarter, int etid, int n0, int t0, const TileOut& o, int bar = 1) {
   const int lane = etid & 31, col = quarter * 32 + lane;
   const int rows = min(COLS, o.t_end - t0);
   const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
@@ -41,7 +41,7 @@ VE_DEVINL void store_tile(uint8_t* stage, uint32_t tmem, int quarter, int etid, 
       for (int j = 0; j < 16; ++j) reinterpret_cast<__nv_bfloat16*>(stage + (c0 + j) * 272)[col] = f2bf(fmaf(__uint_as_float(r[j]), o.alpha, b));
     }
   }
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
   const int live = min(128, o.N - n0);
   if (o.out_f32) {
     const bool vec = !((uintptr_t)o.out_f32 & 15) && o.ldo % 4 == 0;
@@ -91,7 +91,7 @@ VE_DEVINL void store_tile(uint8_t* stage, uint32_t tmem, int quarter, int etid, 
       }
     }
   }
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+  asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory");
 }
 
 }  // namespace ve
