@@ -49,7 +49,8 @@ struct GgufTile {
   VE_DEVINL void init(const BlockGemmParams& p, int expert, int n0, int warp, int lane) {
     g = lane >> 2; t = lane & 3;
     // rows of an octet go to quads 0, 2, 4, 6, 1, 3, 5, 7: the 8-byte stores of half a warp then meet all eight 16-byte slots of the swizzle
-    row = warp * 16 + (((g & 3) << 1) | (g >> 2));
+    // (16-byte stores of a quarter warp: rows 0 and 4, 1 and 5, ...)
+    row = warp * 16 + (F::kVec8 ? ((g & 1) << 2) | (g >> 1) : ((g & 3) << 1) | (g >> 2));
     end = p.W_end;
     chunks = p.K >> 5;
 #pragma unroll
@@ -79,11 +80,22 @@ struct GgufTile {
       const int c = sub * 2 + cc;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
+        if constexpr (F::kVec8) {                              // three values a vector, rounded once each and picked by the codes
+          const uint8_t* u = raw + (r * 8 + g) * kPitch + (int)((uintptr_t)(rp[r] + (size_t)unit * F::kUnit) & 15);
+          uint32_t lut, f[4];
+          const uint32_t codes = vec8_codes<TYPE>(u, c, t, tab, lut);
+          const float dl = vec8_scale<TYPE>(u) * u2f(2 * (lut & 7) + 1), sh = lut & 8 ? -0.125f : 0.125f;
+          const __nv_bfloat162 v01 = __floats2bfloat162_rn(dl * (-1.f + sh), dl * sh), v2 = __floats2bfloat162_rn(dl * (1.f + sh), 0.f);
+          const uint32_t p01 = *reinterpret_cast<const uint32_t*>(&v01), p2 = *reinterpret_cast<const uint32_t*>(&v2);
+          vec8_expand(codes, __byte_perm(p01, p2, 0x6420), __byte_perm(p01, p2, 0x7531), f);
+          *reinterpret_cast<uint4*>(a + (row + 8 * r) * 128 + (((cc * 4 + t) ^ (row & 7)) << 4)) = make_uint4(f[0], f[1], f[2], f[3]);
+          continue;
+        }
         uint32_t q[4] = {0u, 0u, 0u, 0u};
         float s[2] = {0.f, 0.f}, m[2] = {0.f, 0.f};
         if (F::kBig || unit * F::kChunks + c < chunks) {
           const uint8_t* u = raw + (r * 8 + g) * kPitch + (int)((uintptr_t)(rp[r] + (size_t)unit * F::kUnit) & 15);
-          frag<TYPE>(u, c, t, tab, q, s, m);
+          if constexpr (!F::kVec8) frag<TYPE>(u, c, t, tab, q, s, m);
         }
         if (!F::kScale16) s[1] = s[0];
         if (F::kMin == 1) m[1] = m[0];

@@ -280,17 +280,20 @@ struct Fmt {
   static constexpr int kChunks = TYPE == kQ8_0 ? 4 : 8;
   static constexpr int kUnit = kBig ? kBytes : kBytes * kChunks;
   static constexpr bool kWords = kBytes % 4 == 0;                       // fields lie on 4-byte boundaries (where the rows do)
-  static constexpr bool kScale16 = TYPE == kQ2_K || TYPE == kQ3_K || TYPE == kQ6_K || TYPE == kIQ2_XS || TYPE == kIQ2_S || TYPE == kIQ1_M;
+  static constexpr bool kScale16 = TYPE == kQ2_K || TYPE == kQ3_K || TYPE == kQ6_K || TYPE == kIQ2_XS || TYPE == kIQ2_S;
   static constexpr int kMin = TYPE == kQ2_K ? 2 : (TYPE == kQ4_K || TYPE == kQ5_K || TYPE == kQ4_1 || TYPE == kQ5_1) ? 1 : 0;
   // codebook in shared memory
+  // IQ1: a lane takes a whole codebook vector, 8 weights, and the odd scale factors 1..15 are part of the integers
+  static constexpr bool kVec8 = TYPE == kIQ1_S || TYPE == kIQ1_M;
   static constexpr int kTable = TYPE == kIQ2_XXS ? 2048 : TYPE == kIQ2_XS ? 4096 : TYPE == kIQ2_S ? 8192 : TYPE == kIQ3_XXS ? 1024
-      : TYPE == kIQ3_S ? 2048 : TYPE == kIQ1_S || TYPE == kIQ1_M ? 4096 : TYPE == kIQ4_NL || TYPE == kIQ4_XS ? 1024 : 0;
+      : TYPE == kIQ3_S ? 2048 : TYPE == kIQ1_S || TYPE == kIQ1_M ? 8192 + 128 : TYPE == kIQ4_NL || TYPE == kIQ4_XS ? 1024 : 0;
   static constexpr bool kSigns = TYPE == kIQ2_XXS || TYPE == kIQ2_XS || TYPE == kIQ3_XXS;
   static constexpr int kTabBytes = kTable + (kSigns ? 128 : 0);
 };
 
 // The block's threads copy the format's codebook to `tab` (16-byte aligned): grid bytes as they are with the sign table behind them;
-// IQ1: 16 bits per vector, two per value (value + 1); IQ4: the bf16 levels of two nibbles.
+// IQ1: 32 bits per vector, four per value (value + 1: a byte-permute selector), and behind them, for scale s and sign of the shift
+// (index s + 8 * negative), the low and the high bytes of the bf16 values (2 s + 1) * (value +- 1/8); IQ4: the bf16 levels of two nibbles.
 template <int TYPE>
 VE_DEVINL void load_table(uint8_t* tab) {
   if (TYPE == kIQ4_NL || TYPE == kIQ4_XS) {
@@ -303,8 +306,19 @@ VE_DEVINL void load_table(uint8_t* tab) {
       const uint2 g = *reinterpret_cast<const uint2*>(kIqGrids + kOff1s + i * 8);
       uint32_t v = 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v |= ((((j < 4 ? g.x : g.y) >> (8 * (j & 3))) + 1) & 3) << (2 * j);      // -1, 0, 1 as 0, 1, 2
-      reinterpret_cast<unsigned short*>(tab)[i] = (unsigned short)v;
+      for (int j = 0; j < 8; ++j) v |= ((((j < 4 ? g.x : g.y) >> (8 * (j & 3))) + 1) & 3) << (4 * j);      // -1, 0, 1 as 0, 1, 2
+      reinterpret_cast<uint32_t*>(tab)[i] = v;
+    }
+    if (threadIdx.x < 16) {
+      const float m = (float)(2 * (threadIdx.x & 7) + 1), dl = threadIdx.x & 8 ? -0.125f : 0.125f;
+      uint32_t lo = 0, hi = 0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const uint32_t v = __bfloat16_as_ushort(__float2bfloat16_rn(m * ((float)(j - 1) + dl)));              // at most 8 bits: exact
+        lo |= (v & 255) << (8 * j);
+        hi |= (v >> 8) << (8 * j);
+      }
+      reinterpret_cast<uint2*>(tab + 8192)[threadIdx.x] = make_uint2(lo, hi);
     }
   } else if (Fmt<TYPE>::kTable > 0) {
     constexpr int off = TYPE == kIQ2_XXS ? kOff2xxs : TYPE == kIQ2_XS ? kOff2xs : TYPE == kIQ2_S ? kOff2s : TYPE == kIQ3_XXS ? kOff3xxs : kOff3s;
@@ -391,15 +405,13 @@ VE_DEVINL void frag(const uint8_t* u, int c, int t, const uint8_t* tab, uint32_t
       }
   } else if (TYPE == kQ4_K || TYPE == kQ5_K) {
     const uint32_t w0 = ld32<W>(u + 4), w1 = ld32<W>(u + 8), w2 = ld32<W>(u + 12);
-    uint32_t sc, mn;
-    if (c < 4) { sc = (w0 >> (8 * c)) & 63; mn = (w1 >> (8 * c)) & 63; }
-    else {
-      const int e = 8 * (c - 4);
-      sc = ((w2 >> e) & 15) | (((w0 >> (e + 6)) & 3) << 4);
-      mn = ((w2 >> (e + 4)) & 15) | (((w1 >> (e + 6)) & 3) << 4);
-    }
-    s[0] = half_at(u) * u2f(sc);
-    m[0] = half_at(u + 2) * u2f(mn);
+    // four scales (minima) of six bits in the bytes of a word, for chunks 0..3 and 4..7
+    const uint32_t sw = c < 4 ? w0 & 0x3f3f3f3fu : (w2 & 0x0f0f0f0fu) | ((w0 >> 2) & 0x30303030u);
+    const uint32_t mw = c < 4 ? w1 & 0x3f3f3f3fu : ((w2 >> 4) & 0x0f0f0f0fu) | ((w1 >> 2) & 0x30303030u);
+    // d * byte: the byte as 2^23 + byte, the 2^23 taken off inside the FMA (d * 2^23 is exact)
+    const float d = half_at(u), dmin = half_at(u + 2);
+    s[0] = fmaf(d, __uint_as_float(__byte_perm(sw, 0x4B000000u, 0x7440u | (c & 3))), -8388608.f * d);
+    m[0] = fmaf(dmin, __uint_as_float(__byte_perm(mw, 0x4B000000u, 0x7440u | (c & 3))), -8388608.f * dmin);
     const uint8_t* q = u + (TYPE == kQ4_K ? 16 : 48) + (c >> 1) * 32;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -447,36 +459,6 @@ VE_DEVINL void frag(const uint8_t* u, int c, int t, const uint8_t* tab, uint32_t
       a[2 * i] = u7_bf16(b01(w), 0x43044304u);
       a[2 * i + 1] = u7_bf16(b23(w), 0x43044304u);
     }
-  } else if (TYPE == kIQ1_S || TYPE == kIQ1_M) {
-    uint32_t hi[2], neg[2];                             // index bits 8..10 and the sign of the shift of this lane's vector
-    uint32_t qs;
-    const int v = t >> 1;                               // the vector of the group that holds this lane's weights
-    if (TYPE == kIQ1_S) {
-      qs = ld32<W>(u + 2 + c * 4);
-      const uint32_t qh = ld16(u + 34 + 2 * c);
-      s[0] = half_at(u) * u2f(2 * ((qh >> 12) & 7) + 1);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) { hi[i] = (qh >> (3 * (2 * i + v))) & 7; neg[i] = qh & 0x8000u; }
-    } else {
-      qs = ld32<W>(u + c * 4);
-      const uint32_t qh = ld16(u + 32 + 2 * c) >> (4 * v);
-      const uint32_t s01 = ld32<W>(u + 48), s23 = ld32<W>(u + 52);
-      const float d = __half2float(__ushort_as_half((unsigned short)(((s01 >> 12) & 0xf) | ((s01 >> 24) & 0xf0) | ((s23 >> 4) & 0xf00) |
-                                                                     ((s23 >> 16) & 0xf000))));
-      const uint32_t sw = ((c >> 1) < 2 ? s01 : s23) >> (16 * ((c >> 1) & 1) + 6 * (c & 1));
-      s[0] = d * u2f(2 * (sw & 7) + 1);
-      s[1] = d * u2f(2 * ((sw >> 3) & 7) + 1);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) { hi[i] = (qh >> (8 * i)) & 7; neg[i] = (qh >> (8 * i)) & 8; }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint32_t idx = ((qs >> (16 * i + 8 * v)) & 255) | (hi[i] << 8);
-      const uint32_t k = tab[2 * idx + (t & 1)];        // four values plus one, two bits each
-      const uint32_t off = neg[i] ? 0x41124112u : 0x410E410Eu;               // 9 -+ 1/8; bf16 8.0 = 0x4100 with an ulp of 1/16
-      a[2 * i] = bsub2(((k * 0x40010u) & 0x00300030u) | 0x41004100u, off);
-      a[2 * i + 1] = bsub2((k & 0x30u) | ((k << 14) & 0x300000u) | 0x41004100u, off);
-    }
   } else {                                              // IQ2 / IQ3: grid bytes (below 128) with signs
     const int v = t >> 1;
 #pragma unroll
@@ -516,6 +498,39 @@ VE_DEVINL void frag(const uint8_t* u, int c, int t, const uint8_t* tab, uint32_t
       a[2 * i + 1] = u7_bf16(b23(g), 0x43004300u);
       flip4(sg >> (4 * (t & 1)), a + 2 * i);
     }
+  }
+}
+
+// IQ1: lane t takes weights 8 t .. 8 t + 7 of chunk c, one vector. vec8_codes: its selector word; `lut` = scale s (bits 0..2) and sign of the
+// shift (bit 3) of the vector. vec8_scale: the block's scale, w = d * (2 s + 1) * (value +- 1/8).
+template <int TYPE>
+VE_DEVINL uint32_t vec8_codes(const uint8_t* u, int c, int t, const uint8_t* tab, uint32_t& lut) {
+  uint32_t idx;
+  if (TYPE == kIQ1_M) {
+    const uint32_t h = (uint32_t)u[32 + 2 * c + (t >> 1)] >> (4 * (t & 1));
+    const uint32_t sw = ld32<Fmt<TYPE>::kWords>(u + (c < 4 ? 48 : 52)) >> (3 * (t >> 1));
+    lut = ((sw >> (16 * ((c >> 1) & 1) + 6 * (c & 1))) & 7) | (h & 8);
+    idx = u[c * 4 + t] | ((h & 7) << 8);
+  } else {
+    const uint32_t qh = ld16(u + 34 + 2 * c);
+    lut = ((qh >> 12) & 15);
+    idx = u[2 + c * 4 + t] | (((qh >> (3 * t)) & 7) << 8);
+  }
+  return reinterpret_cast<const uint32_t*>(tab)[idx];
+}
+template <int TYPE>
+VE_DEVINL float vec8_scale(const uint8_t* u) {
+  if (TYPE == kIQ1_S) return half_at(u);
+  const uint32_t s01 = ld32<Fmt<TYPE>::kWords>(u + 48), s23 = ld32<Fmt<TYPE>::kWords>(u + 52);
+  return __half2float(__ushort_as_half((unsigned short)(((s01 >> 12) & 0xf) | ((s01 >> 24) & 0xf0) | ((s23 >> 4) & 0xf00) | ((s23 >> 16) & 0xf000))));
+}
+// Eight selectors -> four bf16 pairs, from the low and the high bytes of the three values.
+VE_DEVINL void vec8_expand(uint32_t codes, uint32_t lo, uint32_t hi, uint32_t* a) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t l = __byte_perm(lo, 0u, codes >> (16 * i)), h = __byte_perm(hi, 0u, codes >> (16 * i));
+    a[2 * i] = __byte_perm(l, h, 0x5140);
+    a[2 * i + 1] = __byte_perm(l, h, 0x7362);
   }
 }
 

@@ -167,7 +167,6 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
   float* const red = reinterpret_cast<float*>(smem_raw + C::kTab);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   uint8_t* const ring = smem_raw + C::kTab + 2 * C::kRed * 4 + warp * C::kStages * C::kStage;
-  grid_dep_launch();
   if (C::kTab) load_table<TYPE>(tab);
   if (MODE != 0) grid_dep_wait();                       // the routes come from the kernel in front (weights do not: MODE 0 starts on them)
 
@@ -234,9 +233,10 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
   int item = 0;
   for (int ti = 0; ti < ntile; ++ti) {
     const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
+    if (ti == ntile - 1) grid_dep_launch();              // (blocks of the kernel behind would wait beside this one's and slow it)
     const uint8_t* rp[2 * RT];
     const bool here = rows_of(ti, rp);
-    const __nv_bfloat16* xr = p.x + (MODE != 0 ? (long)(tile / p.tiles_per_route / p.x_div) * p.x_stride : 0) + 4 * t;
+    const __nv_bfloat16* xr = p.x + (MODE != 0 ? (long)(tile / p.tiles_per_route / p.x_div) * p.x_stride : 0) + (F::kVec8 ? 8 : 4) * t;
     float acc[RT][NT][4];
 #pragma unroll
     for (int i = 0; i < RT; ++i)
@@ -255,6 +255,13 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
 #pragma unroll
       for (int r = 0; r < 2 * RT; ++r)
         up[r] = st + (r * 8 + g) * C::kPitch + (int)((uintptr_t)(rp[r] + (size_t)ui * F::kUnit) & 15);
+      float blk[RT][NT][4];                               // (IQ1)
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) blk[i][j][e] = 0.f;
 #pragma unroll
       for (int h = 0; h < F::kChunks; h += 4) {
         uint2 xv[4][NT][2];                               // this lane's activations of four chunks
@@ -264,12 +271,36 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
           for (int j = 0; j < NT; ++j) {
             const bool live = (MODE != 0 ? g == 0 : j * 8 + g < p.M) && (F::kBig || c0 + h + c < chunks);
             const __nv_bfloat16* q = xr + (MODE == 0 ? (long)(j * 8 + g) * p.x_stride : 0) + (long)(c0 + h + c) * 32;
-            xv[c][j][0] = live ? *reinterpret_cast<const uint2*>(q) : make_uint2(0u, 0u);
-            xv[c][j][1] = live ? *reinterpret_cast<const uint2*>(q + 16) : make_uint2(0u, 0u);
+            if (F::kVec8) {
+              const uint4 v = live ? *reinterpret_cast<const uint4*>(q) : make_uint4(0u, 0u, 0u, 0u);
+              xv[c][j][0] = make_uint2(v.x, v.y);
+              xv[c][j][1] = make_uint2(v.z, v.w);
+            } else {
+              xv[c][j][0] = live ? *reinterpret_cast<const uint2*>(q) : make_uint2(0u, 0u);
+              xv[c][j][1] = live ? *reinterpret_cast<const uint2*>(q + 16) : make_uint2(0u, 0u);
+            }
           }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (!F::kBig && c0 + h + c >= chunks) break;
+          if constexpr (F::kVec8) {                       // the block's products are summed before its one scale
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+              uint32_t f[2][4];
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                uint32_t lut;
+                const uint32_t codes = vec8_codes<TYPE>(up[2 * i + r], h + c, t, tab, lut);
+                const uint2 v = reinterpret_cast<const uint2*>(tab + 8192)[lut];
+                vec8_expand(codes, v.x, v.y, f[r]);
+              }
+#pragma unroll
+              for (int j = 0; j < NT; ++j) {
+                mma_bf16_16816(blk[i][j], f[0][0], f[1][0], f[0][1], f[1][1], xv[c][j][0].x, xv[c][j][0].y);
+                mma_bf16_16816(blk[i][j], f[0][2], f[1][2], f[0][3], f[1][3], xv[c][j][1].x, xv[c][j][1].y);
+              }
+            }
+          } else {
           float sx[NT][2][2];                             // sums of x over the group (formats with minima), columns 2 t and 2 t + 1
           if (F::kMin) {
 #pragma unroll
@@ -308,6 +339,19 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
                 ac[2] = fmaf(-mb[k], sx[j][k][0], ac[2]); ac[3] = fmaf(-mb[k], sx[j][k][1], ac[3]);
               }
             }
+          }
+          }
+        }
+      }
+      if constexpr (F::kVec8) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          const float da = vec8_scale<TYPE>(up[2 * i]), db = vec8_scale<TYPE>(up[2 * i + 1]);
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            float* ac = acc[i][j];
+            ac[0] = fmaf(da, blk[i][j][0], ac[0]); ac[1] = fmaf(da, blk[i][j][1], ac[1]);
+            ac[2] = fmaf(db, blk[i][j][2], ac[2]); ac[3] = fmaf(db, blk[i][j][3], ac[3]);
           }
         }
       }
