@@ -95,3 +95,28 @@ def test_bf16_matvec_edges(N, K):
     assert _rel(full.cpu(), x.double() @ W.double().t()) < 1e-5
     for M in (1, 2, 3, 7, 8, 9, 16):
         assert torch.equal(K_.bf16_gemv_f32(W.cuda(), x[:M].cuda()), full[:M]), M
+
+
+@pytest.mark.parametrize("bits", [1, 3, 4, 6, 8])
+def test_exl3_matvec_units_and_groups(bits):
+    """More and fewer units than resident blocks, units of fewer than four column tiles, K of fewer k-tiles than warps, groups without an
+    expert between others, codes that start on a 4-byte boundary; against the product with the matrix decoded to bf16 (2^-8)."""
+    from volta_engine_b200.ops.linear_exl3 import exl3_gemv, exl3_reconstruct
+    g = torch.Generator().manual_seed(bits)
+    for E, K, N, groups, M in ((1, 16, 16, 1, 16), (3, 80, 48, 7, 1), (2, 1040, 176, 300, 2), (2, 256, 64, 5, 9), (2, 272, 112, 200, 1)):
+        n = (K // 16) * (N // 16) * 16 * bits
+        raw = torch.randint(-32768, 32768, (E * n + 8,), generator=g, dtype=torch.int32).to(torch.int16).cuda()
+        x = torch.randn(groups * M, K, generator=g).half().cuda()
+        e = torch.randint(-1, E, (groups,), generator=g, dtype=torch.int32).cuda()
+        e[0] = 0
+        for shift in (0, 2):
+            codes = raw[shift:shift + E * n]
+            y = exl3_gemv(codes, x, M, K, N, bits, 2, out=torch.full((groups * M, N), 7.0, device="cuda"), expert=e, expert_stride=n, groups=groups)
+            for gi in range(0, groups, 1 if groups < 20 else 23):
+                got = y[gi * M:(gi + 1) * M]
+                if int(e[gi]) < 0:
+                    assert bool((got == 7.0).all())
+                    continue
+                w = exl3_reconstruct(codes[int(e[gi]) * n:(int(e[gi]) + 1) * n].clone(), K, N, bits, 2)
+                want = x[gi * M:(gi + 1) * M].double() @ w.double().t()
+                assert _rel(got, want) < 2 ** -8, (bits, K, N, gi)

@@ -6,7 +6,7 @@
 // p*bits + bits - 16. In that order lane `lane` of a warp holds exactly the two B fragments of
 // mma.m16n8k16 for the tile (k = 2t + (i&1) + 8*((i>>1)&1), n = g + 8*(i>>2), g = lane>>2, t = lane&3), so the
 // decoded fp16 pairs go to the tensor core without any shuffle; the activations (<= 16 rows, fp16, already
-// rotated) are the A operand, read through L1. One CTA owns 16 output columns, its 8 warps split K
+// rotated) are the A operand, read through L1. A CTA's 8 warps split K
 // in a fixed order, and the cross-warp sum is a fixed tree: results do not depend on M or on the grid.
 // Codebooks: 2 = MUL1 (x = w*0x83DCD12D, byte sum s, value = fma(1024+s, h(0x1eee), h(0xc931)) in fp16),
 // 0 = 3INST (x = w*89226354+64248484), 1 = MCG (x = w*0xCBAC1FED), both y = (x & 0x8fff8fff) ^ 0x3b603b60,
@@ -26,115 +26,151 @@ VE_DEVINL void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
 constexpr int kExl3Warps = 8;
 
 // x: fp16 [groups][M][K] rotated activations (read through L1: at most 16 x K halves, re-used by every warp);
-// y: fp32 [groups][M][N]; group = blockIdx.y, its weights start at codes + expert[group] * expert_stride
-// (expert == nullptr: one shared matrix). The column tiles of a group are split evenly over gridDim.x CTAs (the host
-// sizes the grid to the number of CTAs that are resident at once, so every CTA gets the same work to within one tile
-// and there is no partial last wave); a CTA walks its range in units of 4, 2 or 1 adjacent column tiles. In a unit every
-// warp walks its share of K and reads NTW * 32 * BITS contiguous bytes per k-tile.
-template <int BITS, int CB, int MH, int NTW>   // MH: 8 or 16 activation rows held by the A fragment
-VE_DEVINL void exl3_gemv_unit(const uint32_t* __restrict__ base, size_t tstride, const __half* __restrict__ xlo,
-                              const __half* __restrict__ xhi, bool row_lo, bool row_hi, float* __restrict__ y, float* red,
-                              int M, int KT, int N, int nt0) {
+// y: fp32 [groups][M][N]; the weights of a group start at codes + expert[group] * expert_stride (expert == nullptr: one shared matrix; a
+// negative expert: nothing is written).
+//
+// A unit is UT = 4, 2 or 1 adjacent column tiles of one group, as wide as still gives every block two units; the units of all groups are
+// split evenly over the blocks that are resident at once, so every block gets the same work to within one unit whatever the number of
+// groups is. In a unit the eight warps split K, and each brings its k-tiles, 4 / UT at a time, through a cp.async ring of its own that runs
+// several stages ahead and on into the next unit. One k-tile ahead in registers (and a grid of groups x columns) a unit cost sixteen memory
+// latencies in a row: 108 us for 160 routes of 2048 x 512 weights at 4 bits, now 70 us; their bytes take 13 us. What bounds it now is the
+// decoding, five to six instructions a weight.
+template <int BITS, int MH>
+struct Exl3Gemv {
+  static constexpr int kStage = 4 * 32 * BITS, kStages = BITS <= 4 ? 8 : 4;      // bytes of four tiles; stages of the ring
+  static constexpr int kRed = kExl3Warps * MH * 64;                               // floats, one of two buffers (units of four tiles)
+  static constexpr int kSmem = 2 * kRed * 4 + kExl3Warps * kStages * kStage;
+};
+
+template <int BITS, int CB, int MH, int UT>   // MH: 8 or 16 activation rows held by the A fragment
+__global__ void __launch_bounds__(kExl3Warps * 32, 2)
+exl3_gemv_kernel(const uint16_t* __restrict__ codes, const __half* __restrict__ x, float* __restrict__ y,
+                 int M, int K, int N, const int* __restrict__ expert, long expert_stride, int groups) {
+  using C = Exl3Gemv<BITS, MH>;
+  constexpr int KU = 4 / UT, W = 16 * UT;                           // k-tiles of a stage, columns of a unit
+  extern __shared__ __align__(16) uint8_t exl3_smem[];
+  float* const red = reinterpret_cast<float*>(exl3_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  uint8_t* const ring = exl3_smem + 2 * C::kRed * 4 + warp * C::kStages * C::kStage;
+  const bool row_lo = g < M, row_hi = MH == 16 && g + 8 < M;
+  const int KT = K >> 4, NT = N >> 4, per_group = (NT + UT - 1) / UT;
+  const long total = (long)groups * per_group;
+  const int u0 = (int)(total * blockIdx.x / gridDim.x), u1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
   const int per = (KT + kExl3Warps - 1) / kExl3Warps;
-  const int kt0 = warp * per, kt1 = min(KT, kt0 + per);
+  const int kt0 = min(KT, warp * per), kt1 = min(KT, kt0 + per);
+  const size_t tstride = (size_t)NT * (32 * BITS);                  // bytes from one k-tile to the next
+
+  int l_unit = u0, l_kt = kt0, l_slot = 0, l_live = 0;             // what is loaded next
+  const uint8_t* l_base = nullptr;
+  auto load = [&]() {
+    if (l_unit < u1 && kt0 < kt1) {
+      if (l_kt == kt0) {
+        const int grp = l_unit / per_group, nt0 = (l_unit - grp * per_group) * UT;
+        const int e = expert ? expert[grp] : 0;
+        l_live = e < 0 ? 0 : min(UT, NT - nt0) * 2 * BITS;          // 16-byte pieces of a k-tile
+        l_base = reinterpret_cast<const uint8_t*>(codes + (size_t)max(e, 0) * expert_stride) + (size_t)nt0 * (32 * BITS);
+      }
+      const uint8_t* src = l_base + (size_t)l_kt * tstride;
+      uint8_t* dst = ring + l_slot * C::kStage;
+      constexpr int P = 2 * BITS * UT;
+      if (!((uintptr_t)src & 15)) {
+#pragma unroll
+        for (int i = 0; i < (8 * BITS + 31) / 32; ++i) {
+          const int j = lane + 32 * i, ku = j / P, piece = j % P;
+          if (ku < KU && piece < l_live && l_kt + ku < kt1)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + j * 16)), "l"(src + ku * tstride + piece * 16) : "memory");
+        }
+      } else {                                                       // codes that start between 16-byte boundaries: word by word
+        for (int j = lane; j < 4 * 8 * BITS; j += 32) {
+          const int ku = j / (4 * P), word = j % (4 * P);
+          if (word < 4 * l_live && l_kt + ku < kt1)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + j * 4)), "l"(src + ku * tstride + word * 4) : "memory");
+        }
+      }
+      l_slot = l_slot + 1 == C::kStages ? 0 : l_slot + 1;
+      l_kt += KU;
+      if (l_kt >= kt1) { l_kt = kt0; ++l_unit; }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < C::kStages - 1; ++i) load();
+
   const Exl3Lane<BITS> L(lane);
   constexpr int NW = Exl3Lane<BITS>::NW;
-  base += (size_t)nt0 * (8 * BITS);
-  float acc[NTW][2][4];
+  int slot = 0, buf = 0;
+  for (int unit = u0; unit < u1; ++unit) {
+    const int grp = unit / per_group, nt0 = (unit - grp * per_group) * UT;
+    const bool here = !expert || expert[grp] >= 0;
+    const __half* xlo = x + ((size_t)grp * M + (row_lo ? g : 0)) * K + 2 * t;
+    const __half* xhi = x + ((size_t)grp * M + (row_hi ? g + 8 : 0)) * K + 2 * t;
+    float acc[UT][2][4];
 #pragma unroll
-  for (int j = 0; j < NTW; ++j)
+    for (int j = 0; j < UT; ++j)
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[j][h][i] = 0.f;
-  constexpr int UK = (NW == 2 ? 4 : 2) / NTW > 0 ? (NW == 2 ? 4 : 2) / NTW : 1;   // k-tiles per step of a warp
-  // Two register buffers: the words of step i + 1 are requested before step i is decoded, so a warp's memory latency
-  // overlaps its own arithmetic (the warps of a CTA run in lock-step and would otherwise all wait at the same time).
-  uint32_t wn[UK][NTW][NW], an[UK][4];
-  auto fetch = [&](int kt) {
+        for (int i = 0; i < 4; ++i) acc[j][h][i] = 0.f;
+    uint32_t an[KU][4];
+    auto fetch = [&](int kt) {                                      // the A fragments of a stage, one ahead
 #pragma unroll
-    for (int u = 0; u < UK; ++u) {
-      const int k = min(kt + u, kt1 - 1);                           // tail: re-read the last tile, its math is skipped
+      for (int u = 0; u < KU; ++u) {
+        const int ko = min(kt + u, kt1 - 1) * 16;
+        an[u][0] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko)) : 0u;
+        an[u][2] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko + 8)) : 0u;
+        an[u][1] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko)) : 0u;
+        an[u][3] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko + 8)) : 0u;
+      }
+    };
+    if (kt0 < kt1 && here) fetch(kt0);
+    for (int kt = kt0; kt < kt1; kt += KU) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(C::kStages - 2) : "memory");
+      __syncwarp();                                                  // the stage is here for every lane, the slot in front of it is free
+      load();
+      const uint32_t* st = reinterpret_cast<const uint32_t*>(ring + slot * C::kStage);
+      slot = slot + 1 == C::kStages ? 0 : slot + 1;
+      if (!here) continue;
+      uint32_t a[KU][4];
 #pragma unroll
-      for (int j = 0; j < NTW; ++j) L.load(base + (size_t)k * tstride + j * (8 * BITS), wn[u][j]);
-      const int ko = k * 16;                                        // the A fragment of the same k-tile (L1 resident)
-      an[u][0] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko)) : 0u;
-      an[u][2] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko + 8)) : 0u;
-      an[u][1] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko)) : 0u;
-      an[u][3] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko + 8)) : 0u;
-    }
-  };
-  if (kt0 < kt1) fetch(kt0);
-  for (int kt = kt0; kt < kt1; kt += UK) {
-    uint32_t w[UK][NTW][NW], a[UK][4];
+      for (int u = 0; u < KU; ++u)
 #pragma unroll
-    for (int u = 0; u < UK; ++u) {
+        for (int i = 0; i < 4; ++i) a[u][i] = an[u][i];
+      if (kt + KU < kt1) fetch(kt + KU);
 #pragma unroll
-      for (int j = 0; j < NTW; ++j)
+      for (int u = 0; u < KU; ++u) {
+        if (kt + u >= kt1) break;
 #pragma unroll
-        for (int i = 0; i < NW; ++i) w[u][j][i] = wn[u][j][i];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[u][i] = an[u][i];
-    }
-    if (kt + UK < kt1) fetch(kt + UK);
-#pragma unroll
-    for (int u = 0; u < UK; ++u) {
-      if (kt + u < kt1) {
-#pragma unroll
-        for (int j = 0; j < NTW; ++j) {
-          uint32_t f[4];
-          L.template decode<CB>(w[u][j], f);
+        for (int j = 0; j < UT; ++j) {                               // (tiles behind the matrix: old bytes of the ring, not stored)
+          uint32_t w[NW], f[4];
+          L.load_shared(st + (u * UT + j) * (8 * BITS), w);
+          L.template decode<CB>(w, f);
           mma_f16(acc[j][0], a[u], f[0], f[1]);
           mma_f16(acc[j][1], a[u], f[2], f[3]);
         }
       }
     }
-  }
-  // C fragment: c[0],c[1] -> row g, cols 2t,2t+1; c[2],c[3] -> row g+8.
-  constexpr int W = 16 * NTW;
-  __syncthreads();                                                  // the previous unit's sums have been read
-  float* r = red + warp * 16 * W;
+    if (!here) continue;                                             // (the same answer in every warp of the block)
+    // C fragment: c[0],c[1] -> row g, cols 2t,2t+1; c[2],c[3] -> row g+8. Warp sums are added in warp order.
+    float* rb = red + buf * C::kRed;                                 // (sums of the unit in front were read, or are, from the other)
+    buf ^= 1;
+    float* r = rb + warp * MH * W;
 #pragma unroll
-  for (int j = 0; j < NTW; ++j)
+    for (int j = 0; j < UT; ++j)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = j * 16 + h * 8 + 2 * t;
-      r[g * W + c] = acc[j][h][0]; r[g * W + c + 1] = acc[j][h][1];
-      r[(g + 8) * W + c] = acc[j][h][2]; r[(g + 8) * W + c + 1] = acc[j][h][3];
+      for (int h = 0; h < 2; ++h) {
+        const int c = j * 16 + h * 8 + 2 * t;
+        *reinterpret_cast<float2*>(r + g * W + c) = make_float2(acc[j][h][0], acc[j][h][1]);
+        if (MH == 16) *reinterpret_cast<float2*>(r + (g + 8) * W + c) = make_float2(acc[j][h][2], acc[j][h][3]);
+      }
+    __syncthreads();
+    for (int i = tid; i < M * W; i += kExl3Warps * 32) {
+      const int m = i / W, n = i % W;
+      if (nt0 * 16 + n >= N) continue;
+      float s = 0.f;
+#pragma unroll
+      for (int wv = 0; wv < kExl3Warps; ++wv) s += rb[wv * MH * W + m * W + n];
+      y[((size_t)grp * M + m) * N + nt0 * 16 + n] = s;
     }
-  __syncthreads();
-  for (int i = tid; i < M * W; i += blockDim.x) {
-    const int m = i / W, n = i % W;
-    float s = 0.f;
-#pragma unroll
-    for (int wv = 0; wv < kExl3Warps; ++wv) s += red[wv * 16 * W + m * W + n];
-    y[(size_t)m * N + nt0 * 16 + n] = s;
-  }
-}
-
-template <int BITS, int CB, int MH>
-__global__ void __launch_bounds__(kExl3Warps * 32, 2)
-exl3_gemv_kernel(const uint16_t* __restrict__ codes, const __half* __restrict__ x, float* __restrict__ y,
-                 int M, int K, int N, const int* __restrict__ expert, long expert_stride) {
-  __shared__ float red[kExl3Warps * 256 * 4];                       // [warps][16 rows][16 * NTW cols], NTW <= 4
-  const int grp = blockIdx.y;
-  if (expert) { const int e = expert[grp]; if (e < 0) return; codes += (size_t)e * expert_stride; }
-  x += (size_t)grp * M * K; y += (size_t)grp * M * N;
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const bool row_lo = g < M, row_hi = MH == 16 && g + 8 < M;
-  const __half* xlo = x + (size_t)(row_lo ? g : 0) * K + 2 * t;
-  const __half* xhi = x + (size_t)(row_hi ? g + 8 : 0) * K + 2 * t;
-  const int KT = K >> 4, NT = N >> 4;
-  const uint32_t* base = reinterpret_cast<const uint32_t*>(codes);
-  const size_t tstride = (size_t)NT * (8 * BITS);
-  int nt = (int)((long)NT * blockIdx.x / gridDim.x);
-  const int nt_end = (int)((long)NT * (blockIdx.x + 1) / gridDim.x);
-  while (nt < nt_end) {
-    const int left = nt_end - nt;
-    if (left >= 4) { exl3_gemv_unit<BITS, CB, MH, 4>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 4; }
-    else if (left >= 2) { exl3_gemv_unit<BITS, CB, MH, 2>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 2; }
-    else { exl3_gemv_unit<BITS, CB, MH, 1>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 1; }
   }
 }
 
@@ -273,37 +309,51 @@ __global__ void __launch_bounds__(256) exl3_reconstruct_kernel(const uint16_t* _
 
 using namespace ve;
 
-// Grid: as many CTAs as are resident at once (occupancy x SMs), shared between the groups; never more than the column
-// tiles of a group.
-template <int BITS, int CB, int MH>
-static int exl3_gemv_grid() {
+template <int BITS, int CB, int MH, int UT>
+static int exl3_gemv_blocks(int* blocks) {                           // blocks that are resident at once, found on the first call
   static int ctas = 0;
   if (!ctas) {
     int per_sm = 0, dev = 0, sms = 148;
+    constexpr int smem = Exl3Gemv<BITS, MH>::kSmem;
+    const cudaError_t e = cudaFuncSetAttribute(exl3_gemv_kernel<BITS, CB, MH, UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exl3_gemv_kernel<BITS, CB, MH>, kExl3Warps * 32, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exl3_gemv_kernel<BITS, CB, MH, UT>, kExl3Warps * 32, smem) != cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
     ctas = per_sm * sms;
   }
-  return ctas;
+  *blocks = ctas;
+  return 0;
+}
+
+template <int BITS, int CB, int MH>
+static int exl3_gemv_run(const void* codes, const void* x, void* y, int M, int K, int N, const int* expert, long stride, int groups,
+                         cudaStream_t st) {
+  int n = 0, rc = exl3_gemv_blocks<BITS, CB, MH, 4>(&n);
+  if (rc) return rc;
+  const int NT = N / 16;
+  // units of four tiles decode with the fewest loads and barriers a weight; fewer than two a block leave blocks idle in the last round
+  const long four = (long)groups * ((NT + 3) / 4), two = (long)groups * ((NT + 1) / 2), one = (long)groups * NT;
+#define VE_UNITS(UT, TOTAL)                                                                                                      \
+  do {                                                                                                                           \
+    if ((rc = exl3_gemv_blocks<BITS, CB, MH, UT>(&n))) return rc;                                                                \
+    exl3_gemv_kernel<BITS, CB, MH, UT><<<(unsigned)(TOTAL < n ? TOTAL : n), kExl3Warps * 32, Exl3Gemv<BITS, MH>::kSmem, st>>>(   \
+        (const uint16_t*)codes, (const __half*)x, (float*)y, M, K, N, expert, stride, groups);                                   \
+  } while (0)
+  if (four >= 2 * n) VE_UNITS(4, four);
+  else if (two >= 2 * n) VE_UNITS(2, two);
+  else VE_UNITS(1, one);
+#undef VE_UNITS
+  VE_CHECK_LAUNCH();
 }
 
 template <int BITS, int CB>
 static int exl3_gemv_launch(const void* codes, const void* x, void* y, int M, int K, int N, const int* expert,
                             long stride, int groups, cudaStream_t st) {
-  const int NT = N / 16;
-  if (M <= 8) {
-    const int gx = max(1, min(NT, exl3_gemv_grid<BITS, CB, 8>() / groups));
-    exl3_gemv_kernel<BITS, CB, 8><<<dim3(gx, groups), kExl3Warps * 32, 0, st>>>((const uint16_t*)codes, (const __half*)x,
-                                                                                 (float*)y, M, K, N, expert, stride);
-  } else {
-    const int gx = max(1, min(NT, exl3_gemv_grid<BITS, CB, 16>() / groups));
-    exl3_gemv_kernel<BITS, CB, 16><<<dim3(gx, groups), kExl3Warps * 32, 0, st>>>((const uint16_t*)codes, (const __half*)x,
-                                                                                  (float*)y, M, K, N, expert, stride);
-  }
-  VE_CHECK_LAUNCH();
+  return M <= 8 ? exl3_gemv_run<BITS, CB, 8>(codes, x, y, M, K, N, expert, stride, groups, st)
+                : exl3_gemv_run<BITS, CB, 16>(codes, x, y, M, K, N, expert, stride, groups, st);
 }
 
 extern "C" {
