@@ -56,55 +56,120 @@ __global__ void mla_rope_store_kernel(__nv_bfloat16* __restrict__ q, long q_stri
 }
 
 // q_abs[row, h, 0:512] = q[row, h, 0:nope] @ W_uk[h] (nope x 512) ; q_abs[row, h, 512:576] = q_rope.
-// grid (rows, heads), 128 threads: thread t owns 4 latent columns.
-__global__ void mla_absorb_q_kernel(const __nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int nope,
-                                    const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ q_abs, int heads) {
-  __shared__ float qs[256];
-  const int row = blockIdx.x, h = blockIdx.y;
-  const __nv_bfloat16* qv = q + (long)row * q_stride + (long)h * q_dim;
-  for (int i = threadIdx.x; i < nope; i += blockDim.x) qs[i] = bf2f(qv[i]);
-  __syncthreads();
-  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  const int c0 = threadIdx.x * 4;
-#pragma unroll 8                                   // eight independent row loads in flight (the loop is latency-bound)
-  for (int d = 0; d < nope; ++d) {
-    const uint2 t = *reinterpret_cast<const uint2*>(w + (long)d * kLat + c0);
-    const float qd = qs[d];
-    acc[0] = fmaf(qd, __uint_as_float(t.x << 16), acc[0]);
-    acc[1] = fmaf(qd, __uint_as_float(t.x & 0xffff0000u), acc[1]);
-    acc[2] = fmaf(qd, __uint_as_float(t.y << 16), acc[2]);
-    acc[3] = fmaf(qd, __uint_as_float(t.y & 0xffff0000u), acc[3]);
-  }
-  __nv_bfloat16* o = q_abs + ((long)row * heads + h) * kLatRow;
-  *reinterpret_cast<__nv_bfloat162*>(o + c0) = __floats2bfloat162_rn(acc[0], acc[1]);
-  *reinterpret_cast<__nv_bfloat162*>(o + c0 + 2) = __floats2bfloat162_rn(acc[2], acc[3]);
-  if (threadIdx.x < kRope) o[kLat + threadIdx.x] = qv[q_dim - kRope + threadIdx.x];
-}
-
-// out[row, h, 0:vdim] = o_lat[row, h, 0:512] @ W_uv[h]^T  (W_uv [heads, vdim, 512]). grid (rows, heads), vdim threads.
-__global__ void mla_expand_out_kernel(const __nv_bfloat16* __restrict__ o_lat, const __nv_bfloat16* __restrict__ w_uv,
-                                      __nv_bfloat16* __restrict__ out, long out_stride, int heads, int vdim) {
-  __shared__ float os[kLat];
-  const int row = blockIdx.x, h = blockIdx.y;
-  const __nv_bfloat16* o = o_lat + ((long)row * heads + h) * kLat;
-  for (int i = threadIdx.x; i < kLat; i += blockDim.x) os[i] = bf2f(o[i]);
-  __syncthreads();
-  const int v = threadIdx.x;
-  if (v >= vdim) return;
-  const __nv_bfloat16* w = w_uv + ((long)h * vdim + v) * kLat;
-  float acc = 0.f;
-#pragma unroll 8
-  for (int c = 0; c < kLat; c += 8) {
-    const bf16x8 t = *reinterpret_cast<const bf16x8*>(w + c);
+// One block a head, 512 threads: thread t of group w owns latent columns 4 t .. 4 t + 3 and 32 of every 128 rows of W_uk, which it asks for
+// at once; eight activation rows share them, and the four groups' sums are added in order. Bound by the 16.8 MB of 128 heads (3 us): a block
+// per (row, head) read them once per row behind a chain of eight loads, 18 us.
+constexpr int kAbsRows = 8;
+__global__ void __launch_bounds__(512) mla_absorb_q_kernel(const __nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int nope,
+                                                           const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ q_abs, int rows,
+                                                           int heads) {
+  __shared__ float qs[256][kAbsRows];
+  __shared__ float red[4][kAbsRows / 2][kLat];
+  const int h = blockIdx.x, tid = threadIdx.x, grp = tid >> 7, c0 = (tid & 127) * 4;
+  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat + c0;
+  for (int r0 = 0; r0 < rows; r0 += kAbsRows) {
+    const int n = min(kAbsRows, rows - r0);
+    const __nv_bfloat16* qv = q + (long)r0 * q_stride + (long)h * q_dim;
+    for (int i = tid; i < nope * kAbsRows; i += 512) {
+      const int r = i / nope, d = i - r * nope;
+      qs[d][r] = r < n ? bf2f(qv[(long)r * q_stride + d]) : 0.f;
+    }
+    for (int i = tid; i < n * kRope; i += 512)
+      q_abs[((long)(r0 + i / kRope) * heads + h) * kLatRow + kLat + i % kRope] = qv[(long)(i / kRope) * q_stride + q_dim - kRope + i % kRope];
+    float acc[kAbsRows][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(t.v[j]);
-      acc = fmaf(f.x, os[c + 2 * j], acc);
-      acc = fmaf(f.y, os[c + 2 * j + 1], acc);
+    for (int r = 0; r < kAbsRows; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
+    bool ready = false;
+    for (int d0 = grp * 32; d0 < (nope + 127) / 128 * 128; d0 += 128) {
+      uint2 t[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) t[i] = d0 + i < nope ? *reinterpret_cast<const uint2*>(w + (long)(d0 + i) * kLat) : make_uint2(0u, 0u);
+      if (!ready) { __syncthreads(); ready = true; }          // qs (every group makes the same number of rounds)
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        if (d0 + i >= nope) break;
+        const float w0 = __uint_as_float(t[i].x << 16), w1 = __uint_as_float(t[i].x & 0xffff0000u);
+        const float w2 = __uint_as_float(t[i].y << 16), w3 = __uint_as_float(t[i].y & 0xffff0000u);
+#pragma unroll
+        for (int r = 0; r < kAbsRows; r += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(&qs[d0 + i][r]);
+          const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc[r + j][0] = fmaf(xs[j], w0, acc[r + j][0]);
+            acc[r + j][1] = fmaf(xs[j], w1, acc[r + j][1]);
+            acc[r + j][2] = fmaf(xs[j], w2, acc[r + j][2]);
+            acc[r + j][3] = fmaf(xs[j], w3, acc[r + j][3]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+      for (int r = 0; r < kAbsRows / 2; ++r) {
+        const float* v = acc[half * (kAbsRows / 2) + r];
+        *reinterpret_cast<float4*>(&red[grp][r][c0]) = make_float4(v[0], v[1], v[2], v[3]);
+      }
+      __syncthreads();
+      // group g writes row half * 4 + g
+      const int row = half * (kAbsRows / 2) + grp;
+      if (row < n) {
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = ((red[0][grp][c0 + j] + red[1][grp][c0 + j]) + red[2][grp][c0 + j]) + red[3][grp][c0 + j];
+        __nv_bfloat16* dst = q_abs + ((long)(r0 + row) * heads + h) * kLatRow + c0;
+        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(o[0], o[1]);
+        *reinterpret_cast<__nv_bfloat162*>(dst + 2) = __floats2bfloat162_rn(o[2], o[3]);
+      }
+      __syncthreads();
     }
   }
-  out[(long)row * out_stride + (long)h * vdim + v] = f2bf(acc);
+}
+
+// out[row, h, 0:vdim] = o_lat[row, h, 0:512] @ W_uv[h]^T  (W_uv [heads, vdim, 512]). grid (vdim / 16, heads, rows / 16), 128 threads: 16 columns of
+// a head, up to 16 rows; the four warps split the 512 latent columns, lane (g, t) holds 8 of every 32 of them for W_uv rows g and g + 8 and
+// o_lat row g (and g + 8). Steps leave the tensor core one by one and are added in fp32. Bound by the 16.8 MB of W_uv of 128 heads (3 us);
+// a thread per output column walked its kilobyte of W_uv alone, once per row: 123 us at eight rows.
+__global__ void __launch_bounds__(128) mla_expand_out_kernel(const __nv_bfloat16* __restrict__ o_lat, const __nv_bfloat16* __restrict__ w_uv,
+                                                             __nv_bfloat16* __restrict__ out, long out_stride, int rows, int heads, int vdim) {
+  __shared__ float part[4][16][17];
+  const int v0 = blockIdx.x * 16, h = blockIdx.y, r0 = blockIdx.z * 16, n = min(16, rows - r0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const __nv_bfloat16* w = w_uv + (long)h * vdim * kLat + warp * 128 + 8 * t;
+  uint4 a[4][2], x[4][2];
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a[c][i] = *reinterpret_cast<const uint4*>(w + (long)min(v0 + g + 8 * i, vdim - 1) * kLat + c * 32);
+      x[c][i] = g + 8 * i < n ? *reinterpret_cast<const uint4*>(o_lat + ((long)(r0 + g + 8 * i) * heads + h) * kLat + warp * 128 + 8 * t + c * 32)
+                              : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i && n <= 8) break;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_bf16_16816(d, a[c][0].x, a[c][1].x, a[c][0].y, a[c][1].y, x[c][i].x, x[c][i].y);
+      mma_bf16_16816(d, a[c][0].z, a[c][1].z, a[c][0].w, a[c][1].w, x[c][i].z, x[c][i].w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] += d[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) part[warp][i * 8 + 2 * t + (e & 1)][(e >> 1) * 8 + g] = acc[e];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * 16; i += 128) {
+    const int m = i >> 4, v = i & 15;
+    if (v0 + v < vdim)
+      out[(long)(r0 + m) * out_stride + (long)h * vdim + v0 + v] =
+          f2bf(((part[0][m][v] + part[1][m][v]) + part[2][m][v]) + part[3][m][v]);
+  }
 }
 
 struct MlaParams {
@@ -343,6 +408,33 @@ __global__ void mla_reduce_kernel(const float* __restrict__ o_part, const float*
 
 using namespace ve;
 
+namespace ve {
+
+// Keys and values of a context expanded per head, as pages [page][head][64][nope + 64] and [page][head][64][vd]: up [ctx, heads * (nope + vd)]
+// holds the expanded parts, lat [ctx, 576] the rotary key behind the latent. One warp a (position, head), 16-byte pieces; bound by the copy
+// (280 MB for 1900 positions of 128 heads: 81 us, where fills and strided copies of padded pages took 500).
+__global__ void __launch_bounds__(256) mla_expand_kv_kernel(const __nv_bfloat16* __restrict__ up, const __nv_bfloat16* __restrict__ lat,
+                                                            __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v, long total, int heads,
+                                                            int nope, int vd) {
+  const long unit = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (unit >= total) return;
+  const long pos = unit / heads;
+  const int h = (int)(unit % heads);
+  const long row = ((pos >> 6) * heads + h) * 64 + (pos & 63);
+  const int lane = threadIdx.x & 31, nk = nope / 8, nv = vd / 8;
+  const uint4* src = reinterpret_cast<const uint4*>(up + (pos * heads + h) * (nope + vd));
+  const uint4* rope = reinterpret_cast<const uint4*>(lat + pos * 576 + 512);
+  uint4* dk = reinterpret_cast<uint4*>(k + row * (nope + 64));
+  uint4* dv = reinterpret_cast<uint4*>(v + row * vd);
+  for (int c = lane; c < nk + 8 + nv; c += 32) {
+    if (c < nk) dk[c] = src[c];
+    else if (c < nk + 8) dk[c] = rope[c - nk];
+    else dv[c - nk - 8] = src[c - 8];
+  }
+}
+
+}  // namespace ve
+
 extern "C" {
 
 int ve_mla_rope_store(void* q, long q_stride, int q_dim, int heads, const void* ckv, long ckv_stride, const void* krope,
@@ -360,9 +452,8 @@ int ve_mla_absorb_q(const void* q, long q_stride, int q_dim, int nope, const voi
                     cudaStream_t st) {
   if (rows <= 0) return 0;
   if (nope > 256) return cudaErrorInvalidValue;
-  dim3 grid(rows, heads);
-  mla_absorb_q_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)q, q_stride, q_dim, nope, (const __nv_bfloat16*)w_uk,
-                                            (__nv_bfloat16*)q_abs, heads);
+  mla_absorb_q_kernel<<<heads, 512, 0, st>>>((const __nv_bfloat16*)q, q_stride, q_dim, nope, (const __nv_bfloat16*)w_uk,
+                                             (__nv_bfloat16*)q_abs, rows, heads);
   VE_CHECK_LAUNCH();
 }
 
@@ -370,9 +461,9 @@ int ve_mla_expand_out(const void* o_lat, const void* w_uv, void* out, long out_s
                       cudaStream_t st) {
   if (rows <= 0) return 0;
   if (vdim > 256) return cudaErrorInvalidValue;
-  dim3 grid(rows, heads);
-  mla_expand_out_kernel<<<grid, ((vdim + 31) / 32) * 32, 0, st>>>((const __nv_bfloat16*)o_lat, (const __nv_bfloat16*)w_uv,
-                                                                  (__nv_bfloat16*)out, out_stride, heads, vdim);
+  dim3 grid((vdim + 15) / 16, heads, (rows + 15) / 16);
+  mla_expand_out_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)o_lat, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, out_stride, rows,
+                                              heads, vdim);
   VE_CHECK_LAUNCH();
 }
 
@@ -462,6 +553,16 @@ int ve_latent_decode(const void* q_abs, void* o_part, void* lse_part, const void
   else if (nb == 4) VE_LD(4);
   else VE_LD(8);
 #undef VE_LD
+  VE_CHECK_LAUNCH();
+}
+
+// up [ctx, heads * (nope + vd)], lat [ctx, 576] (both dense, 16-byte aligned; nope and vd multiples of 8) -> k, v pages of ctx / 64 pages.
+int ve_mla_expand_kv(const void* up, const void* lat, void* k, void* v, int ctx, int heads, int nope, int vd, cudaStream_t st) {
+  if (ctx <= 0) return 0;
+  if (heads <= 0 || nope % 8 || vd % 8 || ctx % 64) return cudaErrorInvalidValue;
+  const long total = (long)ctx * heads;
+  mla_expand_kv_kernel<<<(unsigned)((total + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)up, (const __nv_bfloat16*)lat, (__nv_bfloat16*)k,
+                                                                    (__nv_bfloat16*)v, total, heads, nope, vd);
   VE_CHECK_LAUNCH();
 }
 
