@@ -148,7 +148,6 @@ bf16_gemv_f32_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
   __shared__ float part[WARPS][COLS][ROWS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * ROWS;
-  grid_dep_launch();
   grid_dep_wait();                   // x and, where they were just decoded, the weights come from kernels in front
   const __nv_bfloat16 *wr[2 * NT], *xr[NT];
 #pragma unroll
@@ -163,11 +162,14 @@ bf16_gemv_f32_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
   const int steps = (K + 31) / 32;
-  for (int c0 = warp; c0 < steps; c0 += WARPS * U) {
+  // four steps in a row a warp: 256 contiguous bytes of each weight row (64 a warp, dealt in turn: 5.8 TB/s instead of 6.6)
+  for (int b0 = warp * 4; b0 < steps; b0 += WARPS * 4)
+#pragma unroll
+  for (int c0 = b0; c0 < b0 + 4; c0 += U) {
     uint4 w[U][2 * NT], v[U][NT];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int k = (c0 + u * WARPS) * 32;
+      const int k = (c0 + u) * 32;
       const bool live = k + 8 * t < K;
 #pragma unroll
       for (int r = 0; r < 2 * NT; ++r) w[u][r] = live ? __ldcs(reinterpret_cast<const uint4*>(wr[r] + k)) : make_uint4(0u, 0u, 0u, 0u);
@@ -189,6 +191,7 @@ bf16_gemv_f32_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* _
           for (int e = 0; e < 4; ++e) acc[i][j][e] += d[e];
         }
   }
+  grid_dep_launch();                 // (not before: blocks that wait beside this one's take their issue slots)
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -254,7 +257,7 @@ int ve_bf16_gemv_f32(const void* W, const void* x, long x_stride, void* out, lon
     if (N <= 16 * 148) {
       if (nt == 1) VE_LAUNCH(1, 16); else VE_LAUNCH(2, 16);
     } else {
-      if (nt == 1) VE_LAUNCH(1, 4); else VE_LAUNCH(2, 4);
+      if (nt == 1) VE_LAUNCH(1, 8); else VE_LAUNCH(2, 8);
     }
 #undef VE_LAUNCH
   }
