@@ -607,7 +607,7 @@ extern "C" {
 
 // warps: 1 (decode / verify: <= 16 packed rows per tile, one warp), 104 (same tiles, four warps that split the
 // keys of every page), 4 (prefill: <= 64 packed rows, 16 per warp) or 8 (prefill on tcgen05: <= 128 packed rows per tile,
-// bf16 cache, head_dim 128, one split).
+// bf16 cache, head_dim 128 or 256, one split).
 int ve_attention(const void* q, long q_stride, void* out, long out_stride, const void* gate, long gate_stride,
                  void* o_part, void* lse_part, const void* pos, const void* slot, const void* key_end,
                  const void* tile_first, const void* tile_count, int ntiles, int rows, const void* page_table,
@@ -657,7 +657,7 @@ int ve_attention(const void* q, long q_stride, void* out, long out_stride, const
     if (!stages) { const char* e = getenv("VOLTA_ATTN_STAGES"); stages = (e && e[0] == '2') ? 2 : 3; }   // 3: -8 % at 16K keys
     p.nst = (warps == 104 && hd <= 128) ? stages : 2;
   }
-  if (warps == 8 && (hd != 128 || kv_fp8 != 0 || nsplit != 1 || ((uintptr_t)q & 15) || (q_stride & 7) ||
+  if (warps == 8 && ((hd != 128 && hd != 256) || kv_fp8 != 0 || nsplit != 1 || ((uintptr_t)q & 15) || (q_stride & 7) ||
                      ((uintptr_t)out & 15) || (out_stride & 7) || ((uintptr_t)gate & 15) || (gate_stride & 7)))
     return cudaErrorInvalidValue;
   CUtensorMap kmap, vmap;
@@ -697,7 +697,8 @@ int ve_attention(const void* q, long q_stride, void* out, long out_stride, const
     else return cudaErrorInvalidValue;
   }
 #undef VE_ATTN_TREE
-  else if (warps == 8) { rc = launch_attn_tc<128>(p, kmap, vmap, ntiles, st); }
+  else if (warps == 8 && hd == 128) { rc = launch_attn_tc<128, 128, 2, 4, 4>(p, kmap, vmap, ntiles, st); }
+  else if (warps == 8) { rc = launch_attn_tc<256, 256, 1, 3, 2>(p, kmap, vmap, ntiles, st); }
   else if (kv_fp8 == 2 && hd == 128) { VE_ATTNQ(128, 2) }
   else if (kv_fp8 == 2 && hd == 256) { VE_ATTNQ(256, 2) }
   else if (kv_fp8 == 3 && hd == 128) { VE_ATTNQ(128, 3) }
@@ -714,6 +715,37 @@ int ve_attention(const void* q, long q_stride, void* out, long out_stride, const
     rc = (int)cudaGetLastError();
   }
   return rc;
+}
+
+// Prefill attention with keys of 192 and values of 128 columns (latent attention with its keys and values expanded per head): q [rows,
+// heads * 192], out [rows, heads * 128], pages [pool_pages][heads][64][192 | 128]; tiles of at most 128 rows of one sequence.
+int ve_attention_k192_v128(const void* q, long q_stride, void* out, long out_stride, const void* pos, const void* slot, const void* tile_first,
+                           const void* tile_count, int ntiles, const void* page_table, int max_pages, const void* kpool, const void* vpool,
+                           long pool_pages, int heads, float scale, void* status, cudaStream_t st) {
+  if (ntiles <= 0) return 0;
+  if (heads <= 0 || ((uintptr_t)q & 15) || (q_stride & 7) || ((uintptr_t)out & 15) || (out_stride & 7)) return cudaErrorInvalidValue;
+  AttnParams p = {};
+  p.q = (const __nv_bfloat16*)q;
+  p.q_stride = q_stride;
+  p.out = (__nv_bfloat16*)out;
+  p.out_stride = out_stride;
+  p.pos = (const int*)pos;
+  p.slot = (const int*)slot;
+  p.tile_first = (const int*)tile_first;
+  p.tile_count = (const int*)tile_count;
+  p.page_table = (const int*)page_table;
+  p.max_pages = max_pages;
+  p.nq = p.nkv = heads;
+  p.nsplit = 1;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.status = (int*)status;
+  CUtensorMap kmap, vmap;
+  const uint64_t rows = (uint64_t)pool_pages * heads * kPageTok;
+  int rc = make_tmap_2d(&kmap, kpool, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 192, 384, kPageTok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc) return rc;
+  rc = make_tmap_2d(&vmap, vpool, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 128, 256, kPageTok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc) return rc;
+  return launch_attn_tc<192, 128, 2, 4, 4>(p, kmap, vmap, ntiles, st);
 }
 
 }  // extern "C"

@@ -1,17 +1,20 @@
 // Prefill attention on the fifth-generation tensor cores (tcgen05, accumulators in TMEM). Included by attention.cu.
 //
 // One CTA = one query tile of up to 128 packed rows ((token, head-in-group) pairs of one kv head, one TMEM lane per
-// row) against the pages of its sequence, bf16 cache, head_dim 128, no key split. Per 64-key page:
-//     S  = Q K^T      tcgen05.mma 128 x 64 x 128   (Q and the K page K-major in 128B-swizzled shared memory)
-//     P  = exp2(S * scale - m)                      (softmax warps: tcgen05.ld of one row per thread, bf16 P written to
-//                                                    shared memory in the K-major swizzled layout)
-//     O += P V        tcgen05.mma 128 x 128 x 64   (V page as it lands from TMA: the MN-major operand form)
-// Warp roles (320 threads): warp 0 streams pages by TMA (four stages), warp 1 issues the MMAs, warps 2..5 and 6..9 are two
-// softmax groups of 128 threads (one row per thread each). The pages are dealt to two independent streams, even pages to
-// the first group and odd pages to the second, each with its own S buffers (2 x 64 TMEM columns), its own running
-// (reference maximum, row sum) and its own O accumulator (128 columns), so the exponentials of one stream run under the
-// MMAs of the other and two warps per scheduler hide the TMEM-load and barrier latencies; the two partial results are
-// merged like split-KV partials in the epilogue (both accumulators live in the same TMEM lanes, so a thread reads both).
+// row) against the pages of its sequence, bf16 cache, keys of DK and values of DV columns, no key split. Per 64-key page:
+//     S  = Q K^T      tcgen05.mma 128 x 64 x DK    (Q and the K page K-major in 128B-swizzled shared memory)
+//     P  = exp2(S * scale - m)                      (softmax warps: tcgen05.ld of one row per thread; bf16 P goes back into the
+//                                                    first 32 columns of the S buffer it came from)
+//     O += P V        tcgen05.mma 128 x DV x 64    (P from TMEM, the V page as it lands from TMA: the MN-major operand form)
+// Warp roles: warp 0 streams pages by TMA (K and V through rings of their own: a K page is free as soon as its S is done), warp 1 issues
+// the MMAs, then four softmax warps per stream (one row per thread). Values of 128 columns leave TMEM room for two streams: the pages are
+// dealt to them alternately, each with its own S buffers (2 x 64 TMEM columns; one stream: 3), its own running (reference maximum, row
+// sum) and its own O accumulator, so the exponentials of one stream run under the MMAs of the other and two warps per scheduler hide the
+// TMEM-load and barrier latencies; the two partial results are merged like split-KV partials in the epilogue (both accumulators live in
+// the same TMEM lanes, so a thread reads both). Values of 256 columns take one stream: a page is then 1024 cycles of tensor work against
+// about 700 of softmax, which runs under the S of the next page and the PV of the one in front.
+// Measured against the mma.sync kernel (attn_kernel): 2048 rows of 24 heads of 256 782 to 172 us, 16 heads 219 to 56 us; 1900 rows of 128
+// heads with keys of 192 and values of 128 (there padded to 256) 1654 to 311 us.
 // The reference maximum is only moved when a page raises it by more than 2^8 (then the O row is rescaled in TMEM by
 // the thread that owns it); otherwise the old reference stays, probabilities are at most 2^8 and the final division by
 // the row sum makes the result the same. The exponent is one FMA (score * scale - reference) and one ex2.approx.
@@ -23,27 +26,27 @@
 namespace ve {
 
 constexpr int kTcRows = 128;        // query rows of a tile
-constexpr int kTcThreads = 320;
 constexpr float kTcLazyLog2 = 8.f;  // the reference maximum moves only when a page raises it by more than this
 
-template <int HD, int NST>
-__global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
-                                                                        const __grid_constant__ CUtensorMap vmap) {
-  static_assert(HD == 128, "the tcgen05 prefill kernel is written for head_dim 128");
-  constexpr int TILE = kPageTok * HD * 2;       // one K or V page: 16 KB, two 64-column chunks of 8 KB
-  constexpr int Q_BYTES = kTcRows * HD * 2;     // 32 KB, two 64-column chunks of 16 KB
-  constexpr int P_BYTES = kTcRows * kPageTok * 2;
-  // TMEM columns: S of stream t, buffer b at t * 128 + b * 64; O of stream t at 256 + t * 128
-  constexpr uint32_t TMEM_COLS = 512, O_COL = 256;
+template <int DK, int DV, int STREAMS, int NK, int NV>
+__global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
+                                                                               const __grid_constant__ CUtensorMap vmap) {
+  constexpr int NB = STREAMS == 1 ? 3 : 2;       // S / P buffers of a stream
+  static_assert(DK % 64 == 0 && DV % 64 == 0 && STREAMS * (NB * 64 + DV) <= 512, "S and O of every stream share the tensor memory");
+  constexpr int K_TILE = kPageTok * DK * 2, V_TILE = kPageTok * DV * 2;      // 64-column chunks of 8 KB
+  constexpr int Q_BYTES = kTcRows * DK * 2;                                   // 64-column chunks of 16 KB
+  // TMEM columns: S of stream t, buffer b at (t * NB + b) * 64; O of stream t behind them
+  constexpr uint32_t TMEM_COLS = 512, O_COL = STREAMS * NB * 64;
   const float NEG_INF = __int_as_float(0xff800000);
   grid_dep_launch();
   grid_dep_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* q_s = smem;
-  uint8_t* kv_s = smem + Q_BYTES;               // [NST][K page | V page]
-  uint8_t* p_s = kv_s + NST * 2 * TILE;         // [2 streams][128 rows x 64 keys]
-  __shared__ uint64_t full[NST], empty[NST], s_full[2][2], p_full[2], pv_done[2];
+  uint8_t* k_s = smem + Q_BYTES;                // [NK] pages
+  uint8_t* v_s = k_s + NK * K_TILE;             // [NV] pages
+  __shared__ uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[STREAMS][NB], p_full[STREAMS][NB], pv_done[STREAMS][NB];
+  __shared__ float s_ml[STREAMS][2][kTcRows];   // (reference maximum, row sum) of the streams' rows
   __shared__ uint32_t tmem_holder;
   __shared__ int s_fail;
 
@@ -68,15 +71,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
   const int n = kt_end - kt_begin;
 
   if (tid == 0) {
-    for (int i = 0; i < NST; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i][0], 1);
-      mbar_init(&s_full[i][1], 1);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&pv_done[i], 1);
+    for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < STREAMS; ++i) {
+      for (int b = 0; b < NB; ++b) { mbar_init(&s_full[i][b], 1); mbar_init(&p_full[i][b], 128); mbar_init(&pv_done[i][b], 1); }
     }
     s_fail = 0;
     mbar_fence_init();
@@ -94,12 +92,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
   const int r_pos = p.pos[r_tok];
   const int r_lim = p.key_end ? p.key_end[r_tok] : r_pos;
   if (warp >= 2) {
-    // each stream's threads bring in one 64-column half of their row of Q
-    const uint4* src = reinterpret_cast<const uint4*>(p.q + (long)r_tok * p.q_stride + (long)r_head * HD) + strm * 8;
+    // the streams' threads share the 64-column chunks of their row of Q
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      const uint4 v = r_ok ? src[ch] : make_uint4(0u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(q_s + strm * (kTcRows * 128) + r * 128 + ((ch ^ (r & 7)) << 4)) = v;
+    for (int c = 0; c < DK / 64; ++c) {
+      if (STREAMS == 2 && (c & 1) != strm) continue;
+      const uint4* src = reinterpret_cast<const uint4*>(p.q + (long)r_tok * p.q_stride + (long)r_head * DK) + c * 8;
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        const uint4 v = r_ok ? src[ch] : make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(q_s + c * (kTcRows * 128) + r * 128 + ((ch ^ (r & 7)) << 4)) = v;
+      }
     }
     fence_proxy_async_smem();
   }
@@ -113,81 +115,91 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
     if (elect_one()) {
       prefetch_tmap(&kmap);
       prefetch_tmap(&vmap);
-      for (int j = 0; j < n; ++j) {
-        const int st = j % NST;
-        if (j >= NST && !mbar_wait(&empty[st], ((j / NST) - 1) & 1)) {
-          atomicExch(&s_fail, 1);
-          break;
-        }
-        const int page = p.page_table[(long)s * p.max_pages + kt_begin + j];
-        const int row = (page * p.nkv + kvh) * kPageTok;
-        uint8_t* kb = kv_s + st * 2 * TILE;
-        uint8_t* vb = kb + TILE;
-        mbar_expect_tx(&full[st], 2 * TILE);
-        tma_load_2d(kb, &kmap, &full[st], 0, row);
-        tma_load_2d(kb + 8192, &kmap, &full[st], 64, row);
-        tma_load_2d(vb, &vmap, &full[st], 0, row);
-        tma_load_2d(vb + 8192, &vmap, &full[st], 64, row);
+      auto row_of = [&](int j) { return (p.page_table[(long)s * p.max_pages + kt_begin + j] * p.nkv + kvh) * kPageTok; };
+      auto load_k = [&](int j) {
+        const int st = j % NK;
+        if (j >= NK && !mbar_wait(&k_empty[st], ((j / NK) - 1) & 1)) return false;
+        const int row = row_of(j);
+        mbar_expect_tx(&k_full[st], K_TILE);
+#pragma unroll
+        for (int c = 0; c < DK / 64; ++c) tma_load_2d(k_s + st * K_TILE + c * 8192, &kmap, &k_full[st], c * 64, row);
+        return true;
+      };
+      auto load_v = [&](int j) {
+        const int st = j % NV;
+        if (j >= NV && !mbar_wait(&v_empty[st], ((j / NV) - 1) & 1)) return false;
+        const int row = row_of(j);
+        mbar_expect_tx(&v_full[st], V_TILE);
+#pragma unroll
+        for (int c = 0; c < DV / 64; ++c) tma_load_2d(v_s + st * V_TILE + c * 8192, &vmap, &v_full[st], c * 64, row);
+        return true;
+      };
+      // the scores of a page are asked for in front of the product of the page before
+      bool ok = load_k(0);
+      for (int j = 0; j < n && ok; ++j) {
+        if (j + 1 < n) ok = load_k(j + 1);
+        if (ok) ok = load_v(j);
       }
+      if (!ok) atomicExch(&s_fail, 1);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issue
     if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_f16(1, 1, kTcRows, kPageTok);
-      constexpr uint32_t idesc_pv = make_idesc_f16(1, 1, kTcRows, HD) | (1u << 16);      // B (the V page) is MN-major
-      const uint32_t q_a = smem_u32(q_s), kv_a = smem_u32(kv_s), p_a = smem_u32(p_s);
+      constexpr uint32_t idesc_pv = make_idesc_f16(1, 1, kTcRows, DV) | (1u << 16);      // B (the V page) is MN-major
+      const uint32_t q_a = smem_u32(q_s), k_a = smem_u32(k_s), v_a = smem_u32(v_s);
       bool ok = true;
-      // page j belongs to stream j & 1 and is that stream's page j >> 1
+      // page j belongs to stream j % STREAMS and is that stream's page j / STREAMS
       auto issue_s = [&](int j) {
-        const int st = j % NST, t = j & 1, b = (j >> 1) & 1;
-        if (!mbar_wait(&full[st], (j / NST) & 1)) return false;
+        const int st = j % NK, t = j % STREAMS, i = j / STREAMS, b = i % NB;
+        // the buffer held P of the stream's page i - NB: MMAs of different shapes are not ordered, so its PV has to be complete
+        if (i >= NB && !mbar_wait(&pv_done[t][b], (i / NB - 1) & 1)) return false;
+        if (!mbar_wait(&k_full[st], (j / NK) & 1)) return false;
         tc_fence_after();
-        const uint32_t kb = kv_a + st * 2 * TILE;
+        const uint32_t kb = k_a + st * K_TILE;
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
+        for (int kk = 0; kk < DK / 16; ++kk) {
           const int c = kk >> 2, off = (kk & 3) * 2;
-          tc_mma_f16(tmem_base + t * 128 + b * kPageTok, make_desc_sw128(q_a + c * (kTcRows * 128)) + off,
+          tc_mma_f16(tmem_base + (t * NB + b) * kPageTok, make_desc_sw128(q_a + c * (kTcRows * 128)) + off,
                      make_desc_sw128(kb + c * 8192) + off, idesc_s, kk ? 1u : 0u);
         }
+        tc_commit(&k_empty[st]);
         tc_commit(&s_full[t][b]);
         return true;
       };
-      ok = issue_s(0);
-      if (ok && n > 1) ok = issue_s(1);
+      for (int j = 0; j < STREAMS && j < n && ok; ++j) ok = issue_s(j);
       for (int j = 0; j < n && ok; ++j) {
-        // the S buffer page j + 2 lands in was read by the softmax of page j - 2, which ended before its P arrived
-        if (j + 2 < n) ok = issue_s(j + 2);
+        if (j + STREAMS < n) ok = issue_s(j + STREAMS);
         if (!ok) break;
-        const int t = j & 1, i = j >> 1;
-        ok = mbar_wait(&p_full[t], i & 1);
+        const int t = j % STREAMS, i = j / STREAMS;
+        ok = mbar_wait(&p_full[t][i % NB], (i / NB) & 1) && mbar_wait(&v_full[j % NV], (j / NV) & 1);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t vb = kv_a + (j % NST) * 2 * TILE + TILE;
+        const uint32_t vb = v_a + (j % NV) * V_TILE;
 #pragma unroll
         for (int ks = 0; ks < kPageTok / 16; ++ks)
-          tc_mma_f16(tmem_base + O_COL + t * HD, make_desc_sw128(p_a + t * P_BYTES) + ks * 2,
-                     make_desc_sw128_mn(vb + ks * 2048, 8192u, 1024u), idesc_pv, (i | ks) ? 1u : 0u);
-        tc_commit(&pv_done[t]);
-        tc_commit(&empty[j % NST]);
+          tc_mma_f16_ta(tmem_base + O_COL + t * DV, tmem_base + (t * NB + i % NB) * kPageTok + ks * 8,
+                        make_desc_sw128_mn(vb + ks * 2048, 8192u, 1024u), idesc_pv, (i | ks) ? 1u : 0u);
+        tc_commit(&pv_done[t][i % NB]);
+        tc_commit(&v_empty[j % NV]);
       }
       if (!ok) atomicExch(&s_fail, 1);
     }
   } else {
     // ------------------------------------------------------------------ softmax and correction of one stream
     const uint32_t t_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t o_col = O_COL + strm * HD;
-    const int n_mine = (n - strm + 1) >> 1;
+    const uint32_t o_col = O_COL + strm * DV;
+    const int n_mine = (n - strm + STREAMS - 1) / STREAMS;
     float m_ref = NEG_INF, l0 = 0.f, l1 = 0.f;
     bool ok = true;
-    uint8_t* prow = p_s + strm * P_BYTES + r * 128;
     for (int i = 0; i < n_mine; ++i) {
-      const int b = i & 1, key0 = (kt_begin + 2 * i + strm) * kPageTok;
-      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[strm][b], (i >> 1) & 1));
+      const int b = i % NB, key0 = (kt_begin + STREAMS * i + strm) * kPageTok;
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[strm][b], (i / NB) & 1));
       if (!ok) break;
       tc_fence_after();
       float sv[kPageTok];
-      tmem_ld32(t_lane + strm * 128 + b * kPageTok, reinterpret_cast<uint32_t*>(sv));
-      tmem_ld32(t_lane + strm * 128 + b * kPageTok + 32, reinterpret_cast<uint32_t*>(sv) + 32);
+      tmem_ld32(t_lane + (strm * NB + b) * kPageTok, reinterpret_cast<uint32_t*>(sv));
+      tmem_ld32(t_lane + (strm * NB + b) * kPageTok + 32, reinterpret_cast<uint32_t*>(sv) + 32);
       tmem_ld_wait();
       if (!r_ok || key0 + kPageTok - 1 > r_lim || (p.window > 0 && key0 <= r_pos - p.window)) {
 #pragma unroll
@@ -213,14 +225,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
         m_ref = mx;
       }
       const bool fix = i > 0 && __any_sync(0xffffffffu, grow);
-      // The stream's previous PV read the P buffer this page is about to overwrite and is the last writer of O: a row
-      // correction waits for it now, otherwise the exponentials run first and only the stores of P wait.
+      // The stream's previous PV is the last writer of O: a row correction waits for it. (P goes to the buffer of its own S, which no MMA
+      // in flight reads.)
       if (fix) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[strm], (i - 1) & 1));
+        ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[strm][(i - 1) % NB], ((i - 1) / NB) & 1));
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
-        for (int c0 = 0; c0 < HD; c0 += 32) {
+        for (int c0 = 0; c0 < DV; c0 += 32) {
           uint32_t ov[32];
           tmem_ld32(t_lane + o_col + c0, ov);
           tmem_ld_wait();
@@ -242,45 +254,38 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
         l1 += p1;
         w[e] = pack_bf16(p0, p1);
       }
-      if (i > 0 && !fix) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[strm], (i - 1) & 1));
-        if (!ok) break;
-      }
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch)
-        *reinterpret_cast<uint4*>(prow + ((ch ^ (r & 7)) << 4)) = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
-      fence_proxy_async_smem();
+      __syncwarp();                                // (masks and maxima let lanes part; the store wants the whole warp)
+      tmem_st32(t_lane + (strm * NB + b) * kPageTok, w);
+      tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_full[strm]);
+      mbar_arrive(&p_full[strm][b]);              // (a barrier a buffer: a fast warp may be a page ahead of a slow one)
     }
-    if (n_mine > 0) ok = __all_sync(0xffffffffu, ok && mbar_wait(&pv_done[strm], (n_mine - 1) & 1));
+    if (n_mine > 0) ok = __all_sync(0xffffffffu, ok && mbar_wait(&pv_done[strm][(n_mine - 1) % NB], ((n_mine - 1) / NB) & 1));
     if (!ok) atomicExch(&s_fail, 1);
-    // the stream's P buffer is free now (its last PV has completed): it carries (maximum, sum) to the merge
-    reinterpret_cast<float*>(p_s + strm * P_BYTES)[r] = m_ref;
-    reinterpret_cast<float*>(p_s + strm * P_BYTES)[kTcRows + r] = l0 + l1;
+    s_ml[strm][0][r] = m_ref;
+    s_ml[strm][1][r] = l0 + l1;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (warp >= 2 && !s_fail) {
     // ------------------------------------------------------------------ merge of the two streams and output
-    // stream 0's threads write columns 0..63 of their row, stream 1's threads columns 64..127
+    // each stream's threads write their share of the columns of their row
     const uint32_t t_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    const float* ml0 = reinterpret_cast<const float*>(p_s);
-    const float* ml1 = reinterpret_cast<const float*>(p_s + P_BYTES);
-    const float m0 = ml0[r], m1 = ml1[r];
+    const bool two = STREAMS == 2 && n > 1;                  // (a one-page tile never wrote the second accumulator)
+    const float m0 = s_ml[0][0][r], m1 = two ? s_ml[STREAMS - 1][0][r] : NEG_INF;
     const float m = fmaxf(m0, m1);
-    const float a0 = m == NEG_INF ? 0.f : ex2_approx(m0 - m), a1 = (m == NEG_INF || n < 2) ? 0.f : ex2_approx(m1 - m);
-    const float l = ml0[kTcRows + r] * a0 + (n < 2 ? 0.f : ml1[kTcRows + r] * a1);
+    const float a0 = m == NEG_INF ? 0.f : ex2_approx(m0 - m), a1 = (m == NEG_INF || !two) ? 0.f : ex2_approx(m1 - m);
+    const float l = s_ml[0][1][r] * a0 + (two ? s_ml[STREAMS - 1][1][r] * a1 : 0.f);
     const float inv = l > 0.f ? 1.f / l : 0.f;
     const float f0 = a0 * inv, f1 = a1 * inv;
-    __nv_bfloat16* orow = p.out + (long)r_tok * p.out_stride + (long)r_head * HD;
-    const __nv_bfloat16* grow_ = p.gate ? p.gate + (long)r_tok * p.gate_stride + (long)r_head * HD : nullptr;
+    __nv_bfloat16* orow = p.out + (long)r_tok * p.out_stride + (long)r_head * DV;
+    const __nv_bfloat16* grow_ = p.gate ? p.gate + (long)r_tok * p.gate_stride + (long)r_head * DV : nullptr;
 #pragma unroll 1
-    for (int c0 = strm * 64; c0 < strm * 64 + 64; c0 += 32) {
+    for (int c0 = strm * (DV / STREAMS); c0 < (strm + 1) * (DV / STREAMS); c0 += 32) {
       uint32_t ov[32], ow[32];
       tmem_ld32(t_lane + O_COL + c0, ov);
-      if (n > 1) tmem_ld32(t_lane + O_COL + HD + c0, ow);     // a one-page tile never wrote the second accumulator
+      if (two) tmem_ld32(t_lane + O_COL + DV + c0, ow);
       tmem_ld_wait();
       if (r_ok) {
 #pragma unroll
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             float a = __uint_as_float(ov[q4 * 8 + 2 * e]) * f0, c = __uint_as_float(ov[q4 * 8 + 2 * e + 1]) * f0;
-            if (n > 1) {
+            if (two) {
               a = fmaf(__uint_as_float(ow[q4 * 8 + 2 * e]), f1, a);
               c = fmaf(__uint_as_float(ow[q4 * 8 + 2 * e + 1]), f1, c);
             }
@@ -319,22 +324,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const At
   if (tid == 0 && s_fail && p.status) atomicExch(p.status, (int)kErrMbarTimeout);
 }
 
-template <int HD, int NST>
-static int launch_attn_tc_n(const AttnParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int ntiles, cudaStream_t st) {
-  constexpr int smem = kTcRows * HD * 2 + NST * 2 * kPageTok * HD * 2 + 2 * kTcRows * kPageTok * 2 + 1024;
+template <int DK, int DV, int STREAMS, int NK, int NV>
+static int launch_attn_tc(const AttnParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int ntiles, cudaStream_t st) {
+  constexpr int smem = kTcRows * DK * 2 + NK * kPageTok * DK * 2 + NV * kPageTok * DV * 2 + 1024;
+  static_assert(smem <= 225 * 1024, "shared memory budget (beside 2 KB of barriers and row sums)");
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DK, DV, STREAMS, NK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  launch_pdl(attn_prefill_tc_kernel<HD, NST>, dim3(ntiles, p.nkv, 1), dim3(kTcThreads), smem, st, p, kmap, vmap);
+  launch_pdl(attn_prefill_tc_kernel<DK, DV, STREAMS, NK, NV>, dim3(ntiles, p.nkv, 1), dim3(64 + 128 * STREAMS), smem, st, p, kmap, vmap);
   return (int)cudaGetLastError();
-}
-
-template <int HD>
-static int launch_attn_tc(const AttnParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int ntiles, cudaStream_t st) {
-  return launch_attn_tc_n<HD, 4>(p, kmap, vmap, ntiles, st);      // a fifth stage measured the same (804 vs 803 TFLOP/s)
 }
 
 }  // namespace ve

@@ -1,4 +1,4 @@
-// Prefill linear with NVFP4 weights and bf16 activations on 256-feature x 192-token output tiles:
+// Prefill linear with NVFP4 weights and bf16 activations on 256-feature x 192-token (or shorter) output tiles:
 //   out[t, n] = alpha * sum_k W[n, k] * X[t, k],   W dequantised to bf16 inside the tile loader (exact products).
 //
 // Two things bounded the form in front of this one (256 x 256 tiles, dequantised weights in shared memory, a block per tile):
@@ -7,7 +7,7 @@
 //    weights go to tensor memory, from where the MMA takes its A operand: 92 KB, 720 cycles for 768 cycles of tensor work. Two accumulators
 //    of 192 columns and two buffers of 2 x 32 columns of weights fill the 512 columns, hence the 192 tokens.
 //  * the last wave: 2048 tokens x 5120 features are 160 tiles of 256 x 256 on 148 SMs. Here the blocks are persistent, and the tiles of the
-//    last wave and of the partial wave behind it are dealt to the blocks by k steps: a tile cut in two or three leaves fp32 partial
+//    partial last wave (or of the last two) are dealt to the blocks by k steps where that is shorter: a cut tile leaves fp32 partial
 //    sums in a workspace, and the block that arrives last adds them up in the order of k and stores. No block waits for another.
 //
 // Warp roles (320 threads): warp 0 TMA producer, warp 1 TMEM owner + MMA issuer, warps 2..9 dequantise (one weight row of 64 a thread and step,
@@ -26,29 +26,42 @@ constexpr int W_SMEM = W_STAGES * W_STAGE + 2 * W_STORE + 1024;
 constexpr int W_ACC = 2 * W_T;                                         // first TMEM column of the weight buffers
 constexpr int W_GRID = 148;
 
-// How the output tiles are dealt: the first `cut` tiles by k steps (multiples of `quantum`) to all blocks, the others whole.
+// How the output tiles are dealt: the first `cut` tiles by k steps (multiples of `quantum`) to the first `cutters` blocks, the others whole.
 struct WidePlan {
-  int tiles_n, tiles_t, tiles, nkt, grid, cut, quantum;
+  int tile_t;                     // tokens of a tile, a multiple of 16
+  int tiles_n, tiles_t, tiles, nkt, grid, cut, cutters, quantum;
   // first of block c's steps of the cut tiles
   __host__ __device__ int begin(int c) const {
     const long q = (long)cut * (nkt / quantum);                        // quanta in all
-    return (int)(q * c / grid) * quantum;
+    return c >= cutters ? cut * nkt : (int)(q * c / cutters) * quantum;
   }
 };
+// Costs in k steps of a 192-token tile (0.5 to 0.8 us): a block that leaves a piece of a tile spends about eight on writing it, and the block that
+// adds a tile up about six for each of its pieces (2048 tokens, 5120 x 5120: 44 us for two pieces a block and 2.5 a tile). So tiles are
+// cut where that is less than what the last, partly filled wave wastes: the remainder alone, in at most eight pieces a tile (220 tiles:
+// 148 whole and 72 in two), or with one whole wave (160 tiles), whichever is shorter; a short K or a handful of tiles stay whole
+// (44 tiles of 32 steps: 39 us whole, 68 us cut).
 static inline WidePlan wide_plan(int T, int N, int K) {
   WidePlan p;
   p.tiles_n = (N + 255) / 256; p.tiles_t = (T + W_T - 1) / W_T; p.tiles = p.tiles_n * p.tiles_t; p.nkt = K / W_KT;
+  p.tile_t = ((T + p.tiles_t - 1) / p.tiles_t + 15) / 16 * 16;          // (no taller than the tokens ask for: 452 are 3 x 160)
   p.quantum = 1;
   for (int q = p.nkt / 16; q > 1; --q)
     if (p.nkt % q == 0) { p.quantum = q; break; }
-  const int waves = (p.tiles + W_GRID - 1) / W_GRID;
-  // steps of the longest block either way; storing and adding partial sums costs about as much as 16 steps
-  const long whole = (long)waves * p.nkt, split = ((long)p.tiles * p.nkt + W_GRID - 1) / W_GRID + 16;
+  const int waves = (p.tiles + W_GRID - 1) / W_GRID, rest = p.tiles % W_GRID;
   p.grid = p.tiles < W_GRID ? p.tiles : W_GRID;
   p.cut = 0;
-  if (split < whole) {
-    p.grid = W_GRID;
-    p.cut = p.tiles <= W_GRID ? p.tiles : p.tiles % W_GRID + W_GRID;
+  p.cutters = 1;
+  long best = (long)waves * p.nkt;
+  if (rest) {
+    for (int n = 2; n <= 8 && rest * n <= W_GRID + rest; ++n) {           // n pieces a tile, as far as there are blocks
+      const int blocks = rest * n < W_GRID ? rest * n : W_GRID;
+      const long cost = (long)(waves - 1) * p.nkt + ((long)rest * p.nkt + blocks - 1) / blocks + 8 + 6 * (n + (blocks < rest * n));
+      if (cost < best) { best = cost; p.cut = rest; p.cutters = blocks; }
+    }
+    const long cost = ((long)p.tiles * p.nkt + W_GRID - 1) / W_GRID + 16 + 6 * 3;
+    if (waves > 1 && cost < best) { best = cost; p.cut = rest + W_GRID; p.cutters = W_GRID; }
+    if (p.cut && p.grid < p.cutters) p.grid = p.cutters;
   }
   return p;
 }
@@ -62,7 +75,7 @@ struct WideParams {
   const __nv_bfloat16* residual;
   long ldr;
   const uint8_t* sfa;     // [N/128][K/128][128][8] E4M3 scales
-  float* partial;         // [2 * grid][W_T][256]: a block's first and last piece of a cut tile
+  float* partial;         // [2 * cutters][W_T][256]: a block's first and last piece of a cut tile
   int* arrived;           // [cut] zeros
   int* status;
 };
@@ -90,16 +103,6 @@ struct WideItems {
     return true;
   }
 };
-
-// D[tmem] (+)= A[tmem] * B[smem desc], bf16 operands: A's 128 rows are the TMEM lanes, two k a column.
-VE_DEVINL void tc_mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 
 VE_DEVINL void w_e2m1x8_to_bf16x8(uint32_t w, uint32_t* o) {
   // table lookup on the byte-permute unit: bf16 patterns of {0, .5, 1, 1.5, 2, 3, 4, 6}
@@ -157,7 +160,7 @@ gemm_w4a16_wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap a
       int i = 0;                                   // steps so far, over all items
       bool ok = true;
       while (ok && it.next()) {
-        const int tn = it.tile / p.plan.tiles_t, t0 = (it.tile - tn * p.plan.tiles_t) * W_T, n0 = tn * 256;
+        const int tn = it.tile / p.plan.tiles_t, t0 = (it.tile - tn * p.plan.tiles_t) * p.plan.tile_t, n0 = tn * 256;
         // (a matrix of an odd number of 128-feature tiles: the second one's codes read as zero, its scales are the first one's)
         const int sf1 = n0 + 128 < p.N ? 2 * tn + 1 : 2 * tn;
         for (int kt = it.k0; kt < it.k1; ++kt, ++i) {
@@ -165,7 +168,7 @@ gemm_w4a16_wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap a
           ok = mbar_wait(&empty[s], ((i / W_STAGES) & 1) ^ 1);
           if (!ok) break;
           uint8_t* st = stage_ptr(s);
-          mbar_expect_tx(&full[s], 2 * W_RAW + W_B + 2 * W_SF);
+          mbar_expect_tx(&full[s], 2 * W_RAW + p.plan.tile_t * 128 + 2 * W_SF);
           tma_load_2d(st + OFF_RAW, &amap, &full[s], kt * 32, n0);
           tma_load_2d(st + OFF_RAW + W_RAW, &amap, &full[s], kt * 32, n0 + 128);
           tma_load_2d(st, &bmap, &full[s], kt * W_KT, t0);
@@ -177,7 +180,7 @@ gemm_w4a16_wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap a
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_f16(1, 1, 128, W_T);
+      const uint32_t idesc = make_idesc_f16(1, 1, 128, p.plan.tile_t);
       int i = 0, item = 0;
       bool ok = true;
       while (ok && it.next()) {
@@ -249,14 +252,14 @@ gemm_w4a16_wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap a
       asm volatile("bar.sync 3, 256;" ::: "memory");          // one answer for the eight warps: they meet at barriers below
       ok = !*(volatile int*)&s_fail;
       if (!ok) break;
-      const int tn = it.tile / p.plan.tiles_t, t0 = (it.tile - tn * p.plan.tiles_t) * W_T, n0 = tn * 256;
-      const int rows = min(W_T, p.T - t0);
+      const int tn = it.tile / p.plan.tiles_t, t0 = (it.tile - tn * p.plan.tiles_t) * p.plan.tile_t, n0 = tn * 256;
+      const int rows = min(p.plan.tile_t, p.T - t0);
       const bool piece = it.k0 > 0 || it.k1 < p.plan.nkt;
       if (!piece) {
         if (n0 + sub * 128 < p.N)
           for (int t = 0; t < rows; t += 32)
             store_tile<32>(staging, tmem_base + sub * W_T + t, quarter, etid, n0 + sub * 128, t0 + t,
-                           TileOut{p.N, p.T, p.alpha, p.out, nullptr, p.ldo, p.residual, p.ldr}, 1 + sub);
+                           TileOut{p.N, t0 + rows, p.alpha, p.out, nullptr, p.ldo, p.residual, p.ldr}, 1 + sub);
       } else {
         float* mine = p.partial + (size_t)(2 * blockIdx.x + (it.first ? 0 : 1)) * (W_T * 256) + sub * 128 + row;
 #pragma unroll 1
@@ -290,23 +293,23 @@ gemm_w4a16_wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap a
           const int f = ((threadIdx.x - 64) & 63) * 4, n = n0 + f;
           const bool vec = !((uintptr_t)p.out & 7) && p.ldo % 4 == 0 && (!p.residual || (!((uintptr_t)p.residual & 7) && p.ldr % 4 == 0));
           if (n < p.N)
-            for (int t = (threadIdx.x - 64) >> 6; t < rows; t += 32) {
-              float4 sum[8];
+            for (int t = (threadIdx.x - 64) >> 6; t < rows; t += 64) {
+              float4 sum[16];                        // (sixteen loads in flight a thread)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+              for (int j = 0; j < 16; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
               for (int c = c_lo; c <= c_hi; ++c) {
                 const int b0 = p.plan.begin(c);
                 if (p.plan.begin(c + 1) == b0) continue;
                 const float* src = p.partial + (size_t)(2 * c + (b0 >= begin ? 0 : 1)) * (W_T * 256) + f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
+                for (int j = 0; j < 16; ++j)
                   if (t + 4 * j < rows) {
                     const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(t + 4 * j) * 256));
                     sum[j].x += v.x; sum[j].y += v.y; sum[j].z += v.z; sum[j].w += v.w;
                   }
               }
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
+              for (int j = 0; j < 16; ++j) {
                 if (t + 4 * j >= rows) continue;
                 float o[4] = {sum[j].x * p.alpha, sum[j].y * p.alpha, sum[j].z * p.alpha, sum[j].w * p.alpha};
                 __nv_bfloat16* dst = p.out + (long)(t0 + t + 4 * j) * p.ldo + n;
@@ -345,7 +348,7 @@ extern "C" {
 long ve_gemm_w4a16_wide_scratch(int T, int N, int K) {
   if (T <= 0 || N <= 0 || K < W_KT) return 0;
   const WidePlan pl = wide_plan(T, N, K);
-  return pl.cut ? (long)2 * pl.grid * W_T * 256 * 4 + (long)pl.cut * 4 : 0;
+  return pl.cut ? (long)2 * pl.cutters * W_T * 256 * 4 + (long)pl.cut * 4 : 0;
 }
 
 // Wp [N, K/2] bytes, sfa [N/128][K/128][128][8], X [T, K] bf16 (pitch ldx). N % 128 == 0, K % 128 == 0. scratch: 16-byte aligned,
@@ -359,7 +362,7 @@ int ve_gemm_w4a16_wide(const void* Wp, const void* sfa, const void* X, long ldx,
   CUtensorMap amap, bmap;
   int rc = make_tmap_2d(&amap, Wp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, (uint64_t)K / 2, 128, 32, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc) return rc;
-  rc = make_tmap_2d(&bmap, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, K, (uint64_t)ldx * 2, W_T, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  rc = make_tmap_2d(&bmap, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, K, (uint64_t)ldx * 2, pl.tile_t, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -368,7 +371,7 @@ int ve_gemm_w4a16_wide(const void* Wp, const void* sfa, const void* X, long ldx,
     attr_set = true;
   }
   float* partial = (float*)scratch;
-  int* arrived = pl.cut ? (int*)(partial + (size_t)2 * pl.grid * W_T * 256) : nullptr;
+  int* arrived = pl.cut ? (int*)(partial + (size_t)2 * pl.cutters * W_T * 256) : nullptr;
   if (pl.cut) {
     const cudaError_t e = cudaMemsetAsync(arrived, 0, (size_t)pl.cut * 4, st);
     if (e != cudaSuccess) return (int)e;

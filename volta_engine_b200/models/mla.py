@@ -183,7 +183,8 @@ class MLAModel(MoEModel):
         return L.o_proj.forward(att, out=pbuf)
 
     def _attn_prefill_expanded(self, L, q, b: BatchRows, kv, pool):
-        """Expand K / V per head for the context of the chunk's sequence and run the dense paged kernel (hd 256)."""
+        """Expand K / V per head for the context of the chunk's sequence and run the paged prefill kernel: keys of 192 and values of 128
+        columns as they are, other widths padded to 256."""
         cfg = self.cfg
         n, hl, nope, vd = q.shape[0], self.heads, cfg.qk_nope, cfg.v_head_dim
         slot = b.host_slots[0]
@@ -193,6 +194,17 @@ class MLAModel(MoEModel):
         pages = kv.host_table[slot, :npages].long().to(q.device)
         lat = pool[pages, 0].reshape(npages * 64, LAT_ROW)                       # [ctx_pad, 576]
         up = L.w_ukv.forward(lat[:, :LAT].contiguous())                          # [ctx_pad, hl * (nope + vd)]
+        if self.qd == 192 and vd == 128 and nope == 128 and K.ATTN_PREFILL_TC and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0:
+            kp = torch.empty(npages, hl, 64, 192, dtype=q.dtype, device=q.device)
+            vp = torch.empty(npages, hl, 64, 128, dtype=q.dtype, device=q.device)
+            call("mla_expand_kv", "ppppiiii", ptr(up), ptr(lat), ptr(kp), ptr(vp), npages * 64, hl, nope, vd)
+            table = torch.arange(npages, dtype=torch.int32, device=q.device).reshape(1, npages)
+            slot0 = torch.zeros(n, dtype=torch.int32, device=q.device)
+            tf, tc, ntiles = K.make_prefill_tiles([0] * n, 1, q.device, 128, False)
+            out = torch.empty(n, hl * 128, dtype=q.dtype, device=q.device)
+            call("attention_k192_v128", "plplppppipipplifp", ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(b.pos), ptr(slot0), ptr(tf), ptr(tc),
+                 ntiles, ptr(table), npages, ptr(kp), ptr(vp), npages, hl, float(self.scale), ptr(K.status_word(q.device)))
+            return out
         up = up.reshape(npages, 64, hl, nope + vd)
         kfull = torch.zeros(npages, hl, 64, 256, dtype=q.dtype, device=q.device)
         vfull = torch.zeros(npages, hl, 64, 256, dtype=q.dtype, device=q.device)

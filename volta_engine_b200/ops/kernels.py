@@ -197,7 +197,7 @@ ATTN_DECODE_WARPS = 1 if os.environ.get("VOLTA_ATTN_DECODE", "ksplit") == "1warp
 # "fused": the split CTA that finishes last merges the partials itself. Measured slower than the parallel merge kernel
 # (one CTA walks 32 splits x 5 heads serially: 166 vs 192 tok/s on the 27B decode), so the kernel form is the default.
 ATTN_FUSED_MERGE = os.environ.get("VOLTA_ATTN_MERGE", "kernel") == "fused"
-# prefill tiles on the tcgen05 kernel where it applies (bf16 cache, head_dim 128); "mma" keeps the mma.sync kernel
+# prefill tiles on the tcgen05 kernel where it applies (bf16 cache, head_dim 128 or 256); "mma" keeps the mma.sync kernel
 ATTN_PREFILL_TC = os.environ.get("VOLTA_ATTN_PREFILL", "tc") != "mma"
 
 
@@ -217,7 +217,7 @@ def attention(q, pos, slot, page_table, kpool, vpool, nq, nkv, hd, scale, *, out
 
     ``tiles`` = (tile_first, tile_count, ntiles[, wide]) int32 device tensors grouping consecutive rows of one
     sequence for prefill (<= 64 // G tokens per tile); None = one row per tile (decode / verify). ``wide`` is the same
-    grouping at <= 128 // G tokens per tile: with a bf16 cache and head_dim 128 the prefill runs on the tcgen05 kernel
+    grouping at <= 128 // G tokens per tile: with a bf16 cache and head_dim 128 or 256 the prefill runs on the tcgen05 kernel
     (128 query rows per CTA, accumulators in TMEM), otherwise on the mma.sync kernel over the 64-row tiles.
     ``tree`` = (base int32 [rows], mask int64 [rows]): rows of a verification tree. Keys at cache positions >= base[r]
     are the tree's own nodes and row r sees node j only if bit j of mask[r] is set (its ancestors and itself).
@@ -240,7 +240,7 @@ def attention(q, pos, slot, page_table, kpool, vpool, nq, nkv, hd, scale, *, out
     else:
         tf, tc, ntiles = tiles[:3]
         warps = 4
-        if (ATTN_PREFILL_TC and len(tiles) > 3 and tiles[3] is not None and hd == 128 and fmt == 0 and nsplit == 1
+        if (ATTN_PREFILL_TC and len(tiles) > 3 and tiles[3] is not None and hd in (128, 256) and fmt == 0 and nsplit == 1
                 and q.data_ptr() % 16 == 0 and q.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0
                 and (gate is None or (gate.data_ptr() % 16 == 0 and gate.stride(0) % 8 == 0))):
             tf, tc, ntiles = tiles[3]
