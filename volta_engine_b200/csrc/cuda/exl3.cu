@@ -203,22 +203,69 @@ template <int DT> VE_DEVINL void had_store4(void* p, size_t i, const float* v) {
   }
 }
 
-// In-warp 128-point Walsh-Hadamard transform (natural order, scaled by 1/sqrt(128)); lane holds elements 4l..4l+3.
-VE_DEVINL void wht128(float* v, int lane) {
-  float a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], d = v[2] - v[3];
-  v[0] = a + c; v[1] = b + d; v[2] = a - c; v[3] = b - d;
+// 16 consecutive values; vec: the address is 16-byte aligned (else 8 bytes, fp32 16).
+template <int DT> VE_DEVINL void had_load16(const void* p, size_t i, bool vec, float* v) {
+  if (DT == 1 || !vec) {
 #pragma unroll
-  for (int m = 1; m < 32; m <<= 1) {
+    for (int j = 0; j < 16; j += 4) had_load4<DT>(p, i + j, v + j);
+  } else {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p) + i);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 u = src[h];
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = DT == 0 ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]))
+                                 : __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+        v[h * 8 + 2 * j] = f.x; v[h * 8 + 2 * j + 1] = f.y;
+      }
+    }
+  }
+}
+template <int DT> VE_DEVINL void had_store16(void* p, size_t i, bool vec, const float* v) {
+  if (DT == 1 || !vec) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) had_store4<DT>(p, i + j, v + j);
+  } else {
+    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(p) + i);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (DT == 0) { const __nv_bfloat162 r = __floats2bfloat162_rn(v[h * 8 + 2 * j], v[h * 8 + 2 * j + 1]); w[j] = *reinterpret_cast<const uint32_t*>(&r); }
+        else { const __half2 r = __floats2half2_rn(v[h * 8 + 2 * j], v[h * 8 + 2 * j + 1]); w[j] = *reinterpret_cast<const uint32_t*>(&r); }
+      }
+      dst[h] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+// 128-point Walsh-Hadamard transform (natural order, scaled by 1/sqrt(128)) over eight lanes of 16 consecutive values each: strides
+// 1 to 8 inside the lane, 16 to 64 by shuffles, in rising order.
+VE_DEVINL void wht128(float* v, int lane) {
+#pragma unroll
+  for (int m = 1; m < 16; m <<= 1)
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (!(j & m)) {
+        const float a = v[j], b = v[j | m];
+        v[j] = a + b;
+        v[j | m] = a - b;
+      }
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1) {
     const bool up = lane & m;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 16; ++j) {
       const float o = __shfl_xor_sync(0xffffffffu, v[j], m);
       v[j] = up ? o - v[j] : v[j] + o;
     }
   }
   const float s = 0.08838834764831845f;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] *= s;
+  for (int j = 0; j < 16; ++j) v[j] *= s;
 }
 
 struct HadArgs {
@@ -227,6 +274,7 @@ struct HadArgs {
   const int* expert; long scale_stride;
   const int* src;                // null: input row = row / in_div; else src[row] / in_div
   int rows, C, post, in_div, rows_per_group, act;
+  bool vec;                      // every row of 16-bit values starts on a 16-byte boundary
 };
 
 VE_DEVINL float act_apply(float x, int act) {
@@ -234,48 +282,62 @@ VE_DEVINL float act_apply(float x, int act) {
   return x / (1.f + __expf(-x));
 }
 
-// One warp per 128-block. post == 0: out = had(in * scale); post == 1: out = had(in) * scale; with in2:
+// Eight lanes per 128-block. post == 0: out = had(in * scale); post == 1: out = had(in) * scale; with in2:
 // out = act(had(in) * scale) * (had(in2) * scale2).
+// Bound by the rows read and written; with four values a lane the transform took 20 shuffles a block, and they took the time (52 us for the
+// average rotation of 20480 rows of 2048 or 512 columns): 16 values a lane take 12, and the same sums in the same order.
 template <int DI, int DO>
 __global__ void __launch_bounds__(256) had128_kernel(HadArgs a) {
   const int lane = threadIdx.x & 31;
   const int nb = a.C >> 7;
   const long total = (long)a.rows * nb;
-  for (long blk = (long)blockIdx.x * 8 + (threadIdx.x >> 5); blk < total; blk += (long)gridDim.x * 8) {
-    const int row = (int)(blk / nb), cb = (int)(blk % nb);
-    const int col = cb * 128 + lane * 4;
+  for (long b0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; b0 < total; b0 += (long)gridDim.x * 32) {
+    const long blk = b0 + (lane >> 3);
+    const bool in = blk < total;                          // (every lane takes part in the shuffles)
+    const int row = in ? (int)(blk / nb) : 0, cb = in ? (int)(blk % nb) : 0;
+    const int col = cb * 128 + (lane & 7) * 16;
     long soff = col;
+    int e = 0;
     if (a.expert) {
-      const int e = a.expert[row / a.rows_per_group];
-      if (e < 0) {                                     // another rank's route: zeros
-        const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-        if (!a.src) had_store4<DO>(a.out, (size_t)row * a.C + col, zero);      // (rows behind the sorted routes stay unwritten)
-        continue;
-      }
-      soff += (long)e * a.scale_stride;
+      e = a.expert[row / a.rows_per_group];
+      if (e > 0) soff += (long)e * a.scale_stride;
     }
-    const size_t in_row = (size_t)((a.src ? a.src[row] : row) / a.in_div) * a.C;
-    float s[4] = {1.f, 1.f, 1.f, 1.f}, v[4];
-    if (a.scale) had_load4<2>(a.scale, soff, s);
-    had_load4<DI>(a.in, in_row + col, v);
+    const bool live = in && e >= 0;
+    float s[16], v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) { s[j] = 1.f; v[j] = 0.f; }
+    size_t in_row = 0;
+    if (live) {
+      in_row = (size_t)((a.src ? a.src[row] : row) / a.in_div) * a.C;
+      if (a.scale) had_load16<2>(a.scale, soff, a.vec, s);
+      had_load16<DI>(a.in, in_row + col, a.vec, v);
+    }
     if (!a.post) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] *= s[j];
+      for (int j = 0; j < 16; ++j) v[j] *= s[j];
     }
     wht128(v, lane);
     if (a.post) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] *= s[j];
+      for (int j = 0; j < 16; ++j) v[j] *= s[j];
     }
     if (a.in2) {
-      float u[4], s2[4] = {1.f, 1.f, 1.f, 1.f};
-      if (a.scale2) had_load4<2>(a.scale2, soff, s2);
-      had_load4<DI>(a.in2, in_row + col, u);
+      float u[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) { s[j] = 1.f; u[j] = 0.f; }
+      if (live) {
+        if (a.scale2) had_load16<2>(a.scale2, soff, a.vec, s);
+        had_load16<DI>(a.in2, in_row + col, a.vec, u);
+      }
       wht128(u, lane);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = act_apply(v[j], a.act) * (u[j] * s2[j]);
+      for (int j = 0; j < 16; ++j) v[j] = act_apply(v[j], a.act) * (u[j] * s[j]);
     }
-    had_store4<DO>(a.out, (size_t)row * a.C + col, v);
+    if (in && e < 0) {                                    // another rank's route: zeros (rows behind the sorted routes stay unwritten)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = 0.f;
+    }
+    if (live || (in && !a.src)) had_store16<DO>(a.out, (size_t)row * a.C + col, a.vec, v);
   }
 }
 
@@ -415,7 +477,8 @@ int ve_had128(const void* in, const void* in2, void* out, const void* scale, con
   if (rows < 1 || C % 128 || in_div < 1 || rows_per_group < 1) return cudaErrorInvalidValue;
   HadArgs a{in, in2, out, (const __half*)scale, (const __half*)scale2, (const int*)expert, scale_stride,
             (const int*)src, rows, C, post, in_div, rows_per_group, act};
-  const long blocks_needed = ((long)rows * (C / 128) + 7) / 8;
+  a.vec = !(((uintptr_t)in | (uintptr_t)in2 | (uintptr_t)out | (uintptr_t)scale | (uintptr_t)scale2) & 15) && scale_stride % 8 == 0;
+  const long blocks_needed = ((long)rows * (C / 128) + 31) / 32;
   const int blocks = (int)(blocks_needed < 148 * 8 ? blocks_needed : 148 * 8);
   if (dt_in == 0 && dt_out == 2) had128_kernel<0, 2><<<blocks, 256, 0, st>>>(a);
   else if (dt_in == 1 && dt_out == 0) had128_kernel<1, 0><<<blocks, 256, 0, st>>>(a);
