@@ -21,28 +21,30 @@ namespace ve {
 
 constexpr int kLat = 512, kRope = 64, kLatRow = 576, kMlaPage = 64;
 
-// grid (rows, heads + 1): blocks [0, heads) rotate q_rope of one head in place; block `heads` rotates k_rope and
-// writes the latent row. q [rows, heads, q_dim] with the rope part at [q_dim - 64, q_dim). 32 threads per block.
+// grid (rows, head groups), 8 warps: warps rotate q_rope of their heads in place; the one behind the last head rotates k_rope and writes
+// the latent row. q [rows, heads, q_dim] with the rope part at [q_dim - 64, q_dim). A lane takes its pair's sine and cosine once for all
+// its heads: a warp-sized block per (row, head) took 129 us for 1900 rows of 128 heads.
 __global__ void mla_rope_store_kernel(__nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int heads,
                                       const __nv_bfloat16* __restrict__ ckv, long ckv_stride,
                                       const __nv_bfloat16* __restrict__ krope, long krope_stride,
                                       const int* __restrict__ pos, const int* __restrict__ slot,
                                       const int* __restrict__ page_table, int max_pages, __nv_bfloat16* __restrict__ pool,
                                       float theta, int interleaved) {
-  const int row = blockIdx.x, h = blockIdx.y, i = threadIdx.x;   // i: rotation pair 0..31
+  const int row = blockIdx.x, i = threadIdx.x & 31;   // i: rotation pair 0..31
   const int p = pos[row];
   const float inv_freq = exp2f(-log2f(theta) * (2.f * (float)i / (float)kRope));
   float sn, cs;
   sincosf((float)p * inv_freq, &sn, &cs);
   const int i0 = interleaved ? 2 * i : i, i1 = interleaved ? 2 * i + 1 : i + kRope / 2;
-  if (h < heads) {
+  int h = blockIdx.y * 8 + (threadIdx.x >> 5);
+  for (; h < heads; h += gridDim.y * 8) {
     __nv_bfloat16* v = q + (long)row * q_stride + (long)h * q_dim + (q_dim - kRope);
     const float a0 = bf2f(v[i0]), a1 = bf2f(v[i1]);
     // output always in half-split order so that q and k agree whatever the checkpoint's pairing
     v[i0] = f2bf(a0 * cs - a1 * sn);
     v[i1] = f2bf(a1 * cs + a0 * sn);
-    return;
   }
+  if (h != heads) return;
   const int s = slot ? slot[row] : 0;
   if (s < 0) return;
   const int page = page_table[(long)s * max_pages + p / kMlaPage];
@@ -441,8 +443,8 @@ int ve_mla_rope_store(void* q, long q_stride, int q_dim, int heads, const void* 
                       long krope_stride, const void* pos, const void* slot, const void* page_table, int max_pages,
                       void* pool, int rows, float theta, int interleaved, cudaStream_t st) {
   if (rows <= 0) return 0;
-  dim3 grid(rows, heads + 1);
-  mla_rope_store_kernel<<<grid, 32, 0, st>>>((__nv_bfloat16*)q, q_stride, q_dim, heads, (const __nv_bfloat16*)ckv, ckv_stride,
+  dim3 grid(rows, rows >= 512 ? 1 : (heads + 8) / 8);
+  mla_rope_store_kernel<<<grid, 256, 0, st>>>((__nv_bfloat16*)q, q_stride, q_dim, heads, (const __nv_bfloat16*)ckv, ckv_stride,
                                              (const __nv_bfloat16*)krope, krope_stride, (const int*)pos, (const int*)slot,
                                              (const int*)page_table, max_pages, (__nv_bfloat16*)pool, theta, interleaved);
   VE_CHECK_LAUNCH();
