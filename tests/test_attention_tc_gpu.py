@@ -1,4 +1,4 @@
-"""Prompt attention on the tcgen05 kernel at the key and value widths beside 128 x 128, against 64-bit torch."""
+"""Prompt attention on the tcgen05 kernel at heads of 128 and 256 columns, against 64-bit torch."""
 import math
 
 import pytest
@@ -57,28 +57,16 @@ def test_prompt_attention_pages_streams_and_maxima(hd, nq, nkv, start, n, window
     assert K.check_status(torch.device("cuda")) == 0
 
 
-@pytest.mark.parametrize("heads,start,n", [(1, 0, 1), (3, 0, 64), (5, 200, 129), (16, 37, 300), (32, 0, 1900)])
-def test_latent_prompt_attention_keys_of_192(heads, start, n):
-    """Keys and values expanded from the latent rows, then attention at 192 / 128 columns; the context ends inside a page."""
+@pytest.mark.parametrize("heads,npages,nope,vd", [(1, 1, 128, 128), (5, 3, 64, 72), (3, 2, 192, 256)])
+def test_latent_keys_and_values_expanded_into_pages(heads, npages, nope, vd):
+    """Bytes as they are, zeros behind the columns in use."""
     from volta_engine_b200._lib import call, ptr
-    g = torch.Generator().manual_seed(n)
-    npages = (start + n + 63) // 64
-    up = torch.randn(npages * 64, heads * 256, generator=g).to(torch.bfloat16).cuda()
-    lat = torch.randn(npages * 64, 576, generator=g).to(torch.bfloat16).cuda()
-    kp = torch.empty(npages, heads, 64, 192, dtype=torch.bfloat16, device="cuda")
-    vp = torch.empty(npages, heads, 64, 128, dtype=torch.bfloat16, device="cuda")
-    call("mla_expand_kv", "ppppiiii", ptr(up), ptr(lat), ptr(kp), ptr(vp), npages * 64, heads, 128, 128)
-    u = up.reshape(-1, heads, 256)
-    k = torch.cat([u[..., :128], lat[:, None, 512:].expand(-1, heads, -1)], -1)
-    v = u[..., 128:]
-    assert torch.equal(kp.transpose(1, 2).reshape(-1, heads, 192), k) and torch.equal(vp.transpose(1, 2).reshape(-1, heads, 128), v)
-    q = torch.randn(n, heads * 192, generator=g).to(torch.bfloat16).cuda()
-    pos = torch.arange(start, start + n, dtype=torch.int32).cuda()
-    slot = torch.zeros(n, dtype=torch.int32, device="cuda")
-    table = torch.arange(npages, dtype=torch.int32, device="cuda").reshape(1, npages)
-    tf, tc, nt = K.make_prefill_tiles([0] * n, 1, "cuda", 128, False)
-    out = torch.empty(n, heads * 128, dtype=torch.bfloat16, device="cuda")
-    call("attention_k192_v128", "plplppppipipplifp", ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(pos), ptr(slot), ptr(tf), ptr(tc), nt,
-         ptr(table), npages, ptr(kp), ptr(vp), npages, heads, 0.07, ptr(K.status_word(q.device)))
-    assert _err(out.reshape(n, heads, 128), _want(q.reshape(n, heads, 192), k, v, pos, 0, 0.07)) < 2 ** -8 + 2 ** -9
-    assert K.check_status(torch.device("cuda")) == 0
+    up = torch.randn(npages * 64, heads * (nope + vd)).to(torch.bfloat16).cuda()
+    lat = torch.randn(npages * 64, 576).to(torch.bfloat16).cuda()
+    k, v = (torch.full((npages, heads, 64, 256), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    call("mla_expand_kv", "ppppiiii", ptr(up), ptr(lat), ptr(k), ptr(v), npages * 64, heads, nope, vd)
+    u = up.reshape(-1, heads, nope + vd)
+    k, v = (t.transpose(1, 2).reshape(-1, heads, 256) for t in (k, v))
+    assert torch.equal(k[..., :nope], u[..., :nope]) and torch.equal(v[..., :vd], u[..., nope:])
+    assert torch.equal(k[..., nope:nope + 64], lat[:, None, 512:].expand(-1, heads, -1))
+    assert not k[..., nope + 64:].any() and not v[..., vd:].any()

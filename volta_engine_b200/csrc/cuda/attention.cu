@@ -717,35 +717,4 @@ int ve_attention(const void* q, long q_stride, void* out, long out_stride, const
   return rc;
 }
 
-// Prefill attention with keys of 192 and values of 128 columns (latent attention with its keys and values expanded per head): q [rows,
-// heads * 192], out [rows, heads * 128], pages [pool_pages][heads][64][192 | 128]; tiles of at most 128 rows of one sequence.
-int ve_attention_k192_v128(const void* q, long q_stride, void* out, long out_stride, const void* pos, const void* slot, const void* tile_first,
-                           const void* tile_count, int ntiles, const void* page_table, int max_pages, const void* kpool, const void* vpool,
-                           long pool_pages, int heads, float scale, void* status, cudaStream_t st) {
-  if (ntiles <= 0) return 0;
-  if (heads <= 0 || ((uintptr_t)q & 15) || (q_stride & 7) || ((uintptr_t)out & 15) || (out_stride & 7)) return cudaErrorInvalidValue;
-  AttnParams p = {};
-  p.q = (const __nv_bfloat16*)q;
-  p.q_stride = q_stride;
-  p.out = (__nv_bfloat16*)out;
-  p.out_stride = out_stride;
-  p.pos = (const int*)pos;
-  p.slot = (const int*)slot;
-  p.tile_first = (const int*)tile_first;
-  p.tile_count = (const int*)tile_count;
-  p.page_table = (const int*)page_table;
-  p.max_pages = max_pages;
-  p.nq = p.nkv = heads;
-  p.nsplit = 1;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  p.status = (int*)status;
-  CUtensorMap kmap, vmap;
-  const uint64_t rows = (uint64_t)pool_pages * heads * kPageTok;
-  int rc = make_tmap_2d(&kmap, kpool, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 192, 384, kPageTok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-  if (rc) return rc;
-  rc = make_tmap_2d(&vmap, vpool, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, 128, 256, kPageTok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-  if (rc) return rc;
-  return launch_attn_tc<192, 128, 2, 4, 4>(p, kmap, vmap, ntiles, st);
-}
-
 }  // extern "C"

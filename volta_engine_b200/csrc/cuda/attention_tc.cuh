@@ -13,8 +13,7 @@
 // TMEM-load and barrier latencies; the two partial results are merged like split-KV partials in the epilogue (both accumulators live in
 // the same TMEM lanes, so a thread reads both). Values of 256 columns take one stream: a page is then 1024 cycles of tensor work against
 // about 700 of softmax, which runs under the S of the next page and the PV of the one in front.
-// Measured against the mma.sync kernel (attn_kernel): 2048 rows of 24 heads of 256 782 to 172 us, 16 heads 219 to 56 us; 1900 rows of 128
-// heads with keys of 192 and values of 128 (there padded to 256) 1654 to 311 us.
+// Measured against the mma.sync kernel (attn_kernel): 2048 rows of 24 heads of 256 782 to 172 us, 16 heads 219 to 56 us.
 // The reference maximum is only moved when a page raises it by more than 2^8 (then the O row is rescaled in TMEM by
 // the thread that owns it); otherwise the old reference stays, probabilities are at most 2^8 and the final division by
 // the row sum makes the result the same. The exponent is one FMA (score * scale - reference) and one ex2.approx.

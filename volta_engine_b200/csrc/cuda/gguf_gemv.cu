@@ -403,6 +403,182 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
   }
 }
 
+// The mat-vecs of Q8_0 (dense) and IQ1_M (routed) in scalar fp32, in the order of gguf_gemv_kernel: chunk c of 32 weights belongs to lane
+// c % 32, its products are added one after the other, chunks in turn, lanes by a butterfly. Sums stay those of the byte-by-byte kernels bit for bit,
+// so what a router picks behind them does not depend on which of the two ran: a group-limited router at its edge picked other experts for
+// about one token in a hundred with the tensor-core sums. 7168 x 16384 Q8_0: one row 71 us, eight rows 133 us (gguf_mma_kernel 79 and 70 us,
+// byte by byte about 2400 us at eight); IQ1_M, gate / up and down of 64 routes of 2048 x 7168: 949 us (777 us, 2120 us). A warp takes two rows (MODE 2: a gate and an up row); steps of
+// 1024 weights of its rows and of x come through double buffers by 16-byte cp.async, x chunks 80 bytes apart (no bank conflicts).
+template <int TYPE, int MT>
+struct OrderedCfg {
+  static constexpr int kStepBytes = TYPE == kQ8_0 ? 32 * 34 : 4 * 56;
+  static constexpr int kPitch = (kStepBytes + 15 + 15) / 16 * 16;
+  static constexpr int kTab = (Fmt<TYPE>::kTabBytes + 15) / 16 * 16;
+  static constexpr int kX = 32 * 80;                                          // a step of one row of x
+  static constexpr int kSmem = kTab + 2 * MT * kX + 8 * 2 * 2 * kPitch;
+};
+
+template <int TYPE, int MODE, int MT>
+__global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p) {
+  using C = OrderedCfg<TYPE, MT>;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  uint8_t* const tab = smem_raw;
+  uint8_t* const xs = smem_raw + C::kTab;                                     // [2][MT][kX]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* const ws = xs + 2 * MT * C::kX + warp * 2 * 2 * C::kPitch;         // [2][2 rows][kPitch]
+  if (C::kTab) load_table<TYPE>(tab);
+  if (MODE != 0) grid_dep_wait();
+  const int route = blockIdx.y;
+  int e = 0;
+  if (MODE != 0) e = p.ids[route] - p.e0;
+  const bool here = MODE == 0 || (e >= 0 && e < p.e_local);
+  const int half_n = p.N >> 1, n_out = MODE == 2 ? half_n : p.N;
+  const int tiles = (n_out + (MODE == 2 ? 7 : 15)) / (MODE == 2 ? 8 : 16);
+  const __nv_bfloat16* x = p.x + (MODE != 0 ? (long)(route / p.x_div) * p.x_stride : 0);
+  const int chunks = p.K >> 5, steps = (chunks + 31) / 32, M = MODE != 0 ? 1 : p.M;
+  bool waited = MODE != 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int first = tile * (MODE == 2 ? 8 : 16) + warp * (MODE == 2 ? 1 : 2);
+    const uint8_t* rp[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int n = MODE == 2 ? min(first, half_n - 1) + r * half_n : min(first + r, p.N - 1);
+      rp[r] = p.W + ((size_t)(here ? e : 0) * p.N + n) * p.row_bytes;
+    }
+    auto load_w = [&](int i) {
+      const int bytes = TYPE == kQ8_0 ? min(32, chunks - i * 32) * 34 : min(4, (chunks - i * 32) / 8) * 56;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint8_t* src = rp[r] + (size_t)i * C::kStepBytes;
+        const int off = (int)((uintptr_t)src & 15);       // whole 16-byte pieces: inside the allocation, but for the one the matrix ends in
+        src -= off;
+        uint8_t* dst = ws + ((i & 1) * 2 + r) * C::kPitch;
+        for (int j = lane; j < (off + bytes + 15) >> 4; j += 32) {
+          const long left = p.W_end - (src + j * 16);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + j * 16)), "l"(src + j * 16), "r"(left < 16 ? (int)left : 16)
+                       : "memory");
+        }
+      }
+    };
+    auto load_x = [&](int i) {
+      const int n = min(32, chunks - i * 32) * 4;         // 16-byte pieces of a row
+      for (int j = threadIdx.x; j < M * 128; j += 256) {
+        const int m = j >> 7, c = j & 127;
+        if (c < n)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + ((i & 1) * MT + m) * C::kX + (c >> 2) * 80 + (c & 3) * 16)),
+                       "l"(x + (long)m * p.x_stride + (long)i * 1024 + c * 8)
+                       : "memory");
+      }
+    };
+    float acc[2][MT];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+    if (here) {
+      load_w(0);
+      if (!waited) { grid_dep_wait(); waited = true; }
+      load_x(0);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      for (int i = 0; i < steps; ++i) {
+        if (i + 1 < steps) { load_w(i + 1); load_x(i + 1); }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                  // this step is here for every thread
+        if (i * 32 + lane < chunks) {
+          float w[2][32];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const uint8_t* b = ws + ((i & 1) * 2 + r) * C::kPitch + (int)((uintptr_t)(rp[r] + (size_t)i * C::kStepBytes) & 15);
+            if (TYPE == kQ8_0) {
+              b += lane * 34;
+              const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)b & ~(uintptr_t)3);
+              const int sh = (int)((uintptr_t)b & 2) * 8;
+              uint32_t v[9];
+#pragma unroll
+              for (int j = 0; j < 9; ++j) v[j] = q[j];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[j] = __funnelshift_r(v[j], v[j + 1], sh);
+              v[8] >>= sh;
+              const float d = __half2float(__ushort_as_half((unsigned short)v[0]));
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {               // byte j + 2: 2^23 + 128 + value, less 2^23 + 128
+                const uint32_t u = v[(j + 2) >> 2] ^ 0x80808080u;
+                w[r][j] = d * (__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7440u | ((j + 2) & 3))) - 8388736.f);
+              }
+            } else {
+              b += (lane >> 3) * 56;
+              const int c = lane & 7;
+              const uint32_t qs = ld32<true>(b + c * 4), qh = ld16(b + 32 + 2 * c);
+              const float d = vec8_scale<TYPE>(b);
+              const uint32_t sw = ld16(b + 48 + 2 * (c >> 1)) >> (6 * (c & 1));
+              const float dl[2] = {d * u2f(2 * (sw & 7) + 1), d * u2f(2 * ((sw >> 3) & 7) + 1)};
+#pragma unroll
+              for (int l = 0; l < 4; ++l) {
+                const uint32_t h = qh >> (4 * l);
+                const uint32_t codes = reinterpret_cast<const uint32_t*>(tab)[((qs >> (8 * l)) & 255) | ((h & 7) << 8)];
+                const uint2 val = reinterpret_cast<const uint2*>(tab + 8192)[h & 8];
+                uint32_t f[4];
+                vec8_expand(codes, val.x, val.y, f);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  w[r][8 * l + 2 * j] = dl[l >> 1] * __uint_as_float(f[j] << 16);
+                  w[r][8 * l + 2 * j + 1] = dl[l >> 1] * __uint_as_float(f[j] & 0xffff0000u);
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            if (m >= M) break;
+            const uint4* xv = reinterpret_cast<const uint4*>(xs + ((i & 1) * MT + m) * C::kX + lane * 80);
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 t = xv[j];
+              const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float lo = __uint_as_float(u[k] << 16), hi = __uint_as_float(u[k] & 0xffff0000u);
+                s0 = fmaf(w[0][8 * j + 2 * k], lo, s0);
+                s1 = fmaf(w[1][8 * j + 2 * k], lo, s1);
+                s0 = fmaf(w[0][8 * j + 2 * k + 1], hi, s0);
+                s1 = fmaf(w[1][8 * j + 2 * k + 1], hi, s1);
+              }
+            }
+            acc[0][m] += s0;
+            acc[1][m] += s1;
+          }
+        }
+        __syncthreads();                                  // every thread is done with the buffers that the next round fills
+      }
+    }
+    if (tile + (int)gridDim.x >= tiles) grid_dep_launch();
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      if (m >= M) break;
+      const float v0 = warp_sum(acc[0][m]), v1 = warp_sum(acc[1][m]);
+      if (lane != 0) continue;
+      if (MODE == 2) {
+        // the unfused pair rounds both projections to bf16 before the activation: the same rounding points here
+        float gate = bf2f(f2bf(v0)), up = bf2f(f2bf(v1));
+        if (p.limit > 0.f) { gate = fminf(gate, p.limit); up = fminf(fmaxf(up, -p.limit), p.limit); }
+        const float a = p.act ? 0.5f * gate * (1.f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate)))
+                              : gate / (1.f + __expf(-gate));
+        if (first < n_out) p.out[(long)route * p.out_stride + first] = f2bf(here ? a * up : 0.f);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          if (first + r >= n_out) continue;
+          const long at = (long)(MODE == 1 ? route : m) * p.out_stride + first + r;
+          const float v = r ? v1 : v0;
+          if (MODE == 0 && p.out_f32) p.out_f32[at] = v;
+          else p.out[at] = f2bf(v);
+        }
+      }
+    }
+  }
+}
+
 template <int TYPE>
 __global__ void gguf_dequant_kernel(const uint8_t* __restrict__ W, long row_bytes, __nv_bfloat16* __restrict__ out,
                                     long N, int K) {
@@ -441,6 +617,24 @@ static int launch_gguf_mma(GgufGemvArgs a, cudaStream_t st) {
   VE_CHECK_LAUNCH();
 }
 
+template <int TYPE, int MODE, int MT>
+static int launch_gguf_ordered(const GgufGemvArgs& a, int routes, cudaStream_t st) {
+  constexpr int smem = OrderedCfg<TYPE, MT>::kSmem;
+  static bool attr_set = false;
+  if (!attr_set) {
+    const cudaError_t e = cudaFuncSetAttribute(gguf_ordered_kernel<TYPE, MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  const int per = MODE == 2 ? 8 : 16, n = MODE == 2 ? a.N / 2 : a.N;
+  // routed: up to eight tiles a block, so that the codebook is laid out once for them, as long as every SM keeps eight blocks
+  const int tiles = (n + per - 1) / per;
+  long share = MODE == 0 ? 1 : (long)tiles * routes / (148 * 8);
+  share = share < 1 ? 1 : share > 8 ? 8 : share;
+  launch_pdl(gguf_ordered_kernel<TYPE, MODE, MT>, dim3((unsigned)((tiles + share - 1) / share), routes), dim3(256), smem, st, a);
+  VE_CHECK_LAUNCH();
+}
+
 // fields of a block are read from shared memory in words of their natural alignment, which the row addresses must keep
 template <int TYPE>
 static bool block_aligned(const void* W, long row_bytes) {
@@ -453,12 +647,19 @@ static int run_gguf_gemv(GgufGemvArgs a, cudaStream_t st) {
     gguf_gemv_kernel<TYPE><<<(a.N + 7) / 8, 256, 0, st>>>(a.W, a.row_bytes, a.x, a.x_stride, a.out, a.out_stride, a.out_f32, a.M, a.N, a.K);
     VE_CHECK_LAUNCH();
   }
+  if constexpr (TYPE == kQ8_0) {
+    if (a.M == 1) return launch_gguf_ordered<TYPE, 0, 1>(a, 1, st);
+    if (a.M <= 4) return launch_gguf_ordered<TYPE, 0, 4>(a, 1, st);
+    if (a.M <= 8) return launch_gguf_ordered<TYPE, 0, 8>(a, 1, st);
+    return launch_gguf_ordered<TYPE, 0, 16>(a, 1, st);
+  } else {
   // 32 weight rows a tile where several rows of x would otherwise be read again for every 16 of a large matrix; the sums are the same
   a.tiles = (a.N + 15) / 16;
   if (a.M <= 4 || (a.M <= 8 && a.N < 32 * 148)) return launch_gguf_mma<TYPE, 0, 1, 1>(a, st);
   a.tiles = (a.N + 31) / 32;
   if (a.M <= 8) return launch_gguf_mma<TYPE, 0, 1, 2>(a, st);
   return launch_gguf_mma<TYPE, 0, 2, 2>(a, st);
+  }
 }
 
 template <int TYPE>
@@ -473,9 +674,13 @@ static int run_gguf_moe(GgufGemvArgs a, int routes, int fuse_act, cudaStream_t s
                                                           a.out_stride, a.N, a.K, a.act, a.limit);
     VE_CHECK_LAUNCH();
   }
+  if constexpr (TYPE == kIQ1_M) {
+    return fuse_act ? launch_gguf_ordered<TYPE, 2, 1>(a, routes, st) : launch_gguf_ordered<TYPE, 1, 1>(a, routes, st);
+  } else {
   a.tiles_per_route = fuse_act ? (a.N / 2 + 7) / 8 : (a.N + 15) / 16;
   a.tiles = a.tiles_per_route * routes;
   return fuse_act ? launch_gguf_mma<TYPE, 2, 1, 1>(a, st) : launch_gguf_mma<TYPE, 1, 1, 1>(a, st);
+  }
 }
 
 template <int TYPE>

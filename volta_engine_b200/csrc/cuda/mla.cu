@@ -58,119 +58,93 @@ __global__ void mla_rope_store_kernel(__nv_bfloat16* __restrict__ q, long q_stri
 }
 
 // q_abs[row, h, 0:512] = q[row, h, 0:nope] @ W_uk[h] (nope x 512) ; q_abs[row, h, 512:576] = q_rope.
-// One block a head, 512 threads: thread t of group w owns latent columns 4 t .. 4 t + 3 and 32 of every 128 rows of W_uk, which it asks for
-// at once; eight activation rows share them, and the four groups' sums are added in order. Bound by the 16.8 MB of 128 heads (3 us): a block
-// per (row, head) read them once per row behind a chain of eight loads, 18 us.
+// One block a head, thread = latent column; it asks for 32 rows of W_uk at once, and up to eight activation rows share them. Bound by the 16.8 MB
+// of 128 heads (3 us): a block per (row, head) read them once per row behind a chain of eight loads, 18 us. Sums run over d in order.
 constexpr int kAbsRows = 8;
 __global__ void __launch_bounds__(512) mla_absorb_q_kernel(const __nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int nope,
                                                            const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ q_abs, int rows,
                                                            int heads) {
-  __shared__ float qs[256][kAbsRows];
-  __shared__ float red[4][kAbsRows / 2][kLat];
-  const int h = blockIdx.x, tid = threadIdx.x, grp = tid >> 7, c0 = (tid & 127) * 4;
-  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat + c0;
+  __shared__ __align__(16) float qs[256][kAbsRows];
+  const int h = blockIdx.x, tid = threadIdx.x;
+  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat + tid;
   for (int r0 = 0; r0 < rows; r0 += kAbsRows) {
     const int n = min(kAbsRows, rows - r0);
     const __nv_bfloat16* qv = q + (long)r0 * q_stride + (long)h * q_dim;
+    __syncthreads();
     for (int i = tid; i < nope * kAbsRows; i += 512) {
       const int r = i / nope, d = i - r * nope;
       qs[d][r] = r < n ? bf2f(qv[(long)r * q_stride + d]) : 0.f;
     }
     for (int i = tid; i < n * kRope; i += 512)
       q_abs[((long)(r0 + i / kRope) * heads + h) * kLatRow + kLat + i % kRope] = qv[(long)(i / kRope) * q_stride + q_dim - kRope + i % kRope];
-    float acc[kAbsRows][4];
+    __syncthreads();
+    float acc[kAbsRows];
 #pragma unroll
-    for (int r = 0; r < kAbsRows; ++r)
+    for (int r = 0; r < kAbsRows; ++r) acc[r] = 0.f;
+    for (int d0 = 0; d0 < nope; d0 += 32) {
+      __nv_bfloat16 t[32];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
-    bool ready = false;
-    for (int d0 = grp * 32; d0 < (nope + 127) / 128 * 128; d0 += 128) {
-      uint2 t[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) t[i] = d0 + i < nope ? *reinterpret_cast<const uint2*>(w + (long)(d0 + i) * kLat) : make_uint2(0u, 0u);
-      if (!ready) { __syncthreads(); ready = true; }          // qs (every group makes the same number of rounds)
+      for (int i = 0; i < 32; ++i) t[i] = d0 + i < nope ? w[(long)(d0 + i) * kLat] : __float2bfloat16(0.f);
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         if (d0 + i >= nope) break;
-        const float w0 = __uint_as_float(t[i].x << 16), w1 = __uint_as_float(t[i].x & 0xffff0000u);
-        const float w2 = __uint_as_float(t[i].y << 16), w3 = __uint_as_float(t[i].y & 0xffff0000u);
+        const float wf = bf2f(t[i]);
 #pragma unroll
         for (int r = 0; r < kAbsRows; r += 4) {
           const float4 x = *reinterpret_cast<const float4*>(&qs[d0 + i][r]);
-          const float xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[r + j][0] = fmaf(xs[j], w0, acc[r + j][0]);
-            acc[r + j][1] = fmaf(xs[j], w1, acc[r + j][1]);
-            acc[r + j][2] = fmaf(xs[j], w2, acc[r + j][2]);
-            acc[r + j][3] = fmaf(xs[j], w3, acc[r + j][3]);
-          }
+          acc[r] = fmaf(x.x, wf, acc[r]);
+          acc[r + 1] = fmaf(x.y, wf, acc[r + 1]);
+          acc[r + 2] = fmaf(x.z, wf, acc[r + 2]);
+          acc[r + 3] = fmaf(x.w, wf, acc[r + 3]);
         }
       }
     }
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-#pragma unroll
-      for (int r = 0; r < kAbsRows / 2; ++r) {
-        const float* v = acc[half * (kAbsRows / 2) + r];
-        *reinterpret_cast<float4*>(&red[grp][r][c0]) = make_float4(v[0], v[1], v[2], v[3]);
-      }
-      __syncthreads();
-      // group g writes row half * 4 + g
-      const int row = half * (kAbsRows / 2) + grp;
-      if (row < n) {
-        float o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = ((red[0][grp][c0 + j] + red[1][grp][c0 + j]) + red[2][grp][c0 + j]) + red[3][grp][c0 + j];
-        __nv_bfloat16* dst = q_abs + ((long)(r0 + row) * heads + h) * kLatRow + c0;
-        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(o[0], o[1]);
-        *reinterpret_cast<__nv_bfloat162*>(dst + 2) = __floats2bfloat162_rn(o[2], o[3]);
-      }
-      __syncthreads();
-    }
+    for (int r = 0; r < kAbsRows; ++r)
+      if (r < n) q_abs[((long)(r0 + r) * heads + h) * kLatRow + tid] = f2bf(acc[r]);
   }
 }
 
-// out[row, h, 0:vdim] = o_lat[row, h, 0:512] @ W_uv[h]^T  (W_uv [heads, vdim, 512]). grid (vdim / 16, heads, rows / 16), 128 threads: 16 columns of
-// a head, up to 16 rows; the four warps split the 512 latent columns, lane (g, t) holds 8 of every 32 of them for W_uv rows g and g + 8 and
-// o_lat row g (and g + 8). Steps leave the tensor core one by one and are added in fp32. Bound by the 16.8 MB of W_uv of 128 heads (3 us);
-// a thread per output column walked its kilobyte of W_uv alone, once per row: 123 us at eight rows.
+// out[row, h, 0:vdim] = o_lat[row, h, 0:512] @ W_uv[h]^T  (W_uv [heads, vdim, 512]). grid (vdim / 32, heads, rows / 8), 128 threads: 32 rows of a
+// head's W_uv come to shared memory once (rows 1040 bytes apart: no bank conflicts) for eight activation rows, two a warp; lane = column.
+// Bound by the 16.8 MB of W_uv of 128 heads (3 us); a thread per output column walked its kilobyte of W_uv alone, once per row: 123 us at
+// eight rows. Sums run over the latent columns in order.
 __global__ void __launch_bounds__(128) mla_expand_out_kernel(const __nv_bfloat16* __restrict__ o_lat, const __nv_bfloat16* __restrict__ w_uv,
                                                              __nv_bfloat16* __restrict__ out, long out_stride, int rows, int heads, int vdim) {
-  __shared__ float part[4][16][17];
-  const int v0 = blockIdx.x * 16, h = blockIdx.y, r0 = blockIdx.z * 16, n = min(16, rows - r0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const __nv_bfloat16* w = w_uv + (long)h * vdim * kLat + warp * 128 + 8 * t;
-  uint4 a[4][2], x[4][2];
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      a[c][i] = *reinterpret_cast<const uint4*>(w + (long)min(v0 + g + 8 * i, vdim - 1) * kLat + c * 32);
-      x[c][i] = g + 8 * i < n ? *reinterpret_cast<const uint4*>(o_lat + ((long)(r0 + g + 8 * i) * heads + h) * kLat + warp * 128 + 8 * t + c * 32)
-                              : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (i && n <= 8) break;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      mma_bf16_16816(d, a[c][0].x, a[c][1].x, a[c][0].y, a[c][1].y, x[c][i].x, x[c][i].y);
-      mma_bf16_16816(d, a[c][0].z, a[c][1].z, a[c][0].w, a[c][1].w, x[c][i].z, x[c][i].w);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] += d[e];
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) part[warp][i * 8 + 2 * t + (e & 1)][(e >> 1) * 8 + g] = acc[e];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  uint8_t* const wsm = smem_raw;                                              // [32][1040]
+  float* const os = reinterpret_cast<float*>(smem_raw + 32 * 1040);           // [8][512]
+  const int v0 = blockIdx.x * 32, h = blockIdx.y, r0 = blockIdx.z * 8, n = min(8, rows - r0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < 32 * 64; i += 128) {
+    const int v = i >> 6, c = i & 63;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(wsm + v * 1040 + c * 16)),
+                 "l"(w_uv + ((long)h * vdim + min(v0 + v, vdim - 1)) * kLat + c * 8) : "memory");
   }
+  for (int i = threadIdx.x; i < 8 * kLat; i += 128) {
+    const int r = i >> 9, c = i & 511;
+    os[i] = r < n ? bf2f(o_lat[((long)(r0 + r) * heads + h) * kLat + c]) : 0.f;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  for (int i = threadIdx.x; i < n * 16; i += 128) {
-    const int m = i >> 4, v = i & 15;
-    if (v0 + v < vdim)
-      out[(long)(r0 + m) * out_stride + (long)h * vdim + v0 + v] =
-          f2bf(((part[0][m][v] + part[1][m][v]) + part[2][m][v]) + part[3][m][v]);
+  const float *xa = os + warp * 2 * kLat, *xb = xa + kLat;
+  float a = 0.f, b = 0.f;
+#pragma unroll 8
+  for (int c = 0; c < kLat; c += 8) {
+    const bf16x8 t = *reinterpret_cast<const bf16x8*>(wsm + lane * 1040 + c * 2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(t.v[j]);
+      a = fmaf(f.x, xa[c + 2 * j], a);
+      b = fmaf(f.x, xb[c + 2 * j], b);
+      a = fmaf(f.y, xa[c + 2 * j + 1], a);
+      b = fmaf(f.y, xb[c + 2 * j + 1], b);
+    }
+  }
+  if (v0 + lane < vdim) {
+    __nv_bfloat16* dst = out + (long)(r0 + warp * 2) * out_stride + (long)h * vdim + v0 + lane;
+    if (warp * 2 < n) dst[0] = f2bf(a);
+    if (warp * 2 + 1 < n) dst[out_stride] = f2bf(b);
   }
 }
 
@@ -412,9 +386,9 @@ using namespace ve;
 
 namespace ve {
 
-// Keys and values of a context expanded per head, as pages [page][head][64][nope + 64] and [page][head][64][vd]: up [ctx, heads * (nope + vd)]
-// holds the expanded parts, lat [ctx, 576] the rotary key behind the latent. One warp a (position, head), 16-byte pieces; bound by the copy
-// (280 MB for 1900 positions of 128 heads: 81 us, where fills and strided copies of padded pages took 500).
+// Keys and values of a context expanded per head, as pages [page][head][64][256] with zeros behind their nope + 64 and vd columns: up [ctx,
+// heads * (nope + vd)] holds the expanded parts, lat [ctx, 576] the rotary key behind the latent. One warp a (position, head), 16-byte
+// pieces; bound by the copy (380 MB for 1900 positions of 128 heads), where fills and strided copies took 500 us.
 __global__ void __launch_bounds__(256) mla_expand_kv_kernel(const __nv_bfloat16* __restrict__ up, const __nv_bfloat16* __restrict__ lat,
                                                             __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v, long total, int heads,
                                                             int nope, int vd) {
@@ -423,16 +397,12 @@ __global__ void __launch_bounds__(256) mla_expand_kv_kernel(const __nv_bfloat16*
   const long pos = unit / heads;
   const int h = (int)(unit % heads);
   const long row = ((pos >> 6) * heads + h) * 64 + (pos & 63);
-  const int lane = threadIdx.x & 31, nk = nope / 8, nv = vd / 8;
+  const int c = threadIdx.x & 31, nk = nope / 8, nv = vd / 8;      // 16-byte piece of a row of 256
   const uint4* src = reinterpret_cast<const uint4*>(up + (pos * heads + h) * (nope + vd));
   const uint4* rope = reinterpret_cast<const uint4*>(lat + pos * 576 + 512);
-  uint4* dk = reinterpret_cast<uint4*>(k + row * (nope + 64));
-  uint4* dv = reinterpret_cast<uint4*>(v + row * vd);
-  for (int c = lane; c < nk + 8 + nv; c += 32) {
-    if (c < nk) dk[c] = src[c];
-    else if (c < nk + 8) dk[c] = rope[c - nk];
-    else dv[c - nk - 8] = src[c - 8];
-  }
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  reinterpret_cast<uint4*>(k + row * 256)[c] = c < nk ? src[c] : c < nk + 8 ? rope[c - nk] : zero;
+  reinterpret_cast<uint4*>(v + row * 256)[c] = c < nv ? src[nk + c] : zero;
 }
 
 }  // namespace ve
@@ -463,8 +433,15 @@ int ve_mla_expand_out(const void* o_lat, const void* w_uv, void* out, long out_s
                       cudaStream_t st) {
   if (rows <= 0) return 0;
   if (vdim > 256) return cudaErrorInvalidValue;
-  dim3 grid((vdim + 15) / 16, heads, (rows + 15) / 16);
-  mla_expand_out_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)o_lat, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, out_stride, rows,
+  constexpr int smem = 32 * 1040 + 8 * kLat * 4;
+  static bool attr_set = false;
+  if (!attr_set) {
+    const cudaError_t e = cudaFuncSetAttribute(mla_expand_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  dim3 grid((vdim + 31) / 32, heads, (rows + 7) / 8);
+  mla_expand_out_kernel<<<grid, 128, smem, st>>>((const __nv_bfloat16*)o_lat, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, out_stride, rows,
                                               heads, vdim);
   VE_CHECK_LAUNCH();
 }
@@ -558,10 +535,10 @@ int ve_latent_decode(const void* q_abs, void* o_part, void* lse_part, const void
   VE_CHECK_LAUNCH();
 }
 
-// up [ctx, heads * (nope + vd)], lat [ctx, 576] (both dense, 16-byte aligned; nope and vd multiples of 8) -> k, v pages of ctx / 64 pages.
+// up [ctx, heads * (nope + vd)], lat [ctx, 576] (both dense, 16-byte aligned; nope and vd multiples of 8, nope <= 192, vd <= 256) -> k, v: ctx / 64 pages.
 int ve_mla_expand_kv(const void* up, const void* lat, void* k, void* v, int ctx, int heads, int nope, int vd, cudaStream_t st) {
   if (ctx <= 0) return 0;
-  if (heads <= 0 || nope % 8 || vd % 8 || ctx % 64) return cudaErrorInvalidValue;
+  if (heads <= 0 || nope % 8 || nope > 192 || vd % 8 || vd > 256 || ctx % 64) return cudaErrorInvalidValue;
   const long total = (long)ctx * heads;
   mla_expand_kv_kernel<<<(unsigned)((total + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)up, (const __nv_bfloat16*)lat, (__nv_bfloat16*)k,
                                                                     (__nv_bfloat16*)v, total, heads, nope, vd);

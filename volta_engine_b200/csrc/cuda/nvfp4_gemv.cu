@@ -132,6 +132,71 @@ nvfp4_gemv_kernel(const uint8_t* __restrict__ Wp, const uint8_t* __restrict__ Ws
   }
 }
 
+// bf16 weights of few rows (routers, 256 to 512 rows), fp32 output, fp32 FMAs in one fixed order: up to four activation rows a pass. The
+// matrix stays in L2 between the passes, so what the tensor cores would save (14 to 5 us at 16 rows of 512 x 2048) is small, and a router's
+// scores keep their bits.
+template <int MR>
+__global__ void __launch_bounds__(kGemvWarps * 32)
+bf16_gemv_few_kernel(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ x, long x_stride,
+                     float* __restrict__ out, long out_stride, int M, int N, int K, int m0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n0 = blockIdx.x * kGemvRows;
+  __shared__ float part[kGemvWarps][kGemvRows][MR];
+  grid_dep_launch();
+  grid_dep_wait();                   // x is the output of the kernel in front (this launch is a programmatic dependent)
+  float acc[kGemvRows][MR];
+#pragma unroll
+  for (int r = 0; r < kGemvRows; ++r)
+#pragma unroll
+    for (int m = 0; m < MR; ++m) acc[r][m] = 0.f;
+  const int kchunks = K >> 3;
+  for (int c = threadIdx.x; c < kchunks; c += kGemvWarps * 32) {
+    float2 xv[MR][4];
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      const uint4 t = *reinterpret_cast<const uint4*>(x + (long)min(m0 + m, M - 1) * x_stride + (long)c * 8);
+      const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        xv[m][j] = make_float2(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xffff0000u));
+    }
+#pragma unroll
+    for (int r = 0; r < kGemvRows; ++r) {
+      const int n = min(n0 + r, N - 1);
+      const uint4 t = __ldcs(reinterpret_cast<const uint4*>(W + (long)n * K) + c);
+      const uint32_t u[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 wf = make_float2(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xffff0000u));
+#pragma unroll
+        for (int m = 0; m < MR; ++m) {
+          acc[r][m] = fmaf(wf.x, xv[m][j].x, acc[r][m]);
+          acc[r][m] = fmaf(wf.y, xv[m][j].y, acc[r][m]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kGemvRows; ++r)
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      float v = acc[r][m];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) part[warp][r][m] = v;
+    }
+  __syncthreads();
+  if (threadIdx.x < kGemvRows * MR) {
+    const int r = threadIdx.x / MR, m = threadIdx.x % MR;
+    if (n0 + r < N && m0 + m < M) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < kGemvWarps; ++w) v += part[w][r][m];
+      out[(long)(m0 + m) * out_stride + n0 + r] = v;
+    }
+  }
+}
+
 // bf16 weights, fp32 output (LM head, routers: logits stay fp32 for argmax / top-k / LSE), up to 8 * NT activation rows in one pass.
 //
 // Bound by the weights' DRAM traffic (1.55 GB and 235 us for a 151936 x 5120 head), so they are read once whatever M is: a block takes 16 * NT
@@ -246,19 +311,28 @@ int ve_nvfp4_gemv(const void* Wp, const void* Ws, float gscale, const void* x, l
 int ve_bf16_gemv_f32(const void* W, const void* x, long x_stride, void* out, long out_stride, int M, int N, int K,
                      cudaStream_t st) {
   if (K % 8 || M <= 0 || N <= 0) return cudaErrorInvalidValue;
+  if (N <= 16 * 148) {
+    const int blocks = (N + kGemvRows - 1) / kGemvRows;
+    for (int m0 = 0; m0 < M;) {
+      const int left = M - m0;
+#define VE_FEW(MR)                                                                                           \
+  launch_pdl(bf16_gemv_few_kernel<MR>, dim3(blocks), dim3(kGemvWarps * 32), 0, st, (const __nv_bfloat16*)W, \
+             (const __nv_bfloat16*)x, x_stride, (float*)out, out_stride, M, N, K, m0)
+      if (left >= 4) { VE_FEW(4); m0 += 4; }
+      else if (left >= 2) { VE_FEW(2); m0 += 2; }
+      else { VE_FEW(1); m0 += 1; }
+#undef VE_FEW
+    }
+    VE_CHECK_LAUNCH();
+  }
   for (int m0 = 0; m0 < M; m0 += 16) {
     const int m = M - m0 < 16 ? M - m0 : 16, nt = m > 8 ? 2 : 1;
     const __nv_bfloat16* xm = (const __nv_bfloat16*)x + (long)m0 * x_stride;
     float* om = (float*)out + (long)m0 * out_stride;
     const dim3 grid((N + 16 * nt - 1) / (16 * nt));
-    // few weight rows (a router: 256 to 512): 16 warps share a block's K, so that its chain of loads stays short
 #define VE_LAUNCH(NT, WARPS)                                                                                               \
   launch_pdl(bf16_gemv_f32_kernel<NT, WARPS>, grid, dim3(32 * WARPS), 0, st, (const __nv_bfloat16*)W, xm, x_stride, om, out_stride, m, N, K)
-    if (N <= 16 * 148) {
-      if (nt == 1) VE_LAUNCH(1, 16); else VE_LAUNCH(2, 16);
-    } else {
-      if (nt == 1) VE_LAUNCH(1, 8); else VE_LAUNCH(2, 8);
-    }
+    if (nt == 1) VE_LAUNCH(1, 8); else VE_LAUNCH(2, 8);
 #undef VE_LAUNCH
   }
   VE_CHECK_LAUNCH();

@@ -183,8 +183,9 @@ class MLAModel(MoEModel):
         return L.o_proj.forward(att, out=pbuf)
 
     def _attn_prefill_expanded(self, L, q, b: BatchRows, kv, pool):
-        """Expand K / V per head for the context of the chunk's sequence and run the paged prefill kernel: keys of 192 and values of 128
-        columns as they are, other widths padded to 256."""
+        """Expand K / V per head for the context of the chunk's sequence and run the dense paged kernel (hd 256). On its 64-row tiles: the
+        tcgen05 form rounds P against another maximum, and a group-limited router behind it then picks other experts for about one token
+        in a hundred."""
         cfg = self.cfg
         n, hl, nope, vd = q.shape[0], self.heads, cfg.qk_nope, cfg.v_head_dim
         slot = b.host_slots[0]
@@ -194,28 +195,22 @@ class MLAModel(MoEModel):
         pages = kv.host_table[slot, :npages].long().to(q.device)
         lat = pool[pages, 0].reshape(npages * 64, LAT_ROW)                       # [ctx_pad, 576]
         up = L.w_ukv.forward(lat[:, :LAT].contiguous())                          # [ctx_pad, hl * (nope + vd)]
-        if self.qd == 192 and vd == 128 and nope == 128 and K.ATTN_PREFILL_TC and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0:
-            kp = torch.empty(npages, hl, 64, 192, dtype=q.dtype, device=q.device)
-            vp = torch.empty(npages, hl, 64, 128, dtype=q.dtype, device=q.device)
-            call("mla_expand_kv", "ppppiiii", ptr(up), ptr(lat), ptr(kp), ptr(vp), npages * 64, hl, nope, vd)
-            table = torch.arange(npages, dtype=torch.int32, device=q.device).reshape(1, npages)
-            slot0 = torch.zeros(n, dtype=torch.int32, device=q.device)
-            tf, tc, ntiles = K.make_prefill_tiles([0] * n, 1, q.device, 128, False)
-            out = torch.empty(n, hl * 128, dtype=q.dtype, device=q.device)
-            call("attention_k192_v128", "plplppppipipplifp", ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(b.pos), ptr(slot0), ptr(tf), ptr(tc),
-                 ntiles, ptr(table), npages, ptr(kp), ptr(vp), npages, hl, float(self.scale), ptr(K.status_word(q.device)))
-            return out
-        up = up.reshape(npages, 64, hl, nope + vd)
-        kfull = torch.zeros(npages, hl, 64, 256, dtype=q.dtype, device=q.device)
-        vfull = torch.zeros(npages, hl, 64, 256, dtype=q.dtype, device=q.device)
-        kfull[..., :nope] = up[..., :nope].permute(0, 2, 1, 3)
-        kfull[..., nope:nope + ROPE] = lat[:, LAT:].reshape(npages, 1, 64, ROPE)
-        vfull[..., :vd] = up[..., nope:].permute(0, 2, 1, 3)
+        kfull = torch.empty(npages, hl, 64, 256, dtype=q.dtype, device=q.device)
+        vfull = torch.empty(npages, hl, 64, 256, dtype=q.dtype, device=q.device)
+        if nope % 8 == 0 and vd % 8 == 0 and nope + ROPE <= 256 and vd <= 256:
+            call("mla_expand_kv", "ppppiiii", ptr(up), ptr(lat), ptr(kfull), ptr(vfull), npages * 64, hl, nope, vd)
+        else:
+            up = up.reshape(npages, 64, hl, nope + vd)
+            kfull.zero_()
+            vfull.zero_()
+            kfull[..., :nope] = up[..., :nope].permute(0, 2, 1, 3)
+            kfull[..., nope:nope + ROPE] = lat[:, LAT:].reshape(npages, 1, 64, ROPE)
+            vfull[..., :vd] = up[..., nope:].permute(0, 2, 1, 3)
         q256 = torch.zeros(n, hl, 256, dtype=q.dtype, device=q.device)
         q256[..., : self.qd] = q.reshape(n, hl, self.qd)
         table = torch.arange(npages, dtype=torch.int32, device=q.device).reshape(1, npages)
         slot0 = torch.zeros(n, dtype=torch.int32, device=q.device)
-        tiles = K.make_prefill_tiles([0] * n, 1, q.device)
+        tiles = K.make_prefill_tiles([0] * n, 1, q.device, wide=False)
         out = K.attention(q256.reshape(n, hl * 256), b.pos, slot0, table, kfull, vfull, hl, hl, 256, self.scale, tiles=tiles)
         return out.reshape(n, hl, 256)[..., :vd].reshape(n, hl * vd).contiguous()
 

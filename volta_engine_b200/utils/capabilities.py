@@ -25,7 +25,7 @@ TABLE = {
     "exl3_gemv": ("LinearTrellis", P), "exl3_reconstruct": ("LinearTrellis", P), "exl3_reconstruct_batch": ("MoE (EXL3 experts)", P), "exl3_viterbi": ("EXL3 quantiser", P), "exl3_viterbi_scratch": ("EXL3 quantiser", P), "had128": ("LinearTrellis", P),
     "gguf_gemv": ("LinearGguf", P), "gguf_dequant": ("LinearGguf", P), "gguf_set_iq_grids": ("LinearGguf", P),
     "gguf_moe_gemv": ("MoEGguf", P), "gemm_grouped_gguf": ("MoEGguf", P), "gemm_grouped_exl3": ("MoE (EXL3 experts)", P),
-    "mla_expand_kv": ("MLALatent", P), "attention_k192_v128": ("MLALatent", P), "moe_unsort": ("MoE", P), "moe_row_experts": ("MoE (EXL3 experts)", P),
+    "mla_expand_kv": ("MLALatent", P), "moe_unsort": ("MoE", P), "moe_row_experts": ("MoE (EXL3 experts)", P),
     "mla_rope_store": ("MLALatent", P), "mla_absorb_q": ("MLALatent", P), "mla_decode": ("MLALatent", P),
     "mla_expand_out": ("MLALatent", P),
     "latent_rope_store": ("LatentAttention", P), "latent_absorb": ("LatentAttention", P), "latent_attn": ("LatentAttention", P),
