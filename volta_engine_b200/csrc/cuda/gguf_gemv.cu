@@ -406,8 +406,8 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
 // The mat-vecs of Q8_0 (dense) and IQ1_M (routed) in scalar fp32, in the order of gguf_gemv_kernel: chunk c of 32 weights belongs to lane
 // c % 32, its products are added one after the other, chunks in turn, lanes by a butterfly. Sums stay those of the byte-by-byte kernels bit for bit,
 // so what a router picks behind them does not depend on which of the two ran: a group-limited router at its edge picked other experts for
-// about one token in a hundred with the tensor-core sums. 7168 x 16384 Q8_0: one row 71 us, eight rows 133 us (gguf_mma_kernel 79 and 70 us,
-// byte by byte about 2400 us at eight); IQ1_M, gate / up and down of 64 routes of 2048 x 7168: 949 us (777 us, 2120 us). A warp takes two rows (MODE 2: a gate and an up row); steps of
+// about one token in a hundred with the tensor-core sums. 7168 x 16384 Q8_0: one row 71 us, eight rows 133 us (gguf_mma_kernel 79 and 70 us);
+// IQ1_M, gate / up and down of 64 routes of 2048 x 7168: 949 us (gguf_mma_kernel 777 us). A warp takes two rows (MODE 2: a gate and an up row); steps of
 // 1024 weights of its rows and of x come through double buffers by 16-byte cp.async, x chunks 80 bytes apart (no bank conflicts).
 template <int TYPE, int MT>
 struct OrderedCfg {
