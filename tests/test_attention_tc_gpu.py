@@ -57,6 +57,28 @@ def test_prompt_attention_pages_streams_and_maxima(hd, nq, nkv, start, n, window
     assert K.check_status(torch.device("cuda")) == 0
 
 
+@pytest.mark.parametrize("hd", [128, 256])
+def test_prompt_rows_whose_window_lies_behind_their_key_limit(hd):
+    """A tile without a page to read writes zeros, as the 64-row kernel does; its neighbours, in the same launch, see their keys."""
+    n, nq, nkv, window = 70, 4, 2, 64
+    g = torch.Generator().manual_seed(hd)
+    kp, vp = (torch.randn(20, nkv, 64, hd, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    table = torch.arange(20, dtype=torch.int32).reshape(1, 20).cuda()
+    pos = torch.arange(1000, 1000 + n, dtype=torch.int32).cuda()
+    key_end = pos.clone()
+    key_end[:64] = 10                              # G = 2: the first tile of 64 tokens sees nothing, the second one all
+    q = torch.randn(n, nq * hd, generator=g).to(torch.bfloat16).cuda()
+    slot = torch.zeros(n, dtype=torch.int32).cuda()
+    out = []
+    for wide in (True, False):
+        tiles = K.make_prefill_tiles([0] * n, nq // nkv, "cuda", wide=wide)
+        out.append(K.attention(q, pos, slot, table, kp, vp, nq, nkv, hd, 1 / 16, out=torch.full((n, nq * hd), 7.0, dtype=torch.bfloat16, device="cuda"),
+                               tiles=tiles, window=window, key_end=key_end))
+    assert not out[0][:64].any() and not out[1][:64].any()
+    assert _err(out[0][64:], out[1][64:].double()) < 2 ** -7
+    assert K.check_status(torch.device("cuda")) == 0
+
+
 @pytest.mark.parametrize("heads,npages,nope,vd", [(1, 1, 128, 128), (5, 3, 64, 72), (3, 2, 192, 256)])
 def test_latent_keys_and_values_expanded_into_pages(heads, npages, nope, vd):
     """Bytes as they are, zeros behind the columns in use."""

@@ -68,6 +68,16 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   const int kt_end = lim_max / kPageTok + 1;
   const int kt_begin = p.window > 0 ? max(0, pos_min - p.window + 1) / kPageTok : 0;
   const int n = kt_end - kt_begin;
+  if (n <= 0) {
+    // every key limit lies in front of the window: the rows see no key and their output is zero. Uniform, before any barrier or TMEM use;
+    // no page may be asked for, since nobody would wait for it before the block ends.
+    for (int i = tid; i < count * G * (DV / 8); i += blockDim.x) {
+      const int r = i / (DV / 8);
+      *reinterpret_cast<uint4*>(p.out + (long)(first + r / G) * p.out_stride + (long)(kvh * G + r % G) * DV + i % (DV / 8) * 8) =
+          make_uint4(0u, 0u, 0u, 0u);
+    }
+    return;
+  }
 
   if (tid == 0) {
     for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
