@@ -62,6 +62,26 @@ def test_gguf_experts_decoded_in_tiles(spec, rows):
     assert K.check_status("cuda") == 0
 
 
+@pytest.mark.parametrize("spec,gu_at,dn_at", [("gguf_q4_k+q6_k", 2, 0), ("gguf_q6_k+q4_k", 2, 2), ("gguf_iq1_s+q4_1", 4, 2), ("gguf_q8_0+q8_0", 2, 6)])
+def test_gguf_experts_at_any_even_address(spec, gu_at, dn_at):
+    """A bank inside a larger allocation gives what it gives at the start of one, whichever way its formats and addresses let it take."""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank, parse_expert_quant
+    gt, dt = parse_expert_quant(spec)
+    E, I, H, k, rows = 3, 256, 512, 2, 50
+    bank = GGUFExpertBank.random(E, I, H, gt, dt, seed=5, amp=0.05, device="cuda")
+
+    def at(raw, off):
+        buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[off:off + raw.numel()] = raw.reshape(-1)
+        return buf[off:off + raw.numel()].reshape(raw.shape)
+    moved = GGUFExpertBank(at(bank.gu_raw, gu_at), gt, at(bank.dn_raw, dn_at), dt, 0, I, H)
+    assert moved.gu_raw.data_ptr() % 16 == gu_at and moved.dn_raw.data_ptr() % 16 == dn_at
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(rows)]).to(torch.int32).cuda()
+    assert _rel(moved.routes_prefill(x, ids, 0, 0.0), bank._routes_prefill_slabs(x, ids, 0, 0.0)) < 1e-3
+
+
 @pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
 @pytest.mark.parametrize("cb", [0, 1, 2])
 def test_exl3_experts_decoded_in_tiles(bits, cb):

@@ -46,6 +46,26 @@ def test_moe_model_with_gguf_experts_runs_on_cpu():
     assert float((bank.dequant("dn", 0) - dn[0]).abs().max()) < 3e-2
 
 
+@pytest.mark.parametrize("spec", ["gguf_q4_k+q6_k", "gguf_q6_k+q4_k", "gguf_q8_0+q4_1", "gguf_iq1_m+iq1_s", "gguf_q4_0+q4_0"])
+@pytest.mark.parametrize("gu_at,dn_at", [(0, 0), (2, 0), (0, 2), (2, 2), (4, 6), (1, 0), (0, 3)])
+def test_a_bank_is_decoded_in_tiles_only_where_every_block_is_readable(spec, gu_at, dn_at):
+    """Blocks of a multiple of 4 bytes are read in 4-byte words, the others in 2-byte words; each matrix of a bank of two types by its own."""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank, parse_expert_quant
+    gt, dt = parse_expert_quant(spec)
+    E, I, H = 2, 256, 512
+
+    def at(raw, off):
+        buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8)
+        off += -buf.data_ptr() % 16
+        buf[off:off + raw.numel()] = raw.reshape(-1)
+        return buf[off:off + raw.numel()].reshape(raw.shape)
+    bank = GGUFExpertBank(at(G.random_blocks(gt, E * 2 * I, H).reshape(E, 2 * I, -1), gu_at), gt,
+                          at(G.random_blocks(dt, E * H, I).reshape(E, H, -1), dn_at), dt, 0, I, H)
+    assert bank.gu_raw.data_ptr() % 16 == gu_at and bank.dn_raw.data_ptr() % 16 == dn_at
+    word = {t: 4 if G.BLOCK[t][1] % 4 == 0 else 2 for t in (gt, dt)}
+    assert bank._decodes_in_tiles(32) == (gu_at % word[gt] == 0 and dn_at % word[dt] == 0)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("t", IQ)
 def test_gpu_iq_dequant_and_matvec_match_the_statement(t):

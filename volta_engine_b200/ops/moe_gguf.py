@@ -106,10 +106,14 @@ class GGUFExpertBank:
 
     def _decodes_in_tiles(self, routes: int) -> bool:
         """Whether the grouped GEMM decodes the blocks in its tile loader, once per 128 rows of an expert. FUSED_ROWS says up to how
-        many rows an expert this is the faster way; blocks at odd addresses and rows that are no multiple of 16 bytes stay with the other."""
-        words = 4 if gq.row_bytes(self.gu_type, self.hidden) % 4 == 0 and gq.row_bytes(self.dn_type, self.inter) % 4 == 0 else 2
+        many rows an expert this is the faster way; rows of x or out that are no multiple of 16 bytes stay with the other, and so does a
+        matrix whose blocks the loader could not read: it takes their fields in words of 4 bytes where the block is a multiple of 4 bytes
+        long, else of 2, so each matrix has to lie, row by row, on multiples of its own word."""
+        def readable(raw, ggml_type):
+            word = 4 if gq.BLOCK[ggml_type][1] % 4 == 0 else 2
+            return (raw.data_ptr() | raw.shape[2]) % word == 0
         return (routes <= FUSED_ROWS * self.e_local and self.hidden % 8 == 0 and self.inter % 8 == 0
-                and self.gu_raw.data_ptr() % words == 0 and self.dn_raw.data_ptr() % words == 0)
+                and readable(self.gu_raw, self.gu_type) and readable(self.dn_raw, self.dn_type))
 
     def routes_prefill(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
         """Same result layout as :meth:`routes_decode` for a chunk of rows, through the grouped tensor-core GEMM."""
