@@ -104,6 +104,23 @@ def test_exl3_experts_decoded_in_tiles(bits, cb):
     assert K.check_status("cuda") == 0
 
 
+@pytest.mark.parametrize("rows", [1, 5, 40])
+def test_exl3_experts_take_ids_of_any_integer_type_and_stride(rows):
+    """Decode rows and a prompt: 64-bit, 16-bit and strided ids name the same experts as dense 32-bit ones."""
+    from volta_engine_b200.ops.moe_exl3 import EXL3ExpertBank
+    E, I, H, k = 4, 128, 256, 2
+    bank = EXL3ExpertBank.random(E, I, H, 4, e0=1, seed=7, device="cuda", std=0.05)
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(6, generator=g)[:k] for _ in range(rows)]).to(torch.int32).cuda()
+    want = bank.routes(x, ids, 0, 0.0)
+    wide = torch.full((rows, 3 * k), 3, dtype=torch.int32, device="cuda")
+    wide[:, ::3] = ids
+    for form in (ids.long(), ids.short(), wide[:, ::3], ids.t().contiguous().t(), ids.long().t().contiguous().t()):
+        assert torch.equal(bank.routes(x, form, 0, 0.0), want), (form.dtype, form.stride())
+    assert want.any()
+
+
 @pytest.mark.parametrize("N,K", [(1, 8), (17, 40), (512, 7168), (2368, 264), (2369, 1032), (5000, 2048)])
 def test_bf16_matvec_edges(N, K):
     """Row counts on both sides of the warp-count rule, K that ends inside a 32-wide step, every count of activation rows up to more than

@@ -77,6 +77,7 @@ class EXL3ExpertBank:
 
     # ------------------------------------------------------------------------------------------ decode rows
     def routes_decode(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
+        ids = ids.to(torch.int32).contiguous()                      # (the kernels read dense 32-bit words)
         rows, H = x.shape
         k = ids.shape[1]
         R, I, dev = rows * k, self.inter, x.device
@@ -105,6 +106,7 @@ class EXL3ExpertBank:
     def routes_prefill(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
         if limit > 0:
             raise NotImplementedError("clamped gated activation on the EXL3 expert path")
+        ids = ids.to(torch.int32).contiguous()
         rows, H = x.shape
         k = ids.shape[1]
         R, I, dev, E = rows * k, self.inter, x.device, self.e_local
