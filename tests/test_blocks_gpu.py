@@ -37,6 +37,59 @@ def test_gguf_matvec_edges(t, shift):
         assert _rel(lin.forward(x[:3].cuda()).cpu(), want[:3]) < 2 ** -8      # bf16 output: half a unit in the last place
 
 
+def _non_finite(K):
+    """Four rows of activations: none, an infinity, an infinity of each sign in different chunks, values whose products with a block's
+    integers overflow where those with its weights do not."""
+    x = torch.randn(4, K, generator=torch.Generator().manual_seed(K)).to(torch.bfloat16)
+    x[1, 37] = float("inf")
+    x[2, 5], x[2, K - 3] = float("inf"), float("-inf")
+    x[3, ::2] = 3e37
+    return x.cuda()
+
+
+def _same_where_not_finite(got, want, bound):
+    """Infinities and NaN in the same places with the same signs; numbers within 1e-5 of the sum of the products' magnitudes."""
+    fine = torch.isfinite(want)
+    assert torch.equal(got[~fine].nan_to_num(7.0), want[~fine].nan_to_num(7.0))
+    assert bool((((got - want).double().abs() <= 1e-5 * bound)[fine]).all())
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_gguf_matvec_of_infinite_and_huge_activations(t):
+    """Blocks at even addresses against blocks at an odd one, which are summed weight by weight."""
+    N, K = 40, 512
+    raw = gq.random_blocks(t, N, K, seed=t, amp=0.01)
+    buf = torch.zeros(raw.numel() + 64, dtype=torch.uint8, device="cuda")
+    odd = buf[1:1 + raw.numel()].view(N, -1)
+    odd.copy_(raw.reshape(N, -1))
+    x = _non_finite(K)
+    got, want = (LinearGGUF(r, t, N, K).forward(x, out_f32=True) for r in (raw.cuda(), odd))
+    w = gq.dequantize(raw, t, K).double().cuda()
+    _same_where_not_finite(got, want, x.double().nan_to_num(0.0, 0.0, 0.0).abs() @ w.abs().t())
+    assert torch.isinf(want[1]).any()
+
+
+@pytest.mark.parametrize("spec", ["gguf_q4_k+q2_k", "gguf_q5_1+q4_1", "gguf_q5_k+q6_k", "gguf_iq1_m+iq2_s"])
+def test_gguf_experts_of_infinite_and_huge_activations(spec):
+    """The routed mat-vecs, the gated pair among them; outputs are bf16."""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank, parse_expert_quant
+    gt, dt = parse_expert_quant(spec)
+    E, I, H = 3, 256, 512
+    bank = GGUFExpertBank.random(E, I, H, gt, dt, seed=5, amp=0.01, device="cuda")
+
+    def odd(raw):
+        buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[1:1 + raw.numel()] = raw.reshape(-1)
+        return buf[1:1 + raw.numel()].reshape(raw.shape)
+    other = GGUFExpertBank(odd(bank.gu_raw), gt, odd(bank.dn_raw), dt, 0, I, H)
+    ids = torch.tensor([[0, 2], [1, 0], [2, 5], [0, 1]], dtype=torch.int32, device="cuda")
+    x = _non_finite(H)
+    got, want = bank.routes_decode(x, ids, 0, 0.0).float(), other.routes_decode(x, ids, 0, 0.0).float()
+    fine = torch.isfinite(want)
+    assert torch.equal(got[~fine].nan_to_num(7.0), want[~fine].nan_to_num(7.0)) and not fine.all()
+    assert bool(((got - want).abs() <= 2 ** -6 * want.abs().amax(-1, keepdim=True))[fine].all())
+
+
 @pytest.mark.parametrize("spec", ["gguf_q8_0+q4_0", "gguf_q4_k+q5_1", "gguf_iq1_m+iq2_xs", "gguf_q6_k+q3_k", "gguf_q2_k+iq4_xs"])
 @pytest.mark.parametrize("rows", [17, 130, 700])
 def test_gguf_experts_decoded_in_tiles(spec, rows):

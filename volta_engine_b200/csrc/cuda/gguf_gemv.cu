@@ -126,6 +126,33 @@ __global__ void __launch_bounds__(128) gguf_moe_gemv_kernel(const uint8_t* __res
   }
 }
 
+// One product of a packed row with one row of x by a warp, in the order of the two kernels above. For sums whose tensor-core form is not
+// finite: an infinite or huge activation meets the block's integers there before their scale and minimum, so it gave NaN (0 * inf, or
+// inf - inf between s * q and m) or an overflow where the sum over the weights themselves is an infinity or a number.
+template <int TYPE>
+__device__ __noinline__ float ordered_dot(const uint8_t* __restrict__ row, const __nv_bfloat16* __restrict__ xr, int chunks) {
+  const int lane = threadIdx.x & 31;
+  float acc = 0.f;
+  for (int c = lane; c < chunks; c += 32) {
+    float w[32];
+    decode32<TYPE>(row, c, w);
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      const bf16x8 t = *reinterpret_cast<const bf16x8*>(xr + (long)c * 32 + j);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 f = __bfloat1622float2(t.v[u]);
+        s = fmaf(w[j + 2 * u], f.x, s);
+        s = fmaf(w[j + 2 * u + 1], f.y, s);
+      }
+    }
+    acc += s;
+  }
+  return warp_sum(acc);
+}
+VE_DEVINL bool not_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
+
 struct GgufGemvArgs {
   const uint8_t* W; long row_bytes; const uint8_t* W_end;
   const __nv_bfloat16* x; long x_stride;
@@ -372,33 +399,52 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
     }
     __syncthreads();                                      // (the other buffer's sums were read in front of this barrier)
     const int nw = min(8, units);
+    // sums that are not finite are formed again by their warp (all lanes take part), weight by weight
+    auto again = [&](float v, bool bad, auto row_of, auto x_of) {
+      for (uint32_t left = __ballot_sync(0xffffffffu, bad); left; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const float d = ordered_dot<TYPE>(row_of(src), x_of(src), chunks);
+        if (lane == src) v = d;
+      }
+      return v;
+    };
     if (MODE == 0) {
-      for (int i = threadIdx.x; i < 16 * RT * C::kCols; i += 256) {
+      for (int i = threadIdx.x; i < 16 * RT * C::kCols; i += 256) {          // (whole warps: a multiple of 32)
         const int row = i % (16 * RT), m = i / (16 * RT), n = tile * 16 * RT + row;
-        if (m < p.M && n < p.N) {
-          float v = 0.f;
-          for (int w = 0; w < nw; ++w) v += rb[w * C::kRed / 8 + i];
+        const bool in = m < p.M && n < p.N;
+        float v = 0.f;
+        for (int w = 0; w < nw; ++w) v += rb[w * C::kRed / 8 + i];
+        v = again(v, in && not_finite(v), [&](int src) { return p.W + (size_t)(tile * 16 * RT + (i - lane + src) % (16 * RT)) * p.row_bytes; },
+                  [&](int src) { return p.x + (long)((i - lane + src) / (16 * RT)) * p.x_stride; });
+        if (in) {
           if (p.out_f32) p.out_f32[(long)m * p.out_stride + n] = v;
           else p.out[(long)m * p.out_stride + n] = f2bf(v);
         }
       }
-    } else if (threadIdx.x < (MODE == 2 ? 8 : 16)) {
-      const int route = tile / p.tiles_per_route, n = (tile - route * p.tiles_per_route) * (MODE == 2 ? 8 : 16) + threadIdx.x;
-      if (n < (MODE == 2 ? half_n : p.N)) {
-        float v = 0.f, u = 0.f;
-        if (here) {
-          for (int w = 0; w < nw; ++w) v += rb[w * 16 + threadIdx.x];
-          if (MODE == 2) {
-            for (int w = 0; w < nw; ++w) u += rb[w * 16 + 8 + threadIdx.x];
-            // the unfused pair rounds both projections to bf16 before the activation: the same rounding points here
-            float gate = bf2f(f2bf(v)), upv = bf2f(f2bf(u));
-            if (p.limit > 0.f) { gate = fminf(gate, p.limit); upv = fminf(fmaxf(upv, -p.limit), p.limit); }
-            v = (p.act ? 0.5f * gate * (1.f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate)))
-                       : gate / (1.f + __expf(-gate))) * upv;
+    } else if (warp == 0) {
+      constexpr int per = MODE == 2 ? 8 : 16;
+      const int route = tile / p.tiles_per_route, n0 = (tile - route * p.tiles_per_route) * per, n = n0 + lane, n_out = MODE == 2 ? half_n : p.N;
+      const bool in = lane < per && n < n_out;
+      float v = 0.f, u = 0.f;
+      if (here) {
+        if (in)
+          for (int w = 0; w < nw; ++w) {
+            v += rb[w * 16 + lane];
+            if (MODE == 2) u += rb[w * 16 + 8 + lane];
           }
+        const uint8_t* base = p.W + (size_t)(p.ids[route] - p.e0) * p.N * p.row_bytes;
+        auto x_of = [&](int) { return p.x + (long)(route / p.x_div) * p.x_stride; };
+        v = again(v, in && not_finite(v), [&](int src) { return base + (size_t)(n0 + src) * p.row_bytes; }, x_of);
+        if (MODE == 2) {
+          u = again(u, in && not_finite(u), [&](int src) { return base + (size_t)(n0 + src + half_n) * p.row_bytes; }, x_of);
+          // the unfused pair rounds both projections to bf16 before the activation: the same rounding points here
+          float gate = bf2f(f2bf(v)), upv = bf2f(f2bf(u));
+          if (p.limit > 0.f) { gate = fminf(gate, p.limit); upv = fminf(fmaxf(upv, -p.limit), p.limit); }
+          v = (p.act ? 0.5f * gate * (1.f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate)))
+                     : gate / (1.f + __expf(-gate))) * upv;
         }
-        p.out[(long)route * p.out_stride + n] = f2bf(v);
       }
+      if (in) p.out[(long)route * p.out_stride + n] = f2bf(v);
     }
   }
 }
