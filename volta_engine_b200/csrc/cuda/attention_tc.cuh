@@ -68,16 +68,6 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   const int kt_end = lim_max / kPageTok + 1;
   const int kt_begin = p.window > 0 ? max(0, pos_min - p.window + 1) / kPageTok : 0;
   const int n = kt_end - kt_begin;
-  if (n <= 0) {
-    // every key limit lies in front of the window: the rows see no key and their output is zero. Uniform, before any barrier or TMEM use;
-    // no page may be asked for, since nobody would wait for it before the block ends.
-    for (int i = tid; i < count * G * (DV / 8); i += blockDim.x) {
-      const int r = i / (DV / 8);
-      *reinterpret_cast<uint4*>(p.out + (long)(first + r / G) * p.out_stride + (long)(kvh * G + r % G) * DV + i % (DV / 8) * 8) =
-          make_uint4(0u, 0u, 0u, 0u);
-    }
-    return;
-  }
 
   if (tid == 0) {
     for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
@@ -144,7 +134,8 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         return true;
       };
       // the scores of a page are asked for in front of the product of the page before
-      bool ok = load_k(0);
+      // (a tile whose key limits all lie in front of its window has no page: a load that nobody waits for must not be in flight when it ends)
+      bool ok = n <= 0 || load_k(0);
       for (int j = 0; j < n && ok; ++j) {
         if (j + 1 < n) ok = load_k(j + 1);
         if (ok) ok = load_v(j);
@@ -296,6 +287,10 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
       tmem_ld32(t_lane + O_COL + c0, ov);
       if (two) tmem_ld32(t_lane + O_COL + DV + c0, ow);
       tmem_ld_wait();
+      if (n <= 0) {                                          // (nothing was accumulated: the row is zero)
+#pragma unroll
+        for (int e = 0; e < 32; ++e) ov[e] = 0u;
+      }
       if (r_ok) {
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
