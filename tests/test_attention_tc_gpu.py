@@ -79,6 +79,27 @@ def test_prompt_rows_whose_window_lies_behind_their_key_limit(hd):
     assert K.check_status(torch.device("cuda")) == 0
 
 
+@pytest.mark.parametrize("nq,nkv,start,n,window,peak", [(24, 4, 0, 300, 0, 1.0), (16, 2, 200, 900, 0, 4.0), (8, 1, 1500, 300, 256, 3.0), (4, 4, 0, 700, 0, 8.0)])
+def test_prompt_attention_of_256_columns_is_as_near_as_the_64_row_kernel(nq, nkv, start, n, window, peak):
+    """Its probabilities are rounded from the same numbers, so its distance to 64 bits is the other kernel's but for the order of fp32 sums."""
+    hd, g = 256, torch.Generator().manual_seed(n)
+    maxp = (start + n + 63) // 64
+    table = torch.arange(maxp, dtype=torch.int32).reshape(1, maxp).cuda()
+    kp = (torch.randn(maxp, nkv, 64, hd, generator=g) * peak).to(torch.bfloat16).cuda()
+    vp = torch.randn(maxp, nkv, 64, hd, generator=g).to(torch.bfloat16).cuda()
+    pos = torch.arange(start, start + n, dtype=torch.int32).cuda()
+    q = torch.randn(n, nq * hd, generator=g).to(torch.bfloat16).cuda()
+    slot = torch.zeros(n, dtype=torch.int32).cuda()
+    k, v = (t.transpose(1, 2).reshape(-1, nkv, hd) for t in (kp, vp))
+    want = _want(q.reshape(n, nq, hd), k, v, pos, window, 1 / 16)
+    far = []
+    for wide in (True, False):
+        tiles = K.make_prefill_tiles([0] * n, nq // nkv, "cuda", wide=wide)
+        far.append(_err(K.attention(q, pos, slot, table, kp, vp, nq, nkv, hd, 1 / 16, tiles=tiles, window=window).reshape(n, nq, hd), want))
+    assert far[0] < 1.005 * far[1], far
+    assert K.check_status(torch.device("cuda")) == 0
+
+
 @pytest.mark.parametrize("heads,npages,nope,vd", [(1, 1, 128, 128), (5, 3, 64, 72), (3, 2, 192, 256)])
 def test_latent_keys_and_values_expanded_into_pages(heads, npages, nope, vd):
     """Bytes as they are, zeros behind the columns in use."""

@@ -697,8 +697,8 @@ int ve_attention(const void* q, long q_stride, void* out, long out_stride, const
     else return cudaErrorInvalidValue;
   }
 #undef VE_ATTN_TREE
-  else if (warps == 8 && hd == 128) { rc = launch_attn_tc<128, 128, 2, 4, 4>(p, kmap, vmap, ntiles, st); }
-  else if (warps == 8) { rc = launch_attn_tc<256, 256, 1, 3, 2>(p, kmap, vmap, ntiles, st); }
+  else if (warps == 8 && hd == 128) { rc = launch_attn_tc<128, 2, 4, 4>(p, kmap, vmap, ntiles, st); }
+  else if (warps == 8) { rc = launch_attn_tc<256, 1, 3, 2>(p, kmap, vmap, ntiles, st); }
   else if (kv_fp8 == 2 && hd == 128) { VE_ATTNQ(128, 2) }
   else if (kv_fp8 == 2 && hd == 256) { VE_ATTNQ(256, 2) }
   else if (kv_fp8 == 3 && hd == 128) { VE_ATTNQ(128, 3) }

@@ -1,22 +1,26 @@
 // Prefill attention on the fifth-generation tensor cores (tcgen05, accumulators in TMEM). Included by attention.cu.
 //
 // One CTA = one query tile of up to 128 packed rows ((token, head-in-group) pairs of one kv head, one TMEM lane per
-// row) against the pages of its sequence, bf16 cache, keys of DK and values of DV columns, no key split. Per 64-key page:
-//     S  = Q K^T      tcgen05.mma 128 x 64 x DK    (Q and the K page K-major in 128B-swizzled shared memory)
+// row) against the pages of its sequence, bf16 cache, head_dim HD, no key split. Per 64-key page:
+//     S  = Q K^T      tcgen05.mma 128 x 64 x HD    (Q and the K page K-major in 128B-swizzled shared memory)
 //     P  = exp2(S * scale - m)                      (softmax warps: tcgen05.ld of one row per thread; bf16 P goes back into the
 //                                                    first 32 columns of the S buffer it came from)
-//     O += P V        tcgen05.mma 128 x DV x 64    (P from TMEM, the V page as it lands from TMA: the MN-major operand form)
+//     O += P V        tcgen05.mma 128 x HD x 64    (P from TMEM, the V page as it lands from TMA: the MN-major operand form)
 // Warp roles: warp 0 streams pages by TMA (K and V through rings of their own: a K page is free as soon as its S is done), warp 1 issues
-// the MMAs, then four softmax warps per stream (one row per thread). Values of 128 columns leave TMEM room for two streams: the pages are
+// the MMAs, then four softmax warps per stream (one row per thread). Heads of 128 columns leave TMEM room for two streams: the pages are
 // dealt to them alternately, each with its own S buffers (2 x 64 TMEM columns; one stream: 3), its own running (reference maximum, row
 // sum) and its own O accumulator, so the exponentials of one stream run under the MMAs of the other and two warps per scheduler hide the
 // TMEM-load and barrier latencies; the two partial results are merged like split-KV partials in the epilogue (both accumulators live in
-// the same TMEM lanes, so a thread reads both). Values of 256 columns take one stream: a page is then 1024 cycles of tensor work against
+// the same TMEM lanes, so a thread reads both). Heads of 256 columns take one stream: a page is then 1024 cycles of tensor work against
 // about 700 of softmax, which runs under the S of the next page and the PV of the one in front.
-// Measured against the mma.sync kernel (attn_kernel): 2048 rows of 24 heads of 256 782 to 172 us, 16 heads 219 to 56 us.
-// The reference maximum is only moved when a page raises it by more than 2^8 (then the O row is rescaled in TMEM by
-// the thread that owns it); otherwise the old reference stays, probabilities are at most 2^8 and the final division by
-// the row sum makes the result the same. The exponent is one FMA (score * scale - reference) and one ex2.approx.
+// Measured against the mma.sync kernel (attn_kernel): 2048 rows of 24 heads of 256 behind 2048 others 1072 to 245 us, without them 418 to
+// 108 us; 16 heads 715 to 155 and 280 to 65 us. Prompts of a single page are slower, 10 to 13 us (fixed costs of the larger tile).
+// Reference maximum of a row. Heads of 128 columns: it is only moved when a page raises it by more than 2^8 (then the O row is rescaled in
+// TMEM by the thread that owns it); otherwise the old reference stays, probabilities are at most 2^8 and the final division by the row sum
+// makes the result the same. The exponent is one FMA (score * scale - reference) and one ex2.approx. Heads of 256 columns: it is the running
+// maximum itself, and the scaled score is rounded before the maximum is taken off, as in attn_kernel, whose rows of these heads this kernel
+// took over: P is then rounded to bf16 from the same numbers (the largest probability of a page that holds the maximum is one, exactly).
+// With a reference that lags, P lay up to 24 % further from 64 bits (2048 rows, scores of a few units: 0.00209 against 0.00173).
 // Every wait is bounded; on expiry the CTA records a status code, skips its stores and frees its TMEM.
 // Semantics are those of attn_kernel (causal limit / key_end, sliding window, optional sigmoid gate); reference:
 // src/kernels/slang/ref_attention.slang:1-10,47-50,65-70.
@@ -27,13 +31,14 @@ namespace ve {
 constexpr int kTcRows = 128;        // query rows of a tile
 constexpr float kTcLazyLog2 = 8.f;  // the reference maximum moves only when a page raises it by more than this
 
-template <int DK, int DV, int STREAMS, int NK, int NV>
+template <int HD, int STREAMS, int NK, int NV>
 __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
                                                                                const __grid_constant__ CUtensorMap vmap) {
   constexpr int NB = STREAMS == 1 ? 3 : 2;       // S / P buffers of a stream
-  static_assert(DK % 64 == 0 && DV % 64 == 0 && STREAMS * (NB * 64 + DV) <= 512, "S and O of every stream share the tensor memory");
-  constexpr int K_TILE = kPageTok * DK * 2, V_TILE = kPageTok * DV * 2;      // 64-column chunks of 8 KB
-  constexpr int Q_BYTES = kTcRows * DK * 2;                                   // 64-column chunks of 16 KB
+  static_assert(HD % 64 == 0 && STREAMS * (NB * 64 + HD) <= 512, "S and O of every stream share the tensor memory");
+  constexpr bool LAZY = STREAMS == 2;            // see kTcLazyLog2
+  constexpr int TILE = kPageTok * HD * 2;        // a K or V page: 64-column chunks of 8 KB
+  constexpr int Q_BYTES = kTcRows * HD * 2;                                   // 64-column chunks of 16 KB
   // TMEM columns: S of stream t, buffer b at (t * NB + b) * 64; O of stream t behind them
   constexpr uint32_t TMEM_COLS = 512, O_COL = STREAMS * NB * 64;
   const float NEG_INF = __int_as_float(0xff800000);
@@ -43,7 +48,7 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* q_s = smem;
   uint8_t* k_s = smem + Q_BYTES;                // [NK] pages
-  uint8_t* v_s = k_s + NK * K_TILE;             // [NV] pages
+  uint8_t* v_s = k_s + NK * TILE;             // [NV] pages
   __shared__ uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[STREAMS][NB], p_full[STREAMS][NB], pv_done[STREAMS][NB];
   __shared__ float s_ml[STREAMS][2][kTcRows];   // (reference maximum, row sum) of the streams' rows
   __shared__ uint32_t tmem_holder;
@@ -93,9 +98,9 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   if (warp >= 2) {
     // the streams' threads share the 64-column chunks of their row of Q
 #pragma unroll
-    for (int c = 0; c < DK / 64; ++c) {
+    for (int c = 0; c < HD / 64; ++c) {
       if (STREAMS == 2 && (c & 1) != strm) continue;
-      const uint4* src = reinterpret_cast<const uint4*>(p.q + (long)r_tok * p.q_stride + (long)r_head * DK) + c * 8;
+      const uint4* src = reinterpret_cast<const uint4*>(p.q + (long)r_tok * p.q_stride + (long)r_head * HD) + c * 8;
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch) {
         const uint4 v = r_ok ? src[ch] : make_uint4(0u, 0u, 0u, 0u);
@@ -119,18 +124,18 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         const int st = j % NK;
         if (j >= NK && !mbar_wait(&k_empty[st], ((j / NK) - 1) & 1)) return false;
         const int row = row_of(j);
-        mbar_expect_tx(&k_full[st], K_TILE);
+        mbar_expect_tx(&k_full[st], TILE);
 #pragma unroll
-        for (int c = 0; c < DK / 64; ++c) tma_load_2d(k_s + st * K_TILE + c * 8192, &kmap, &k_full[st], c * 64, row);
+        for (int c = 0; c < HD / 64; ++c) tma_load_2d(k_s + st * TILE + c * 8192, &kmap, &k_full[st], c * 64, row);
         return true;
       };
       auto load_v = [&](int j) {
         const int st = j % NV;
         if (j >= NV && !mbar_wait(&v_empty[st], ((j / NV) - 1) & 1)) return false;
         const int row = row_of(j);
-        mbar_expect_tx(&v_full[st], V_TILE);
+        mbar_expect_tx(&v_full[st], TILE);
 #pragma unroll
-        for (int c = 0; c < DV / 64; ++c) tma_load_2d(v_s + st * V_TILE + c * 8192, &vmap, &v_full[st], c * 64, row);
+        for (int c = 0; c < HD / 64; ++c) tma_load_2d(v_s + st * TILE + c * 8192, &vmap, &v_full[st], c * 64, row);
         return true;
       };
       // the scores of a page are asked for in front of the product of the page before
@@ -146,7 +151,7 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
     // ------------------------------------------------------------------ MMA issue
     if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_f16(1, 1, kTcRows, kPageTok);
-      constexpr uint32_t idesc_pv = make_idesc_f16(1, 1, kTcRows, DV) | (1u << 16);      // B (the V page) is MN-major
+      constexpr uint32_t idesc_pv = make_idesc_f16(1, 1, kTcRows, HD) | (1u << 16);      // B (the V page) is MN-major
       const uint32_t q_a = smem_u32(q_s), k_a = smem_u32(k_s), v_a = smem_u32(v_s);
       bool ok = true;
       // page j belongs to stream j % STREAMS and is that stream's page j / STREAMS
@@ -156,9 +161,9 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         if (i >= NB && !mbar_wait(&pv_done[t][b], (i / NB - 1) & 1)) return false;
         if (!mbar_wait(&k_full[st], (j / NK) & 1)) return false;
         tc_fence_after();
-        const uint32_t kb = k_a + st * K_TILE;
+        const uint32_t kb = k_a + st * TILE;
 #pragma unroll
-        for (int kk = 0; kk < DK / 16; ++kk) {
+        for (int kk = 0; kk < HD / 16; ++kk) {
           const int c = kk >> 2, off = (kk & 3) * 2;
           tc_mma_f16(tmem_base + (t * NB + b) * kPageTok, make_desc_sw128(q_a + c * (kTcRows * 128)) + off,
                      make_desc_sw128(kb + c * 8192) + off, idesc_s, kk ? 1u : 0u);
@@ -175,10 +180,10 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         ok = mbar_wait(&p_full[t][i % NB], (i / NB) & 1) && mbar_wait(&v_full[j % NV], (j / NV) & 1);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t vb = v_a + (j % NV) * V_TILE;
+        const uint32_t vb = v_a + (j % NV) * TILE;
 #pragma unroll
         for (int ks = 0; ks < kPageTok / 16; ++ks)
-          tc_mma_f16_ta(tmem_base + O_COL + t * DV, tmem_base + (t * NB + i % NB) * kPageTok + ks * 8,
+          tc_mma_f16_ta(tmem_base + O_COL + t * HD, tmem_base + (t * NB + i % NB) * kPageTok + ks * 8,
                         make_desc_sw128_mn(vb + ks * 2048, 8192u, 1024u), idesc_pv, (i | ks) ? 1u : 0u);
         tc_commit(&pv_done[t][i % NB]);
         tc_commit(&v_empty[j % NV]);
@@ -188,7 +193,7 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   } else {
     // ------------------------------------------------------------------ softmax and correction of one stream
     const uint32_t t_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t o_col = O_COL + strm * DV;
+    const uint32_t o_col = O_COL + strm * HD;
     const int n_mine = (n - strm + STREAMS - 1) / STREAMS;
     float m_ref = NEG_INF, l0 = 0.f, l1 = 0.f;
     bool ok = true;
@@ -218,7 +223,7 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         mx3 = fmaxf(mx3, sv[e + 3]);
       }
       const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;     // the scale is positive
-      const bool grow = mx > m_ref + kTcLazyLog2;
+      const bool grow = mx > (LAZY ? m_ref + kTcLazyLog2 : m_ref);
       float alpha = 1.f;
       if (grow) {
         alpha = ex2_approx(m_ref - mx);          // 0 for the first keys a row sees
@@ -232,7 +237,7 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
-        for (int c0 = 0; c0 < DV; c0 += 32) {
+        for (int c0 = 0; c0 < HD; c0 += 32) {
           uint32_t ov[32];
           tmem_ld32(t_lane + o_col + c0, ov);
           tmem_ld_wait();
@@ -248,8 +253,8 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
       uint32_t w[kPageTok / 2];
 #pragma unroll
       for (int e = 0; e < kPageTok / 2; ++e) {
-        const float p0 = ex2_approx(fmaf(sv[2 * e], p.scale_log2, neg_m));
-        const float p1 = ex2_approx(fmaf(sv[2 * e + 1], p.scale_log2, neg_m));
+        const float p0 = ex2_approx(LAZY ? fmaf(sv[2 * e], p.scale_log2, neg_m) : __fadd_rn(__fmul_rn(sv[2 * e], p.scale_log2), neg_m));
+        const float p1 = ex2_approx(LAZY ? fmaf(sv[2 * e + 1], p.scale_log2, neg_m) : __fadd_rn(__fmul_rn(sv[2 * e + 1], p.scale_log2), neg_m));
         l0 += p0;
         l1 += p1;
         w[e] = pack_bf16(p0, p1);
@@ -279,13 +284,13 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
     const float l = s_ml[0][1][r] * a0 + (two ? s_ml[STREAMS - 1][1][r] * a1 : 0.f);
     const float inv = l > 0.f ? 1.f / l : 0.f;
     const float f0 = a0 * inv, f1 = a1 * inv;
-    __nv_bfloat16* orow = p.out + (long)r_tok * p.out_stride + (long)r_head * DV;
-    const __nv_bfloat16* grow_ = p.gate ? p.gate + (long)r_tok * p.gate_stride + (long)r_head * DV : nullptr;
+    __nv_bfloat16* orow = p.out + (long)r_tok * p.out_stride + (long)r_head * HD;
+    const __nv_bfloat16* grow_ = p.gate ? p.gate + (long)r_tok * p.gate_stride + (long)r_head * HD : nullptr;
 #pragma unroll 1
-    for (int c0 = strm * (DV / STREAMS); c0 < (strm + 1) * (DV / STREAMS); c0 += 32) {
+    for (int c0 = strm * (HD / STREAMS); c0 < (strm + 1) * (HD / STREAMS); c0 += 32) {
       uint32_t ov[32], ow[32];
       tmem_ld32(t_lane + O_COL + c0, ov);
-      if (two) tmem_ld32(t_lane + O_COL + DV + c0, ow);
+      if (two) tmem_ld32(t_lane + O_COL + HD + c0, ow);
       tmem_ld_wait();
       if (n <= 0) {                                          // (nothing was accumulated: the row is zero)
 #pragma unroll
@@ -328,17 +333,17 @@ __global__ void __launch_bounds__(64 + 128 * STREAMS, 1) attn_prefill_tc_kernel(
   if (tid == 0 && s_fail && p.status) atomicExch(p.status, (int)kErrMbarTimeout);
 }
 
-template <int DK, int DV, int STREAMS, int NK, int NV>
+template <int HD, int STREAMS, int NK, int NV>
 static int launch_attn_tc(const AttnParams& p, const CUtensorMap& kmap, const CUtensorMap& vmap, int ntiles, cudaStream_t st) {
-  constexpr int smem = kTcRows * DK * 2 + NK * kPageTok * DK * 2 + NV * kPageTok * DV * 2 + 1024;
+  constexpr int smem = kTcRows * HD * 2 + NK * kPageTok * HD * 2 + NV * kPageTok * HD * 2 + 1024;
   static_assert(smem <= 225 * 1024, "shared memory budget (beside 2 KB of barriers and row sums)");
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DK, DV, STREAMS, NK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, STREAMS, NK, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  launch_pdl(attn_prefill_tc_kernel<DK, DV, STREAMS, NK, NV>, dim3(ntiles, p.nkv, 1), dim3(64 + 128 * STREAMS), smem, st, p, kmap, vmap);
+  launch_pdl(attn_prefill_tc_kernel<HD, STREAMS, NK, NV>, dim3(ntiles, p.nkv, 1), dim3(64 + 128 * STREAMS), smem, st, p, kmap, vmap);
   return (int)cudaGetLastError();
 }
 
