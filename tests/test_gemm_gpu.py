@@ -99,3 +99,19 @@ def test_gemm_w4a16_wide_cut_tiles(T, N, Kd):
     K.gemm_w4a16(p, sf, g, x, out=odd)
     assert torch.equal(odd, first)
     assert K.check_status(DEV) == 0
+
+
+@pytest.mark.parametrize("N,Kd", [(128, 128), (640, 2048), (5120, 1280), (9216, 256), (16384, 128)])
+def test_gemm_w4a16_rows_do_not_depend_on_the_rows_beside_them(N, Kd):
+    """A prompt row has the same bits in portions of any length: one-wave and many-wave launches, tiles of either shape and of every height."""
+    w = rnd(N, Kd, std=0.02, seed=27, dtype=torch.float32)
+    p, s, g = qn.quantize_nvfp4(w, search=False)
+    sf = qn.scales_blocked_k128(s)
+    x = rnd(2500, Kd, seed=28)
+    whole = K.gemm_w4a16(p, sf, g, x)
+    for T in (129, 192, 193, 256, 257, 450, 600, 953, 1500, 2048):
+        assert torch.equal(K.gemm_w4a16(p, sf, g, x[:T]), whole[:T]), T
+        assert torch.equal(K.gemm_w4a16(p, sf, g, x[2500 - T:]), whole[2500 - T:]), T
+    want = x.double() @ qn.dequantize_nvfp4(p, s, g).double().t()
+    assert float((whole.double() - want).norm() / want.norm()) < 2 ** -8
+    assert K.check_status(DEV) == 0

@@ -110,15 +110,6 @@ def call(name: str, sig: str, *args) -> None:
         raise NativeError(f"ve_{name} failed with CUDA error {rc}")
 
 
-def query(name: str, sig: str, *args) -> int:
-    """Value of the kernel library's host function ``ve_<name>`` (no launch, no stream argument)."""
-    key = "q:" + name
-    fn = _bound.get(key)
-    if fn is None:
-        fn = _bound[key] = _bind(kernels(), "ve_" + name, sig, ctypes.c_long)
-    return fn(*args)
-
-
 def hcall(name: str, sig: str, *args, restype=ctypes.c_int):
     """Call a host-library function ``vh_<name>`` (no stream argument)."""
     key = "h:" + name

@@ -10,7 +10,7 @@ import os
 import torch
 
 from .. import _lib
-from .._lib import call, ptr, query
+from .._lib import call, ptr
 from . import reference as ref
 
 PAGE = ref.PAGE
@@ -561,12 +561,10 @@ def gemm_w4a16(packed, sf_blocked, gscale, x, out=None, residual=None):
     if out is None:
         out = torch.empty(T, N, dtype=torch.bfloat16, device=x.device)
     if T > 128 and N % 128 == 0 and K % 128 == 0 and GEMM_WIDE and out.dtype == torch.bfloat16:
-        # prefill chunks: 256 x 192 tiles, weights dequantised into tensor memory (csrc/cuda/gemm_w4a16_wide.cu)
-        need = query("gemm_w4a16_wide_scratch", "iii", T, N, K)
-        scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
-        call("gemm_w4a16_wide", "ppplplpliiifpp", ptr(packed), ptr(sf_blocked), ptr(x), x.stride(0), ptr(out), out.stride(0),
+        # prefill chunks: weights dequantised into tensor memory (csrc/cuda/gemm_w4a16_wide.cu)
+        call("gemm_w4a16_wide", "ppplplpliiifp", ptr(packed), ptr(sf_blocked), ptr(x), x.stride(0), ptr(out), out.stride(0),
              ptr(residual), residual.stride(0) if residual is not None else 0, T, N, K, float(gscale),
-             ptr(status_word(x.device)), ptr(scratch))
+             ptr(status_word(x.device)))
         return out
     call("gemm_w4a16", "ppplplppliiifp", ptr(packed), ptr(sf_blocked), ptr(x), x.stride(0), ptr(out),
          out.stride(0), 0, ptr(residual), residual.stride(0) if residual is not None else 0, T, N, K,
