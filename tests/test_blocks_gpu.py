@@ -37,6 +37,21 @@ def test_gguf_matvec_edges(t, shift):
         assert _rel(lin.forward(x[:3].cuda()).cpu(), want[:3]) < 2 ** -8      # bf16 output: half a unit in the last place
 
 
+@pytest.mark.parametrize("t", TYPES)
+def test_gguf_matvec_is_as_near_as_sums_weight_by_weight(t):
+    """Distance to 64 bits over a long K against that of the same blocks at an odd address, which are summed weight by weight in fp32."""
+    N, K, far = 64, 17408, []
+    raw = gq.random_blocks(t, N, K, seed=t, amp=0.05)
+    w = gq.dequantize(raw, t, K).double().cuda()
+    x = torch.randn(16, K, generator=torch.Generator().manual_seed(t)).to(torch.bfloat16).cuda()
+    for shift in (0, 1):
+        buf = torch.zeros(raw.numel() + 64, dtype=torch.uint8, device="cuda")
+        view = buf[shift:shift + raw.numel()].view(N, -1)
+        view.copy_(raw.reshape(N, -1))
+        far.append(_rel(LinearGGUF(view, t, N, K).forward(x, out_f32=True), x.double() @ w.t()))
+    assert far[0] < 1.1 * far[1], (t, far)
+
+
 def _non_finite(K):
     """Four rows of activations: none, an infinity, an infinity of each sign in different chunks, values whose products with a block's
     integers overflow where those with its weights do not."""

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
 #pragma unroll
       for (int r = 0; r < 2 * RT; ++r)
         up[r] = st + (r * 8 + g) * C::kPitch + (int)((uintptr_t)(rp[r] + (size_t)ui * F::kUnit) & 15);
-      float blk[RT][NT][4];                               // (IQ1)
+      float blk[RT][NT][4];                               // sums of the unit
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
             frag<TYPE>(up[2 * i + 1], h + c, t, tab, fb, sb, mb);
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
-              float* ac = acc[i][j];
+              float* ac = blk[i][j];
               float d[4] = {0.f, 0.f, 0.f, 0.f};
               mma_bf16_16816(d, fa[0], fb[0], fa[1], fb[1], xv[c][j][0].x, xv[c][j][0].y);
               if (F::kScale16) {
@@ -381,6 +381,13 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
             ac[2] = fmaf(db, blk[i][j][2], ac[2]); ac[3] = fmaf(db, blk[i][j][3], ac[3]);
           }
         }
+      } else {                                            // (in two levels: one chain over all of K rounds off twice as much at K = 17408)
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][j][e] += blk[i][j][e];
       }
     }
     // warp sums -> shared memory [warp][column][row], added in warp order
