@@ -38,6 +38,49 @@ def test_gguf_matvec_edges(t, shift):
 
 
 @pytest.mark.parametrize("t", TYPES)
+def test_gguf_matvec_in_lane_order(t):
+    """Asked for it, the mat-vec gives bit for bit what the byte-by-byte kernel gives, which the same blocks at an odd address take: every
+    count of rows a launch is built for, K of less than one step of 1024 weights to several with a partial last one."""
+    big = gq.BLOCK[t][0] == 256
+    for N, K in ((1, 256), (17, 1024), (35, 2304), (16, 4608)) if big else ((1, 32), (17, 1024), (35, 1056), (16, 4448)):
+        raw = gq.random_blocks(t, N, K, seed=t + K, amp=0.05)
+        x = torch.randn(16, K, generator=torch.Generator().manual_seed(N)).to(torch.bfloat16).cuda()
+        lins = []
+        for shift in (1, 0, 2, 6):
+            buf = torch.zeros(raw.numel() + 64, dtype=torch.uint8, device="cuda")
+            view = buf[shift:shift + raw.numel()].view(N, -1)
+            view.copy_(raw.reshape(N, -1))
+            lins.append(LinearGGUF(view, t, N, K, ordered=True))
+        for M in (1, 2, 4, 5, 8, 9, 16):
+            want = lins[0].forward(x[:M], out_f32=True)
+            for lin in lins[1:]:
+                assert torch.equal(lin.forward(x[:M], out_f32=True), want), (t, N, K, M)
+            assert torch.equal(lins[1].forward(x[:M]), lins[0].forward(x[:M]))
+
+
+@pytest.mark.parametrize("spec", ["gguf_iq1_m", "gguf_q8_0+q4_k", "gguf_q2_k+q6_k", "gguf_iq3_s+iq4_xs", "gguf_q5_0+q4_1", "gguf_iq2_xxs+iq4_nl"])
+def test_gguf_experts_in_lane_order(spec):
+    """The same for routed mat-vecs, with both activations and a limit; experts elsewhere give zeros."""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank, parse_expert_quant
+    gt, dt = parse_expert_quant(spec)
+    E, I, H = 4, 256, 1536
+    bank = GGUFExpertBank.random(E, I, H, gt, dt, e0=1, seed=5, amp=0.05, device="cuda")
+
+    def odd(raw):
+        buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[1:1 + raw.numel()] = raw.reshape(-1)
+        return buf[1:1 + raw.numel()].reshape(raw.shape)
+    other = GGUFExpertBank(odd(bank.gu_raw), gt, odd(bank.dn_raw), dt, 1, I, H)
+    g = torch.Generator().manual_seed(9)
+    x = torch.randn(7, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(6, generator=g)[:3] for _ in range(7)]).to(torch.int32).cuda()
+    for act, limit in ((0, 0.0), (1, 0.0), (0, 0.5)):
+        got = bank.routes(x, ids, act, limit, ordered=True)
+        assert torch.equal(got, other.routes(x, ids, act, limit)) and got.any()
+    assert not got[((ids < 1) | (ids >= 5)).reshape(-1)].any()
+
+
+@pytest.mark.parametrize("t", TYPES)
 def test_gguf_matvec_is_as_near_as_sums_weight_by_weight(t):
     """Distance to 64 bits over a long K against that of the same blocks at an odd address, which are summed weight by weight in fp32."""
     N, K, far = 64, 17408, []

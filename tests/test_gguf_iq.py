@@ -46,6 +46,50 @@ def test_moe_model_with_gguf_experts_runs_on_cpu():
     assert float((bank.dequant("dn", 0) - dn[0]).abs().max()) < 3e-2
 
 
+@pytest.mark.parametrize("groups", [1, 2])
+def test_group_limited_routers_have_one_order_of_sums_in_front_of_them(groups):
+    """Every GGUF linear and the experts of such a model are asked for it, drawn and loaded ones; without groups none is."""
+    from volta_engine_b200.models.mla import MLAConfig, MLAModel
+    from volta_engine_b200.models.moe_loader import keep_order
+    from volta_engine_b200.ops.linear import LinearBF16, LinearGroup
+    from volta_engine_b200.ops.linear_gguf import LinearGGUF
+    cfg = MLAConfig.tiny_mla(n_group=groups, topk_group=1, quant="gguf_q8_0", expert_quant="gguf_q8_0", first_dense_layers=1, mtp_layers=0)
+    m = MLAModel(cfg, "cpu").init_random(seed=1)
+    lins = [lin for L in m.layers for lin in (L.qkv_a, L.q_b, L.o_proj, L.gate_up if L.dense_ffn else L.shared_gu)]
+    assert m.ordered == (groups > 1) and all(isinstance(lin, LinearGGUF) and lin.ordered == m.ordered for lin in lins)
+    for lin in lins:
+        lin.ordered = False
+    L = m.layers[0]
+    L.gate_up = LinearGroup([LinearGGUF(L.gate_up.raw[:512], G.GGML_Q8_0, 512, 256), LinearBF16(torch.zeros(512, 256))])
+    keep_order(m.layers)
+    assert L.q_b.ordered and L.gate_up.parts[0].ordered and m.layers[1].shared_gu.ordered
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("groups", [1, 2])
+def test_gpu_group_limited_models_ask_their_experts_for_one_order(groups):
+    """Decode rows of the model against the same model whose weights lie at odd addresses, where the byte-by-byte kernels add in that order."""
+    from volta_engine_b200.models.moe import MoEConfig, MoEModel
+    cfg = MoEConfig.tiny_moe(n_group=groups, topk_group=1, quant="gguf_q4_k", expert_quant="gguf_iq2_xs+q5_k", hidden=512, expert_ffn=256, shared_ffn=256)
+    m = MoEModel(cfg, "cuda").init_random(seed=3)
+    L = m.layers[0]
+    asked, routes = [], L.bank.routes
+    L.bank.routes = lambda *a, **kw: asked.append(kw["ordered"]) or routes(*a, **kw)
+    x = torch.randn(5, 512, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).cuda()
+    y = m.ffn_block(0, L, x, None, None)
+    assert asked == [groups > 1]
+
+    def odd(raw):
+        buf = torch.zeros(raw.numel() + 16, dtype=torch.uint8, device="cuda")
+        buf[1:1 + raw.numel()] = raw.reshape(-1)
+        return buf[1:1 + raw.numel()].reshape(raw.shape)
+    for lin in (L.shared_gu, L.shared_dn):
+        lin.raw = odd(lin.raw)
+    L.bank.gu_raw, L.bank.dn_raw = odd(L.bank.gu_raw), odd(L.bank.dn_raw)
+    if groups > 1:
+        assert torch.equal(m.ffn_block(0, L, x, None, None), y)
+
+
 @pytest.mark.parametrize("spec", ["gguf_q4_k+q6_k", "gguf_q6_k+q4_k", "gguf_q8_0+q4_1", "gguf_iq1_m+iq1_s", "gguf_q4_0+q4_0"])
 @pytest.mark.parametrize("gu_at,dn_at", [(0, 0), (2, 0), (0, 2), (2, 2), (4, 6), (1, 0), (0, 3)])
 def test_a_bank_is_decoded_in_tiles_only_where_every_block_is_readable(spec, gu_at, dn_at):

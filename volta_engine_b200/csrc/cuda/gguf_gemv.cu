@@ -3,8 +3,11 @@
 //   Q8_0, Q4_0, Q4_1, Q5_0, Q5_1, IQ4_NL (32-value blocks), Q2_K, Q3_K, Q4_K, Q5_K, Q6_K, IQ4_XS and the codebook
 //   formats IQ1_S, IQ1_M, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S (256-value super-blocks), bf16 activations, fp32
 //   accumulation.
-// Summation order of an output is fixed by K alone (chunks of 32 weights dealt to eight warps, warp sums added in order), so it does
-// not depend on M, on N or on what else is in the batch.
+// Two orders of summation, each fixed by K alone, so that a row's result does not depend on M, on N or on what else is in the batch:
+//   * gguf_mma_kernel: units of 256 weights (128 for Q8_0) dealt to eight warps, sums of a unit added up first, then a warp's units, then the
+//     warps in order. The form for every format, unless the caller asks for the other.
+//   * lane order (gguf_ordered_kernel; gguf_gemv_kernel and gguf_moe_gemv_kernel for blocks whose address the others cannot read): chunk c of 32
+//     weights belongs to lane c % 32, its products are added one after the other, chunks in turn, lanes by a butterfly.
 // Reference counterparts: src/kernels/cuda/gguf/gguf_linear.cu:38-160 (gemv on q8_1 activations) and the
 // vendored dequantize kernels; block layouts as in quant/gguf.py.
 #include "gguf_blocks.cuh"
@@ -456,17 +459,19 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
   }
 }
 
-// The mat-vecs of Q8_0 (dense) and IQ1_M (routed) in scalar fp32, in the order of gguf_gemv_kernel: chunk c of 32 weights belongs to lane
-// c % 32, its products are added one after the other, chunks in turn, lanes by a butterfly. Sums stay those of the byte-by-byte kernels bit for bit,
-// so what a router picks behind them does not depend on which of the two ran: a group-limited router at its edge picked other experts for
-// about one token in a hundred with the tensor-core sums. 7168 x 16384 Q8_0: one row 71 us, eight rows 133 us (gguf_mma_kernel 79 and 70 us);
-// IQ1_M, gate / up and down of 64 routes of 2048 x 7168: 949 us (gguf_mma_kernel 777 us). A warp takes two rows (MODE 2: a gate and an up row); steps of
-// 1024 weights of its rows and of x come through double buffers by 16-byte cp.async, x chunks 80 bytes apart (no bank conflicts).
+// The mat-vecs in scalar fp32 and in lane order, bit for bit the sums of gguf_gemv_kernel and gguf_moe_gemv_kernel, for callers that ask for it:
+// models whose router picks groups of experts first. At such a router's edge any change of rounding in front of it picks other experts, for about
+// one token in a hundred with the sums of gguf_mma_kernel, although their error against 64 bits is no larger.
+// Times (gguf_mma_kernel in brackets): 7168 x 16384 Q8_0 one row 58 us (65), eight 127 us (62); Q4_K 72 (44) and 137 us (42); gate / up and down of 64
+// routes of 2048 x 7168 IQ1_M 944 us (750), Q4_K 1217 us (870), Q8_0 965 us (1270). The byte-by-byte kernels: 174 and 999 us, 165 and 987 us; 2121,
+// 2578 and 2638 us.
+// A warp takes two rows (MODE 2: a gate and an up row); steps of 1024 weights of its rows and of x come through double buffers by 16-byte
+// cp.async, x chunks 80 bytes apart (no bank conflicts). Q8_0 and IQ1_M have decoders of whole words, the other formats go byte by byte.
 template <int TYPE, int MT>
 struct OrderedCfg {
-  static constexpr int kStepBytes = TYPE == kQ8_0 ? 32 * 34 : 4 * 56;
+  static constexpr int kStepBytes = Fmt<TYPE>::kBig ? 4 * Fmt<TYPE>::kBytes : 32 * Fmt<TYPE>::kBytes;
   static constexpr int kPitch = (kStepBytes + 15 + 15) / 16 * 16;
-  static constexpr int kTab = (Fmt<TYPE>::kTabBytes + 15) / 16 * 16;
+  static constexpr int kTab = TYPE == kIQ1_M ? (Fmt<TYPE>::kTabBytes + 15) / 16 * 16 : 0;
   static constexpr int kX = 32 * 80;                                          // a step of one row of x
   static constexpr int kSmem = kTab + 2 * MT * kX + 8 * 2 * 2 * kPitch;
 };
@@ -499,7 +504,7 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
       rp[r] = p.W + ((size_t)(here ? e : 0) * p.N + n) * p.row_bytes;
     }
     auto load_w = [&](int i) {
-      const int bytes = TYPE == kQ8_0 ? min(32, chunks - i * 32) * 34 : min(4, (chunks - i * 32) / 8) * 56;
+      const int bytes = (Fmt<TYPE>::kBig ? min(4, (chunks - i * 32) / 8) : min(32, chunks - i * 32)) * Fmt<TYPE>::kBytes;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const uint8_t* src = rp[r] + (size_t)i * C::kStepBytes;
@@ -542,7 +547,7 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             const uint8_t* b = ws + ((i & 1) * 2 + r) * C::kPitch + (int)((uintptr_t)(rp[r] + (size_t)i * C::kStepBytes) & 15);
-            if (TYPE == kQ8_0) {
+            if constexpr (TYPE == kQ8_0) {
               b += lane * 34;
               const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)b & ~(uintptr_t)3);
               const int sh = (int)((uintptr_t)b & 2) * 8;
@@ -558,7 +563,7 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
                 const uint32_t u = v[(j + 2) >> 2] ^ 0x80808080u;
                 w[r][j] = d * (__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7440u | ((j + 2) & 3))) - 8388736.f);
               }
-            } else {
+            } else if constexpr (TYPE == kIQ1_M) {
               b += (lane >> 3) * 56;
               const int c = lane & 7;
               const uint32_t qs = ld32<true>(b + c * 4), qh = ld16(b + 32 + 2 * c);
@@ -578,6 +583,8 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
                   w[r][8 * l + 2 * j + 1] = dl[l >> 1] * __uint_as_float(f[j] & 0xffff0000u);
                 }
               }
+            } else {
+              decode32<TYPE>(b, lane, w[r]);
             }
           }
 #pragma unroll
@@ -695,28 +702,24 @@ static bool block_aligned(const void* W, long row_bytes) {
 }
 
 template <int TYPE>
-static int run_gguf_gemv(GgufGemvArgs a, cudaStream_t st) {
+static int run_gguf_gemv(GgufGemvArgs a, int ordered, cudaStream_t st) {
   if (!block_aligned<TYPE>(a.W, a.row_bytes)) {          // blocks at odd addresses: byte by byte
     gguf_gemv_kernel<TYPE><<<(a.N + 7) / 8, 256, 0, st>>>(a.W, a.row_bytes, a.x, a.x_stride, a.out, a.out_stride, a.out_f32, a.M, a.N, a.K);
     VE_CHECK_LAUNCH();
   }
-  if constexpr (TYPE == kQ8_0) {
-    if (a.M == 1) return launch_gguf_ordered<TYPE, 0, 1>(a, 1, st);
-    if (a.M <= 4) return launch_gguf_ordered<TYPE, 0, 4>(a, 1, st);
-    if (a.M <= 8) return launch_gguf_ordered<TYPE, 0, 8>(a, 1, st);
-    return launch_gguf_ordered<TYPE, 0, 16>(a, 1, st);
-  } else {
+  if (ordered)
+    return a.M == 1 ? launch_gguf_ordered<TYPE, 0, 1>(a, 1, st) : a.M <= 4 ? launch_gguf_ordered<TYPE, 0, 4>(a, 1, st)
+         : a.M <= 8 ? launch_gguf_ordered<TYPE, 0, 8>(a, 1, st) : launch_gguf_ordered<TYPE, 0, 16>(a, 1, st);
   // 32 weight rows a tile where several rows of x would otherwise be read again for every 16 of a large matrix; the sums are the same
   a.tiles = (a.N + 15) / 16;
   if (a.M <= 4 || (a.M <= 8 && a.N < 32 * 148)) return launch_gguf_mma<TYPE, 0, 1, 1>(a, st);
   a.tiles = (a.N + 31) / 32;
   if (a.M <= 8) return launch_gguf_mma<TYPE, 0, 1, 2>(a, st);
   return launch_gguf_mma<TYPE, 0, 2, 2>(a, st);
-  }
 }
 
 template <int TYPE>
-static int run_gguf_moe(GgufGemvArgs a, int routes, int fuse_act, cudaStream_t st) {
+static int run_gguf_moe(GgufGemvArgs a, int routes, int fuse_act, int ordered, cudaStream_t st) {
   if (!block_aligned<TYPE>(a.W, a.row_bytes)) {
     const dim3 grid(((fuse_act ? a.N / 2 : a.N) + 3) / 4, routes);
     if (fuse_act)
@@ -727,13 +730,10 @@ static int run_gguf_moe(GgufGemvArgs a, int routes, int fuse_act, cudaStream_t s
                                                           a.out_stride, a.N, a.K, a.act, a.limit);
     VE_CHECK_LAUNCH();
   }
-  if constexpr (TYPE == kIQ1_M) {
-    return fuse_act ? launch_gguf_ordered<TYPE, 2, 1>(a, routes, st) : launch_gguf_ordered<TYPE, 1, 1>(a, routes, st);
-  } else {
+  if (ordered) return fuse_act ? launch_gguf_ordered<TYPE, 2, 1>(a, routes, st) : launch_gguf_ordered<TYPE, 1, 1>(a, routes, st);
   a.tiles_per_route = fuse_act ? (a.N / 2 + 7) / 8 : (a.N + 15) / 16;
   a.tiles = a.tiles_per_route * routes;
   return fuse_act ? launch_gguf_mma<TYPE, 2, 1, 1>(a, st) : launch_gguf_mma<TYPE, 1, 1, 1>(a, st);
-  }
 }
 
 template <int TYPE>
@@ -773,14 +773,15 @@ int ve_gguf_set_iq_grids(const void* table) {
   return 0;
 }
 
+// ordered: sums in lane order (see gguf_ordered_kernel).
 int ve_gguf_gemv(const void* W, int ggml_type, long row_bytes, const void* x, long x_stride, void* out, long out_stride,
-                 int out_is_f32, int M, int N, int K, cudaStream_t st) {
+                 int out_is_f32, int M, int N, int K, int ordered, cudaStream_t st) {
   if (M <= 0 || M > 16 || N <= 0 || K % 32) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
   if (!iq_grids_ready(ggml_type)) return cudaErrorNotReady;
   GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)N * row_bytes, (const __nv_bfloat16*)x, x_stride,
                  out_is_f32 ? nullptr : (__nv_bfloat16*)out, out_is_f32 ? (float*)out : nullptr, out_stride, M, N, K};
-#define VE_CALL(T) run_gguf_gemv<T>(a, st)
+#define VE_CALL(T) run_gguf_gemv<T>(a, ordered, st)
   VE_GGUF_TYPES(ggml_type, VE_CALL)
 #undef VE_CALL
 }
@@ -789,14 +790,14 @@ int ve_gguf_gemv(const void* W, int ggml_type, long row_bytes, const void* x, lo
 // output has N/2 columns act(gate) * up (act 0 SiLU, 1 tanh-GELU; limit > 0 clamps gate from above and up to +-limit).
 int ve_gguf_moe_gemv(const void* W, int ggml_type, long row_bytes, const void* ids, int e0, int e_local, const void* x,
                      long x_stride, int x_div, void* out, long out_stride, int routes, int N, int K, int fuse_act, int act,
-                     float limit, cudaStream_t st) {
+                     float limit, int ordered, cudaStream_t st) {
   if (routes <= 0) return 0;
   if (N <= 0 || K % 32 || x_div <= 0 || (fuse_act && N % 2)) return cudaErrorInvalidValue;
   if (ggml_type >= kQ2_K && ggml_type != kIQ4_NL && K % 256) return cudaErrorInvalidValue;
   if (!iq_grids_ready(ggml_type)) return cudaErrorNotReady;
   GgufGemvArgs a{(const uint8_t*)W, row_bytes, (const uint8_t*)W + (size_t)e_local * N * row_bytes, (const __nv_bfloat16*)x, x_stride,
                  (__nv_bfloat16*)out, nullptr, out_stride, 1, N, K, 0, (const int*)ids, e0, e_local, x_div, act, 0, limit};
-#define VE_CALL(T) run_gguf_moe<T>(a, routes, fuse_act, st)
+#define VE_CALL(T) run_gguf_moe<T>(a, routes, fuse_act, ordered, st)
   VE_GGUF_TYPES(ggml_type, VE_CALL)
 #undef VE_CALL
 }

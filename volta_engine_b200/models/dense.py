@@ -121,6 +121,17 @@ class DenseModel:
         self.lm_head = None
         self.attn_ws = None
 
+    @property
+    def ordered(self) -> bool:
+        """Whether what is computed keeps to one order of summation where kernels offer two (GGUF mat-vecs of decode rows, prompt attention of
+        256-column heads). A router that picks groups of experts first wants it: near its edge any change of rounding in front of it picks
+        other experts, for about one token in a hundred."""
+        return getattr(self.cfg, "n_group", 1) > 1
+
+    def prompt_tiles(self, b: BatchRows):
+        """The rows' attention tiles; without the wide ones where they would change the order of sums (see ``ordered``)."""
+        return b.tiles[:3] if b.tiles is not None and self.hd == 256 and self.ordered else b.tiles
+
     # ------------------------------------------------------------------------------------- weights
     def _make_linear(self, w: torch.Tensor, search: bool, whole=None):
         """``whole``: the full matrices this rank's shard ``w`` was cut from (a tensor or several). The NVFP4 tensor
@@ -138,7 +149,7 @@ class DenseModel:
             from ..quant import gguf as gq
             gtype = {"gguf_q8_0": gq.GGML_Q8_0, "gguf_q4_0": gq.GGML_Q4_0, "gguf_q4_k": gq.GGML_Q4_K,
                      "gguf_q6_k": gq.GGML_Q6_K}[self.cfg.quant]
-            return LinearGGUF.from_dense(w, gtype, act_q8=self.cfg.gemm_mode == "q8_act")
+            return LinearGGUF.from_dense(w, gtype, act_q8=self.cfg.gemm_mode == "q8_act", ordered=self.ordered)
         return LinearBF16(w.to(torch.bfloat16))
 
     def init_random(self, seed: int = 1, std: float = 0.02, search: bool = False):
@@ -499,7 +510,7 @@ class DenseModel:
             qkv = L.qkv.forward_rope(x, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.rot,
                                      self.layer_theta(li))
             att = K.attention(qkv, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.hd,
-                              self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=b.tiles,
+                              self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=self.prompt_tiles(b),
                               nsplit=1 if b.tiles is not None else b.nsplit, ws=self.attn_ws)
             return self._row_parallel(L.o_proj, att, pbuf)
         qkv = L.qkv.forward(x)
@@ -516,7 +527,7 @@ class DenseModel:
         K.rope_store(qkv, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.hd, self.rot,
                      self.layer_theta(li), cfg.rope_interleaved, mrope=mrope)
         att = K.attention(qkv, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.hd,
-                          self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=b.tiles,
+                          self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=self.prompt_tiles(b),
                           nsplit=1 if b.tiles is not None else b.nsplit, ws=self.attn_ws, tree=b.tree)
         return self._row_parallel(L.o_proj, att, pbuf)
 
@@ -534,7 +545,7 @@ class DenseModel:
         K.rope_store(qkv, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.hd, self.rot,
                      self.layer_theta(li), cfg.rope_interleaved, mrope=mrope)
         att = K.attention(qkv, b.pos, b.slot, kv.page_table, kpool, vpool, self.nq, self.nkv, self.hd,
-                          self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=b.tiles,
+                          self.scale, window=self.layer_window(li), key_end=b.key_end, tiles=self.prompt_tiles(b),
                           nsplit=1 if b.tiles is not None else b.nsplit, ws=self.attn_ws)
         hs.accumulate(li, 2, att)
         return self._row_parallel(L.o_proj, att, pbuf)

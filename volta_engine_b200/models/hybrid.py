@@ -245,7 +245,7 @@ class HybridModel(SlotStates, MoEModel):
                 a_slot = torch.where(b.slot < 0, b.slot, ar[:b.n])
                 nsplit = min(nsplit, 8)
         att = K.attention(qkv, a_pos, a_slot, a_table, a_k, a_v, self.nq, self.nkv, self.hd, self.scale,
-                          window=cfg.sliding_window, key_end=b.key_end, gate=gate, tiles=b.tiles,
+                          window=cfg.sliding_window, key_end=b.key_end, gate=gate, tiles=self.prompt_tiles(b),
                           nsplit=1 if b.tiles is not None else nsplit, ws=self.attn_ws)
         return L.o_proj.forward(att, out=pbuf)
 

@@ -298,8 +298,8 @@ class MoEModel(DenseModel):
         I = bank.inter
         tier = getattr(L, "tier", None)
         if hasattr(bank, "routes"):
-            # experts held as GGUF blocks: fused dequant mat-vec per route, or per-slab dequantise + grouped GEMM
-            d, inv = bank.routes(x, ids, act, cfg.act_limit), None
+            # experts held as GGUF blocks or trellis codes: fused mat-vec per route, or a grouped GEMM that decodes them
+            d, inv = bank.routes(x, ids, act, cfg.act_limit, ordered=self.ordered), None
         elif tier is not None or rows <= 16 or bank.gu_sf is None:
             # tiered residency: per-expert base pointers (device slot or pinned host memory) instead of the stacked bank
             stager = getattr(self, "expert_stager", None)

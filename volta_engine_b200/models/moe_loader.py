@@ -12,6 +12,7 @@ from __future__ import annotations
 import torch
 
 from ..ops.linear import LinearBF16, LinearNVFP4, fuse_linears
+from ..ops.linear_gguf import LinearGGUF
 from ..quant import nvfp4 as qn
 from .factory import TensorSource, dense_config_from_hf
 from .mla import LAT, ROPE, MLAConfig, MLAModel
@@ -215,4 +216,16 @@ def load_moe_family(hf: dict, src: TensorSource, device, comm, gemm_mode="w4a16"
         model.mtp = {"layer": block, "fc": model._make_linear(fc, True), "norm_e": src.tensor(p + "enorm.weight", dev, bf),
                      "norm_h": src.tensor(p + "hnorm.weight", dev, bf),
                      "norm_out": src.tensor(p + "shared_head.norm.weight", dev, bf), "cache_layer": cfg.n_layers}
+    if model.ordered:
+        keep_order(model.layers + ([model.mtp["layer"]] if getattr(model, "mtp", None) else []))
     return model
+
+
+def keep_order(layers) -> None:
+    """Decode rows through the layers' GGUF linears add in lane order (see ``DenseModel.ordered``)."""
+    for L in layers:
+        for name in (n for c in type(L).__mro__ for n in getattr(c, "__slots__", ())):
+            lin = getattr(L, name, None)
+            for part in getattr(lin, "parts", [lin]):
+                if isinstance(part, LinearGGUF):
+                    part.ordered = True

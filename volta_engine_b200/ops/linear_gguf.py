@@ -39,18 +39,20 @@ def ensure_iq_grids(device) -> None:
 
 
 class LinearGGUF:
-    def __init__(self, raw: torch.Tensor, ggml_type: int, out_features: int, in_features: int, act_q8: bool = False):
+    def __init__(self, raw: torch.Tensor, ggml_type: int, out_features: int, in_features: int, act_q8: bool = False,
+                 ordered: bool = False):
+        """``ordered``: decode rows add in lane order (see csrc/cuda/gguf_gemv.cu): what stands in front of a group-limited router."""
         self.raw = raw.contiguous().reshape(out_features, -1)
         self.ggml_type, self.out_features, self.in_features = ggml_type, out_features, in_features
         self.row_bytes = self.raw.shape[1]
         assert self.row_bytes == gq.row_bytes(ggml_type, in_features)
-        self.act_q8 = act_q8
+        self.act_q8, self.ordered = act_q8, ordered
         if self.raw.is_cuda and ggml_type in gq.IQ_TYPES:
             ensure_iq_grids(self.raw.device)
 
     @classmethod
-    def from_dense(cls, w: torch.Tensor, ggml_type: int, act_q8: bool = False):
-        return cls(gq.quantize(w, ggml_type), ggml_type, w.shape[0], w.shape[1], act_q8)
+    def from_dense(cls, w: torch.Tensor, ggml_type: int, act_q8: bool = False, ordered: bool = False):
+        return cls(gq.quantize(w, ggml_type), ggml_type, w.shape[0], w.shape[1], act_q8, ordered)
 
     def dequant(self) -> torch.Tensor:
         if self.raw.is_cuda and self.ggml_type in gq.IQ_TYPES:
@@ -79,9 +81,9 @@ class LinearGGUF:
             if out is None:
                 out = torch.empty(rows, self.out_features, dtype=torch.float32 if out_f32 else torch.bfloat16,
                                   device=x.device)
-            call("gguf_gemv", "pilplpliiii", ptr(self.raw), self.ggml_type, self.row_bytes, ptr(x), x.stride(0),
+            call("gguf_gemv", "pilplpliiiii", ptr(self.raw), self.ggml_type, self.row_bytes, ptr(x), x.stride(0),
                  ptr(out), out.stride(0), 1 if out.dtype == torch.float32 else 0, rows, self.out_features,
-                 self.in_features)
+                 self.in_features, 1 if self.ordered else 0)
             return out
         w = self.dequant()
         if rows <= 16 and out_f32 and residual is None:

@@ -212,7 +212,8 @@ class EXL3ExpertBank:
                 d[t * k + j] = ex.linear_reference(a, self.down[e], self.bits, s["d_suh"][e], s["d_svh"][e], self.cb).to(x.dtype)[0]
         return d
 
-    def routes(self, x: torch.Tensor, ids: torch.Tensor, act: int = 0, limit: float = 0.0) -> torch.Tensor:
+    def routes(self, x: torch.Tensor, ids: torch.Tensor, act: int = 0, limit: float = 0.0, ordered: bool = False) -> torch.Tensor:
+        """(The trellis mat-vec has one order of summation: ``ordered`` changes nothing here.)"""
         if not x.is_cuda:
             return self.routes_reference(x, ids, act, limit)
         if x.shape[0] <= 16:

@@ -85,18 +85,19 @@ class GGUFExpertBank:
         return gq.dequantize(raw[e], t, k)
 
     # ------------------------------------------------------------------------------------------ decode rows
-    def routes_decode(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float) -> torch.Tensor:
+    def routes_decode(self, x: torch.Tensor, ids: torch.Tensor, act: int, limit: float, ordered: bool = False) -> torch.Tensor:
         """x [rows, H] bf16, ids [rows, k] int32 -> d [rows * k, H]: the down projection of every route (zeros for
-        experts of other ranks)."""
+        experts of other ranks). ``ordered``: sums in lane order (see csrc/cuda/gguf_gemv.cu)."""
         rows, H = x.shape
         k = ids.shape[1]
         routes, I = rows * k, self.inter
         a = torch.empty(routes, I, dtype=x.dtype, device=x.device)
-        call("gguf_moe_gemv", "pilpiiplipliiiiif", ptr(self.gu_raw), self.gu_type, self.gu_raw.shape[2], ptr(ids), self.e0,
-             self.e_local, ptr(x), x.stride(0), k, ptr(a), a.stride(0), routes, 2 * I, H, 1, act, float(limit))
+        call("gguf_moe_gemv", "pilpiiplipliiiiifi", ptr(self.gu_raw), self.gu_type, self.gu_raw.shape[2], ptr(ids), self.e0,
+             self.e_local, ptr(x), x.stride(0), k, ptr(a), a.stride(0), routes, 2 * I, H, 1, act, float(limit),
+             1 if ordered else 0)
         d = torch.empty(routes, H, dtype=x.dtype, device=x.device)
-        call("gguf_moe_gemv", "pilpiiplipliiiiif", ptr(self.dn_raw), self.dn_type, self.dn_raw.shape[2], ptr(ids), self.e0,
-             self.e_local, ptr(a), a.stride(0), 1, ptr(d), d.stride(0), routes, H, I, 0, act, 0.0)
+        call("gguf_moe_gemv", "pilpiiplipliiiiifi", ptr(self.dn_raw), self.dn_type, self.dn_raw.shape[2], ptr(ids), self.e0,
+             self.e_local, ptr(a), a.stride(0), 1, ptr(d), d.stride(0), routes, H, I, 0, act, 0.0, 1 if ordered else 0)
         return d
 
     # ------------------------------------------------------------------------------------------ prefill chunks
@@ -194,11 +195,11 @@ class GGUFExpertBank:
                 d[t * k + j] = (a.float() @ self.dequant("dn", e).t()).to(x.dtype)[0]
         return d
 
-    def routes(self, x: torch.Tensor, ids: torch.Tensor, act: int = 0, limit: float = 0.0) -> torch.Tensor:
+    def routes(self, x: torch.Tensor, ids: torch.Tensor, act: int = 0, limit: float = 0.0, ordered: bool = False) -> torch.Tensor:
         if not x.is_cuda:
             return self.routes_reference(x, ids, act, limit)
         if self.gu_type in gq.IQ_TYPES or self.dn_type in gq.IQ_TYPES:
             ensure_iq_grids(x.device)             # (a bank moved to the device after it was built has not done this yet)
         if x.shape[0] <= 16:
-            return self.routes_decode(x, ids, act, limit)
+            return self.routes_decode(x, ids, act, limit, ordered)
         return self.routes_prefill(x, ids, act, limit)
