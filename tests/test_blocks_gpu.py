@@ -268,3 +268,26 @@ def test_exl3_matvec_units_and_groups(bits):
                 w = exl3_reconstruct(codes[int(e[gi]) * n:(int(e[gi]) + 1) * n].clone(), K, N, bits, 2)
                 want = x[gi * M:(gi + 1) * M].double() @ w.double().t()
                 assert _rel(got, want) < 2 ** -8, (bits, K, N, gi)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices")
+def test_kernels_of_much_shared_memory_run_on_every_device():
+    """What a kernel is allowed belongs to a device: one process may use a second one after the first."""
+    from volta_engine_b200._lib import call, ptr
+    from volta_engine_b200.ops.linear_exl3 import exl3_gemv
+    out = []
+    for dev in (0, 1, 0):
+        with torch.cuda.device(dev):
+            g = torch.Generator().manual_seed(1)
+            x = torch.randn(9, 512, generator=g).to(torch.bfloat16).cuda()
+            raw = gq.random_blocks(12, 64, 512, seed=1, amp=0.05).cuda()
+            ys = [LinearGGUF(raw, 12, 64, 512, ordered=o).forward(x) for o in (False, True)]
+            codes = torch.randint(-32768, 32768, (32 * 8 * 64,), generator=g, dtype=torch.int32).to(torch.int16).cuda()
+            e = torch.zeros(60, dtype=torch.int32, device="cuda")
+            ys.append(exl3_gemv(codes, torch.randn(60, 512, generator=g).half().cuda(), 1, 512, 128, 4, 2, expert=e, expert_stride=codes.numel(), groups=60))
+            o, w = torch.randn(3, 2, 512, generator=g).to(torch.bfloat16).cuda(), torch.randn(2, 64, 512, generator=g).to(torch.bfloat16).cuda()
+            y = torch.empty(3, 128, dtype=torch.bfloat16, device="cuda")
+            call("mla_expand_out", "pppliii", ptr(o), ptr(w), ptr(y), y.stride(0), 3, 2, 64)
+            out.append([t.cpu() for t in ys + [y]])
+    for other in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(out[0], other))

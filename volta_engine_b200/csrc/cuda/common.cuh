@@ -1,6 +1,7 @@
 // Shared device helpers for the sm_100a kernels: warp/block reductions, mbarrier, TMA (no cluster
 // multicast anywhere), tcgen05 (alloc / mma / commit / ld), and bounded spin-waits.
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -124,6 +125,20 @@ static inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.attrs = at;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Dynamic shared memory of a kernel beyond 48 KB: the attribute belongs to the device, so it is set once on each that launches the kernel.
+template <auto KERNEL>
+static inline cudaError_t allow_smem(int bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 
 VE_DEVINL uint64_t globaltimer_ns() {

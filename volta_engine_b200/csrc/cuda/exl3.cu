@@ -374,17 +374,15 @@ using namespace ve;
 template <int BITS, int CB, int MH, int UT>
 static int exl3_gemv_blocks(int* blocks) {                           // blocks that are resident at once, found on the first call
   static int ctas = 0;
+  constexpr int smem = Exl3Gemv<BITS, MH>::kSmem;
+  const cudaError_t e = allow_smem<exl3_gemv_kernel<BITS, CB, MH, UT>>(smem);
+  if (e != cudaSuccess) return (int)e;
   if (!ctas) {
-    int per_sm = 0, dev = 0, sms = 148;
-    constexpr int smem = Exl3Gemv<BITS, MH>::kSmem;
-    const cudaError_t e = cudaFuncSetAttribute(exl3_gemv_kernel<BITS, CB, MH, UT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exl3_gemv_kernel<BITS, CB, MH, UT>, kExl3Warps * 32, smem) != cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
-    ctas = per_sm * sms;
+    ctas = per_sm * 148;
   }
   *blocks = ctas;
   return 0;

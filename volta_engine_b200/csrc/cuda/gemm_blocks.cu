@@ -271,12 +271,8 @@ __global__ void __launch_bounds__(64 + 32 * kBgWarps, 2) gemm_blocks_kernel(cons
 
 template <class D>
 static int launch_blocks(const BlockGemmParams& p, const CUtensorMap& bmap, int n_tiles, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_blocks_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, BgCfg<D>::kSmem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  const cudaError_t e = allow_smem<gemm_blocks_kernel<D>>(BgCfg<D>::kSmem);
+  if (e != cudaSuccess) return (int)e;
   gemm_blocks_kernel<D><<<dim3((p.N + 127) / 128, n_tiles), 64 + 32 * kBgWarps, BgCfg<D>::kSmem, st>>>(p, bmap);
   return (int)cudaGetLastError();
 }

@@ -665,9 +665,10 @@ static int launch_gguf_mma(GgufGemvArgs a, cudaStream_t st) {
   static_assert(C::kSmem <= 200 * 1024, "shared memory of an SM");
   static int per_sm = 0;                                 // resident blocks an SM, found once (the same on every B200)
   int n = per_sm;
+  const cudaError_t a_rc = allow_smem<gguf_mma_kernel<TYPE, MODE, NT, RT>>(C::kSmem);
+  if (a_rc != cudaSuccess) return (int)a_rc;
   if (n == 0) {
-    cudaError_t e = cudaFuncSetAttribute(gguf_mma_kernel<TYPE, MODE, NT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gguf_mma_kernel<TYPE, MODE, NT, RT>, 256, C::kSmem);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gguf_mma_kernel<TYPE, MODE, NT, RT>, 256, C::kSmem);
     if (e != cudaSuccess) return (int)e;
     if (n < 1) n = 1;
     per_sm = n;
@@ -680,12 +681,8 @@ static int launch_gguf_mma(GgufGemvArgs a, cudaStream_t st) {
 template <int TYPE, int MODE, int MT>
 static int launch_gguf_ordered(const GgufGemvArgs& a, int routes, cudaStream_t st) {
   constexpr int smem = OrderedCfg<TYPE, MT>::kSmem;
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(gguf_ordered_kernel<TYPE, MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  const cudaError_t e = allow_smem<gguf_ordered_kernel<TYPE, MODE, MT>>(smem);
+  if (e != cudaSuccess) return (int)e;
   const int per = MODE == 2 ? 8 : 16, n = MODE == 2 ? a.N / 2 : a.N;
   // routed: up to eight tiles a block, so that the codebook is laid out once for them, as long as every SM keeps eight blocks
   const int tiles = (n + per - 1) / per;

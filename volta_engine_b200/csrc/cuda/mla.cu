@@ -434,12 +434,8 @@ int ve_mla_expand_out(const void* o_lat, const void* w_uv, void* out, long out_s
   if (rows <= 0) return 0;
   if (vdim > 256) return cudaErrorInvalidValue;
   constexpr int smem = 32 * 1040 + 8 * kLat * 4;
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(mla_expand_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  const cudaError_t e = allow_smem<mla_expand_out_kernel>(smem);
+  if (e != cudaSuccess) return (int)e;
   dim3 grid((vdim + 31) / 32, heads, (rows + 7) / 8);
   mla_expand_out_kernel<<<grid, 128, smem, st>>>((const __nv_bfloat16*)o_lat, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, out_stride, rows,
                                               heads, vdim);
