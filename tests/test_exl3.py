@@ -269,3 +269,21 @@ def test_gpu_quantize_whole_matrix_with_the_device_encoder():
     eff = ex.effective_weight(codes.cpu(), 4, suh.cpu(), svh.cpu())
     rel = float((eff - W).norm() / W.norm())
     assert rel < 0.12, rel                                         # 4 bits per weight: about 7-9 % relative error
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [2, 3, 4, 6, 8])
+@pytest.mark.parametrize("K,N,M", [(256, 128, 1), (1040, 176, 3), (2048, 64, 16)])
+def test_gpu_matvec_of_few_and_of_many_groups_gives_the_same_bits(bits, K, N, M):
+    """Groups on both sides of the rule that picks the kernel."""
+    from volta_engine_b200.ops.linear_exl3 import exl3_gemv
+    g = torch.Generator().manual_seed(bits + K)
+    E, n = 3, (K // 16) * (N // 16) * 16 * bits
+    codes = torch.randint(-32768, 32767, (E * n,), generator=g, dtype=torch.int32).to(torch.int16).cuda()
+    x = torch.randn(64 * M, K, generator=g).half().cuda()
+    e = torch.randint(-1, E, (64,), generator=g, dtype=torch.int32).cuda()
+    whole = exl3_gemv(codes, x, M, K, N, bits, 2, out=torch.full((64 * M, N), 7.0, device="cuda"), expert=e, expert_stride=n, groups=64)
+    for groups in (1, 7, 47, 48):
+        part = exl3_gemv(codes, x[:groups * M], M, K, N, bits, 2, out=torch.full((groups * M, N), 7.0, device="cuda"), expert=e[:groups].contiguous(),
+                         expert_stride=n, groups=groups)
+        assert torch.equal(part, whole[:groups * M]), groups

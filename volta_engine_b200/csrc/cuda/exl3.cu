@@ -25,7 +25,121 @@ VE_DEVINL void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
 
 constexpr int kExl3Warps = 8;
 
+// Few groups (a dense matrix, the routes of a few rows): see exl3_gemv_launch.
 // x: fp16 [groups][M][K] rotated activations (read through L1: at most 16 x K halves, re-used by every warp);
+// y: fp32 [groups][M][N]; group = blockIdx.y, its weights start at codes + expert[group] * expert_stride
+// (expert == nullptr: one shared matrix). The column tiles of a group are split evenly over gridDim.x CTAs (the host
+// sizes the grid to the number of CTAs that are resident at once, so every CTA gets the same work to within one tile
+// and there is no partial last wave); a CTA walks its range in units of 4, 2 or 1 adjacent column tiles. In a unit every
+// warp walks its share of K and reads NTW * 32 * BITS contiguous bytes per k-tile.
+template <int BITS, int CB, int MH, int NTW>   // MH: 8 or 16 activation rows held by the A fragment
+VE_DEVINL void exl3_gemv_unit(const uint32_t* __restrict__ base, size_t tstride, const __half* __restrict__ xlo,
+                              const __half* __restrict__ xhi, bool row_lo, bool row_hi, float* __restrict__ y, float* red,
+                              int M, int KT, int N, int nt0) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int per = (KT + kExl3Warps - 1) / kExl3Warps;
+  const int kt0 = warp * per, kt1 = min(KT, kt0 + per);
+  const Exl3Lane<BITS> L(lane);
+  constexpr int NW = Exl3Lane<BITS>::NW;
+  base += (size_t)nt0 * (8 * BITS);
+  float acc[NTW][2][4];
+#pragma unroll
+  for (int j = 0; j < NTW; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[j][h][i] = 0.f;
+  constexpr int UK = (NW == 2 ? 4 : 2) / NTW > 0 ? (NW == 2 ? 4 : 2) / NTW : 1;   // k-tiles per step of a warp
+  // Two register buffers: the words of step i + 1 are requested before step i is decoded, so a warp's memory latency
+  // overlaps its own arithmetic (the warps of a CTA run in lock-step and would otherwise all wait at the same time).
+  uint32_t wn[UK][NTW][NW], an[UK][4];
+  auto fetch = [&](int kt) {
+#pragma unroll
+    for (int u = 0; u < UK; ++u) {
+      const int k = min(kt + u, kt1 - 1);                           // tail: re-read the last tile, its math is skipped
+#pragma unroll
+      for (int j = 0; j < NTW; ++j) L.load(base + (size_t)k * tstride + j * (8 * BITS), wn[u][j]);
+      const int ko = k * 16;                                        // the A fragment of the same k-tile (L1 resident)
+      an[u][0] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko)) : 0u;
+      an[u][2] = row_lo ? __ldg(reinterpret_cast<const uint32_t*>(xlo + ko + 8)) : 0u;
+      an[u][1] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko)) : 0u;
+      an[u][3] = row_hi ? __ldg(reinterpret_cast<const uint32_t*>(xhi + ko + 8)) : 0u;
+    }
+  };
+  if (kt0 < kt1) fetch(kt0);
+  for (int kt = kt0; kt < kt1; kt += UK) {
+    uint32_t w[UK][NTW][NW], a[UK][4];
+#pragma unroll
+    for (int u = 0; u < UK; ++u) {
+#pragma unroll
+      for (int j = 0; j < NTW; ++j)
+#pragma unroll
+        for (int i = 0; i < NW; ++i) w[u][j][i] = wn[u][j][i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[u][i] = an[u][i];
+    }
+    if (kt + UK < kt1) fetch(kt + UK);
+#pragma unroll
+    for (int u = 0; u < UK; ++u) {
+      if (kt + u < kt1) {
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) {
+          uint32_t f[4];
+          L.template decode<CB>(w[u][j], f);
+          mma_f16(acc[j][0], a[u], f[0], f[1]);
+          mma_f16(acc[j][1], a[u], f[2], f[3]);
+        }
+      }
+    }
+  }
+  // C fragment: c[0],c[1] -> row g, cols 2t,2t+1; c[2],c[3] -> row g+8.
+  constexpr int W = 16 * NTW;
+  __syncthreads();                                                  // the previous unit's sums have been read
+  float* r = red + warp * 16 * W;
+#pragma unroll
+  for (int j = 0; j < NTW; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = j * 16 + h * 8 + 2 * t;
+      r[g * W + c] = acc[j][h][0]; r[g * W + c + 1] = acc[j][h][1];
+      r[(g + 8) * W + c] = acc[j][h][2]; r[(g + 8) * W + c + 1] = acc[j][h][3];
+    }
+  __syncthreads();
+  for (int i = tid; i < M * W; i += blockDim.x) {
+    const int m = i / W, n = i % W;
+    float s = 0.f;
+#pragma unroll
+    for (int wv = 0; wv < kExl3Warps; ++wv) s += red[wv * 16 * W + m * W + n];
+    y[(size_t)m * N + nt0 * 16 + n] = s;
+  }
+}
+
+template <int BITS, int CB, int MH>
+__global__ void __launch_bounds__(kExl3Warps * 32, 2)
+exl3_gemv_few_kernel(const uint16_t* __restrict__ codes, const __half* __restrict__ x, float* __restrict__ y,
+                 int M, int K, int N, const int* __restrict__ expert, long expert_stride) {
+  __shared__ float red[kExl3Warps * 256 * 4];                       // [warps][16 rows][16 * NTW cols], NTW <= 4
+  const int grp = blockIdx.y;
+  if (expert) { const int e = expert[grp]; if (e < 0) return; codes += (size_t)e * expert_stride; }
+  x += (size_t)grp * M * K; y += (size_t)grp * M * N;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const bool row_lo = g < M, row_hi = MH == 16 && g + 8 < M;
+  const __half* xlo = x + (size_t)(row_lo ? g : 0) * K + 2 * t;
+  const __half* xhi = x + (size_t)(row_hi ? g + 8 : 0) * K + 2 * t;
+  const int KT = K >> 4, NT = N >> 4;
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(codes);
+  const size_t tstride = (size_t)NT * (8 * BITS);
+  int nt = (int)((long)NT * blockIdx.x / gridDim.x);
+  const int nt_end = (int)((long)NT * (blockIdx.x + 1) / gridDim.x);
+  while (nt < nt_end) {
+    const int left = nt_end - nt;
+    if (left >= 4) { exl3_gemv_unit<BITS, CB, MH, 4>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 4; }
+    else if (left >= 2) { exl3_gemv_unit<BITS, CB, MH, 2>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 2; }
+    else { exl3_gemv_unit<BITS, CB, MH, 1>(base, tstride, xlo, xhi, row_lo, row_hi, y, red, M, KT, N, nt); nt += 1; }
+  }
+}
+
+// Many groups. x: fp16 [groups][M][K] rotated activations (read through L1: at most 16 x K halves, re-used by every warp);
 // y: fp32 [groups][M][N]; the weights of a group start at codes + expert[group] * expert_stride (expert == nullptr: one shared matrix; a
 // negative expert: nothing is written).
 //
@@ -409,9 +523,34 @@ static int exl3_gemv_run(const void* codes, const void* x, void* y, int M, int K
   VE_CHECK_LAUNCH();
 }
 
+template <int BITS, int CB, int MH>
+static int exl3_gemv_few(const void* codes, const void* x, void* y, int M, int K, int N, const int* expert, long stride, int groups,
+                         cudaStream_t st) {
+  static int ctas = 0;                                             // blocks that are resident at once
+  if (!ctas) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, exl3_gemv_few_kernel<BITS, CB, MH>, kExl3Warps * 32, 0) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    ctas = per_sm * 148;
+  }
+  const int gx = max(1, min(N / 16, ctas / groups));
+  exl3_gemv_few_kernel<BITS, CB, MH><<<dim3(gx, groups), kExl3Warps * 32, 0, st>>>((const uint16_t*)codes, (const __half*)x, (float*)y, M, K, N,
+                                                                                    expert, stride);
+  VE_CHECK_LAUNCH();
+}
+
+// Both kernels add in the same order and give the same bits. A group of blocks for each group of routes has the shorter path from memory to
+// the tensor core and is faster as long as the resident blocks divide among the groups: 5120 x 5120 at 4 bits 18 us (ring 22), 5120 x 34816 61 us
+// (69), ten routes of 2048 x 512 7.8 us (11.0), 32 of 4096 x 1408 at 3 bits 63 us (84). With many groups most of its blocks have no second column
+// tile to take or none at all: 80 routes of 4096 x 1408 195 us (166), 160 of 2048 x 512 100 us (68). At 40 routes the two are level.
+constexpr int kExl3FewGroups = 48;
+
 template <int BITS, int CB>
 static int exl3_gemv_launch(const void* codes, const void* x, void* y, int M, int K, int N, const int* expert,
                             long stride, int groups, cudaStream_t st) {
+  if (groups < kExl3FewGroups)
+    return M <= 8 ? exl3_gemv_few<BITS, CB, 8>(codes, x, y, M, K, N, expert, stride, groups, st)
+                  : exl3_gemv_few<BITS, CB, 16>(codes, x, y, M, K, N, expert, stride, groups, st);
   return M <= 8 ? exl3_gemv_run<BITS, CB, 8>(codes, x, y, M, K, N, expert, stride, groups, st)
                 : exl3_gemv_run<BITS, CB, 16>(codes, x, y, M, K, N, expert, stride, groups, st);
 }
