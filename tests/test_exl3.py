@@ -287,3 +287,24 @@ def test_gpu_matvec_of_few_and_of_many_groups_gives_the_same_bits(bits, K, N, M)
         part = exl3_gemv(codes, x[:groups * M], M, K, N, bits, 2, out=torch.full((groups * M, N), 7.0, device="cuda"), expert=e[:groups].contiguous(),
                          expert_stride=n, groups=groups)
         assert torch.equal(part, whole[:groups * M]), groups
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("C", [128, 384, 5120])
+@pytest.mark.parametrize("post", [False, True])
+def test_gpu_rotation_of_few_and_of_many_rows_gives_the_same_bits(C, post):
+    """Rows on both sides of the rule that picks the values of a lane; types, a second operand with the activation, experts with none among them."""
+    from volta_engine_b200.ops.linear_exl3 import had128
+    rows = 148 * 32 // (C // 128) + 5
+    g = torch.Generator().manual_seed(C)
+    x, x2 = (torch.randn(rows, C, generator=g).cuda() for _ in range(2))
+    s, s2 = (torch.randn(3, C, generator=g).half().cuda() for _ in range(2))
+    e = torch.randint(-1, 3, (rows,), generator=g, dtype=torch.int32).cuda()
+    for cast, out in ((torch.bfloat16, torch.float16), (torch.float32, torch.bfloat16), (torch.float32, torch.float32), (torch.float16, torch.float16)):
+        xs = x.to(cast)
+        whole = had128(xs, s, post=post, out_dtype=out, expert=e, scale_stride=C)
+        for k in (1, 9, rows // 2):
+            assert torch.equal(had128(xs[:k], s, post=post, out_dtype=out, expert=e[:k].contiguous(), scale_stride=C), whole[:k]), (cast, k)
+        assert not whole[e < 0].any()
+    both = had128(x, s, post=True, out_dtype=torch.float16, x2=x2, scale2=s2, act=0, expert=e, scale_stride=C)
+    assert torch.equal(had128(x[:9], s, post=True, out_dtype=torch.float16, x2=x2[:9], scale2=s2, act=0, expert=e[:9].contiguous(), scale_stride=C), both[:9])

@@ -356,30 +356,40 @@ template <int DT> VE_DEVINL void had_store16(void* p, size_t i, bool vec, const 
   }
 }
 
-// 128-point Walsh-Hadamard transform (natural order, scaled by 1/sqrt(128)) over eight lanes of 16 consecutive values each: strides
-// 1 to 8 inside the lane, 16 to 64 by shuffles, in rising order.
+template <int DT, int V> VE_DEVINL void had_load(const void* p, size_t i, bool vec, float* v) {
+  if (V == 16) had_load16<DT>(p, i, vec, v);
+  else had_load4<DT>(p, i, v);
+}
+template <int DT, int V> VE_DEVINL void had_store(void* p, size_t i, bool vec, const float* v) {
+  if (V == 16) had_store16<DT>(p, i, vec, v);
+  else had_store4<DT>(p, i, v);
+}
+
+// 128-point Walsh-Hadamard transform (natural order, scaled by 1/sqrt(128)) over 128 / V lanes of V consecutive values each: strides
+// below V inside the lane, the others by shuffles, in rising order.
+template <int V>
 VE_DEVINL void wht128(float* v, int lane) {
 #pragma unroll
-  for (int m = 1; m < 16; m <<= 1)
+  for (int m = 1; m < V; m <<= 1)
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
+    for (int j = 0; j < V; ++j)
       if (!(j & m)) {
         const float a = v[j], b = v[j | m];
         v[j] = a + b;
         v[j | m] = a - b;
       }
 #pragma unroll
-  for (int m = 1; m < 8; m <<= 1) {
+  for (int m = 1; m < 128 / V; m <<= 1) {
     const bool up = lane & m;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < V; ++j) {
       const float o = __shfl_xor_sync(0xffffffffu, v[j], m);
       v[j] = up ? o - v[j] : v[j] + o;
     }
   }
   const float s = 0.08838834764831845f;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] *= s;
+  for (int j = 0; j < V; ++j) v[j] *= s;
 }
 
 struct HadArgs {
@@ -396,20 +406,22 @@ VE_DEVINL float act_apply(float x, int act) {
   return x / (1.f + __expf(-x));
 }
 
-// Eight lanes per 128-block. post == 0: out = had(in * scale); post == 1: out = had(in) * scale; with in2:
+// 128 / V lanes per 128-block. post == 0: out = had(in * scale); post == 1: out = had(in) * scale; with in2:
 // out = act(had(in) * scale) * (had(in2) * scale2).
-// Bound by the rows read and written; with four values a lane the transform took 20 shuffles a block, and they took the time (52 us for the
-// average rotation of 20480 rows of 2048 or 512 columns): 16 values a lane take 12, and the same sums in the same order.
-template <int DI, int DO>
+// Many rows are bound by what is read and written, and by the shuffles: four values a lane take 20 a block, 16 values 12, for the same sums in
+// the same order (2000 rows of 2048 columns 9.1 to 6.9 us, of 5120 18.6 to 13.8 us). A few rows are bound by latency, which four values a
+// lane keep shorter (1 to 16 rows of 2048 columns 1.9 us against 2.5 us, 160 rows 2.5 against 2.9 us).
+template <int DI, int DO, int V>
 __global__ void __launch_bounds__(256) had128_kernel(HadArgs a) {
   const int lane = threadIdx.x & 31;
   const int nb = a.C >> 7;
   const long total = (long)a.rows * nb;
-  for (long b0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; b0 < total; b0 += (long)gridDim.x * 32) {
-    const long blk = b0 + (lane >> 3);
+  constexpr int LANES = 128 / V, PER = 32 / LANES;          // of a block; blocks of a warp
+  for (long b0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * PER; b0 < total; b0 += (long)gridDim.x * 8 * PER) {
+    const long blk = b0 + lane / LANES;
     const bool in = blk < total;                          // (every lane takes part in the shuffles)
     const int row = in ? (int)(blk / nb) : 0, cb = in ? (int)(blk % nb) : 0;
-    const int col = cb * 128 + (lane & 7) * 16;
+    const int col = cb * 128 + (lane % LANES) * V;
     long soff = col;
     int e = 0;
     if (a.expert) {
@@ -417,41 +429,41 @@ __global__ void __launch_bounds__(256) had128_kernel(HadArgs a) {
       if (e > 0) soff += (long)e * a.scale_stride;
     }
     const bool live = in && e >= 0;
-    float s[16], v[16];
+    float s[V], v[V];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) { s[j] = 1.f; v[j] = 0.f; }
+    for (int j = 0; j < V; ++j) { s[j] = 1.f; v[j] = 0.f; }
     size_t in_row = 0;
     if (live) {
       in_row = (size_t)((a.src ? a.src[row] : row) / a.in_div) * a.C;
-      if (a.scale) had_load16<2>(a.scale, soff, a.vec, s);
-      had_load16<DI>(a.in, in_row + col, a.vec, v);
+      if (a.scale) had_load<2, V>(a.scale, soff, a.vec, s);
+      had_load<DI, V>(a.in, in_row + col, a.vec, v);
     }
     if (!a.post) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] *= s[j];
+      for (int j = 0; j < V; ++j) v[j] *= s[j];
     }
-    wht128(v, lane);
+    wht128<V>(v, lane);
     if (a.post) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] *= s[j];
+      for (int j = 0; j < V; ++j) v[j] *= s[j];
     }
     if (a.in2) {
-      float u[16];
+      float u[V];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) { s[j] = 1.f; u[j] = 0.f; }
+      for (int j = 0; j < V; ++j) { s[j] = 1.f; u[j] = 0.f; }
       if (live) {
-        if (a.scale2) had_load16<2>(a.scale2, soff, a.vec, s);
-        had_load16<DI>(a.in2, in_row + col, a.vec, u);
+        if (a.scale2) had_load<2, V>(a.scale2, soff, a.vec, s);
+        had_load<DI, V>(a.in2, in_row + col, a.vec, u);
       }
-      wht128(u, lane);
+      wht128<V>(u, lane);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = act_apply(v[j], a.act) * (u[j] * s[j]);
+      for (int j = 0; j < V; ++j) v[j] = act_apply(v[j], a.act) * (u[j] * s[j]);
     }
     if (in && e < 0) {                                    // another rank's route: zeros (rows behind the sorted routes stay unwritten)
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = 0.f;
+      for (int j = 0; j < V; ++j) v[j] = 0.f;
     }
-    if (live || (in && !a.src)) had_store16<DO>(a.out, (size_t)row * a.C + col, a.vec, v);
+    if (live || (in && !a.src)) had_store<DO, V>(a.out, (size_t)row * a.C + col, a.vec, v);
   }
 }
 
@@ -615,15 +627,23 @@ int ve_had128(const void* in, const void* in2, void* out, const void* scale, con
   HadArgs a{in, in2, out, (const __half*)scale, (const __half*)scale2, (const int*)expert, scale_stride,
             (const int*)src, rows, C, post, in_div, rows_per_group, act};
   a.vec = !(((uintptr_t)in | (uintptr_t)in2 | (uintptr_t)out | (uintptr_t)scale | (uintptr_t)scale2) & 15) && scale_stride % 8 == 0;
-  const long blocks_needed = ((long)rows * (C / 128) + 31) / 32;
-  const int blocks = (int)(blocks_needed < 148 * 8 ? blocks_needed : 148 * 8);
-  if (dt_in == 0 && dt_out == 2) had128_kernel<0, 2><<<blocks, 256, 0, st>>>(a);
-  else if (dt_in == 1 && dt_out == 0) had128_kernel<1, 0><<<blocks, 256, 0, st>>>(a);
-  else if (dt_in == 1 && dt_out == 2) had128_kernel<1, 2><<<blocks, 256, 0, st>>>(a);
-  else if (dt_in == 2 && dt_out == 2) had128_kernel<2, 2><<<blocks, 256, 0, st>>>(a);
-  else if (dt_in == 0 && dt_out == 0) had128_kernel<0, 0><<<blocks, 256, 0, st>>>(a);
-  else if (dt_in == 1 && dt_out == 1) had128_kernel<1, 1><<<blocks, 256, 0, st>>>(a);
+  const long n = (long)rows * (C / 128);
+  // 16 values a lane once they still give every SM 32 blocks of 128 (at 4700 the two are level)
+  const int per = n < 148 * 32 ? 8 : 32;                            // blocks of 128 a thread block
+  const int blocks = (int)((n + per - 1) / per < 148 * 8 ? (n + per - 1) / per : 148 * 8);
+#define VE_HAD(DI, DO)                                                         \
+  do {                                                                          \
+    if (per == 8) had128_kernel<DI, DO, 4><<<blocks, 256, 0, st>>>(a);        \
+    else had128_kernel<DI, DO, 16><<<blocks, 256, 0, st>>>(a);                \
+  } while (0)
+  if (dt_in == 0 && dt_out == 2) VE_HAD(0, 2);
+  else if (dt_in == 1 && dt_out == 0) VE_HAD(1, 0);
+  else if (dt_in == 1 && dt_out == 1) VE_HAD(1, 1);
+  else if (dt_in == 1 && dt_out == 2) VE_HAD(1, 2);
+  else if (dt_in == 2 && dt_out == 2) VE_HAD(2, 2);
+  else if (dt_in == 0 && dt_out == 0) VE_HAD(0, 0);
   else return cudaErrorInvalidValue;
+#undef VE_HAD
   VE_CHECK_LAUNCH();
 }
 
