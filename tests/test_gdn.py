@@ -93,6 +93,48 @@ def test_gpu_gdn_row_blocks_columns_and_taps(dims, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(16, 48, 128, 128, 4), (16, 48, 128, 128, 3), (14, 14, 64, 256, 4), (4, 12, 128, 128, 4), (2, 2, 64, 64, 9)])
+@pytest.mark.parametrize("n", [1, 33, 100, 300, 1030])
+def test_gpu_gdn_prepare_forms(dims, n):
+    """The convolution, norms and gates in each of their forms (a block a row, a warp a row, 16 rows a warp) against 64 bits: sequences that
+    begin inside the batch, end of one and start of another, padding rows, rows that continue a stored convolution."""
+    from volta_engine_b200._lib import call, ptr
+    d = GDNDims(*dims)
+    nk, nv, dk, dv, kc = dims
+    g = torch.Generator().manual_seed(n)
+    P = _params(d, g)
+    cut = n // 3
+    slot = torch.tensor([1] * cut + [-1] * min(3, n - cut - 1) + [0] * (n - cut - min(3, n - cut - 1)), dtype=torch.int32)
+    pos = torch.tensor([20 + i for i in range(cut)] + [0] * min(3, n - cut - 1) + list(range(n - cut - min(3, n - cut - 1))), dtype=torch.int32)
+    proj = torch.randn(n, d.proj_out, generator=g).to(torch.bfloat16)
+    conv = torch.randn(2, kc - 1, d.conv_dim, generator=g)
+    u, gb = torch.zeros(n, d.conv_dim, device="cuda"), torch.zeros(n, 2 * nv, device="cuda")
+    Pg = {k: v.float().cuda().contiguous() for k, v in P.items()}
+    pg, po, sl, cg = proj.cuda(), pos.cuda(), slot.cuda(), conv.cuda()
+    call("gdn_prepare", "plpppppppp" + "iiiiiii", ptr(pg), pg.stride(0), ptr(po), ptr(sl), ptr(cg), ptr(Pg["conv_w"]), ptr(Pg["A_log"]),
+         ptr(Pg["dt_bias"]), ptr(u), ptr(gb), n, nk, nv, dk, dv, kc, 2)
+    raw, cw = proj[:, :d.conv_dim].double(), P["conv_w"].double()
+    hist = {1: conv[1].double(), 0: torch.zeros(kc - 1, d.conv_dim, dtype=torch.float64)}
+    want = torch.zeros(n, d.conv_dim, dtype=torch.float64)
+    for s in (0, 1):
+        r = (slot == s).nonzero()[:, 0]
+        if len(r):
+            x = torch.cat([hist[s], raw[r]])
+            want[r] = torch.nn.functional.silu(sum(x[j:j + len(r)] * cw[:, j] for j in range(kc)))
+    live = slot >= 0
+    for base, scale in ((0, dk ** -0.5), (nk * dk, 1.0)):
+        q = want[:, base:base + nk * dk].reshape(n, nk, dk)
+        want[:, base:base + nk * dk] = (q * torch.rsqrt((q * q).sum(-1, keepdim=True) + 1e-6) * scale).reshape(n, -1)
+    ba = proj[:, d.conv_dim + nv * dv:].double()
+    decay = torch.exp(-torch.exp(P["A_log"].double()) * torch.nn.functional.softplus(ba[:, nv:2 * nv] + P["dt_bias"].double()))
+    gates = torch.cat([decay, torch.sigmoid(ba[:, :nv])], 1)
+    # (short exponentials: a few parts in 10^6 at most on values of order one)
+    assert float((u.cpu()[live].double() - want[live]).norm() / want[live].norm()) < 2e-6
+    assert float((gb.cpu()[live].double() - gates[live]).abs().max()) < 1e-5
+    assert not u.cpu()[~live].any() and not gb.cpu()[~live].any()
+
+
+@pytest.mark.gpu
 def test_gpu_hybrid_model_generates_and_matches_whole_prefill():
     dev = torch.device("cuda:0")
     cfg = HybridConfig.tiny_hybrid()

@@ -39,6 +39,52 @@ VE_DEVINL int rows_before(const int* slot, const int* pos, int i, int lim) {
   return r;
 }
 
+// A few rows: grid (2*nk + nv + 1, rows), block = max(dk, dv, nv) threads, one channel each. Unit < nk: q head; < 2nk: k head; < 2nk+nv: v head; last: gates.
+__global__ void gdn_prepare_rows_kernel(const GdnArgs a) {
+  __shared__ float red[33];
+  grid_dep_launch();
+  grid_dep_wait();
+  const int unit = blockIdx.x, i = blockIdx.y, tid = threadIdx.x;
+  const int s = a.slot[i];
+  if (s < 0) return;
+  const int C = 2 * a.nk * a.dk + a.nv * a.dv;
+  if (unit == 2 * a.nk + a.nv) {
+    if (tid < a.nv) {
+      const __nv_bfloat16* row = a.proj + (long)i * a.ld + C + a.nv * a.dv;
+      const float b = bf2f(row[tid]), av = bf2f(row[a.nv + tid]);
+      const float x = av + a.dt_bias[tid];
+      const float sp = x > 20.f ? x : log1pf(__expf(x));
+      a.gb[(long)i * 2 * a.nv + tid] = __expf(-__expf(a.A_log[tid]) * sp);
+      a.gb[(long)i * 2 * a.nv + a.nv + tid] = 1.f / (1.f + __expf(-b));
+    }
+    return;
+  }
+  const bool is_v = unit >= 2 * a.nk;
+  const int width = is_v ? a.dv : a.dk;
+  const int c0 = is_v ? 2 * a.nk * a.dk + (unit - 2 * a.nk) * a.dv : unit * a.dk;
+  const int p = a.pos[i];
+  const int r = rows_before(a.slot, a.pos, i, a.kc - 1);
+  float val = 0.f;
+  if (tid < width) {
+    const int c = c0 + tid;
+    float acc = 0.f;
+    for (int d = 0; d < a.kc; ++d) {               // d = distance into the past of the tap
+      if (p - d < 0) break;
+      float x;
+      if (d <= r) x = bf2f(a.proj[(long)(i - d) * a.ld + c]);
+      else x = a.conv_state[((long)s * (a.kc - 1) + (a.kc - 1 - (d - r))) * C + c];
+      acc += x * a.conv_w[(long)c * a.kc + (a.kc - 1 - d)];
+    }
+    val = siluf(acc);
+  }
+  if (!is_v) {
+    const float ss = block_sum(val * val, red);
+    const float inv = rsqrtf(ss + 1e-6f) * (unit < a.nk ? rsqrtf((float)a.dk) : 1.f);
+    val *= inv;
+  }
+  if (tid < width) a.u[(long)i * C + c0 + tid] = val;
+}
+
 // One warp per unit, eight warps a block; each warp walks `per` rows of its unit. Unit < nk: q head; < 2nk: k head; < 2nk+nv: v head;
 // last: gates. The filter of a lane's channels stays in registers, and so do the last KC - 1 inputs where a row continues the one in
 // front of it. Bound by the bf16 rows read and the fp32 rows written (126 MB at 2048 rows of 10240 channels, 20 us at the copy rate): a
@@ -430,8 +476,17 @@ int ve_gdn_prepare(const void* proj, long ld, const void* pos, const void* slot,
             (const float*)conv_w, (const float*)A_log, (const float*)dt_bias, (float*)u, (float*)gb, nullptr,
             rows, nk, nv, dk, dv, kc, slots, nullptr};
   const int units = 2 * nk + nv + 1, width = dk > dv ? dk : dv;
-  // a warp walks 16 rows as soon as that still gives every SM some blocks, else each row has its own warps
-  const int per = rows >= 256 ? 16 : 1;
+  // A block per (unit, row) has the shortest path through a row; warps waste less on many, first one a row, then 16 rows after one another.
+  // us at 81 units (16 key and 48 value heads), block / warp a row / 16 rows a warp: 4 rows 2.6 5.5 -, 64 rows 9.4 10.7 -, 128 rows 16.8 16.1 -,
+  // 255 rows 31.5 26.8 31.6, 512 rows 61 - 34, 2048 rows 240 - 118; at 21 units 255 rows 9.5 11.4 28, 700 rows 22 - 30, 1024 rows 32 - 30.
+  // (Narrow models' warps of a row fill their waves badly: they go from blocks straight to 16 rows.)
+  const long work = (long)units * rows;
+  const int per = work < 7000 || (work < 20500 && units < 40) ? 0 : work < 20500 ? 1 : 16;
+  if (per == 0) {
+    const int threads = ((width > nv ? width : nv) + 31) / 32 * 32;
+    launch_pdl(gdn_prepare_rows_kernel, dim3(units, rows), dim3(threads), 0, st, a);
+    VE_CHECK_LAUNCH();
+  }
   const dim3 grid((units + 7) / 8, (rows + per - 1) / per);
   if (width <= 128 && kc == 4) launch_pdl(gdn_prepare_kernel<4, 4>, grid, dim3(256), 0, st, a, per);
   else if (width <= 128) launch_pdl(gdn_prepare_kernel<4, 0>, grid, dim3(256), 0, st, a, per);
