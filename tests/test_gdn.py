@@ -93,6 +93,33 @@ def test_gpu_gdn_row_blocks_columns_and_taps(dims, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 2, 64, 32, 4), (2, 2, 128, 96, 3), (1, 3, 128, 64, 4), (2, 4, 64, 256, 4)])
+@pytest.mark.parametrize("busy", [[(3, 1)], [(4, 1), (0, 1), (2, 1)], [(1, 5), (3, 4)], [(2, 31), (0, 1)], [(2, 32), (0, 1)], [(4, 3), (1, 60)]])
+def test_gpu_gdn_streams_between_idle_slots(dims, busy):
+    """Launches on both sides of 32 rows with slots that have no row beside, between and behind those that have: idle states keep their bytes.
+    Columns that divide into blocks of 64, of 32 only, and heads of one block."""
+    d = GDNDims(*dims)
+    g = torch.Generator().manual_seed(len(busy))
+    P = _params(d, g)
+    Pg = {k: v.float().cuda().contiguous() for k, v in P.items()}
+    st_c, st_g = GDNState(d, 5, "cpu"), GDNState(d, 5, "cuda")
+    for st in (st_c, st_g):
+        st.rec.copy_(torch.randn(st.rec.shape, generator=torch.Generator().manual_seed(3)) * 0.1)
+        st.conv.copy_(torch.randn(st.conv.shape, generator=torch.Generator().manual_seed(4)))
+    before = st_g.rec.clone(), st_g.conv.clone()
+    pos = torch.tensor([7 + i for _, n in busy for i in range(n)], dtype=torch.int32)
+    slot = torch.tensor([s for s, n in busy for _ in range(n)], dtype=torch.int32)
+    proj = torch.randn(len(pos), d.proj_out, generator=g).to(torch.bfloat16)
+    ref = gdn_reference(proj, pos, slot, st_c, d, eps=1e-6, **P)
+    out = gdn_forward(proj.cuda(), pos.cuda(), slot.cuda(), st_g, d, eps=1e-6, **Pg).float().cpu()
+    assert float((out - ref).norm() / ref.norm()) < 4e-3              # bf16 output: 2^-9 at most per value
+    assert float((st_g.rec.cpu() - st_c.rec).norm() / st_c.rec.norm()) < 1e-5
+    assert torch.equal(st_g.conv.cpu(), st_c.conv)
+    idle = [s for s in range(5) if s not in [b for b, _ in busy]]
+    assert torch.equal(st_g.rec[idle], before[0][idle]) and torch.equal(st_g.conv[idle], before[1][idle])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(16, 48, 128, 128, 4), (16, 48, 128, 128, 3), (14, 14, 64, 256, 4), (4, 12, 128, 128, 4), (2, 2, 64, 64, 9)])
 @pytest.mark.parametrize("n", [1, 33, 100, 300, 1030])
 def test_gpu_gdn_prepare_forms(dims, n):

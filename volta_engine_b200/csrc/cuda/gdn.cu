@@ -194,7 +194,7 @@ VE_DEVINL void cp_async4(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// grid (dv / 16, nv, slots), 64 threads: 16 columns of one head's state; eight lanes share two columns, DK / 8 keys of each in the
+// grid (dv / COLS, nv, slots), 4 COLS threads: COLS columns of one head's state; eight lanes share two columns, DK / 8 keys of each in the
 // registers of a lane.
 //
 // The recurrence is a serial chain over the rows, so what counts is the chain's length per row and how many chains run beside one another.
@@ -203,28 +203,40 @@ VE_DEVINL void cp_async4(void* dst, const void* src) {
 // ahead, the chain of a row is 3 * DK / 8 packed FMAs and three shuffles (the output sums of a block are reduced together behind it, 14
 // shuffles instead of 48), and 384 blocks share the chip. Shared-memory reads of k and q (512 bytes a warp and 16-byte load, also where
 // lanes read the same) bind next: with one column a lane they took 384 cycles a row on an SM with three blocks, 0.65 us a row in all
-// against 0.31 us now (2048 rows of 48 heads: 650 us), of which a row's chain of dependent instructions is most.
-constexpr int kGdnRows = 8, kGdnStages = 3, kGdnCols = 16;
-template <int DK, bool KDA>
+// against 0.29 us now (2048 rows of 48 heads: 596 us; with the kernels in front and behind 743 us), of which a row's chain of
+// dependent instructions is most.
+//
+// Launches of few rows, mostly one a slot, have a form of their own, bound by the state's bytes and by how fast blocks come and go, those of idle
+// slots among them: 64 columns a block, blocks of four rows, a ring of two, registers for half as many warps again. us for 48 heads with the
+// kernels in front and behind (a thread a column / 16 columns a block / now): one row, one slot 12.6 13.2 10.8; one row, 31 idle slots 11.4 18.8
+// 10.0; four rows of one slot 16.6 16.3 10.8; 8 streams 22.5 27.4 24.7; 16 streams 32.2 44.3 40.6, where a thread a column, with whole
+// rows of the state in a warp's load, is still ahead.
+// COLS: columns of a block, a warp eight of them; 16 in the long form, 64 or 32 in the brief one (as dv allows).
+constexpr int kGdnBrief = 32;
+template <int DK, bool KDA, int COLS>
 struct GdnStage {
-  float k[kGdnRows][DK], q[kGdnRows][DK], d[KDA ? kGdnRows : 1][KDA ? DK : 4];
-  float v[kGdnRows][kGdnCols];
-  float gb[kGdnRows][2];
+  static constexpr bool kBrief = COLS > 16;
+  static constexpr int kRows = kBrief ? 4 : 8, kStages = kBrief ? 2 : 3;
+  float k[kRows][DK], q[kRows][DK], d[KDA ? kRows : 1][KDA ? DK : 4];
+  float v[kRows][COLS];
+  float gb[kRows][2];
 };
 
-template <int DK, bool KDA>
-__global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
+template <int DK, bool KDA, int COLS>
+__global__ void __launch_bounds__(4 * COLS, (COLS > 16 ? 192 : 96) / COLS) gdn_recurrent_kernel(const GdnArgs a) {
+  using Stage = GdnStage<DK, KDA, COLS>;
+  constexpr bool BRIEF = Stage::kBrief;
+  constexpr int kGdnRows = Stage::kRows, kGdnStages = Stage::kStages, NT = 4 * COLS;
   extern __shared__ __align__(16) uint8_t gdn_smem[];
-  GdnStage<DK, KDA>* const ring = reinterpret_cast<GdnStage<DK, KDA>*>(gdn_smem);
-  __shared__ int s_first[2], s_count[2];
+  Stage* const ring = reinterpret_cast<Stage*>(gdn_smem);
+  __shared__ int s_first[NT / 32], s_count[NT / 32];
   constexpr int NP = DK / 16;                          // register pairs of a lane's part of a column
-  constexpr int NT = 64;
-  // Blocks of the kernel behind wait on the SMs once they may start, and their polling halves the pace of these few warps (2048 rows:
-  // 0.31 us a row without them, 0.55 us with them): a long walk lets them in only when it ends.
-  const bool brief = a.rows <= 32;
-  if (brief) grid_dep_launch();
+  // A long walk is launched plainly and lets its dependents in when it ends: chains that share an SM slow each other, and both blocks of the
+  // kernel behind that wait there and an uneven first placement (this kernel's blocks let in while the one in front still holds parts of the
+  // chip pile up on the SMs that are free) took 2048 rows of 48 heads from 0.31 us a row to 0.57.
+  if (BRIEF) grid_dep_launch();
   grid_dep_wait();
-  const int c0 = blockIdx.x * kGdnCols, h = blockIdx.y, s = blockIdx.z;
+  const int c0 = blockIdx.x * COLS, h = blockIdx.y, s = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = lane & 7;
   const int col = warp * 8 + (lane >> 3) * 2;           // first of this lane's two columns within the block
   // rows of this slot (consecutive)
@@ -235,8 +247,10 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
   count = __reduce_add_sync(0xffffffffu, count);
   if (lane == 0) { s_first[warp] = first; s_count[warp] = count; }
   __syncthreads();
-  first = min(s_first[0], s_first[1]);
-  count = s_count[0] + s_count[1];
+  first = s_first[0];
+  count = s_count[0];
+#pragma unroll
+  for (int w = 1; w < NT / 32; ++w) { first = min(first, s_first[w]); count += s_count[w]; }
   if (count == 0) return;
   const int C = 2 * a.nk * DK + a.nv * a.dv;
   const int kh = h / (a.nv / a.nk);
@@ -244,7 +258,7 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
 
   auto load = [&](int blk) {                            // one block of rows into its ring stage
     if (blk * kGdnRows < count) {
-      GdnStage<DK, KDA>& st = ring[blk % kGdnStages];
+      Stage& st = ring[blk % kGdnStages];
       const int n = min(kGdnRows, count - blk * kGdnRows);
       const long i0 = first + blk * kGdnRows;
       constexpr int Q = DK / 4;                          // 16-byte pieces of a key
@@ -255,8 +269,12 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
         cp_async16(&st.k[r][c], ui + a.nk * DK);
         if (KDA) cp_async16(&st.d[r][c], a.kdec + ((i0 + r) * a.nv + h) * DK + c);
       }
-      if (tid < n * 4) cp_async16(&st.v[tid >> 2][(tid & 3) * 4], a.u + (i0 + (tid >> 2)) * C + 2 * a.nk * DK + h * a.dv + c0 + (tid & 3) * 4);
-      else if (tid >= 32 && tid < 32 + n * 2) {
+      constexpr int V = COLS / 4;
+      for (int j = tid; j < n * V; j += NT) {
+        const int r = j / V, c = j % V * 4;
+        cp_async16(&st.v[r][c], a.u + (i0 + r) * C + 2 * a.nk * DK + h * a.dv + c0 + c);
+      }
+      if (tid >= 32 && tid < 32 + n * 2) {
         const int r = (tid - 32) >> 1, w = tid & 1;
         cp_async4(&st.gb[r][w], a.gb + (i0 + r) * 2 * a.nv + w * a.nv + h);
       }
@@ -278,7 +296,7 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
     S[1][j] = pack2(lo.y, hi.y);
   }
   float o[2][kGdnRows];
-  auto row = [&](const GdnStage<DK, KDA>& st, int r) {
+  auto row = [&](const Stage& st, int r) {
     uint64_t k2[NP], m[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
     const float2 g = *reinterpret_cast<const float2*>(st.gb[r]);
     const float2 v = *reinterpret_cast<const float2*>(&st.v[r][col]);
@@ -333,7 +351,7 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kGdnStages - 2) : "memory");
     __syncthreads();                                     // this block's rows have landed; the stage in front of it is free
     load(blk + kGdnStages - 1);
-    const GdnStage<DK, KDA>& st = ring[blk % kGdnStages];
+    const Stage& st = ring[blk % kGdnStages];
     const int n = min(kGdnRows, count - blk * kGdnRows);
     if (n == kGdnRows) {
 #pragma unroll
@@ -345,9 +363,14 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
         if (r < n) row(st, r);
       }
     }
-    // sums over the eight lanes of a column: lane `part` ends with row `part`
+    // sums over the eight lanes of a column: lane `part` ends with row `part` (of four rows, `part` and `part` - 4 with the same one)
+    if (kGdnRows == 4)
 #pragma unroll
-    for (int w = 4; w >= 1; w >>= 1) {
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[c][j] += __shfl_xor_sync(0xffffffffu, o[c][j], 4);
+#pragma unroll
+    for (int w = kGdnRows / 2; w >= 1; w >>= 1) {
       const bool up = part & w;
 #pragma unroll
       for (int c = 0; c < 2; ++c)
@@ -360,7 +383,7 @@ __global__ void __launch_bounds__(64) gdn_recurrent_kernel(const GdnArgs a) {
     if (part < n)
       *reinterpret_cast<float2*>(a.o + ((long)(first + blk * kGdnRows + part) * a.nv + h) * a.dv + c0 + col) = make_float2(o[0][0], o[1][0]);
   }
-  if (!brief) grid_dep_launch();
+  if (!BRIEF) grid_dep_launch();
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     const long k = ((j >> 1) * 8 + part) * 4 + (j & 1) * 2;
@@ -437,12 +460,20 @@ __global__ void kda_decay_kernel(const __nv_bfloat16* __restrict__ f, long ld, c
 
 using namespace ve;
 
+template <int DK, bool KDA, int COLS>
+static int launch_recurrent_cols(const GdnArgs& a, cudaStream_t st) {
+  using Stage = GdnStage<DK, KDA, COLS>;
+  constexpr int smem = Stage::kStages * (int)sizeof(Stage);
+  static_assert(smem <= 48 * 1024, "no opt-in to large shared memory is made");
+  const dim3 grid(a.dv / COLS, a.nv, a.slots);
+  if (Stage::kBrief) launch_pdl(gdn_recurrent_kernel<DK, KDA, COLS>, grid, dim3(4 * COLS), smem, st, a);
+  else gdn_recurrent_kernel<DK, KDA, COLS><<<grid, 4 * COLS, smem, st>>>(a);
+  VE_CHECK_LAUNCH();
+}
 template <int DK, bool KDA>
 static int launch_recurrent_dk(const GdnArgs& a, cudaStream_t st) {
-  constexpr int smem = kGdnStages * (int)sizeof(GdnStage<DK, KDA>);
-  static_assert(smem <= 48 * 1024, "no opt-in to large shared memory is made");
-  launch_pdl(gdn_recurrent_kernel<DK, KDA>, dim3(a.dv / kGdnCols, a.nv, a.slots), dim3(64), smem, st, a);
-  VE_CHECK_LAUNCH();
+  if (a.rows > kGdnBrief) return launch_recurrent_cols<DK, KDA, 16>(a, st);
+  return a.dv % 64 == 0 ? launch_recurrent_cols<DK, KDA, 64>(a, st) : launch_recurrent_cols<DK, KDA, 32>(a, st);
 }
 template <bool KDA>
 static int launch_recurrent(const GdnArgs& a, cudaStream_t st) {
