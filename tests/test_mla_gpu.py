@@ -113,3 +113,58 @@ def test_mtp_rounds_run_on_the_device_and_reproduce_plain_greedy():
     assert run2.round_depth() == 3
     from volta_engine_b200.ops import kernels as K
     assert K.check_status(DEV) == 0
+
+
+@pytest.mark.parametrize("heads,nope,vd,shift", [(3, 128, 128, 0), (8, 96, 72, 1), (2, 256, 256, 0), (5, 37, 33, 3)])
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 8, 9, 16, 17, 40])
+def test_query_absorption_and_output_expansion(heads, nope, vd, shift, rows):
+    """Every count of rows a launch is built for and more than one pass, widths that are no multiple of a piece, absorption weights that start
+    between 16-byte boundaries. fp32 sums of exact products, rounded to bf16 once."""
+    from volta_engine_b200._lib import call, ptr
+    g = torch.Generator().manual_seed(rows)
+    q = torch.randn(rows, heads * (nope + 64), generator=g).to(torch.bfloat16).to(DEV)
+    wuk = torch.empty(heads * nope * 512 + 8, dtype=torch.bfloat16, device=DEV)[shift:shift + heads * nope * 512].view(heads, nope, 512)
+    wuk.copy_(torch.randn(heads, nope, 512, generator=g))
+    wuv = torch.randn(heads, vd, 512, generator=g).to(torch.bfloat16).to(DEV)
+    q_abs = torch.full((rows, heads, 576), 7.0, dtype=torch.bfloat16, device=DEV)
+    call("mla_absorb_q", "pliippii", ptr(q), q.stride(0), nope + 64, nope, ptr(wuk), ptr(q_abs), rows, heads)
+    qh = q.view(rows, heads, nope + 64)
+    want = torch.einsum("rhd,hdc->rhc", qh[..., :nope].double(), wuk.double())
+    assert float((q_abs[..., :512].double() - want).norm() / want.norm()) < 2 ** -8
+    assert torch.equal(q_abs[..., 512:], qh[..., nope:])
+    o = torch.randn(rows, heads, 512, generator=g).to(torch.bfloat16).to(DEV)
+    out = torch.full((rows, heads * vd), 7.0, dtype=torch.bfloat16, device=DEV)
+    call("mla_expand_out", "pppliii", ptr(o), ptr(wuv), ptr(out), out.stride(0), rows, heads, vd)
+    want = torch.einsum("rhc,hvc->rhv", o.double(), wuv.double()).reshape(rows, -1)
+    assert float((out.double() - want).norm() / want.norm()) < 2 ** -8
+
+
+@pytest.mark.parametrize("heads", [1, 7, 8, 20])
+@pytest.mark.parametrize("rows", [5, 511, 512, 700])
+@pytest.mark.parametrize("interleaved", [0, 1])
+def test_latent_rotation_and_store_of_many_rows(heads, rows, interleaved):
+    """Both forms of the launch, a block for eight heads of a row and a block for all of them; padding rows store nothing."""
+    from volta_engine_b200._lib import call, ptr
+    from volta_engine_b200.ops.reference import rope_rotate
+    g = torch.Generator().manual_seed(rows + heads)
+    q = torch.randn(rows, heads * 96, generator=g).to(torch.bfloat16)
+    ckv, kr = torch.randn(rows, 512, generator=g).to(torch.bfloat16), torch.randn(rows, 64, generator=g).to(torch.bfloat16)
+    pos = torch.arange(3, 3 + rows, dtype=torch.int32)
+    slot = torch.ones(rows, dtype=torch.int32)
+    slot[1] = -1
+    table = torch.randperm(24, generator=g).int().reshape(2, 12)
+    pool = torch.full((24, 1, 64, 576), 7.0, dtype=torch.bfloat16, device=DEV)
+    a = [t.to(DEV) for t in (q, ckv, kr, pos, slot, table)]
+    call("mla_rope_store", "pliiplplpppipifi", ptr(a[0]), a[0].stride(0), 96, heads, ptr(a[1]), 512, ptr(a[2]), 64, ptr(a[3]), ptr(a[4]),
+         ptr(a[5]), 12, ptr(pool), rows, 10000.0, interleaved)
+    want = q.view(rows, heads, 96).clone()
+    want[..., 32:] = rope_rotate(want[..., 32:].contiguous(), pos, 64, 10000.0, bool(interleaved))
+    got = a[0].cpu().view(rows, heads, 96)
+    assert torch.equal(got[..., :32], q.view(rows, heads, 96)[..., :32])
+    assert float((got.float() - want.float()).abs().max()) < 3e-2                 # (an ulp of bf16 at 4)
+    lat = torch.cat([ckv, rope_rotate(kr.view(rows, 1, 64).clone(), pos, 64, 10000.0, bool(interleaved))[:, 0]], 1)
+    want_pool = torch.full((24, 64, 576), 7.0)
+    for r in range(rows):
+        if slot[r] >= 0:
+            want_pool[table[1, pos[r] // 64], pos[r] % 64] = lat[r].float()
+    assert float((pool.cpu()[:, 0].float() - want_pool).abs().max()) < 3e-2

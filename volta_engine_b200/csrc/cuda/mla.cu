@@ -40,7 +40,7 @@ __global__ void mla_rope_store_kernel(__nv_bfloat16* __restrict__ q, long q_stri
   for (; h < heads; h += gridDim.y * 8) {
     __nv_bfloat16* v = q + (long)row * q_stride + (long)h * q_dim + (q_dim - kRope);
     const float a0 = bf2f(v[i0]), a1 = bf2f(v[i1]);
-    // output always in half-split order so that q and k agree whatever the checkpoint's pairing
+    // (in place: the pairs stay where the checkpoint has them, in q as in k)
     v[i0] = f2bf(a0 * cs - a1 * sn);
     v[i1] = f2bf(a1 * cs + a0 * sn);
   }
@@ -58,51 +58,63 @@ __global__ void mla_rope_store_kernel(__nv_bfloat16* __restrict__ q, long q_stri
 }
 
 // q_abs[row, h, 0:512] = q[row, h, 0:nope] @ W_uk[h] (nope x 512) ; q_abs[row, h, 512:576] = q_rope.
-// One block a head, thread = latent column; it asks for 32 rows of W_uk at once, and up to eight activation rows share them. Bound by the 16.8 MB
-// of 128 heads (3 us): a block per (row, head) read them once per row behind a chain of eight loads, 18 us. Sums run over d in order.
-constexpr int kAbsRows = 8;
-__global__ void __launch_bounds__(512) mla_absorb_q_kernel(const __nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int nope,
-                                                           const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ q_abs, int rows,
-                                                           int heads) {
-  __shared__ __align__(16) float qs[256][kAbsRows];
-  const int h = blockIdx.x, tid = threadIdx.x;
-  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat + tid;
-  for (int r0 = 0; r0 < rows; r0 += kAbsRows) {
-    const int n = min(kAbsRows, rows - r0);
-    const __nv_bfloat16* qv = q + (long)r0 * q_stride + (long)h * q_dim;
-    __syncthreads();
-    for (int i = tid; i < nope * kAbsRows; i += 512) {
-      const int r = i / nope, d = i - r * nope;
-      qs[d][r] = r < n ? bf2f(qv[(long)r * q_stride + d]) : 0.f;
-    }
-    for (int i = tid; i < n * kRope; i += 512)
-      q_abs[((long)(r0 + i / kRope) * heads + h) * kLatRow + kLat + i % kRope] = qv[(long)(i / kRope) * q_stride + q_dim - kRope + i % kRope];
-    __syncthreads();
-    float acc[kAbsRows];
-#pragma unroll
-    for (int r = 0; r < kAbsRows; ++r) acc[r] = 0.f;
-    for (int d0 = 0; d0 < nope; d0 += 32) {
-      __nv_bfloat16 t[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) t[i] = d0 + i < nope ? w[(long)(d0 + i) * kLat] : __float2bfloat16(0.f);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (d0 + i >= nope) break;
-        const float wf = bf2f(t[i]);
-#pragma unroll
-        for (int r = 0; r < kAbsRows; r += 4) {
-          const float4 x = *reinterpret_cast<const float4*>(&qs[d0 + i][r]);
-          acc[r] = fmaf(x.x, wf, acc[r]);
-          acc[r + 1] = fmaf(x.y, wf, acc[r + 1]);
-          acc[r + 2] = fmaf(x.z, wf, acc[r + 2]);
-          acc[r + 3] = fmaf(x.w, wf, acc[r + 3]);
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kAbsRows; ++r)
-      if (r < n) q_abs[((long)(r0 + r) * heads + h) * kLatRow + tid] = f2bf(acc[r]);
+// grid (512 / 256, heads, rows / ROWS), 128 threads: 256 latent columns of a head's W_uk come to shared memory at once, for up to ROWS activation
+// rows; a thread has two columns. ROWS: 1, 4, 8, or 16 once blocks of eight are more than a wave. Bound by latency, one wave of copies behind
+// the launch, and at 128 heads by the FMAs. Sums run over d in order. Warm, us, of a block per (row, head) with a chain of loads / a block a head /
+// now: 8 heads one row 7.2 8.9 4.0, eight rows 7.7 9.5 8.3, 64 rows 8.2 61 8.5; 128 heads one row 7.8 9.2 5.0, eight rows 9.1 9.7 9.9, 16 rows
+// 16.2 17.2 15.6.
+constexpr int kAbsCols = 256;
+template <int ROWS>
+__global__ void __launch_bounds__(kAbsCols / 2) mla_absorb_q_kernel(const __nv_bfloat16* __restrict__ q, long q_stride, int q_dim, int nope,
+                                                                    const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ q_abs,
+                                                                    int rows, int heads, bool vec) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  float* const qs = reinterpret_cast<float*>(smem_raw);                                       // [nope][ROWS]
+  __nv_bfloat16* const ws = reinterpret_cast<__nv_bfloat16*>(smem_raw + (nope * ROWS * 4 + 15) / 16 * 16);      // [nope][kAbsCols]
+  const int c0 = blockIdx.x * kAbsCols, h = blockIdx.y, r0 = blockIdx.z * ROWS, n = min(ROWS, rows - r0), tid = threadIdx.x;
+  const __nv_bfloat16* w = w_uk + (long)h * nope * kLat + c0;
+  for (int i = tid; i < nope * (kAbsCols / 8); i += kAbsCols / 2) {
+    const int d = i / (kAbsCols / 8), c = i % (kAbsCols / 8) * 8;
+    if (vec)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ws + d * kAbsCols + c)), "l"(w + (long)d * kLat + c) : "memory");
+    else                                            // (weights that do not start on a 16-byte boundary)
+      for (int e = 0; e < 8; ++e) ws[d * kAbsCols + c + e] = w[(long)d * kLat + c + e];
   }
+  const __nv_bfloat16* qv = q + (long)r0 * q_stride + (long)h * q_dim;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    for (int d = tid; d < nope; d += kAbsCols / 2) qs[d * ROWS + r] = r < n ? bf2f(qv[(long)r * q_stride + d]) : 0.f;
+  if (blockIdx.x == 0)
+    for (int i = tid; i < n * kRope; i += kAbsCols / 2)
+      q_abs[((long)(r0 + i / kRope) * heads + h) * kLatRow + kLat + i % kRope] = qv[(long)(i / kRope) * q_stride + q_dim - kRope + i % kRope];
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float acc[ROWS][2];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.f;
+#pragma unroll 8
+  for (int d = 0; d < nope; ++d) {
+    const float2 wf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(ws + d * kAbsCols + 2 * tid));
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const float x = qs[d * ROWS + r];
+      acc[r][0] = fmaf(x, wf.x, acc[r][0]);
+      acc[r][1] = fmaf(x, wf.y, acc[r][1]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (r < n)
+      *reinterpret_cast<__nv_bfloat162*>(q_abs + ((long)(r0 + r) * heads + h) * kLatRow + c0 + 2 * tid) = __floats2bfloat162_rn(acc[r][0], acc[r][1]);
+}
+template <int ROWS>
+static int launch_absorb(const void* q, long q_stride, int q_dim, int nope, const void* w_uk, void* q_abs, int rows, int heads, cudaStream_t st) {
+  const int smem = (nope * ROWS * 4 + 15) / 16 * 16 + nope * kAbsCols * 2;       // 68 KB at 128 and eight rows, 136 KB at 256
+  const cudaError_t e = allow_smem<mla_absorb_q_kernel<ROWS>>(256 * (ROWS * 4 + kAbsCols * 2));
+  if (e != cudaSuccess) return (int)e;
+  mla_absorb_q_kernel<ROWS><<<dim3(kLat / kAbsCols, heads, (rows + ROWS - 1) / ROWS), kAbsCols / 2, smem, st>>>(
+      (const __nv_bfloat16*)q, q_stride, q_dim, nope, (const __nv_bfloat16*)w_uk, (__nv_bfloat16*)q_abs, rows, heads, !((uintptr_t)w_uk & 15));
+  VE_CHECK_LAUNCH();
 }
 
 // out[row, h, 0:vdim] = o_lat[row, h, 0:512] @ W_uv[h]^T  (W_uv [heads, vdim, 512]). grid (vdim / 32, heads, rows / 8), 128 threads: 32 rows of a
@@ -424,9 +436,10 @@ int ve_mla_absorb_q(const void* q, long q_stride, int q_dim, int nope, const voi
                     cudaStream_t st) {
   if (rows <= 0) return 0;
   if (nope > 256) return cudaErrorInvalidValue;
-  mla_absorb_q_kernel<<<heads, 512, 0, st>>>((const __nv_bfloat16*)q, q_stride, q_dim, nope, (const __nv_bfloat16*)w_uk,
-                                             (__nv_bfloat16*)q_abs, rows, heads);
-  VE_CHECK_LAUNCH();
+  return rows == 1 ? launch_absorb<1>(q, q_stride, q_dim, nope, w_uk, q_abs, rows, heads, st)
+       : rows <= 4 ? launch_absorb<4>(q, q_stride, q_dim, nope, w_uk, q_abs, rows, heads, st)
+       : rows <= 8 || 2 * heads * ((rows + 7) / 8) <= 3 * 148 ? launch_absorb<8>(q, q_stride, q_dim, nope, w_uk, q_abs, rows, heads, st)
+                   : launch_absorb<16>(q, q_stride, q_dim, nope, w_uk, q_abs, rows, heads, st);
 }
 
 int ve_mla_expand_out(const void* o_lat, const void* w_uv, void* out, long out_stride, int rows, int heads, int vdim,
