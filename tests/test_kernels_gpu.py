@@ -345,3 +345,28 @@ def test_bounded_wait_reports_through_the_status_word():
     assert int(status.item()) == 0
     x = torch.ones(4, device=DEV)
     assert float((x + 1).sum()) == 8.0                                          # the context still works
+
+
+@pytest.mark.parametrize("nq,nkv,hd,rot", [(5, 1, 128, 128), (24, 4, 256, 64), (3, 3, 96, 48), (8, 2, 64, 64)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rope_store_of_many_rows_equals_parts(nq, nkv, hd, rot, interleaved):
+    """A block for all heads of a row (512 rows and more) against the blocks of a few heads that shorter launches take, row for row; the
+    first rows also against the oracle. Padding rows store nothing."""
+    rows = 700
+    qkv = rnd(rows, (nq + 2 * nkv) * hd, seed=nq)
+    pos = torch.arange(2, 2 + rows, dtype=torch.int32, device=DEV)
+    slot = torch.ones(rows, dtype=torch.int32, device=DEV)
+    slot[3] = -1
+    table = torch.randperm(24, generator=torch.Generator().manual_seed(1)).int().reshape(2, 12).to(DEV)
+    kp, vp = rnd(24, nkv, 64, hd, seed=2), rnd(24, nkv, 64, hd, seed=3)
+    part, kq, vq = qkv.clone(), kp.clone(), vp.clone()
+    q_ref, k_ref, v_ref = qkv[:40].cpu().clone(), kp.cpu().clone(), vp.cpu().clone()
+    ref.rope_store(q_ref, pos[:40].cpu(), slot[:40].cpu(), table.cpu(), k_ref, v_ref, nq, nkv, hd, rot, 1e6, interleaved)
+    K.rope_store(qkv, pos, slot, table, kp, vp, nq, nkv, hd, rot, 1e6, interleaved)
+    for a, b in ((0, 40), (40, 41), (41, 500), (500, 700)):
+        K.rope_store(part[a:b], pos[a:b], slot[a:b], table, kq, vq, nq, nkv, hd, rot, 1e6, interleaved)
+        if a == 0:
+            live = torch.arange(40) != 3                     # (the kernel leaves the key of a padding row as it is)
+            assert_close(part[:40].cpu()[live], q_ref[live], name="rope q/k")
+            assert_close(kq.cpu(), k_ref, name="k cache")
+    assert torch.equal(qkv, part) and torch.equal(kp, kq) and torch.equal(vp, vq)

@@ -173,7 +173,6 @@ __global__ void rope_store_kernel(__nv_bfloat16* __restrict__ qkv, const int* __
     const int pr = pos3 ? pos3[(i < sec0 ? 0 : (i < sec0 + sec1 ? 1 : 2)) * (long)gridDim.x + row] : p;
     sincosf((float)pr * pos_scale * inv_freq, &sn, &cs);
   }
-  const long page = s >= 0 ? page_table[(long)s * max_pages + p / kPage] : 0;
   for (int head = blockIdx.y * blockDim.y + threadIdx.y; head < nq + nkv; head += gridDim.y * blockDim.y) {
     __nv_bfloat16* h = qkv + row_off + (long)head * hd;
     float a0 = bf2f(h[i0]), a1 = bf2f(h[i1]);
@@ -190,6 +189,7 @@ __global__ void rope_store_kernel(__nv_bfloat16* __restrict__ qkv, const int* __
     }
     if (s < 0) continue;
     const int kvh = head - nq;
+    const long page = page_table[(long)s * max_pages + p / kPage];
     const long dst = ((page * nkv + kvh) * kPage + (p % kPage)) * hd;
     h[i0] = b0;
     h[i1] = b1;
