@@ -173,6 +173,25 @@ def test_gguf_experts_decoded_in_tiles(spec, rows):
     assert K.check_status("cuda") == 0
 
 
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("I,rows", [(256, 33), (512, 150)])
+def test_gguf_experts_of_every_format_decoded_in_tiles(t, I, rows):
+    """Bit for bit the bank decoded to bf16 first: the same operands in the same chain over K. (Formats of 32-weight blocks also with a K that
+    ends inside a staged unit.)"""
+    from volta_engine_b200.ops.moe_gguf import GGUFExpertBank
+    big = gq.BLOCK[t][0] == 256
+    E, H, k = 3, 512, 2
+    I += 0 if big else 32
+    bank = GGUFExpertBank.random(E, I, H, t, t, seed=t, amp=0.05, device="cuda")
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, H, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(4, generator=g)[:k] for _ in range(rows)]).to(torch.int32).cuda()
+    assert bank._decodes_in_tiles(rows * k)
+    assert torch.equal(bank.routes_prefill(x, ids, 0, 0.0), bank._routes_prefill_slabs(x, ids, 0, 0.0))
+    from volta_engine_b200.ops import kernels as K
+    assert K.check_status("cuda") == 0
+
+
 @pytest.mark.parametrize("spec,gu_at,dn_at", [("gguf_q4_k+q6_k", 2, 0), ("gguf_q6_k+q4_k", 2, 2), ("gguf_iq1_s+q4_1", 4, 2), ("gguf_q8_0+q8_0", 2, 6)])
 def test_gguf_experts_at_any_even_address(spec, gu_at, dn_at):
     """A bank inside a larger allocation gives what it gives at the start of one, whichever way its formats and addresses let it take."""

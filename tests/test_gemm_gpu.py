@@ -79,10 +79,9 @@ def test_gemm_w4a4(T, N, Kd):
 
 
 @pytest.mark.parametrize("T,N,Kd", [(129, 128, 128), (192, 384, 2048), (193, 1280, 5120), (700, 640, 8192), (1000, 5120, 1280), (2048, 8192, 256)])
-def test_gemm_w4a16_wide_cut_tiles(T, N, Kd):
-    """An odd number of 128-feature tiles, tokens around tiles of 192, tiles that stay whole and tiles cut along K into two to eight pieces
-    (few tiles of a long K), a residual, and an output whose rows are no multiple of 16 bytes. Sums in fp32 over at most 8192 exact
-    products and one rounding to bf16 (2^-8)."""
+def test_gemm_w4a16_wide_tiles(T, N, Kd):
+    """An odd number of 128-feature tiles, tokens around tiles of 192 and 256, launches of both tile shapes, a residual, and an output whose rows
+    are no multiple of 16 bytes. Sums in fp32 over at most 8192 exact products and one rounding to bf16 (2^-8)."""
     w = rnd(N, Kd, std=0.02, seed=24, dtype=torch.float32)
     p, s, g = qn.quantize_nvfp4(w, search=False)
     sf = qn.scales_blocked_k128(s)
@@ -93,7 +92,7 @@ def test_gemm_w4a16_wide_cut_tiles(T, N, Kd):
         return float((got.double() - ref).norm() / ref.norm())
     first = K.gemm_w4a16(p, sf, g, x)
     assert off(first, want) < 2 ** -8
-    assert torch.equal(K.gemm_w4a16(p, sf, g, x), first)              # pieces are added in the order of k, whoever arrives last
+    assert torch.equal(K.gemm_w4a16(p, sf, g, x), first)
     assert off(K.gemm_w4a16(p, sf, g, x, residual=res), want + res.double()) < 2 ** -8
     odd = torch.empty(T, N + 3, dtype=torch.bfloat16, device=DEV)[:, :N]
     K.gemm_w4a16(p, sf, g, x, out=odd)

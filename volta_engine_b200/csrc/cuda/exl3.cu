@@ -147,8 +147,8 @@ exl3_gemv_few_kernel(const uint16_t* __restrict__ codes, const __half* __restric
 // split evenly over the blocks that are resident at once, so every block gets the same work to within one unit whatever the number of
 // groups is. In a unit the eight warps split K, and each brings its k-tiles, 4 / UT at a time, through a cp.async ring of its own that runs
 // several stages ahead and on into the next unit. One k-tile ahead in registers (and a grid of groups x columns) a unit cost sixteen memory
-// latencies in a row: 108 us for 160 routes of 2048 x 512 weights at 4 bits, now 70 us; their bytes take 13 us. What bounds it now is the
-// decoding, five to six instructions a weight.
+// latencies in a row: 108 us for 160 routes of 2048 x 512 weights at 4 bits, now 70 us; their bytes take 13 us. What bounds it now is
+// issuing: 8.7 instructions a weight, 72 % of the issue slots of 16 warps an SM.
 template <int BITS, int MH>
 struct Exl3Gemv {
   static constexpr int kStage = 4 * 32 * BITS, kStages = BITS <= 4 ? 8 : 4;      // bytes of four tiles; stages of the ring
@@ -192,13 +192,13 @@ exl3_gemv_kernel(const uint16_t* __restrict__ codes, const __half* __restrict__ 
         for (int i = 0; i < (8 * BITS + 31) / 32; ++i) {
           const int j = lane + 32 * i, ku = j / P, piece = j % P;
           if (ku < KU && piece < l_live && l_kt + ku < kt1)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + j * 16)), "l"(src + ku * tstride + piece * 16) : "memory");
+            cp_async16(dst + j * 16, src + ku * tstride + piece * 16);
         }
       } else {                                                       // codes that start between 16-byte boundaries: word by word
         for (int j = lane; j < 4 * 8 * BITS; j += 32) {
           const int ku = j / (4 * P), word = j % (4 * P);
           if (word < 4 * l_live && l_kt + ku < kt1)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + j * 4)), "l"(src + ku * tstride + word * 4) : "memory");
+            cp_async4(dst + j * 4, src + ku * tstride + word * 4);
         }
       }
       l_slot = l_slot + 1 == C::kStages ? 0 : l_slot + 1;

@@ -187,13 +187,6 @@ VE_DEVINL uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-VE_DEVINL void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-VE_DEVINL void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 // grid (dv / COLS, nv, slots), 4 COLS threads: COLS columns of one head's state; eight lanes share two columns, DK / 8 keys of each in the
 // registers of a lane.
 //
@@ -204,7 +197,7 @@ VE_DEVINL void cp_async4(void* dst, const void* src) {
 // shuffles instead of 48), and 384 blocks share the chip. Shared-memory reads of k and q (512 bytes a warp and 16-byte load, also where
 // lanes read the same) bind next: with one column a lane they took 384 cycles a row on an SM with three blocks, 0.65 us a row in all
 // against 0.29 us now (2048 rows of 48 heads: 596 us; with the kernels in front and behind 743 us), of which a row's chain of
-// dependent instructions is most.
+// dependent instructions is most (138 instructions a row and warp, 41 % of the issue slots at five warps an SM).
 //
 // Launches of few rows, mostly one a slot, have a form of their own, bound by the state's bytes and by how fast blocks come and go, those of idle
 // slots among them: 64 columns a block, blocks of four rows, a ring of two, registers for half as many warps again. us for 48 heads with the

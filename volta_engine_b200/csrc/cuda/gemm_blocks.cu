@@ -7,8 +7,9 @@
 // One CTA: 128 output features x one tile of at most 128 rows of one expert. Warp 0: TMA of the rows' bf16 tiles (boxes of 32 rows, as many
 // as the tile has); warp 1: TMEM and MMA; warps 2..9 decode: each copies the raw blocks of its 16 features (EXL3: its 16-column tiles) with
 // cp.async through a ring of its own, 256 weights of K ahead, and writes bf16 into the stage; warps 2..5 store the tile. Two CTAs share an
-// SM, so one decodes while the other multiplies or stores. What bounds it is the decoding arithmetic (3 to 6 instructions a weight, once
-// per 128 rows), so a tile is as tall as two CTAs' shared memory allows.
+// SM, so one decodes while the other multiplies or stores. What bounds it is issuing the decoding: 9.7 instructions a
+// weight and tile for IQ1_M, 10.7 for trellis codes of 4 bits, 61 and 72 % of the issue slots of 20 warps an SM; next come waits for a stage. So a
+// tile is as tall as two CTAs' shared memory allows.
 // Every wait is bounded; on expiry the kernel records a status code and drains.
 #include "common.cuh"
 #include "exl3_blocks.cuh"
@@ -68,9 +69,7 @@ struct GgufTile {
       const int n16 = (off + bytes + 15) >> 4;
       for (int j = t; j < n16; j += 4) {
         const long left = end - (src + j * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (r * 8 + g) * kPitch + j * 16)),
-                     "l"(src + j * 16), "r"(left < 16 ? (int)left : 16)
-                     : "memory");
+        cp_async16(dst + (r * 8 + g) * kPitch + j * 16, src + j * 16, left < 16 ? (int)left : 16);
       }
     }
   }
@@ -127,8 +126,7 @@ struct Exl3Tile {
     for (int i = 0; i < BITS; ++i) {
       const int j = lane + 32 * i, tile = j / (2 * BITS), piece = j % (2 * BITS), kt = unit * 16 + tile;
       if (kt < kt_all)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + j * 16)), "l"(base + (size_t)kt * kstride + piece * 16)
-                     : "memory");
+        cp_async16(dst + j * 16, base + (size_t)kt * kstride + piece * 16);
     }
   }
   VE_DEVINL void decode(const uint8_t* raw, int unit, int sub, uint8_t* a, const uint8_t*) const {

@@ -8,11 +8,13 @@
 //   * two 128-feature sub-tiles x 192 tokens: accumulators of 2 x 192 columns and two buffers of 2 x 32 columns of weights fill the 512
 //     columns. 92 KB of shared memory a step, 720 cycles for 768 of tensor work; measured 0.75 us a step: the dequantising, one weight row of
 //     64 a thread and step, takes most of it (shorter tiles are no faster).
-//   * one sub-tile x 256 tokens: half a weight row a thread and step, four buffers; 0.52 us a step for two thirds of the products.
+//   * one sub-tile x 256 tokens: half a weight row a thread and step, four buffers; 0.52 us a step for two thirds of the products (34816 x
+//     5120 at 2048 tokens: tensor pipe 61 % busy, issue slots 54 %).
 // The shape that needs less time for its waves of 148 tiles is taken (0.75 : 0.52 is 10 : 7). Times in us of the former kernel, of one
 // sub-tile and of two: 5120 x 5120 600 tokens 84 51 61, 953 tokens 85 98 63, 2048 tokens 166 145 122; 34816 x 5120 256 tokens 90 84 125,
 // 2048 tokens 699 620 657, 8192 tokens 2919 2745 2944; 5120 x 17408 150 tokens 260 164 234, 1500 tokens 262 283 378, 2048 tokens 511 381
-// 379. Where 256 x 256 tiles happened to fill whole waves the former kernel was up to 8 % faster (16384 x 5120 at 452 tokens 90 to 95 us).
+// 379. Where 256 x 256 tiles happened to fill whole waves the former kernel was faster (16384 x 5120 at 452 tokens 90 us against 95,
+// 5120 x 5120 at 3001 tokens 180 against 210).
 //
 // A result depends on its own row of X alone: every tile runs over K in one chain, whatever T and the shape are. (Tiles of a partial last
 // wave cut along K, with fp32 partial sums, would give 5120 x 17408 116 to 140 us at 129 to 256 tokens in place of 162 to 171, but rows that

@@ -172,8 +172,9 @@ struct GgufGemvArgs {
 // A tile is 16 * RT weight rows (MODE 2: eight gate and eight up rows). The eight warps of a block deal its units of 256 weights along K
 // (128 for Q8_0) between them; each warp copies its units through a ring of its own with 16-byte cp.async and turns them into operand
 // fragments, whose products with all activation rows are one tensor-core instruction per 16 weights. Blocks are persistent over tiles and the
-// ring runs on into the next tile. What bounds it is the weights' DRAM traffic, or for the formats of four bits and less decoding, 1.5 to 3
-// instructions a weight. A lane that decoded 32 consecutive weights of its own straight from global memory (one warp a row) read
+// ring runs on into the next tile. What bounds it is issuing: 34816 x 5120 Q4_K at four rows
+// takes 6.4 instructions a weight, 62 % of the issue slots of 16 warps an SM, at a quarter of the copy rate (decoding, the activations of every
+// row tile and the scales; next come waits for dependent results and for the barrier behind a tile). A lane that decoded 32 consecutive weights of its own straight from global memory (one warp a row) read
 // single bytes up to 4352 bytes apart and multiplied every row of x in fp32: 365 us for the average matrix of a 27B-class Q4_K layer at
 // four rows, 538 us for Q8_0 at eight rows of the larger latent-attention shapes.
 template <int TYPE, int MODE, int NT, int RT>
@@ -245,9 +246,7 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
           const int n16 = (off + bytes + 15) >> 4;
           for (int j = t; j < n16; j += 4) {
             const long left = p.W_end - (src + j * 16);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (r * 8 + g) * C::kPitch + j * 16)),
-                         "l"(src + j * 16), "r"(left < 16 ? (int)left : 16)
-                         : "memory");
+            cp_async16(dst + (r * 8 + g) * C::kPitch + j * 16, src + j * 16, left < 16 ? (int)left : 16);
           }
         }
       }
@@ -464,7 +463,7 @@ __global__ void __launch_bounds__(256, 2) gguf_mma_kernel(const GgufGemvArgs p) 
 // one token in a hundred with the sums of gguf_mma_kernel, although their error against 64 bits is no larger.
 // Times (gguf_mma_kernel in brackets): 7168 x 16384 Q8_0 one row 58 us (65), eight 127 us (62); Q4_K 72 (44) and 137 us (42); gate / up and down of 64
 // routes of 2048 x 7168 IQ1_M 944 us (750), Q4_K 1217 us (870), Q8_0 965 us (1270). The byte-by-byte kernels: 174 and 999 us, 165 and 987 us; 2121,
-// 2578 and 2638 us.
+// 2578 and 2638 us. Bound by issuing: IQ1_M takes 10.1 instructions a weight, 84 % of the issue slots.
 // A warp takes two rows (MODE 2: a gate and an up row); steps of 1024 weights of its rows and of x come through double buffers by 16-byte
 // cp.async, x chunks 80 bytes apart (no bank conflicts). Q8_0 and IQ1_M have decoders of whole words, the other formats go byte by byte.
 template <int TYPE, int MT>
@@ -513,8 +512,7 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
         uint8_t* dst = ws + ((i & 1) * 2 + r) * C::kPitch;
         for (int j = lane; j < (off + bytes + 15) >> 4; j += 32) {
           const long left = p.W_end - (src + j * 16);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + j * 16)), "l"(src + j * 16), "r"(left < 16 ? (int)left : 16)
-                       : "memory");
+          cp_async16(dst + j * 16, src + j * 16, left < 16 ? (int)left : 16);
         }
       }
     };
@@ -523,9 +521,7 @@ __global__ void __launch_bounds__(256) gguf_ordered_kernel(const GgufGemvArgs p)
       for (int j = threadIdx.x; j < M * 128; j += 256) {
         const int m = j >> 7, c = j & 127;
         if (c < n)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xs + ((i & 1) * MT + m) * C::kX + (c >> 2) * 80 + (c & 3) * 16)),
-                       "l"(x + (long)m * p.x_stride + (long)i * 1024 + c * 8)
-                       : "memory");
+          cp_async16(xs + ((i & 1) * MT + m) * C::kX + (c >> 2) * 80 + (c & 3) * 16, x + (long)m * p.x_stride + (long)i * 1024 + c * 8);
       }
     };
     float acc[2][MT];

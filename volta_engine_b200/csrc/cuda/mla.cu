@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kAbsCols / 2) mla_absorb_q_kernel(const __nv_b
   for (int i = tid; i < nope * (kAbsCols / 8); i += kAbsCols / 2) {
     const int d = i / (kAbsCols / 8), c = i % (kAbsCols / 8) * 8;
     if (vec)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ws + d * kAbsCols + c)), "l"(w + (long)d * kLat + c) : "memory");
+      cp_async16(ws + d * kAbsCols + c, w + (long)d * kLat + c);
     else                                            // (weights that do not start on a 16-byte boundary)
       for (int e = 0; e < 8; ++e) ws[d * kAbsCols + c + e] = w[(long)d * kLat + c + e];
   }
@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(128) mla_expand_out_kernel(const __nv_bfloat16
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < 32 * 64; i += 128) {
     const int v = i >> 6, c = i & 63;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(wsm + v * 1040 + c * 16)),
-                 "l"(w_uv + ((long)h * vdim + min(v0 + v, vdim - 1)) * kLat + c * 8) : "memory");
+    cp_async16(wsm + v * 1040 + c * 16, w_uv + ((long)h * vdim + min(v0 + v, vdim - 1)) * kLat + c * 8);
   }
   for (int i = threadIdx.x; i < 8 * kLat; i += 128) {
     const int r = i >> 9, c = i & 511;
